@@ -69,8 +69,10 @@ enum { SPC_STEPPER_EULER = 0, SPC_STEPPER_SRK = 1, SPC_STEPPER_RK4 = 2, SPC_STEP
  * (ChimeraSystem.cpp:90-98). */
 enum { SPC_NEIGHBOUR_CELL = 0, SPC_NEIGHBOUR_VERLET = 1 };
 
-/* Precision.  FP64: every value and operation in double, in the reference's
- * order.  FP32C: neighbour sums, sin/cos and stage updates in float with
+/* Precision.  FP64: every value and operation in double, the neighbour terms
+ * added in the reference's order; a term's sine or cosine of the phase
+ * difference comes from each particle's sine and cosine by the
+ * angle-difference identity, within ~4e-16 of the exact value.  FP32C: neighbour sums, sin/cos and stage updates in float with
  * compensated (Kahan) accumulation; the cutoff / minimum-image decision, the
  * wrapped positions and the accumulated phase stay double.
  * FP32X: the per-pair work stays off the FP64 pipe (float prefilter, the
@@ -426,7 +428,7 @@ int spc_batch_retune(spc_batch *b, double dt, int32_t trial_steps, spc_tuning *c
  * start-up.  The caller passes device buffers: d_state (3N doubles, AoS),
  * d_derivative (3N) and d_additional (2N); the work is enqueued on `stream`
  * (a cudaStream_t, NULL for the default stream) and the call returns without
- * waiting.  Intermediates live in one static device array of about 1.1 MB
+ * waiting.  Intermediates live in one static device array of about 1.2 MB
  * that every GPU loading the library keeps until the process exits; limits:
  * n <= 8192 particles and int(L/rho)^2 <= 16384 cells, larger sizes return
  * SPC_ERR_CAPACITY.  The Chimera and vortex models are supported; the

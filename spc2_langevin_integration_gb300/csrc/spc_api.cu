@@ -196,16 +196,6 @@ int spc_create(const spc_params *p, int32_t n, spc_handle **out) {
     const double want = std::max(2.0 * mean, mean + 8.0 * std::sqrt(mean)) + 64.0;
     rc = engine_init_verlet(&h->e, ((int)want + 31) / 32 * 32);
   }
-  // (cells dense enough for the cell-tile kernel by default: the warp-per-cell
-  // kernel of sparse cells keeps no cosines)
-  if (rc == SPC_OK && p->model != SPC_MODEL_VORTEX_ARRAYS && p->stepper == SPC_STEPPER_SRK &&
-      p->precision == SPC_PRECISION_FP64 && p->neighbour == SPC_NEIGHBOUR_CELL && !sc.allpairs &&
-      (double)n / (double)sc.ncell >= kSparseBelowDefault) {
-    // accepted pairs: about pi rho^2 n / L^2 per particle
-    const double mean = 3.141592653589793 * p->rho * p->rho * (double)n / (p->L * p->L);
-    const double want = std::max(2.0 * mean, mean + 8.0 * std::sqrt(mean)) + 64.0;
-    rc = engine_init_tile_cos(&h->e, ((int)std::min(want, (double)n) + 31) / 32 * 32);
-  }
   if (rc == SPC_OK && p->model == SPC_MODEL_VORTEX_ARRAYS && p->stepper == SPC_STEPPER_SRK) {
     // pairs within rho: about pi rho^2 n / L^2 per particle
     const double mean = 3.141592653589793 * p->rho * p->rho * (double)n / (p->L * p->L);
@@ -1121,9 +1111,9 @@ constexpr size_t kNaHist = na_round(4ull * (1u << 11) * kNoAllocMaxTiles);
 constexpr size_t kNaSys = na_round(sizeof(SysDesc));
 // x y phi omega | st_x st_y st_phi | sx sy sphi | dphi_s      (11 double arrays)
 // keys vals keys_alt vals_alt pidx cnt_s dphi_f sys_of_p      (8 32-bit arrays)
-// fxy cs (2 float2 arrays) | cell_start | sys_of_c | hist | system table | all-pairs cell | clamp counter
+// fxy cs (2 float2 arrays) | dcs (double2) | cell_start | sys_of_c | hist | system table | all-pairs cell | clamp counter
 constexpr size_t kNoAllocBytes =
-    11 * kNaD + 8 * kNaF + 2 * kNaF2 + 2 * kNaCells + kNaHist + kNaSys + 256 + 256;
+    11 * kNaD + 8 * kNaF + 2 * kNaF2 + 2 * kNaD + 2 * kNaCells + kNaHist + kNaSys + 256 + 256;
 
 constexpr int kNoAllocMaxDevices = 64;
 std::mutex g_noalloc_mu;
@@ -1261,6 +1251,7 @@ extern "C" int spc_rhs_srk_noalloc(const spc_params *p, int32_t n, const double 
   int *sys_of_p = (int *)take(kNaF);
   a.fxy = (float2 *)take(kNaF2);
   a.cs = (float2 *)take(kNaF2);
+  a.dcs = (double2 *)take(2 * kNaD);
   a.cell_start = (int *)take(kNaCells);
   int *sys_of_c = (int *)take(kNaCells);
   e.hist = (uint32_t *)take(kNaHist);

@@ -304,7 +304,13 @@ int dalloc(Engine *e, T **ptr, size_t count) {
   return SPC_OK;
 }
 
-// The 11-bit scatter needs more than the default 48 KB of dynamic shared
+template <int PREC, int KIND>
+cudaError_t vtile_attribute() {
+  return cudaFuncSetAttribute(k_vtile<PREC, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)sizeof(VStage<PREC, KIND>));
+}
+
+// The 11-bit scatter and the Verlet passes need more than the default 48 KB of dynamic shared
 // memory; the attribute is set with the device current (not a stream
 // operation, so never inside a capture).
 inline cudaError_t set_kernel_attributes() {
@@ -313,6 +319,10 @@ inline cudaError_t set_kernel_attributes() {
   if (ce == cudaSuccess)
     ce = cudaFuncSetAttribute(k_radix_scatter<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)scatter_smem_bytes(11));
+  if (ce == cudaSuccess) ce = vtile_attribute<kPrecFP64, kKindSin>();
+  if (ce == cudaSuccess) ce = vtile_attribute<kPrecFP64, kKindCos2>();
+  if (ce == cudaSuccess) ce = vtile_attribute<kPrecFP32C, kKindSin>();
+  if (ce == cudaSuccess) ce = vtile_attribute<kPrecFP32C, kKindCos2>();
   return ce;
 }
 
@@ -332,6 +342,8 @@ inline void engine_footprint(int stepper, int precision, long long *per_particle
   if (precision != SPC_PRECISION_FP64)  // cell units: round sums, counts, chunk counters, list
     b += kSplitRounds * ((precision == SPC_PRECISION_FP32X ? 16 : 8) + 4) + 4 + kSplitRounds * 8 / 32;
   if (precision == SPC_PRECISION_FP64) b += 8 + 8 + 4;                          // vortex-arrays outputs
+  if (precision != SPC_PRECISION_FP32C) b += 16;                                // dcs
+  if (precision == SPC_PRECISION_FP64 && stepper == SPC_STEPPER_SRK) b += (long long)kMaskWords * 4;  // masks
   b += 12 * 8 + 4 + 4;                       // AoS staging, histogram share
   *per_particle = b;
   // cell_start, sys_of_c; float forms: unit list (two halves' worth), flag, sub-cell split and flag
@@ -380,7 +392,9 @@ inline int engine_init(Engine *e, int stepper, int precision, int pool_cap, int 
     SPC_TRY(dalloc(e, &a.va_vx, N));
     SPC_TRY(dalloc(e, &a.va_vy, N));
     SPC_TRY(dalloc(e, &a.va_cnt2, N));
+    if (stepper == SPC_STEPPER_SRK) SPC_TRY(dalloc(e, &a.nbmask, (size_t)kMaskWords * N));
   }
+  if (precision != SPC_PRECISION_FP32C) SPC_TRY(dalloc(e, &a.dcs, N));
   int *sys_of_p = nullptr, *sys_of_c = nullptr;
   SPC_TRY(dalloc(e, &sys_of_p, N));
   a.sys_of_p = sys_of_p;
@@ -454,8 +468,6 @@ inline int engine_init(Engine *e, int stepper, int precision, int pool_cap, int 
   return SPC_OK;
 }
 
-// Verlet buffers for rows of up to `cap` entries (cap <= 1024, so that the
-// FP32C pass-1 bits of a row fit the 32 mask words of a particle).
 // Vortex-arrays SRK single systems: room for the first pass's records of
 // `cap` pairs within rho per particle (32 B each), within a budget of 4 GB;
 // beyond it (or beyond cap pairs) the second pass recomputes them.
@@ -468,18 +480,8 @@ inline int engine_init_va_cache(Engine *e, int cap) {
   return SPC_OK;
 }
 
-// Cell-tile FP64 SRK single systems: room for the first pass's cosines of
-// `cap` accepted pairs per particle (8 B each), within a budget of 4 GB;
-// beyond it (or beyond cap pairs) the second pass evaluates them.
-inline int engine_init_tile_cos(Engine *e, int cap) {
-  const size_t N = (size_t)e->pool_cap;
-  cap = std::max(32, cap);
-  if ((size_t)cap * N * sizeof(double) > ((size_t)4 << 30)) return SPC_OK;
-  SPC_TRY(dalloc(e, &e->a.tcos, (size_t)cap * N));
-  e->a.tcap = cap;
-  return SPC_OK;
-}
-
+// Verlet buffers for rows of up to `cap` entries (cap <= 1024, so that the
+// pass-1 bits of a row fit the 32 mask words of a particle).
 inline int engine_init_verlet(Engine *e, int cap) {
   const size_t N = (size_t)e->pool_cap;
   cap = std::max(32, std::min(cap, kMaskWords * kWarp));
@@ -493,13 +495,6 @@ inline int engine_init_verlet(Engine *e, int cap) {
   SPC_TRY(dalloc(e, &e->vyb, N));
   SPC_TRY(dalloc(e, &e->vflags, 2));
   SPC_TRY(dalloc(e, &e->vrebuilds, 1));
-  // FP64 SRK: the first pass keeps each accepted row entry's cosine for the
-  // second (sincos gives the cosine bit for bit; spc_check_sincos), within a
-  // budget of 4 GB; above it the second pass evaluates the cosine itself
-  double *vcos = nullptr;
-  if (e->precision == SPC_PRECISION_FP64 && e->stepper == SPC_STEPPER_SRK &&
-      (size_t)cap * N * sizeof(double) <= ((size_t)4 << 30))
-    SPC_TRY(dalloc(e, &vcos, (size_t)cap * N));
   cudaStream_t st = e->stream;
   SPC_CUDA(e, cudaMemsetAsync(e->vrowlen, 0, N * 4, st));
   SPC_CUDA(e, cudaMemsetAsync(e->vsys, 0, N * 4, st));
@@ -515,7 +510,6 @@ inline int engine_init_verlet(Engine *e, int cap) {
   a.vyb = e->vyb;
   a.vflags = e->vflags;
   a.vrebuilds = e->vrebuilds;
-  a.vcos = vcos;
   e->verlet_stale = true;
   return SPC_OK;
 }
@@ -790,7 +784,7 @@ inline void mark(Engine *e, int slot) {
   if (e->profiling) cudaEventRecord(e->prof_ev[slot], e->stream);
 }
 
-inline int eval_cells(Engine *e, KArgs &a, int rk_form, int kq, double kcdt, bool marks = true);
+inline int eval_cells(Engine *e, KArgs &a, int prec, int rk_form, int kq, double kcdt, bool marks = true);
 
 // One evaluation's binning.  Verlet engines: refresh the Verlet-order copies
 // of the stage state and rebuild the rows when the displacement test (or a
@@ -803,12 +797,15 @@ inline int eval_stage(Engine *e, KArgs &a, int rk_form, int kq, double kcdt, boo
   if (!verlet_ok) {
     a.cell_mid = nullptr;
     a.cell_near = nullptr;
+    // they run the FP64 gather and pass: cos / sin of the phases go behind
+    // the results in the AoS staging area (12 doubles per pool particle)
+    a.dcs = reinterpret_cast<double2 *>(e->aos + (((size_t)e->pool_cap + 1) & ~(size_t)1));
   }
-  if (!e->verlet) return eval_cells(e, a, rk_form, kq, kcdt);
   if (!verlet_ok) {
-    e->verlet_stale = true;
-    return eval_cells(e, a, rk_form, kq, kcdt);
+    if (e->verlet) e->verlet_stale = true;
+    return eval_cells(e, a, kPrecFP64, rk_form, kq, kcdt);
   }
+  if (!e->verlet) return eval_cells(e, a, e->precision, rk_form, kq, kcdt);
   const int n = e->n_active;
   cudaStream_t st = e->stream;
   // the gather and the rebuild see the build tables; the caller's arguments
@@ -823,7 +820,7 @@ inline int eval_stage(Engine *e, KArgs &a, int rk_form, int kq, double kcdt, boo
     k_vgather<kPrecFP64><<<blocks_for(n, 256), 256, 0, st>>>(b, rk_form, kq, kcdt);
   SPC_LAUNCHED(e);
   mark(e, 1);
-  SPC_TRY(eval_cells(e, b, rk_form, kq, kcdt, false));
+  SPC_TRY(eval_cells(e, b, e->precision, rk_form, kq, kcdt, false));
   mark(e, 2);
   k_verlet_build<<<std::min(std::max(e->ncell_total, 1), 152 * 16), kVThreads, 0, st>>>(b);
   SPC_LAUNCHED(e);
@@ -833,9 +830,10 @@ inline int eval_stage(Engine *e, KArgs &a, int rk_form, int kq, double kcdt, boo
   return SPC_OK;
 }
 
-// Cell-list binning: stage, sort, cell bounds, cell-order gather.  marks:
-// record the profiling events after each part.
-inline int eval_cells(Engine *e, KArgs &a, int rk_form, int kq, double kcdt, bool marks) {
+// Cell-list binning: stage, sort, cell bounds, cell-order gather (for the
+// passes of precision prec).  marks: record the profiling events after each
+// part.
+inline int eval_cells(Engine *e, KArgs &a, int prec, int rk_form, int kq, double kcdt, bool marks) {
   const int n = e->n_active;
   cudaStream_t st = e->stream;
   const int bits = e->radix_bits;
@@ -868,9 +866,9 @@ inline int eval_cells(Engine *e, KArgs &a, int rk_form, int kq, double kcdt, boo
   if (marks) mark(e, 2);
   a.skeys = kin;
   a.svals = vin;
-  if (e->precision == SPC_PRECISION_FP32C)
+  if (prec == kPrecFP32C)
     k_gather<kPrecFP32C><<<blocks_for(n + 1, 256), 256, 0, st>>>(a);
-  else if (e->precision == SPC_PRECISION_FP32X)
+  else if (prec == kPrecFP32X)
     k_gather<kPrecFP32X><<<blocks_for(n + 1, 256), 256, 0, st>>>(a);
   else
     k_gather<kPrecFP64><<<blocks_for(n + 1, 256), 256, 0, st>>>(a);
@@ -925,7 +923,8 @@ int launch_pass_t(Engine *e, const KArgs &a, int epi) {
   }
   if constexpr (KIND != kKindNb && PREC != kPrecFP32X) {  // FP32X is refused with Verlet rows
     if (e->has_cells && e->verlet) {
-      k_vtile<PREC, KIND><<<std::min(e->ncell_total, 152 * 256), kVThreads, 0, st>>>(a, epi);
+      k_vtile<PREC, KIND>
+          <<<std::min(e->ncell_total, 152 * 256), kVThreads, sizeof(VStage<PREC, KIND>), st>>>(a, epi);
       SPC_LAUNCHED(e);
       return SPC_OK;
     }

@@ -92,6 +92,7 @@ struct KArgs {
   double *sx, *sy, *sphi;
   float2 *fxy;                       // prefilter coordinates relative to the cell origin
   float2 *cs;                        // FP32C: (cos phi, sin phi)
+  double2 *dcs;                      // FP64 passes: (cos phi, sin phi) of the stage phase
   longlong2 *ics;                    // FP32X: (cos phi, sin phi) in fixed point (2^kXQ)
   longlong2 *iws;                    // FP32X SRK: phase rate times (cos phi, sin phi), fixed point (2^xq2)
   double *scos;                      // FP32X SRK: pass-1 sum_j cos(phi_j - phi_i - alpha), cell order
@@ -103,7 +104,7 @@ struct KArgs {
   int *cnt_s;                        // n_i, cell order
   double *va_vx, *va_vy;             // vortex arrays: pass-1 velocity components, cell order
   int *va_cnt2;                      // vortex arrays: cohesion partners, cell order
-  uint32_t *nbmask;                  // FP32C: pass-1 neighbour bitmasks (mask_at), or null
+  uint32_t *nbmask;                  // pass-1 neighbour bitmasks for the SRK second pass (mask_at), or null
   // Cell units of the float cell-tile passes (SPC_TUNE_CELL_UNITS; units
   // null when off): the units k_list_units lists for the units kernel
   // (cell, unit), their count (zeroed by k_gather), per staging
@@ -138,16 +139,11 @@ struct KArgs {
   const int *gate;                   // binning kernels return at once when *gate == 0
   int *vsys, *vcell;                 // build: system and cell of each cell-order slot
   uint16_t *vrows;                   // row entry k of slot v at vrows[((k / 8) * n_active + v) * 8 + k % 8]
-  double *vcos;                      // FP64 SRK: cos of row entry k's phase difference at vcos[k * n_active + v], or null
   // vortex-arrays SRK (single systems): the first pass's record of slot p's
   // k-th pair within rho (k < vacap): strength, its derivative, sin and cos of
   // the phase difference at vacache[(k * n_active + p) * 4 + 0..3], or null
   double *vacache;
   int vacap;
-  // cell-tile FP64 SRK (single systems): cos of slot p's k-th accepted pair
-  // (k < tcap) from the first pass at tcos[k * n_active + p], or null
-  double *tcos;
-  int tcap;
   int *vrowlen;                      // entries of each row, -1: overflow (scan the stencil)
   int vcap;                          // row limit of the current build
   double *vxb, *vyb;                 // stage positions at the build
@@ -297,6 +293,12 @@ __global__ void k_gather(KArgs a) {
     double s, c;
     sincos(ph, &s, &c);
     a.ics[p] = make_longlong2(to_fixed(c, kXQ), to_fixed(s, kXQ));
+    if (sc.allpairs) a.dcs[p] = make_double2(c, s);  // its passes are the FP64 ones
+  }
+  if constexpr (PREC == kPrecFP64) {
+    double s, c;
+    sincos(ph, &s, &c);
+    a.dcs[p] = make_double2(c, s);
   }
 }
 
@@ -363,23 +365,89 @@ struct ILane {
   bool valid;
   float fx, fy; // prefilter coordinates
   double x, y;  // wrapped stage position
-  double phi;   // stage phase
   double card;  // pass 2: n_i from pass 1 (double, as neighborhood_cardinality_)
-  double rcard; // pass 2: 1 / n_i rounded to nearest (ddiv_by)
   double dphi;  // pass 2: own phase rate
   float ca, sa; // FP32C: cos(phi + alpha), sin(phi + alpha)
+  double dca, dsa;  // FP64: the same in double
   float dphif;
 };
+
+// FP64 pair terms.  The reference evaluates sin (SRK second pass: cos) of
+// phi_j - phi_i - alpha per pair (ChimeraSystem.cpp:412, :634-637).  Here both
+// come from the angle-difference identities with each particle's cos phi and
+// sin phi, evaluated once by the gather, and with theta_i = phi_i + alpha by
+// angle addition: two operations of the FP64 pipe per term instead of the ~25
+// of a sine (GB300 runs FP64 at 1/64 of the FP32 rate, and the pair terms
+// filled that pipe: 75% busy).  A term's absolute error is ~1.5e-16, as that
+// of the sine of the twice rounded difference, and the terms are added in the
+// reference's order as before; the mean of 200 terms is 2.4e-17 (uniform
+// phases, before 2.9e-17) to 3.5e-16 (aligned, alpha = 1.45: the same as
+// before) from the exact one.  Vortex SRK step, N = 65,536: 2.96 -> 0.44
+// ms on the cell list.
+__device__ __forceinline__ double pair_sin(double2 cj, const ILane &il) {
+  return __fma_rn(cj.y, il.dca, -dmul(cj.x, il.dsa));
+}
+__device__ __forceinline__ double pair_cos(double2 cj, const ILane &il) {
+  return __fma_rn(cj.x, il.dca, dmul(cj.y, il.dsa));
+}
+// One accepted pair: pass 1 adds the sine, pass 2 the cosine and the cosine
+// weighted by the difference of the phase rates.  The second pass's quotients
+// by n_i are taken once of each sum (finish_pairs).
+template <int KIND>
+__device__ __forceinline__ void add_pair(Acc<kPrecFP64> &acc, const ILane &il, double2 cj, double dj) {
+  if constexpr (KIND == kKindSin) {
+    acc.s0 = dadd(acc.s0, pair_sin(cj, il));
+  } else {
+    const double c = pair_cos(cj, il);
+    acc.s0 = dadd(acc.s0, c);
+    acc.s1 = __fma_rn(dsub(dj, il.dphi), c, acc.s1);
+  }
+}
+template <int KIND>
+__device__ __forceinline__ void finish_pairs(Acc<kPrecFP64> &acc, const ILane &il) {
+  if constexpr (KIND == kKindCos2) {
+    if (il.card > 0.0) {
+      acc.s0 = ddiv(acc.s0, il.card);
+      acc.s1 = ddiv(acc.s1, il.card);
+    }
+  }
+}
+
+// The float test of 32 staged candidates against one particle (FP64 passes):
+// bit 31 - t of the result is the sign of candidate t's d^2 - lo2, set when
+// it is inside for certain.  An undecided one (left to the reference's FP64
+// test) has an offset in [0, hi2 - lo2]; *um gets the smallest bit pattern of
+// the offsets as an unsigned number, in which negative floats come last.  Two
+// fused multiply-adds, one funnel shift and one minimum per candidate.
+__device__ __forceinline__ uint32_t test32(const float2 *__restrict__ xy, float fx, float fy, float nlo,
+                                           uint32_t &um) {
+  uint32_t bits = 0u;
+#pragma unroll
+  for (int t = 0; t < kWarp; t += 2) {
+    const float4 c = *reinterpret_cast<const float4 *>(xy + t);
+    const float dx0 = c.x - fx, dy0 = c.y - fy, dx1 = c.z - fx, dy1 = c.w - fy;
+    const uint32_t o0 = __float_as_uint(cutoff_offset(dx0, dy0, nlo));
+    const uint32_t o1 = __float_as_uint(cutoff_offset(dx1, dy1, nlo));
+    bits = __funnelshift_l(o0, bits, 1);
+    bits = __funnelshift_l(o1, bits, 1);
+    um = min(um, min(o0, o1));
+  }
+  return bits;
+}
+// bits of the first cnt candidates of a block (0 <= cnt <= 32)
+__device__ __forceinline__ uint32_t first_bits(int cnt) {
+  return cnt >= kWarp ? 0xffffffffu : ~(0xffffffffu >> cnt);
+}
+// upper end of the undecided band above lo2, rounded outwards
+__device__ __forceinline__ float undecided_width(float lo2, float hi2) { return (hi2 - lo2) * 1.001f; }
 
 template <int PREC, int KIND>
 __device__ __forceinline__ void accept_pair(const KArgs &a, const SysDesc &sd, const ILane &il,
                                             Acc<PREC> &acc, int pj, float cjc, float cjs,
                                             float dphij_f, long long &wpos) {
-  const SysConst &sc = sd.sc;
   if constexpr (KIND == kKindSin) {
     if constexpr (PREC == kPrecFP64) {
-      // alignment_force_[i] += sin(phi_j - phi_i - alpha_) (ChimeraSystem.cpp:412)
-      acc.s0 = dadd(acc.s0, sin(dsub(dsub(a.sphi[pj], il.phi), sc.alpha)));
+      add_pair<KIND>(acc, il, a.dcs[pj], 0.0);  // ChimeraSystem.cpp:412
     } else {
       // sin(phi_j - (phi_i + alpha)) by the angle-difference identity
       kahan_add(acc.s0, acc.c0, cjs * il.ca - cjc * il.sa);
@@ -387,10 +455,7 @@ __device__ __forceinline__ void accept_pair(const KArgs &a, const SysDesc &sd, c
     acc.n++;
   } else if constexpr (KIND == kKindCos2) {
     if constexpr (PREC == kPrecFP64) {
-      // ChimeraSystem.cpp:634-637
-      const double c = cos(dsub(dsub(a.sphi[pj], il.phi), sc.alpha));
-      acc.s0 = dadd(acc.s0, ddiv_by(c, il.card, il.rcard));
-      acc.s1 = dadd(acc.s1, ddiv_by(dmul(dsub(a.dphi_s[pj], il.dphi), c), il.card, il.rcard));
+      add_pair<KIND>(acc, il, a.dcs[pj], a.dphi_s[pj]);  // ChimeraSystem.cpp:634-637
     } else {
       const float c = cjc * il.ca + cjs * il.sa;
       kahan_add(acc.s0, acc.c0, c);
@@ -401,8 +466,9 @@ __device__ __forceinline__ void accept_pair(const KArgs &a, const SysDesc &sd, c
     if (a.list_idx) a.list_idx[wpos++] = a.pidx[pj] - sd.pool_p0;
     if constexpr (PREC == kPrecFP64) {
       if (a.out_r) {
-        acc.s0 += cos(a.sphi[pj]);
-        acc.s1 += sin(a.sphi[pj]);
+        const double2 cj = a.dcs[pj];
+        acc.s0 += cj.x;
+        acc.s1 += cj.y;
       }
     }
     acc.n++;
@@ -423,7 +489,8 @@ __device__ void epilogue(const KArgs &a, int epi, const SysDesc &sd, const ILane
   if constexpr (KIND == kKindNb) {
     if (epi == kEpiCount) a.out_cnt[q] = acc.n;
     if (epi == kEpiLocalOrder) {
-      const double re = acc.s0 + cos(il.phi), im = acc.s1 + sin(il.phi);
+      const double2 ci = a.dcs[p];
+      const double re = acc.s0 + ci.x, im = acc.s1 + ci.y;
       a.out_r[q] = sqrt(re * re + im * im) / (double)(acc.n + 1);
     }
     return;
@@ -437,9 +504,10 @@ __device__ void epilogue(const KArgs &a, int epi, const SysDesc &sd, const ILane
   const double dt = a.dt;
   if constexpr (PREC == kPrecFP64) {
     if (draws) philox_normal2(sd.seed, sd.system_id, step, (uint32_t)i, z0, z1);
-    // cos / sin of the stage phase: evaluated here, or (FP32X) the gather's
-    // fixed-point values, exact to 2^-53
-    const double cph = cs_known ? cs_known->x : cos(il.phi), sph = cs_known ? cs_known->y : sin(il.phi);
+    // cos / sin of the stage phase from the gather: the doubles, or (FP32X)
+    // its fixed-point values, exact to 2^-53
+    const double2 csp = cs_known ? *cs_known : a.dcs[p];
+    const double cph = csp.x, sph = csp.y;
     const double d0 = dmul(sc.v0, cph), d1 = dmul(sc.v0, sph);  // v_0_ * cos(phi_i) (:419-420)
     if constexpr (KIND == kKindSin) {
       // sigma_ * alignment_force_[i] / neighborhood_cardinality_[i] (:421-424)
@@ -606,7 +674,6 @@ __device__ __forceinline__ void load_i(const KArgs &a, const SysConst &sc, ILane
   if (!valid) return;
   il.x = a.sx[p];
   il.y = a.sy[p];
-  il.phi = a.sphi[p];
   if (!sc.allpairs) {
     const float2 f = a.fxy[p];
     il.fx = f.x;
@@ -619,9 +686,13 @@ __device__ __forceinline__ void load_i(const KArgs &a, const SysConst &sc, ILane
     il.ca = t.x * sc.cos_a - t.y * sc.sin_a;
     il.sa = t.y * sc.cos_a + t.x * sc.sin_a;
   }
+  if constexpr (PREC == kPrecFP64 && KIND != kKindNb) {
+    const double2 t = a.dcs[p];
+    il.dca = dsub(dmul(t.x, sc.cos_ad), dmul(t.y, sc.sin_ad));
+    il.dsa = dadd(dmul(t.y, sc.cos_ad), dmul(t.x, sc.sin_ad));
+  }
   if constexpr (KIND == kKindCos2) {
     il.card = (double)a.cnt_s[p];
-    il.rcard = drcp(il.card);  // unused (and infinite) when n_i = 0: no pairs
     il.dphi = a.dphi_s[p];
     if constexpr (PREC == kPrecFP32C) il.dphif = a.dphi_f[p];
   } else {
@@ -776,19 +847,36 @@ __global__ void __launch_bounds__(kPassThreads) k_cell_pass(KArgs a, int epi) {
 // All pairs (rho > L/4): ChimeraSystem.cpp:117-255.  An all-pairs system's
 // particles form one cell, in index order.  A work item is one block of T
 // particles of one such system, so a large system spreads over many CTAs;
-// one thread per i walks j ascending (the reference's order), with the exact
-// FP64 test on unwrapped stage positions.  T is the CTA width: 128, or 32
+// one thread per i walks j ascending (the reference's order).  T is the CTA width: 128, or 32
 // (one warp per CTA, four times the CTAs) when the all-pairs systems hold too
 // few particles to give every SM work at 128 (each thread's sums are the
 // same either way).
 constexpr int kAllPairsThreads = 128;
 constexpr int kAllPairsThreadsSmall = 32;
 
+// The candidates are tested in float first, as in the cell kernels: for two
+// positions inside the box |dx| <= L, and the reference's minimum image is
+// min(|dx|, L - |dx|).  A position outside the box (an RK4 stage; the all-pairs
+// form does not wrap its copies) is staged as NaN, which is never in the band,
+// and flagged, so that its pairs are decided by the reference's FP64 test
+// alone.  A round of candidates is tested first, which leaves each thread its
+// neighbours as bits in shared memory; then each thread walks its bits, so
+// the FP64 terms run on nearly full warps.
+// Measured, Chimera Euler step of N = 2,000, L = 1, rho = 0.3: the FP64 test
+// of every candidate took 2.74 ms; this form 0.20 ms.
+constexpr int kAllPairsCap = 704;  // candidates staged per round
+
 template <int PREC, int KIND, int T = kAllPairsThreads>
 __global__ void __launch_bounds__(T) k_allpairs_pass(KArgs a, int epi) {
-  __shared__ double tx[T], ty[T];
-  __shared__ float2 tcs[T];
-  __shared__ float td[T];
+  constexpr bool kPair64 = PREC == kPrecFP64 && KIND != kKindNb;
+  constexpr int kWords = kAllPairsCap / kWarp;
+  __shared__ __align__(16) float2 t_xy[kAllPairsCap];
+  __shared__ double2 t_cs[kPair64 ? kAllPairsCap : 1];
+  __shared__ double t_d[kPair64 && KIND == kKindCos2 ? kAllPairsCap : 1];
+  __shared__ float2 t_csf[PREC == kPrecFP32C ? kAllPairsCap : 1];
+  __shared__ float t_df[PREC == kPrecFP32C && KIND == kKindCos2 ? kAllPairsCap : 1];
+  __shared__ uint32_t t_out[kWords];   // candidates outside the box (first_bits order)
+  __shared__ uint32_t t_w[kWords][T];  // each thread's neighbours of the round
   for (int item = blockIdx.x;; item += gridDim.x) {
     // the item's system (w) and particle block (rest), uniform over the CTA
     int w = 0, rest = item, cb = 0, ce = 0;
@@ -804,45 +892,108 @@ __global__ void __launch_bounds__(T) k_allpairs_pass(KArgs a, int epi) {
     const int c = a.ap_cells[w];
     const SysDesc &sd = a.sys[a.sys_of_c[c]];
     const SysConst &sc = sd.sc;
-    {
-      const int ib = cb + rest * T;
-      const int i = ib + threadIdx.x;
-      ILane il;
-      Acc<PREC> acc;
-      load_i<PREC, KIND>(a, sc, il, i, i < ce);
-      acc.init();
-      long long wpos = (a.list_idx && il.valid) ? a.list_off[a.pidx[i]] : 0;
-      for (int jt = cb; jt < ce; jt += T) {
-        const int jl = jt + threadIdx.x;
-        __syncthreads();
-        if (jl < ce) {
-          tx[threadIdx.x] = a.sx[jl];
-          ty[threadIdx.x] = a.sy[jl];
+    const bool exact_all = sc.exact_all != 0;
+    const float Lf = (float)sc.L, nlo = -sc.lo2, wid = undecided_width(sc.lo2, sc.hi2);
+    const int i = cb + rest * T + threadIdx.x;
+    ILane il;
+    Acc<PREC> acc;
+    load_i<PREC, KIND>(a, sc, il, i, i < ce);
+    acc.init();
+    long long wpos = (a.list_idx && il.valid) ? a.list_off[a.pidx[i]] : 0;
+    // the box's upper edge counts as outside: at |dx| = L the reference's
+    // minimum image is L and not 0 (PeriodicBoundaryConditions.cpp:22-35)
+    const double edge = sc.L * (1.0 - 1e-12);
+    auto outside = [&](double x, double y) { return !(x >= 0.0 && x < edge && y >= 0.0 && y < edge); };
+    const bool i_out = il.valid && outside(il.x, il.y);
+    const float fx = il.valid ? (float)il.x : 0.0f, fy = il.valid ? (float)il.y : 0.0f;
+    for (int jt = cb; jt < ce; jt += kAllPairsCap) {
+      const int cnt = min(kAllPairsCap, ce - jt), nw = (cnt + kWarp - 1) / kWarp;
+      __syncthreads();
+      for (int k = threadIdx.x; k < nw * kWarp; k += T) {
+        const int j = jt + k;
+        bool out = false;
+        float2 f = make_float2(__int_as_float(0x7fc00000), 0.0f);
+        if (k < cnt) {
+          const double x = a.sx[j], y = a.sy[j];
+          out = outside(x, y);
+          if (!out) f = make_float2((float)x, (float)y);
+          if constexpr (kPair64) {
+            t_cs[k] = a.dcs[j];
+            if constexpr (KIND == kKindCos2) t_d[k] = a.dphi_s[j];
+          }
           if constexpr (PREC == kPrecFP32C) {
-            tcs[threadIdx.x] = a.cs[jl];
-            if constexpr (KIND == kKindCos2) td[threadIdx.x] = a.dphi_f[jl];
+            t_csf[k] = a.cs[j];
+            if constexpr (KIND == kKindCos2) t_df[k] = a.dphi_f[j];
           }
         }
-        __syncthreads();
-        const int cnt = min(T, ce - jt);
-        if (!il.valid) continue;
-        for (int t = 0; t < cnt; ++t) {
-          const int j = jt + t;
-          if (j == i) continue;
-          if (exact_within(sc, il.x, il.y, tx[t], ty[t])) {
-            float cc = 0.0f, ss = 0.0f, dj = 0.0f;
-            if constexpr (PREC == kPrecFP32C) {
-              cc = tcs[t].x;
-              ss = tcs[t].y;
-              if constexpr (KIND == kKindCos2) dj = td[t];
+        t_xy[k] = f;
+        const uint32_t o = __brev(__ballot_sync(0xffffffffu, out));  // k is a multiple of 32 apart per warp
+        if (threadIdx.x % kWarp == 0) t_out[k / kWarp] = o;
+      }
+      __syncthreads();
+      if (!il.valid) continue;
+      for (int wd = 0; wd < nw; ++wd) {
+        const int j0 = wd * kWarp;
+        uint32_t bits = 0u, um = 0xffffffffu;
+#pragma unroll
+        for (int t = 0; t < kWarp; t += 2) {
+          const float4 cj = *reinterpret_cast<const float4 *>(t_xy + j0 + t);
+          const float ax0 = fabsf(cj.x - fx), ay0 = fabsf(cj.y - fy), ax1 = fabsf(cj.z - fx), ay1 = fabsf(cj.w - fy);
+          const float dx0 = fminf(ax0, Lf - ax0), dy0 = fminf(ay0, Lf - ay0);
+          const float dx1 = fminf(ax1, Lf - ax1), dy1 = fminf(ay1, Lf - ay1);
+          const uint32_t o0 = __float_as_uint(cutoff_offset(dx0, dy0, nlo));
+          const uint32_t o1 = __float_as_uint(cutoff_offset(dx1, dy1, nlo));
+          bits = __funnelshift_l(o0, bits, 1);
+          bits = __funnelshift_l(o1, bits, 1);
+          um = min(um, min(o0, o1));
+        }
+        const uint32_t known = first_bits(cnt - j0) & ~((unsigned)(i - jt - j0) < (unsigned)kWarp
+                                                            ? 0x80000000u >> (i - jt - j0)
+                                                            : 0u);
+        const bool all = exact_all || i_out;
+        if (all || um <= __float_as_uint(wid) || t_out[wd] != 0u) {  // the reference's FP64 test
+          for (int t = 0; t < kWarp; ++t) {
+            const uint32_t b = 0x80000000u >> t;
+            if (!(known & b)) continue;
+            bool ask = all || (t_out[wd] & b) != 0u;
+            if (!ask) {
+              const float2 cj = t_xy[j0 + t];
+              const float ax = fabsf(cj.x - fx), ay = fabsf(cj.y - fy);
+              const float off = cutoff_offset(fminf(ax, Lf - ax), fminf(ay, Lf - ay), nlo);
+              ask = off >= 0.0f && off <= wid;
             }
-            accept_pair<PREC, KIND>(a, sd, il, acc, j, cc, ss, dj, wpos);
+            if (!ask) continue;
+            const int j = jt + j0 + t;
+            bits = exact_within(sc, il.x, il.y, a.sx[j], a.sy[j]) ? bits | b : bits & ~b;
           }
+        }
+        t_w[wd][threadIdx.x] = bits & known;
+      }
+      uint32_t bits = 0u;
+      for (int wd = -1;;) {
+        while (bits == 0u && ++wd < nw) bits = t_w[wd][threadIdx.x];
+        if (bits == 0u) break;
+        const int t = __clz(bits), k = wd * kWarp + t;
+        bits ^= 0x80000000u >> t;
+        if constexpr (kPair64) {
+          add_pair<KIND>(acc, il, t_cs[k], KIND == kKindCos2 ? t_d[k] : 0.0);
+          acc.n++;
+        } else {
+          float cc = 0.0f, ss = 0.0f, dj = 0.0f;
+          if constexpr (PREC == kPrecFP32C) {
+            cc = t_csf[k].x;
+            ss = t_csf[k].y;
+            if constexpr (KIND == kKindCos2) dj = t_df[k];
+          }
+          accept_pair<PREC, KIND>(a, sd, il, acc, jt + k, cc, ss, dj, wpos);
         }
       }
-      if (il.valid) epilogue<PREC, KIND>(a, epi, sd, il, acc, a.pidx[i]);
-      __syncthreads();
     }
+    if (il.valid) {
+      if constexpr (kPair64) finish_pairs<KIND>(acc, il);
+      epilogue<PREC, KIND>(a, epi, sd, il, acc, a.pidx[i]);
+    }
+    __syncthreads();
   }
 }
 

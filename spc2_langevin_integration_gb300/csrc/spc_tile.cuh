@@ -13,11 +13,10 @@
 // are combined in a fixed order, so results are deterministic.
 //
 // FP64 (k_tile_fp64): one thread per particle walks the whole list in order,
-// so each particle's sum keeps the reference's order term for term.  Accepted
-// candidates go into a per-thread FIFO in shared memory and the warp drains
-// the common minimum of its queues after every block of 32 candidates, so the
-// FP64 sin/cos (1/64-rate pipe on GB300) runs on full warps instead of on the
-// few lanes that happen to accept a given candidate.
+// so each particle's sum keeps the reference's order term for term.  The
+// threads first find their neighbours of a staging round as bits and then walk
+// the bits, so that the FP64 terms (1/64-rate pipe on GB300) run on nearly
+// full warps instead of on the few lanes that accept a given candidate.
 //
 // Both decide every pair exactly as the reference: float prefilter on
 // cell-relative coordinates, the reference's FP64 test for pairs within a
@@ -29,10 +28,9 @@
 namespace spc {
 
 constexpr int kTileCap = 1024;      // FP32C: candidates staged per round
-constexpr int kTileCap64 = 768;     // FP64: candidates staged per round (7 CTAs/SM fit)
+constexpr int kTileCap64 = 704;     // FP64: candidates staged per round (7 CTAs/SM fit)
 constexpr int kTileThreads32 = 128; // FP32C CTA: 4 warps
 constexpr int kTileThreads64 = 64;  // FP64 CTA: 2 warps
-constexpr int kQCap = 64;           // FP64 per-thread queue (power of two)
 
 struct Stencil {
   int start[9];    // cell-order start of each stencil cell
@@ -1094,13 +1092,27 @@ __global__ void __launch_bounds__(kTileThreads32, kTileMinBlocks32) k_units_fp32
 }
 
 // ---------------------------------------------------------------------------
+// FP64 passes.  A staging round is tested first: each thread's neighbours of
+// the round become bits, one word per 32 candidates, in its own column of
+// shared memory.  Then each thread walks its bits in order (the reference's
+// visiting order), taking the next word when one is used up, so the lanes of a
+// warp run out of neighbours together (a lane has ~200 +- 14 of them) and the
+// FP64 terms run on ~90% full warps.  The SRK first pass keeps the words of
+// one-round cells in nbmask and the second pass tests nothing again.
+// Bound by the FP64 pipe (3 operations per pair in pass 1, 5 in pass 2).
+// Vortex SRK, N = 65,536: pass 1 2.04 ms -> 171 us, pass 2 0.92 ms ->
+// 250 us (sines per pair and a queue of accepted candidates before; 137 MB
+// of kept cosines are gone).  704 candidates per round leave room for 7 CTAs
+// per SM in pass 2.
+constexpr int kTileWords64 = kTileCap64 / kWarp;
+static_assert(kTileCap64 % kWarp == 0 && (kTileWords64 + 3) / 4 * 4 <= kMaskWords, "FP64 staging round");
+
 template <int KIND>
 __global__ void __launch_bounds__(kTileThreads64) k_tile_fp64(KArgs a, int epi) {
-  __shared__ float2 s_xy[kTileCap64];   // x+shift, y+shift (prefilter)
-  __shared__ double s_phi[kTileCap64];  // stage phase
+  __shared__ __align__(16) float2 s_xy[kTileCap64];  // x+shift, y+shift (prefilter; padded to 32)
+  __shared__ double2 s_cs[kTileCap64];               // cos, sin of the stage phase
   __shared__ double s_d[KIND == kKindCos2 ? kTileCap64 : 1];  // pass 2: phase rate
-  __shared__ int s_p[kTileCap64];
-  __shared__ uint16_t s_q[kQCap][kTileThreads64];
+  __shared__ uint32_t s_w[(kTileWords64 + 3) / 4 * 4][kTileThreads64];
   const int tid = threadIdx.x;
   const int n_all = a.n_active;
   const int nitems = tile_items(a);
@@ -1111,13 +1123,13 @@ __global__ void __launch_bounds__(kTileThreads64) k_tile_fp64(KArgs a, int epi) 
     const SysDesc &sd = a.sys[a.sys_of_c[c]];
     const SysConst &sc = sd.sc;
     if (sc.allpairs) continue;
-    const float lo2 = sc.lo2, hi2 = sc.hi2;
-    const float band = 0.5f * (hi2 - lo2), nmid = -0.5f * (hi2 + lo2);
+    const float nlo = -sc.lo2, wid = undecided_width(sc.lo2, sc.hi2);
     const bool exact_all = sc.exact_all != 0;
     Stencil st;
     stencil_of(a, sd, c, st);
     const int total = st.prefix[9];
     const int rounds = (total + kTileCap64 - 1) / kTileCap64;
+    const bool masked = rounds == 1 && a.nbmask != nullptr && !exact_all;
     for (int ig = cb; ig < ce; ig += kTileThreads64) {
       const int gi = min(kTileThreads64, ce - ig);
       const bool valid = tid < gi;
@@ -1125,87 +1137,84 @@ __global__ void __launch_bounds__(kTileThreads64) k_tile_fp64(KArgs a, int epi) 
       ILane il;
       load_i<kPrecFP64, KIND>(a, sc, il, p, valid);
       if (!valid) {
-        il.fx = il.fy = 3.0e30f;
-        il.x = il.y = il.phi = il.dphi = 0.0;
-        il.card = il.rcard = 1.0;
+        il.fx = il.fy = 3.0e17f;
+        il.x = il.y = 0.0;
       }
       Acc<kPrecFP64> acc;
       acc.init();
       for (int r = 0; r < rounds; ++r) {
         const int rlo = r * kTileCap64, rcnt = min(kTileCap64, total - rlo);
+        const int nw = (rcnt + kWarp - 1) / kWarp;
         if (rounds > 1 || ig == cb) {
           __syncthreads();
-          for (int k = tid; k < rcnt; k += blockDim.x) {
-            int q;
-            const int pj = slot_of(st, rlo + k, q);
-            const float2 f = a.fxy[pj];
-            s_xy[k] = make_float2(f.x + shift_x(q, sc.cell_f), f.y + shift_y(q, sc.cell_f));
-            s_phi[k] = a.sphi[pj];
-            s_p[k] = pj;
-            if constexpr (KIND == kKindCos2) s_d[k] = a.dphi_s[pj];
+          for (int k = tid; k < nw * kWarp; k += blockDim.x) {
+            if (k < rcnt) {
+              int q;
+              const int pj = slot_of(st, rlo + k, q);
+              s_cs[k] = a.dcs[pj];
+              if constexpr (KIND == kKindCos2) s_d[k] = a.dphi_s[pj];
+              if (KIND == kKindCos2 && masked) continue;
+              const float2 f = a.fxy[pj];
+              s_xy[k] = make_float2(f.x + shift_x(q, sc.cell_f), f.y + shift_y(q, sc.cell_f));
+            } else {  // padding: never a neighbour, never near the cutoff
+              s_xy[k] = make_float2(3.0e18f, 3.0e18f);
+            }
           }
           __syncthreads();
         }
-        const int self = st.prefix[4] + (p - c0) - rlo;
-        int qn = 0, qh = 0;
-        // accepted pair number `ord` of this particle (the same in both SRK
-        // passes): single systems keep the first pass's cosine for the second
-        // (sincos gives the bits of cos; spc_check_sincos)
-        auto eval = [&](int j, int ord) {
-          const double dphi_ = dsub(dsub(s_phi[j], il.phi), sc.alpha);
-          double *slot = (a.tcos && ord < a.tcap) ? a.tcos + (size_t)ord * n_all + p : nullptr;
-          if constexpr (KIND == kKindSin) {
-            double sn;
-            if (slot) {
-              double cn;
-              sincos(dphi_, &sn, &cn);
-              *slot = cn;
-            } else {
-              sn = sin(dphi_);
+        if (!valid) continue;
+        uint4 *m4 = reinterpret_cast<uint4 *>(a.nbmask);
+        if (KIND == kKindCos2 && masked) {
+          for (int g = 0; g * 4 < nw; ++g) {
+            const uint4 m = m4[(size_t)g * n_all + p];
+            s_w[4 * g][tid] = m.x;
+            s_w[4 * g + 1][tid] = m.y;
+            s_w[4 * g + 2][tid] = m.z;
+            s_w[4 * g + 3][tid] = m.w;
+          }
+        } else {
+          const int self = st.prefix[4] + (p - c0) - rlo;
+          for (int w = 0; w < nw; ++w) {
+            const int j0 = w * kWarp;
+            uint32_t um = 0xffffffffu;
+            uint32_t bits = test32(s_xy + j0, il.fx, il.fy, nlo, um);
+            uint32_t known = first_bits(rcnt - j0);
+            if ((unsigned)(self - j0) < (unsigned)kWarp) known &= ~(0x80000000u >> (self - j0));
+            // pairs the float test cannot decide: the reference's FP64 test
+            if (exact_all || um <= __float_as_uint(wid)) {
+              for (int t = 0; t < kWarp; ++t) {
+                const uint32_t b = 0x80000000u >> t;
+                if (!(known & b)) continue;
+                const float2 cj = s_xy[j0 + t];
+                const float off = cutoff_offset(cj.x - il.fx, cj.y - il.fy, nlo);
+                if (!(exact_all || (off >= 0.0f && off <= wid))) continue;
+                int q;
+                const int pj = slot_of(st, rlo + j0 + t, q);
+                bits = exact_within(sc, il.x, il.y, a.sx[pj], a.sy[pj]) ? bits | b : bits & ~b;
+              }
             }
-            acc.s0 = dadd(acc.s0, sn);  // ChimeraSystem.cpp:412
-          } else {
-            const double cc = slot ? *slot : cos(dphi_);  // ChimeraSystem.cpp:634-637
-            acc.s0 = dadd(acc.s0, ddiv_by(cc, il.card, il.rcard));
-            acc.s1 = dadd(acc.s1, ddiv_by(dmul(dsub(s_d[j], il.dphi), cc), il.card, il.rcard));
+            bits &= known;
+            acc.n += __popc(bits);
+            s_w[w][tid] = bits;
           }
-        };
-        for (int j0 = 0; j0 < rcnt; j0 += kWarp) {
-          const int je = min(j0 + kWarp, rcnt);
-          for (int j = j0; j < je; ++j) {
-            const float2 cj = s_xy[j];
-            const float off = cutoff_offset(cj.x - il.fx, cj.y - il.fy, nmid);
-            bool in = !exact_all && float_inside(off, band) && (j != self);
-            const bool amb = (exact_all || float_undecided(off, band)) && (j != self) && valid;
-            if (__any_sync(0xffffffffu, amb)) {
-              if (amb) in = exact_within(sc, il.x, il.y, a.sx[s_p[j]], a.sy[s_p[j]]);
-            }
-            if (in) {
-              s_q[qn & (kQCap - 1)][tid] = (uint16_t)j;
-              ++qn;
-            }
-          }
-          // drain the warp's common backlog on full warps, in FIFO order (lanes
-          // past the end of the cell hold no queue and do not bound it)
-          int m = __reduce_min_sync(0xffffffffu, valid ? qn - qh : 0x7fffffff);
-          if (m == 0x7fffffff) m = 0;
-          if (valid) {
-            for (int k = 0; k < m; ++k) eval(s_q[(qh + k) & (kQCap - 1)][tid], acc.n + qh + k);
-            qh += m;
-          }
-          // keep room for the next block of 32
-          while (qn - qh > kQCap - kWarp) {
-            eval(s_q[qh & (kQCap - 1)][tid], acc.n + qh);
-            ++qh;
-          }
+          if (KIND == kKindSin && masked)
+            for (int g = 0; g * 4 < nw; ++g)  // words past the last one are not read
+              m4[(size_t)g * n_all + p] =
+                  make_uint4(s_w[4 * g][tid], s_w[4 * g + 1][tid], s_w[4 * g + 2][tid], s_w[4 * g + 3][tid]);
         }
-        while (qh < qn) {  // tail of this round
-          eval(s_q[qh & (kQCap - 1)][tid], acc.n + qh);
-          ++qh;
+        uint32_t bits = 0u;
+        for (int w = -1;;) {
+          while (bits == 0u && ++w < nw) bits = s_w[w][tid];
+          if (bits == 0u) break;
+          const int t = __clz(bits), j = w * kWarp + t;
+          bits ^= 0x80000000u >> t;
+          add_pair<KIND>(acc, il, s_cs[j], KIND == kKindCos2 ? s_d[j] : 0.0);
         }
-        acc.n += qn;
       }
-      if (valid) epilogue<kPrecFP64, KIND>(a, epi, sd, il, acc, a.pidx[p]);
+      if (valid) {
+        finish_pairs<KIND>(acc, il);
+        epilogue<kPrecFP64, KIND>(a, epi, sd, il, acc, a.pidx[p]);
+      }
       __syncthreads();
     }
   }

@@ -36,7 +36,7 @@ constexpr int kVThreads = 128;
 constexpr int kVMaxR = 3;                 // stencil radius limit (7 x 7 cells)
 constexpr int kVMaxCells = (2 * kVMaxR + 1) * (2 * kVMaxR + 1);
 constexpr int kVStage32 = 1664;           // FP32C / build: candidates staged per round
-constexpr int kVStage64 = 1536;           // FP64: candidates staged per round
+constexpr int kVStage64 = 1664;           // FP64: candidates staged per round
 
 // The (2R+1)^2 stencil of cell c: start of each stencil cell in cell order and
 // the prefix offsets of the staged list, in shared memory.  All threads call it.
@@ -77,7 +77,7 @@ __device__ __forceinline__ int vstencil_entry(const int *s_prefix, int ncells, i
 template <int PREC, int KIND, bool BUILD>
 __device__ __forceinline__ void vstage_round(const KArgs &a, const SysConst &sc, const int *s_start,
                                              const int *s_prefix, int rlo, int rcnt, float4 *c4,
-                                             float2 *xy, float *df, double *phi, double *dd) {
+                                             float2 *xy, float *df, double2 *dcs, double *dd) {
   const int R = sc.vR, D = 2 * R + 1;
   for (int k = threadIdx.x; k < rcnt; k += blockDim.x) {
     const int g = rlo + k;
@@ -93,7 +93,7 @@ __device__ __forceinline__ void vstage_round(const KArgs &a, const SysConst &sc,
     }
     if constexpr (!BUILD && PREC == kPrecFP32C && KIND == kKindCos2) df[k] = a.dphi_f[pj];
     if constexpr (!BUILD && PREC == kPrecFP64) {
-      phi[k] = a.sphi[pj];
+      dcs[k] = a.dcs[pj];
       if constexpr (KIND == kKindCos2) dd[k] = a.dphi_s[pj];
     }
   }
@@ -214,6 +214,11 @@ __global__ void __launch_bounds__(256) k_vgather(KArgs a, int rk_form, int kq, d
       sincosf(reduced_phase_f(ph), &s, &c);
       a.cs[v] = make_float2(c, s);
     }
+    if constexpr (PREC == kPrecFP64) {
+      double s, c;
+      sincos(ph, &s, &c);
+      a.dcs[v] = make_double2(c, s);
+    }
     double ex = x - a.vxb[v], ey = y - a.vyb[v];
     ex = ex > hL ? ex - sc.L : (ex < -hL ? ex + sc.L : ex);
     ey = ey > hL ? ey - sc.L : (ey < -hL ? ey + sc.L : ey);
@@ -241,7 +246,7 @@ template <int KIND>
 struct VStage<kPrecFP64, KIND> {
   static constexpr int kCap = kVStage64;
   float2 xy[kCap];
-  double phi[kCap];
+  double2 dcs[kCap];  // cos, sin of the stage phase
   double dd[KIND == kKindCos2 ? kCap : 1];
 };
 
@@ -249,7 +254,10 @@ template <int PREC, int KIND>
 __global__ void __launch_bounds__(kVThreads) k_vtile(KArgs a, int epi) {
   using Stage = VStage<PREC, KIND>;
   constexpr int kCap = Stage::kCap;
-  __shared__ Stage sm;
+  // dynamic: the FP64 second pass stages 53 KB, so that the 25 cells of a
+  // uniform system's stencil (~1,600 candidates) are one round
+  extern __shared__ __align__(16) unsigned char vtile_smem[];
+  Stage &sm = *reinterpret_cast<Stage *>(vtile_smem);
   __shared__ int s_start[kVMaxCells], s_prefix[kVMaxCells + 1];
   const int n_all = a.n_active, tid = threadIdx.x;
   // the next evaluation's gather raises the flag again if it must
@@ -275,8 +283,8 @@ __global__ void __launch_bounds__(kVThreads) k_vtile(KArgs a, int epi) {
       load_i<PREC, KIND>(a, sc, il, v, valid);
       const int len = valid ? a.vrowlen[v] : 0;
       const bool rows = len >= 0;
-      // FP32C pass 2 reads pass 1's bits of row entries (rows only)
-      const bool masked = PREC == kPrecFP32C && rows && a.nbmask != nullptr && !exact_all;
+      // pass 2 reads pass 1's bits of row entries (rows only)
+      const bool masked = rows && a.nbmask != nullptr && !exact_all;
       const int self = centre + (v - cb);
       Acc<PREC> acc;
       acc.init();
@@ -327,23 +335,7 @@ __global__ void __launch_bounds__(kVThreads) k_vtile(KArgs a, int epi) {
               b1 = fmaf(sm.df[j] - il.dphif, tv, b1);
             }
           } else {
-            const double dp = dsub(dsub(sm.phi[j], il.phi), sc.alpha);
-            // row entries only: k is then the entry's position in the row
-            double *vc = (a.vcos && rows) ? a.vcos + (size_t)k * n_all + v : nullptr;
-            if constexpr (KIND == kKindSin) {
-              double sn, cn;
-              if (vc) {  // keep the cosine for the second pass
-                sincos(dp, &sn, &cn);
-                *vc = cn;
-              } else {
-                sn = sin(dp);
-              }
-              acc.s0 = dadd(acc.s0, sn);  // ChimeraSystem.cpp:412
-            } else {
-              const double cc = vc ? *vc : cos(dp);  // ChimeraSystem.cpp:634-637
-              acc.s0 = dadd(acc.s0, ddiv_by(cc, il.card, il.rcard));
-              acc.s1 = dadd(acc.s1, ddiv_by(dmul(dsub(sm.dd[j], il.dphi), cc), il.card, il.rcard));
-            }
+            add_pair<KIND>(acc, il, sm.dcs[j], KIND == kKindCos2 ? sm.dd[j] : 0.0);
           }
           bits |= 1u << (k & (kWarp - 1));
         }
@@ -353,8 +345,8 @@ __global__ void __launch_bounds__(kVThreads) k_vtile(KArgs a, int epi) {
             kahan_add(acc.s0, acc.c0, b0);
             if constexpr (KIND == kKindCos2) kahan_add(acc.s1, acc.c1, b1);
             b0 = b1 = 0.0f;
-            if (KIND == kKindSin && masked) a.nbmask[(size_t)(k / kWarp) * n_all + v] = bits;
           }
+          if (KIND == kKindSin && masked) a.nbmask[(size_t)(k / kWarp) * n_all + v] = bits;
           bits = 0u;
         }
         ++k;
@@ -367,7 +359,7 @@ __global__ void __launch_bounds__(kVThreads) k_vtile(KArgs a, int epi) {
                                           nullptr, nullptr);
         else
           vstage_round<PREC, KIND, false>(a, sc, s_start, s_prefix, rlo, rcnt, nullptr, sm.xy, nullptr,
-                                          sm.phi, sm.dd);
+                                          sm.dcs, sm.dd);
         __syncthreads();
         if (!valid) continue;
         if (rows && rounds == 1 && !exact_all) {
@@ -415,22 +407,7 @@ __global__ void __launch_bounds__(kVThreads) k_vtile(KArgs a, int epi) {
                       b1 = fmaf(sm.df[j] - il.dphif, tv, b1);
                     }
                   } else {
-                    const double dp = dsub(dsub(sm.phi[j], il.phi), sc.alpha);
-                    double *vc = a.vcos ? a.vcos + (size_t)kk * n_all + v : nullptr;
-                    if constexpr (KIND == kKindSin) {
-                      double sn, cn;
-                      if (vc) {  // keep the cosine for the second pass
-                        sincos(dp, &sn, &cn);
-                        *vc = cn;
-                      } else {
-                        sn = sin(dp);
-                      }
-                      acc.s0 = dadd(acc.s0, sn);  // ChimeraSystem.cpp:412
-                    } else {
-                      const double cc = vc ? *vc : cos(dp);  // ChimeraSystem.cpp:634-637
-                      acc.s0 = dadd(acc.s0, ddiv_by(cc, il.card, il.rcard));
-                      acc.s1 = dadd(acc.s1, ddiv_by(dmul(dsub(sm.dd[j], il.dphi), cc), il.card, il.rcard));
-                    }
+                    add_pair<KIND>(acc, il, sm.dcs[j], KIND == kKindCos2 ? sm.dd[j] : 0.0);
                   }
                   bits |= 1u << (kk & (kWarp - 1));
                 }
@@ -442,8 +419,8 @@ __global__ void __launch_bounds__(kVThreads) k_vtile(KArgs a, int epi) {
                 kahan_add(acc.s0, acc.c0, b0);
                 if constexpr (KIND == kKindCos2) kahan_add(acc.s1, acc.c1, b1);
                 b0 = b1 = 0.0f;
-                if (KIND == kKindSin && masked) a.nbmask[(size_t)(c8 >> 2) * n_all + v] = bits;
               }
+              if (KIND == kKindSin && masked) a.nbmask[(size_t)(c8 >> 2) * n_all + v] = bits;
               bits = 0u;
             }
           }
@@ -470,12 +447,14 @@ __global__ void __launch_bounds__(kVThreads) k_vtile(KArgs a, int epi) {
         if constexpr (PREC == kPrecFP32C) {
           kahan_add(acc.s0, acc.c0, b0);
           if constexpr (KIND == kKindCos2) kahan_add(acc.s1, acc.c1, b1);
-          if (KIND == kKindSin && masked && (k & (kWarp - 1)) != 0)
-            a.nbmask[(size_t)(k / kWarp) * n_all + v] = bits;
           acc.s0 = acc.s0 - acc.c0;
           acc.s1 = acc.s1 - acc.c1;
           acc.c0 = acc.c1 = 0.0f;
+        } else {
+          finish_pairs<KIND>(acc, il);
         }
+        if (KIND == kKindSin && masked && (k & (kWarp - 1)) != 0)
+          a.nbmask[(size_t)(k / kWarp) * n_all + v] = bits;
         epilogue<PREC, KIND>(a, epi, sd, il, acc, a.pidx[v]);
       }
     }

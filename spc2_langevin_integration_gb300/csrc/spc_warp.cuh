@@ -44,7 +44,7 @@ constexpr double kSparseBelowDefault = 24.0;
 // Candidates of the staging round [rlo, rlo + rcnt) into shared memory.
 template <int PREC, int KIND>
 __device__ __forceinline__ void stage_round(const KArgs &a, const SysConst &sc, const Stencil &st, int rlo,
-                                            int rcnt, int lane, float4 *c4, float2 *xy, double *phi,
+                                            int rcnt, int lane, float4 *c4, float2 *xy, double2 *dcs,
                                             float *df, double *dd) {
   for (int k = lane; k < rcnt; k += kWarp) {
     int q;
@@ -57,7 +57,7 @@ __device__ __forceinline__ void stage_round(const KArgs &a, const SysConst &sc, 
       if constexpr (KIND == kKindCos2) df[k] = a.dphi_f[pj];
     } else {
       xy[k] = make_float2(xs, ys);
-      phi[k] = a.sphi[pj];
+      dcs[k] = a.dcs[pj];
       if constexpr (KIND == kKindCos2) dd[k] = a.dphi_s[pj];
     }
   }
@@ -65,8 +65,8 @@ __device__ __forceinline__ void stage_round(const KArgs &a, const SysConst &sc, 
 
 __device__ __forceinline__ void invalid_lane(ILane &il) {
   il.fx = il.fy = 3.0e30f;
-  il.x = il.y = il.phi = il.dphi = 0.0;
-  il.card = il.rcard = 1.0;
+  il.x = il.y = il.dphi = 0.0;
+  il.card = 1.0;
   il.ca = il.sa = il.dphif = 0.0f;
 }
 
@@ -361,7 +361,7 @@ __global__ void __launch_bounds__(kWarpPassThreads, 8) k_warp_fp32x(KArgs a, int
 template <int KIND>
 struct WarpStage64 {
   float2 xy[kWarpCap];  // x+shift, y+shift (prefilter)
-  double phi[kWarpCap];
+  double2 dcs[kWarpCap];  // cos, sin of the stage phase
   double dd[KIND == kKindCos2 ? kWarpCap : 1];  // pass 2: phase rate
   uint8_t acc[2 * kWarp];                       // accepted candidates, in order
 };
@@ -402,15 +402,15 @@ __global__ void __launch_bounds__(kWarpPassThreads) k_warp_fp64(KArgs a, int epi
         const int nwords = (rcnt + kWarp - 1) / kWarp;
         __syncwarp();
         if (rounds > 1 || ib == cb)
-          stage_round<kPrecFP64, KIND>(a, sc, st, rlo, rcnt, lane, nullptr, sm.xy, sm.phi, nullptr, sm.dd);
+          stage_round<kPrecFP64, KIND>(a, sc, st, rlo, rcnt, lane, nullptr, sm.xy, sm.dcs, nullptr, sm.dd);
         __syncwarp();
         for (int i = 0; i < gn; ++i) {
           const float fxi = __shfl_sync(FULL, il.fx, i), fyi = __shfl_sync(FULL, il.fy, i);
           const int self = st.prefix[4] + (ib - cb) + i - rlo;  // staged index of i (may be outside)
-          const double phii = __shfl_sync(FULL, il.phi, i);
-          const double cardi = KIND == kKindCos2 ? __shfl_sync(FULL, il.card, i) : 1.0;
-          const double rcardi = KIND == kKindCos2 ? __shfl_sync(FULL, il.rcard, i) : 1.0;
-          const double dphii = KIND == kKindCos2 ? __shfl_sync(FULL, il.dphi, i) : 0.0;
+          ILane ii;  // particle i's terms
+          ii.dca = __shfl_sync(FULL, il.dca, i);
+          ii.dsa = __shfl_sync(FULL, il.dsa, i);
+          ii.dphi = KIND == kKindCos2 ? __shfl_sync(FULL, il.dphi, i) : 0.0;
           int n_i = 0, nacc = 0;
           // evaluate the first cnt listed candidates (one per lane) and add
           // them on lane i in list order
@@ -418,13 +418,11 @@ __global__ void __launch_bounds__(kWarpPassThreads) k_warp_fp64(KArgs a, int epi
             double v0 = 0.0, v1 = 0.0;
             if (lane < cnt) {
               const int jj = sm.acc[lane];
-              const double dp = dsub(dsub(sm.phi[jj], phii), sc.alpha);
               if constexpr (KIND == kKindSin) {
-                v0 = sin(dp);  // ChimeraSystem.cpp:412
+                v0 = pair_sin(sm.dcs[jj], ii);  // ChimeraSystem.cpp:412
               } else {
-                const double cc = cos(dp);  // ChimeraSystem.cpp:634-637
-                v0 = ddiv_by(cc, cardi, rcardi);
-                v1 = ddiv_by(dmul(dsub(sm.dd[jj], dphii), cc), cardi, rcardi);
+                v0 = pair_cos(sm.dcs[jj], ii);  // ChimeraSystem.cpp:634-637
+                v1 = dsub(sm.dd[jj], ii.dphi);
               }
             }
             for (int k = 0; k < cnt; ++k) {
@@ -432,7 +430,7 @@ __global__ void __launch_bounds__(kWarpPassThreads) k_warp_fp64(KArgs a, int epi
               if (lane == i) my_d0 = dadd(my_d0, t0);
               if constexpr (KIND == kKindCos2) {
                 const double t1 = __shfl_sync(FULL, v1, k);
-                if (lane == i) my_d1 = dadd(my_d1, t1);
+                if (lane == i) my_d1 = __fma_rn(t1, t0, my_d1);
               }
             }
           };
@@ -479,6 +477,7 @@ __global__ void __launch_bounds__(kWarpPassThreads) k_warp_fp64(KArgs a, int epi
         acc.s0 = my_d0;
         acc.s1 = my_d1;
         acc.n = my_n;
+        finish_pairs<KIND>(acc, il);
         epilogue<kPrecFP64, KIND>(a, epi, sd, il, acc, a.pidx[p]);
       }
     }
