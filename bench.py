@@ -50,18 +50,18 @@ ALG_BYTES = {
 }
 ALG_BYTES_STEP = 168 + 8      # survey accounting for the whole SRK step (+ omega)
 # The kernels of each phase, by form (the cell-list forms; a phase that runs
-# the cell-tile and the warp-per-cell kernels, for dense and sparse cells,
+# the cell-tile and the particle-per-lane kernels, for dense and sparse cells,
 # counts both).
 PHASE_KERNELS = {
     "fp32c": {"stage": ["k_stage"], "sort": ["k_scan_digits", "k_radix_scatter"],
               "gather": ["k_gather<1>", "k_list_units (cell units on)"],
-              "pass1": ["k_tile_fp32c<0>", "k_units_fp32c<0> (cell units on)", "k_warp_fp32c<0>"],
-              "pass2": ["k_tile_fp32c<1>", "k_units_fp32c<1> (cell units on)", "k_warp_fp32c<1>"]},
+              "pass1": ["k_tile_fp32c<0>", "k_units_fp32c<0> (cell units on)", "k_lane<1, 0>"],
+              "pass2": ["k_tile_fp32c<1>", "k_units_fp32c<1> (cell units on)", "k_lane<1, 1>"]},
     "fp32x": {"stage": ["k_stage"], "sort": ["k_scan_digits", "k_radix_scatter"],
               "gather": ["k_gather<2>", "k_list_units (cell units on)"],
-              "pass1": ["k_tile_fp32x<0>", "k_units_fp32x<0> (cell units on)", "k_warp_fp32x<0>",
+              "pass1": ["k_tile_fp32x<0>", "k_units_fp32x<0> (cell units on)", "k_lane<2, 0>",
                         "k_epilogue_fp32x<0>"],
-              "pass2": ["k_tile_fp32x<1>", "k_units_fp32x<1> (cell units on)", "k_warp_fp32x<1>",
+              "pass2": ["k_tile_fp32x<1>", "k_units_fp32x<1> (cell units on)", "k_lane<2, 1>",
                         "k_epilogue_fp32x<1>"]},
     "fp64": {"stage": ["k_stage"], "sort": ["k_scan_digits", "k_radix_scatter"],
              "gather": ["k_gather<0>", "k_vgather<0>"], "pass1": ["k_vtile<0,0>", "k_tile_fp64<0>"],
@@ -1166,7 +1166,7 @@ def main():
                          "phase profiles of cell tiles, cell units and sub-cells (float forms)")
     ap.add_argument("--sparse-below", type=float, default=None,
                     help="ensemble: neighbour-kernel tuning (mean particles per cell below "
-                         "which a system runs the warp-per-cell passes)")
+                         "which a system runs the particle-per-lane passes)")
     ap.add_argument("--compare-kernels", action="store_true",
                     help="ensemble: also time every system on the cell-tile passes")
     ap.add_argument("--drift-steps", type=int, default=10000)

@@ -226,7 +226,7 @@ int spc_profile_steps(spc_handle *h, double dt, int32_t nsteps, double *out_ms, 
 /* Tuning knobs (no counterpart in the reference; results do not depend on
  * them beyond floating-point summation order in the FP32C form).
  * SPC_TUNE_SPARSE_BELOW: cell-list systems with fewer particles per cell
- * than this value (on average) run the warp-per-cell neighbour passes, the
+ * than this value (on average) run the particle-per-lane neighbour passes, the
  * others the cell-tile passes; 0 sends every system to the cell-tile passes.
  * Default 24.
  * SPC_TUNE_VERLET_ROW_LIMIT (Verlet handles only): the longest neighbour row
@@ -274,7 +274,7 @@ int spc_get_tuning(const spc_handle *h, int32_t key, double *value);
 /* Autotuner (no counterpart in the reference).  Times `trial_steps` steps
  * (as captured graphs, after one warm-up call) of every candidate on the
  * caller's state and keeps the fastest: the cell-list passes with the
- * cell-tile or the warp-per-cell kernels, and, where the stencil allows
+ * cell-tile or the particle-per-lane kernels, and, where the stencil allows
  * Verlet rows, rows with skins of 0.1, 0.2 and 0.4 rho.  Every candidate
  * computes the same neighbour sets; FP64 results differ between them only by
  * summation order.  omega is required for the vortex model.  On return *best
@@ -298,7 +298,7 @@ typedef struct spc_tuning {
 
 /* Autotuner over every tuning dimension (no counterpart in the reference):
  * the cell-list passes with each kernel choice (all cell-tile, the default
- * split between cell-tile and warp-per-cell, all warp-per-cell) and, for the
+ * split between cell-tile and particle-per-lane, all particle-per-lane) and, for the
  * cell-tile kernels, 1, 2 or 4 CTAs per cell; and Verlet rows with skins of
  * 0.1, 0.2 and 0.4 rho where the stencil and the precision allow.  Each
  * candidate runs trial_steps steps as a captured graph on its own handle

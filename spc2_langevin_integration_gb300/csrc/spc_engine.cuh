@@ -28,7 +28,7 @@
 #include "spc_kernels.cuh"
 #include "spc_sort.cuh"
 #include "spc_tile.cuh"
-#include "spc_warp.cuh"
+#include "spc_lane.cuh"
 #include "spc_verlet.cuh"
 #include "spc_va.cuh"
 
@@ -212,7 +212,7 @@ struct Engine {
   int ncell_tile = 0, ncell_warp = 0, ncell_va = 0;  // cells of the tile, warp and vortex-arrays systems
   bool has_cells = false;
   // tuning: cell-list systems with fewer than sparse_below particles per cell
-  // (on average) run the warp-per-cell passes
+  // (on average) run the particle-per-lane passes
   double sparse_below = kSparseBelowDefault;
   // tuning: CTAs per cell of the cell-tile kernels (0: chosen per layout)
   int tile_split_tune = 0;
@@ -384,7 +384,7 @@ inline int engine_init(Engine *e, int stepper, int precision, int pool_cap, int 
   SPC_TRY(dalloc(e, &a.sx, N));
   SPC_TRY(dalloc(e, &a.sy, N));
   SPC_TRY(dalloc(e, &a.sphi, N));
-  SPC_TRY(dalloc(e, &a.fxy, N));
+  SPC_TRY(dalloc(e, &a.fxy, N + kFxyPad));
   SPC_TRY(dalloc(e, &a.pidx, N));
   SPC_TRY(dalloc(e, &a.dphi_s, N));
   SPC_TRY(dalloc(e, &a.cnt_s, N));
@@ -664,7 +664,7 @@ inline SysDesc desc_of(const SysHost &h, int dense_p0, int c0) {
 }
 
 // 0: cell list, dense cells (cell-tile kernels); 1: cell list, sparse cells
-// (warp-per-cell kernel); 2: vortex-arrays model (its own kernel, cell list or
+// (particle-per-lane kernel); 2: vortex-arrays model (its own kernel, cell list or
 // all pairs); 3: all pairs.
 inline int system_class(const Engine *e, const SysHost &h) {
   if (h.sc.va) return 2;
@@ -687,7 +687,7 @@ inline std::vector<long long> launch_shape(const Engine *e) {
   return {e->nsys, e->n_active, e->ncell_total, e->ntiles, e->radix_bits, e->sort_passes, e->ncell_tile,
           e->ncell_warp, e->ncell_va, e->n_ap_all, e->has_cells, a.n_ap, a.tile_split, a.hist_len,
           e->ap_items, e->ap_items_all, e->ap_items_small, e->ap_items_all_small, a.units != nullptr,
-          a.cell_mid != nullptr};
+          a.cell_mid != nullptr, a.lane_p0, a.lane_p1};
 }
 
 inline int engine_layout(Engine *e) {
@@ -698,9 +698,10 @@ inline int engine_layout(Engine *e) {
   std::vector<int> ap, ap_all;
   int dense = 0, cells = 0;
   std::fill(e->slot_layout.begin(), e->slot_layout.end(), -1);
-  // cell-tile systems first, then warp-per-cell, vortex-arrays and all-pairs
+  // cell-tile systems first, then particle-per-lane, vortex-arrays and all-pairs
   // systems, so that each neighbour kernel covers one contiguous range of cells
-  int ncell_tile = 0, ncell_warp = 0, ncell_va = 0;
+  // and, for the lane kernel, of cell-order slots
+  int ncell_tile = 0, ncell_warp = 0, ncell_va = 0, lane_p0 = 0, lane_p1 = 0;
   e->ap_items = e->ap_items_all = 0;
   e->ap_items_small = e->ap_items_all_small = 0;
   for (int cls = 0; cls < 4; ++cls) {
@@ -727,6 +728,8 @@ inline int engine_layout(Engine *e) {
       if (cls == 1) ncell_warp += h.ncell;
       if (cls == 2) ncell_va += h.ncell;
     }
+    if (cls == 0) lane_p0 = dense;
+    if (cls == 1) lane_p1 = dense;
   }
   e->ncell_tile = ncell_tile;
   e->ncell_warp = ncell_warp;
@@ -753,6 +756,8 @@ inline int engine_layout(Engine *e) {
   a.units = (e->cell_units_tune || sub) ? e->units_buf : nullptr;
   a.cell_mid = sub ? e->cell_mid_buf : nullptr;
   a.cell_near = sub ? e->cell_near_buf : nullptr;
+  a.lane_p0 = lane_p0;
+  a.lane_p1 = e->verlet ? lane_p0 : lane_p1;  // Verlet passes serve every cell-list system
   a.va_c0 = e->ncell_tile + e->ncell_warp;
   a.va_c1 = a.va_c0 + e->ncell_va;
   a.n_ap = (int)ap.size();
@@ -797,6 +802,7 @@ inline int eval_stage(Engine *e, KArgs &a, int rk_form, int kq, double kcdt, boo
   if (!verlet_ok) {
     a.cell_mid = nullptr;
     a.cell_near = nullptr;
+    a.lane_p0 = a.lane_p1 = 0;  // every prefilter coordinate relative to its own cell
     // they run the FP64 gather and pass: cos / sin of the phases go behind
     // the results in the AoS staging area (12 doubles per pool particle)
     a.dcs = reinterpret_cast<double2 *>(e->aos + (((size_t)e->pool_cap + 1) & ~(size_t)1));
@@ -935,8 +941,8 @@ int launch_pass_t(Engine *e, const KArgs &a, int epi) {
       SPC_LAUNCHED(e);
     }
   }
-  if (e->has_cells) {
-    {
+  if constexpr (KIND != kKindNb) {
+    if (e->has_cells) {
       if (e->ncell_tile > 0) {
         const int grid = std::min(e->ncell_tile * std::max(a.tile_split, 1), 152 * 256);
         if constexpr ((PREC == kPrecFP32C || PREC == kPrecFP32X) && KIND != kKindNb) {
@@ -973,19 +979,16 @@ int launch_pass_t(Engine *e, const KArgs &a, int epi) {
           if (a.units) SPC_CUDA(e, cudaStreamWaitEvent(st, e->join_ev, 0));
       }
       if (e->ncell_warp > 0) {
-        const int grid = std::min(blocks_for(e->ncell_warp, kWarpPassWarps), 152 * 64);
-        if constexpr (PREC == kPrecFP32C)
-          k_warp_fp32c<KIND><<<grid, kWarpPassThreads, 0, st>>>(a, epi);
-        else if constexpr (PREC == kPrecFP32X)
-          k_warp_fp32x<KIND><<<grid, kWarpPassThreads, 0, st>>>(a, epi);
-        else
-          k_warp_fp64<KIND><<<grid, kWarpPassThreads, 0, st>>>(a, epi);
+        // one warp per CTA when that spreads the particles over more SMs
+        const int np = a.lane_p1 - a.lane_p0;
+        const int threads = np >= 152 * 4 * kLaneThreads ? kLaneThreads : kWarp;
+        k_lane<PREC, KIND><<<blocks_for(np, threads), threads, 0, st>>>(a, epi);
         SPC_LAUNCHED(e);
       }
-      if constexpr (PREC == kPrecFP32X && KIND != kKindNb) {
-        // the neighbour kernels wrote the sums; the FP64 epilogues run densely
-        if (e->ncell_tile + e->ncell_warp > 0) {
-          k_epilogue_fp32x<KIND><<<blocks_for(e->n_active, 256), 256, 0, st>>>(a, epi);
+      if constexpr (PREC == kPrecFP32X) {
+        // the cell-tile kernels wrote the sums; the FP64 epilogues run densely
+        if (e->ncell_tile > 0) {
+          k_epilogue_fp32x<KIND><<<blocks_for(a.lane_p0, 256), 256, 0, st>>>(a, epi, a.lane_p0);
           SPC_LAUNCHED(e);
         }
       }
@@ -1203,8 +1206,8 @@ inline int engine_get_tuning(const Engine *e, int key, double *value) {
 }
 
 // Kernel-choice candidates of the cell-list passes: the threshold below which
-// systems take the warp-per-cell kernels (all cell-tile, the default, all
-// warp-per-cell) and the cell-tile kernels' CTAs per cell.
+// systems take the particle-per-lane kernel (all cell-tile, the default, all
+// particle-per-lane) and the cell-tile kernels' CTAs per cell.
 struct TuneCand {
   double sparse;
   int split;

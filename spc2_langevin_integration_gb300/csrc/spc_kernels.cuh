@@ -46,6 +46,7 @@ enum Epilogue {
   kEpiLocalOrder = 9,  // per-particle local order parameter
 };
 
+constexpr int kFxyPad = 4;  // the lane kernel reads candidates four at a time
 constexpr int kKSlots = 6;  // RK4 k1..k4 (persistent) + two scratch slots for spc_rhs_rk
 
 // One system of a batch.
@@ -69,7 +70,8 @@ struct KArgs {
   int ncell_total;
   int ncell_tile;                    // cells [0, ncell_tile): cell-tile kernels
   int tile_split;                    // cell-tile kernels: CTAs per cell (0 or 1: one)
-  int va_c0, va_c1;                  // [ncell_tile, va_c0): warp kernel; [va_c0, va_c1): vortex arrays
+  int va_c0, va_c1;                  // [ncell_tile, va_c0): lane kernel; [va_c0, va_c1): vortex arrays
+  int lane_p0, lane_p1;              // cell-order slots of the lane kernel's systems
   const int *sys_of_p;               // dense index -> system
   const int *sys_of_c;               // global cell -> system
   // state pool (structure of arrays)
@@ -90,7 +92,8 @@ struct KArgs {
   uint8_t *cell_near;
   // cell order
   double *sx, *sy, *sphi;
-  float2 *fxy;                       // prefilter coordinates relative to the cell origin
+  float2 *fxy;                       // prefilter coordinates relative to the cell origin (lane kernel's
+                                     // systems: x relative to the column block's), kFxyPad entries more
   float2 *cs;                        // FP32C: (cos phi, sin phi)
   double2 *dcs;                      // FP64 passes: (cos phi, sin phi) of the stage phase
   longlong2 *ics;                    // FP32X: (cos phi, sin phi) in fixed point (2^kXQ)
@@ -248,6 +251,12 @@ __device__ __forceinline__ float reduced_phase_f(double ph) {
   return (float)(ph - two_pi * rint(ph * inv_two_pi));
 }
 
+// Column blocks of a row of nc cells (particle-per-lane passes): blocks of 16,
+// the last one up to 31; the first column of cx's block.
+__device__ __forceinline__ int block_first(int cx, int nc) {
+  return min(cx >> 4, max((nc >> 4) - 1, 0)) << 4;
+}
+
 template <int PREC>
 __global__ void k_gather(KArgs a) {
   if (a.gate && *a.gate == 0) return;
@@ -280,7 +289,8 @@ __global__ void k_gather(KArgs a) {
   if (!sc.allpairs) {
     const int key = cell_of_slot(a, p) - sd.c0;
     const int cx = key % sc.nc, cy = key / sc.nc;
-    a.fxy[p] = make_float2((float)(x - (double)cx * sc.cell), (float)(y - (double)cy * sc.cell));
+    const int ox = p >= a.lane_p0 && p < a.lane_p1 ? block_first(cx, sc.nc) : cx;
+    a.fxy[p] = make_float2((float)(x - (double)ox * sc.cell), (float)(y - (double)cy * sc.cell));
     if (a.cell_mid && fabs(row_offset(sc, y, cy) - 0.5 * sc.cell) < kNearHalf * sc.cell)
       a.cell_near[sd.c0 + key] = 1;
   }
@@ -323,11 +333,9 @@ struct Acc<kPrecFP32C> {
 
 // Word w (< 32) of the pass-1 neighbour bitmask of cell-order slot p among n
 // active particles.  Four consecutive words of a particle share one 16-byte
-// group.  The cell-tile and warp-per-cell kernels of one pass write the same
-// buffer for the particles of their own cells, so both must index it this way:
-// distinct (w, p) never share a word.  (The Verlet kernels keep a word-major
-// layout of their own; a Verlet engine holds one system and runs no other
-// neighbour kernel in the pass.)
+// group, and all kernels of a pass that index a buffer this way never share a
+// word.  (The Verlet kernels keep a word-major layout of their own: a Verlet
+// engine holds one system and runs no other neighbour kernel in the pass.)
 __device__ __forceinline__ size_t mask_at(int w, int p, int n) {
   return ((size_t)(w >> 2) * n + p) * 4 + (w & 3);
 }
@@ -365,6 +373,7 @@ struct ILane {
   bool valid;
   float fx, fy; // prefilter coordinates
   double x, y;  // wrapped stage position
+  double phi;   // stage phase
   double card;  // pass 2: n_i from pass 1 (double, as neighborhood_cardinality_)
   double dphi;  // pass 2: own phase rate
   float ca, sa; // FP32C: cos(phi + alpha), sin(phi + alpha)
@@ -378,29 +387,39 @@ struct ILane {
 // sin phi, evaluated once by the gather, and with theta_i = phi_i + alpha by
 // angle addition: two operations of the FP64 pipe per term instead of the ~25
 // of a sine (GB300 runs FP64 at 1/64 of the FP32 rate, and the pair terms
-// filled that pipe: 75% busy).  A term's absolute error is ~1.5e-16, as that
-// of the sine of the twice rounded difference, and the terms are added in the
-// reference's order as before; the mean of 200 terms is 2.4e-17 (uniform
-// phases, before 2.9e-17) to 3.5e-16 (aligned, alpha = 1.45: the same as
-// before) from the exact one.  Vortex SRK step, N = 65,536: 2.96 -> 0.44
-// ms on the cell list.
-__device__ __forceinline__ double pair_sin(double2 cj, const ILane &il) {
-  return __fma_rn(cj.y, il.dca, -dmul(cj.x, il.dsa));
+// filled that pipe: 75% busy).  A term's absolute error is below 3.5e-16, as
+// that of the sine of the twice rounded difference; a term below 2^-11, whose
+// relative error would pass 7e-13 (1e-12 is the right-hand sides' contract),
+// is evaluated as the reference writes it: 1 term in 1,600 of unrelated
+// phases.  The terms are added in the reference's order as before; the mean of
+// 200 terms is 2.4e-17 (uniform phases, before 2.9e-17) to 3.5e-16 (aligned,
+// alpha = 1.45: the same as before) from the exact one.  Vortex SRK step,
+// N = 65,536: 2.96 -> 0.45 ms on the cell list.
+__device__ __noinline__ double sin_of_difference(double pj, double pi, double alpha) {
+  return sin(dsub(dsub(pj, pi), alpha));
 }
-__device__ __forceinline__ double pair_cos(double2 cj, const ILane &il) {
-  return __fma_rn(cj.x, il.dca, dmul(cj.y, il.dsa));
+__device__ __noinline__ double cos_of_difference(double pj, double pi, double alpha) {
+  return cos(dsub(dsub(pj, pi), alpha));
+}
+// |t| < 2^-11
+__device__ __forceinline__ bool small_term(double t) {
+  return (unsigned)(__double2hiint(t) & 0x7fffffff) < 0x3f400000u;
 }
 // One accepted pair: pass 1 adds the sine, pass 2 the cosine and the cosine
-// weighted by the difference of the phase rates.  The second pass's quotients
-// by n_i are taken once of each sum (finish_pairs).
-template <int KIND>
-__device__ __forceinline__ void add_pair(Acc<kPrecFP64> &acc, const ILane &il, double2 cj, double dj) {
+// weighted by the difference of the phase rates.  phase() gives phi_j.  The
+// second pass's quotients by n_i are taken once of each sum (finish_pairs).
+template <int KIND, class Phase>
+__device__ __forceinline__ void add_pair(Acc<kPrecFP64> &acc, const SysConst &sc, const ILane &il, double2 cj,
+                                         double dj, Phase phase) {
   if constexpr (KIND == kKindSin) {
-    acc.s0 = dadd(acc.s0, pair_sin(cj, il));
+    double t = __fma_rn(cj.y, il.dca, -dmul(cj.x, il.dsa));
+    if (small_term(t)) t = sin_of_difference(phase(), il.phi, sc.alpha);
+    acc.s0 = dadd(acc.s0, t);
   } else {
-    const double c = pair_cos(cj, il);
-    acc.s0 = dadd(acc.s0, c);
-    acc.s1 = __fma_rn(dsub(dj, il.dphi), c, acc.s1);
+    double t = __fma_rn(cj.x, il.dca, dmul(cj.y, il.dsa));
+    if (small_term(t)) t = cos_of_difference(phase(), il.phi, sc.alpha);
+    acc.s0 = dadd(acc.s0, t);
+    acc.s1 = __fma_rn(dsub(dj, il.dphi), t, acc.s1);
   }
 }
 template <int KIND>
@@ -447,7 +466,7 @@ __device__ __forceinline__ void accept_pair(const KArgs &a, const SysDesc &sd, c
                                             float dphij_f, long long &wpos) {
   if constexpr (KIND == kKindSin) {
     if constexpr (PREC == kPrecFP64) {
-      add_pair<KIND>(acc, il, a.dcs[pj], 0.0);  // ChimeraSystem.cpp:412
+      add_pair<KIND>(acc, sd.sc, il, a.dcs[pj], 0.0, [&]() { return a.sphi[pj]; });  // ChimeraSystem.cpp:412
     } else {
       // sin(phi_j - (phi_i + alpha)) by the angle-difference identity
       kahan_add(acc.s0, acc.c0, cjs * il.ca - cjc * il.sa);
@@ -455,7 +474,7 @@ __device__ __forceinline__ void accept_pair(const KArgs &a, const SysDesc &sd, c
     acc.n++;
   } else if constexpr (KIND == kKindCos2) {
     if constexpr (PREC == kPrecFP64) {
-      add_pair<KIND>(acc, il, a.dcs[pj], a.dphi_s[pj]);  // ChimeraSystem.cpp:634-637
+      add_pair<KIND>(acc, sd.sc, il, a.dcs[pj], a.dphi_s[pj], [&]() { return a.sphi[pj]; });  // :634-637
     } else {
       const float c = cjc * il.ca + cjs * il.sa;
       kahan_add(acc.s0, acc.c0, c);
@@ -674,6 +693,7 @@ __device__ __forceinline__ void load_i(const KArgs &a, const SysConst &sc, ILane
   if (!valid) return;
   il.x = a.sx[p];
   il.y = a.sy[p];
+  il.phi = a.sphi[p];
   if (!sc.allpairs) {
     const float2 f = a.fxy[p];
     il.fx = f.x;
@@ -754,16 +774,15 @@ __device__ void epilogue_fp32x(const KArgs &a, int epi, const SysDesc &sd, const
 
 // FP32X epilogues as their own dense launch: one thread per cell-order slot,
 // so the FP64 per-particle work (rates, noise, the stepper update) runs on
-// full warps, while the neighbour kernels, whose warps cover cells of a few
-// particles, only write each particle's sums (xsum, xcnt).  All-pairs systems
-// finish in their own (FP64) kernel.
+// full warps, while the cell-tile kernels only write each particle's sums
+// (xsum, xcnt).  Slots [0, n): the cell-tile systems; the particle-per-lane
+// and all-pairs kernels finish their own.
 template <int KIND>
-__global__ void __launch_bounds__(256) k_epilogue_fp32x(KArgs a, int epi) {
+__global__ void __launch_bounds__(256) k_epilogue_fp32x(KArgs a, int epi, int n) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= a.n_active) return;
+  if (p >= n) return;
   const SysDesc &sd = a.sys[a.sys_of_c[cell_of_slot(a, p)]];
   const SysConst &sc = sd.sc;
-  if (sc.allpairs) return;
   ILane il;
   load_i<kPrecFP32X, KIND>(a, sc, il, p, true);
   const double2 v = a.xsum[p];
@@ -976,7 +995,7 @@ __global__ void __launch_bounds__(T) k_allpairs_pass(KArgs a, int epi) {
         const int t = __clz(bits), k = wd * kWarp + t;
         bits ^= 0x80000000u >> t;
         if constexpr (kPair64) {
-          add_pair<KIND>(acc, il, t_cs[k], KIND == kKindCos2 ? t_d[k] : 0.0);
+          add_pair<KIND>(acc, sc, il, t_cs[k], KIND == kKindCos2 ? t_d[k] : 0.0, [&]() { return a.sphi[jt + k]; });
           acc.n++;
         } else {
           float cc = 0.0f, ss = 0.0f, dj = 0.0f;

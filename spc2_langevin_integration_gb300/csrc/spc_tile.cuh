@@ -1208,7 +1208,10 @@ __global__ void __launch_bounds__(kTileThreads64) k_tile_fp64(KArgs a, int epi) 
           if (bits == 0u) break;
           const int t = __clz(bits), j = w * kWarp + t;
           bits ^= 0x80000000u >> t;
-          add_pair<KIND>(acc, il, s_cs[j], KIND == kKindCos2 ? s_d[j] : 0.0);
+          add_pair<KIND>(acc, sc, il, s_cs[j], KIND == kKindCos2 ? s_d[j] : 0.0, [&]() {
+            int q;
+            return a.sphi[slot_of(st, rlo + j, q)];
+          });
         }
       }
       if (valid) {

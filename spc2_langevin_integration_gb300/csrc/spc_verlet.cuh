@@ -335,7 +335,8 @@ __global__ void __launch_bounds__(kVThreads) k_vtile(KArgs a, int epi) {
               b1 = fmaf(sm.df[j] - il.dphif, tv, b1);
             }
           } else {
-            add_pair<KIND>(acc, il, sm.dcs[j], KIND == kKindCos2 ? sm.dd[j] : 0.0);
+            add_pair<KIND>(acc, sc, il, sm.dcs[j], KIND == kKindCos2 ? sm.dd[j] : 0.0,
+                           [&]() { return a.sphi[vslot_of(sc, s_start, s_prefix, g)]; });
           }
           bits |= 1u << (k & (kWarp - 1));
         }
@@ -407,7 +408,8 @@ __global__ void __launch_bounds__(kVThreads) k_vtile(KArgs a, int epi) {
                       b1 = fmaf(sm.df[j] - il.dphif, tv, b1);
                     }
                   } else {
-                    add_pair<KIND>(acc, il, sm.dcs[j], KIND == kKindCos2 ? sm.dd[j] : 0.0);
+                    add_pair<KIND>(acc, sc, il, sm.dcs[j], KIND == kKindCos2 ? sm.dd[j] : 0.0,
+                           [&]() { return a.sphi[vslot_of(sc, s_start, s_prefix, j)]; });
                   }
                   bits |= 1u << (kk & (kWarp - 1));
                 }
