@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 
 #include "spc_fixed.h"
+#include "spc_math.h"
 
 namespace spc {
 
@@ -46,11 +47,7 @@ __device__ __forceinline__ double dsqrt(double a) { return __dsqrt_rn(a); }
 // 2^62 in magnitude, so the integer sums are exact, and the conversion back
 // (one rounding to double) is the only error of a round's sum.
 constexpr int kXQ = 52;
-// v 2^q is exact (a power-of-two scaling of a normal result), then rounded
-// to the nearest integer
-__device__ __forceinline__ long long to_fixed(double v, int q) {
-  return __double2ll_rn(__dmul_rn(v, pow2i(q)));
-}
+__device__ __forceinline__ long long to_fixed(double v, int q) { return double_to_fixed(v, q); }
 __device__ __forceinline__ double from_fixed(long long v, int q) { return fixed_to_double(v, q); }
 // A particle's whole sum over several staging rounds is kept in 128 bits, so
 // it is one exact integer whatever the kernel's round size, and converted to
@@ -86,6 +83,41 @@ __device__ __forceinline__ void fmaf2_if(float &c, float &s, float d, float x, f
       : "f"(d), "f"(x), "f"(y), "r"((int)p));
 }
 
+// sin and cos of a stage phase (spc_math.h; the library's beyond its range).
+__device__ __noinline__ void sincos_library(double ph, double *s, double *c) { sincos(ph, s, c); }
+__device__ __forceinline__ void sincos_phase(double ph, double &s, double &c) {
+  if (phase_in_range(ph))
+    sincos_in_range(ph, s, c);
+  else
+    sincos_library(ph, &s, &c);
+}
+
+// A neighbour count as a double with its reciprocal rounded to nearest, for
+// ddiv_by: a table of the usual counts in place of a conversion and a division
+// (about ten operations of the FP64 pipe).
+struct Count {
+  double n, r;
+};
+constexpr int kCounts = 512;
+struct CountTable {
+  Count v[kCounts];
+  constexpr CountTable() : v() {
+    for (int i = 0; i < kCounts; ++i) v[i] = Count{(double)i, i ? 1.0 / (double)i : 0.0};
+  }
+};
+static __device__ const CountTable kCountTable = CountTable();
+__device__ __forceinline__ Count count_of(int n) {
+  if ((unsigned)n < (unsigned)kCounts) return kCountTable.v[n];
+  const double d = (double)n;
+  return Count{d, drcp(d)};
+}
+
+// 0 <= x < L, or x = -0.0, by the bit patterns (NaN: false).
+__device__ __forceinline__ bool in_box(double x, double L) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  return b < (unsigned long long)__double_as_longlong(L) || b == 0x8000000000000000ull;
+}
+
 // Per-system constants, the reference's ChimeraSystem / PeriodicBoundaryConditions
 // members (ChimeraSystem.cpp:19-33, PeriodicBoundaryConditions.cpp:13-14).
 struct SysConst {
@@ -101,7 +133,7 @@ struct SysConst {
   float cell_f;
   float lo2, hi2; // prefilter: float dr^2 < lo2 => inside, > hi2 => outside, else decide in FP64
   int exact_all;  // decide every candidate in FP64
-  int L_pow2;     // L is a power of two: x / L == x * (1 / L) exactly
+  double ncd;     // nc as a double
   float cos_a, sin_a;  // FP32C: cos(alpha), sin(alpha) rounded to float
   // FP32X: cos(alpha), sin(alpha) in double, and the fixed-point exponent of
   // the phase-rate-weighted sums of the SRK second pass (sum_j d_j cos phi_j,
@@ -142,8 +174,13 @@ __device__ __forceinline__ bool exact_within(const SysConst &sc, double xi, doub
 // ApplyPeriodicBoundaryConditions (PeriodicBoundaryConditions.cpp:117-121): x - floor(x * rL) * L.
 // When 0 <= x * rL < 1 (an unsigned compare of the bits; -0.0 and NaN fail it)
 // floor gives +0.0 and x - 0.0 * L is x itself, so the result is returned
-// without the floor, the product and the difference.
+// without the floor, the product and the difference.  More than 8 units of
+// L's bit pattern below L the product of two roundings is below 1, and it is
+// not formed either.
 __device__ __forceinline__ double wrap_1d(double x, double rL, double L) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  const unsigned long long l = (unsigned long long)__double_as_longlong(L);
+  if (b < l && l - b > 8ull) return x;
   const double t = dmul(x, rL);
   if ((unsigned long long)__double_as_longlong(t) < 0x3FF0000000000000ull) return x;
   return dsub(x, dmul(floor(t), L));
@@ -152,7 +189,7 @@ __device__ __forceinline__ double wrap_1d(double x, double rL, double L) {
 // The conditional copy-wrap inside the force loops (ChimeraSystem.cpp:299-302):
 // both coordinates are wrapped when either is outside [0, L).
 __device__ __forceinline__ void wrap_if_outside(const SysConst &sc, double &x, double &y) {
-  if (x < 0.0 || x >= sc.L || y < 0.0 || y >= sc.L) {
+  if (!(in_box(x, sc.L) && in_box(y, sc.L))) {
     const double xw = wrap_1d(x, sc.rL, sc.L);
     const double yw = wrap_1d(y, sc.rL, sc.L);
     x = xw;
@@ -163,9 +200,8 @@ __device__ __forceinline__ void wrap_if_outside(const SysConst &sc, double &x, d
 // int(x / x_size_ * num_subcells_x_) (ChimeraSystem.cpp:304-305).  An index
 // outside [0, nc) (x within an ulp of L) is clamped; *clamped is set.
 __device__ __forceinline__ int cell_coord(const SysConst &sc, double x, int &clamped) {
-  // for a power-of-two L the scaling by 1/L is exact, so it equals the division
-  const double q = sc.L_pow2 ? dmul(x, sc.rL) : ddiv(x, sc.L);
-  int c = __double2int_rz(dmul(q, (double)sc.nc));
+  const double q = ddiv_by(x, sc.L, sc.rL);
+  int c = __double2int_rz(dmul(q, sc.ncd));
   if (c < 0) {
     c = 0;
     clamped = 1;
@@ -202,18 +238,17 @@ __device__ __forceinline__ U4 philox4x32_10(U4 c, uint32_t k0, uint32_t k1) {
 }
 
 // Two standard normals for (particle i, step) by Box-Muller on two 53-bit
-// uniforms; u1 in (0, 1] so the logarithm is finite.
+// uniforms; u1 in (0, 1] so the logarithm is finite.  (A caller that uses one
+// of them leaves the other's last product to the compiler.)
 __device__ __forceinline__ void philox_normal2(uint64_t seed, uint32_t system_id, uint64_t step,
                                                uint32_t i, double &z0, double &z1) {
   const U4 o = philox4x32_10(U4{i, system_id, (uint32_t)step, (uint32_t)(step >> 32)},
                              (uint32_t)seed, (uint32_t)(seed >> 32));
   const uint64_t a = ((((uint64_t)o.x) << 32) | o.y) >> 11;
   const uint64_t b = ((((uint64_t)o.z) << 32) | o.w) >> 11;
-  const double u1 = (double)(a + 1) * 0x1.0p-53;
-  const double u2 = (double)b * 0x1.0p-53;
-  const double r = sqrt(-2.0 * log(u1));
+  const double r = sqrt_pos(neg2_log53(a + 1));
   double s, c;
-  sincospi(2.0 * u2, &s, &c);
+  sincos_turn53(b, s, c);
   z0 = r * c;
   z1 = r * s;
 }

@@ -43,12 +43,6 @@ inline std::string &global_error() {
   return s;
 }
 
-// A positive finite power of two (then x / L equals x * (1 / L) exactly).
-inline int is_pow2(double L) {
-  int e = 0;
-  return std::frexp(L, &e) == 0.5 ? 1 : 0;
-}
-
 inline int blocks_for(long long n, int threads) { return (int)((n + threads - 1) / threads); }
 
 inline int noise_per_particle(int stepper) {
@@ -73,6 +67,7 @@ inline SysConst make_sysconst(const spc_params &p, int n) {
   sc.D = p.D_phi;
   sc.allpairs = !(p.rho <= 0.25 * p.L);
   sc.nc = sc.allpairs ? 1 : std::max(1, (int)(p.L / p.rho));
+  sc.ncd = (double)sc.nc;
   sc.ncell = sc.nc * sc.nc;
   sc.cell = p.L / sc.nc;
   sc.cell_f = (float)sc.cell;
@@ -81,7 +76,6 @@ inline SysConst make_sysconst(const spc_params &p, int n) {
   sc.lo2 = (float)(sc.rho2 * (1.0 - 3e-5));
   sc.hi2 = (float)(sc.rho2 * (1.0 + 3e-5));
   sc.exact_all = (p.flags & SPC_FLAG_EXACT_ALL) ? 1 : 0;
-  sc.L_pow2 = is_pow2(p.L);
   sc.cos_a = (float)std::cos(p.alpha);
   sc.sin_a = (float)std::sin(p.alpha);
   sc.s2D = std::sqrt(2.0 * p.D_phi);  // correctly rounded, as the device's sqrt

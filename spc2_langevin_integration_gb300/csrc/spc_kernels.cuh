@@ -290,7 +290,7 @@ __global__ void k_gather(KArgs a) {
     const int key = cell_of_slot(a, p) - sd.c0;
     const int cx = key % sc.nc, cy = key / sc.nc;
     const int ox = p >= a.lane_p0 && p < a.lane_p1 ? block_first(cx, sc.nc) : cx;
-    a.fxy[p] = make_float2((float)(x - (double)ox * sc.cell), (float)(y - (double)cy * sc.cell));
+    a.fxy[p] = make_float2((float)__fma_rn(-(double)ox, sc.cell, x), (float)__fma_rn(-(double)cy, sc.cell, y));
     if (a.cell_mid && fabs(row_offset(sc, y, cy) - 0.5 * sc.cell) < kNearHalf * sc.cell)
       a.cell_near[sd.c0 + key] = 1;
   }
@@ -301,13 +301,13 @@ __global__ void k_gather(KArgs a) {
   }
   if constexpr (PREC == kPrecFP32X) {
     double s, c;
-    sincos(ph, &s, &c);
+    sincos_phase(ph, s, c);
     a.ics[p] = make_longlong2(to_fixed(c, kXQ), to_fixed(s, kXQ));
     if (sc.allpairs) a.dcs[p] = make_double2(c, s);  // its passes are the FP64 ones
   }
   if constexpr (PREC == kPrecFP64) {
     double s, c;
-    sincos(ph, &s, &c);
+    sincos_phase(ph, s, c);
     a.dcs[p] = make_double2(c, s);
   }
 }
@@ -374,7 +374,7 @@ struct ILane {
   float fx, fy; // prefilter coordinates
   double x, y;  // wrapped stage position
   double phi;   // stage phase
-  double card;  // pass 2: n_i from pass 1 (double, as neighborhood_cardinality_)
+  int cnt;      // pass 2: n_i from pass 1
   double dphi;  // pass 2: own phase rate
   float ca, sa; // FP32C: cos(phi + alpha), sin(phi + alpha)
   double dca, dsa;  // FP64: the same in double
@@ -425,9 +425,10 @@ __device__ __forceinline__ void add_pair(Acc<kPrecFP64> &acc, const SysConst &sc
 template <int KIND>
 __device__ __forceinline__ void finish_pairs(Acc<kPrecFP64> &acc, const ILane &il) {
   if constexpr (KIND == kKindCos2) {
-    if (il.card > 0.0) {
-      acc.s0 = ddiv(acc.s0, il.card);
-      acc.s1 = ddiv(acc.s1, il.card);
+    if (il.cnt > 0) {
+      const Count n = count_of(il.cnt);
+      acc.s0 = ddiv_by(acc.s0, n.n, n.r);
+      acc.s1 = ddiv_by(acc.s1, n.n, n.r);
     }
   }
 }
@@ -499,6 +500,13 @@ __device__ __forceinline__ double noise_at(const KArgs &a, int q, int k, double 
   return k == 0 ? z0 : z1;
 }
 
+// v + sdt * 0.0 (StochasticEulerStepper.hpp:43: the position's noise is zero),
+// by the bit pattern: it turns -0.0 into 0.0, or v into NaN with sdt.
+__device__ __forceinline__ double plus_zero(double v, double sdt) {
+  if ((__double2hiint(sdt) & 0x7ff00000) == 0x7ff00000) return dadd(v, dmul(sdt, 0.0));
+  return __double_as_longlong(v) == (long long)0x8000000000000000ull ? 0.0 : v;
+}
+
 // Fused epilogue for the particle in pool slot q (system sd) at cell-order slot p.
 template <int PREC, int KIND>
 __device__ void epilogue(const KArgs &a, int epi, const SysDesc &sd, const ILane &il,
@@ -531,7 +539,8 @@ __device__ void epilogue(const KArgs &a, int epi, const SysDesc &sd, const ILane
     if constexpr (KIND == kKindSin) {
       // sigma_ * alignment_force_[i] / neighborhood_cardinality_[i] (:421-424)
       const bool has = acc.n != 0;
-      const double rate = has ? ddiv(dmul(sc.sigma, acc.s0), (double)acc.n) : 0.0;
+      const Count cn = count_of(acc.n);
+      const double rate = has ? ddiv_by(dmul(sc.sigma, acc.s0), cn.n, cn.r) : 0.0;
       if (epi == kEpiRkK || epi == kEpiRk4Combine) {
         if (!live) return;
         const int k = a.kq_out;
@@ -559,8 +568,8 @@ __device__ void epilogue(const KArgs &a, int epi, const SysDesc &sd, const ILane
         // SRK-Ptr stepper does (StochasticRungeKuttaStepperPtr.hpp:65)
         const double sdt = a.sdt;
         const double sto = dmul(sc.s2D, noise_at(a, q, 0, z0, z1));
-        const double xs = dadd(a.x[q], dadd(dmul(dt, d0), dmul(sdt, 0.0)));
-        const double ys = dadd(a.y[q], dadd(dmul(dt, d1), dmul(sdt, 0.0)));
+        const double xs = dadd(a.x[q], plus_zero(dmul(dt, d0), sdt));
+        const double ys = dadd(a.y[q], plus_zero(dmul(dt, d1), sdt));
         const double drift = sd.is_vortex ? dadd(a.omega[q], rate) : rate;
         a.phi[q] = dadd(a.phi[q], dadd(dmul(dt, drift), dmul(sdt, sto)));
         a.x[q] = wrap_1d(xs, sc.rL, sc.L);
@@ -708,11 +717,11 @@ __device__ __forceinline__ void load_i(const KArgs &a, const SysConst &sc, ILane
   }
   if constexpr (PREC == kPrecFP64 && KIND != kKindNb) {
     const double2 t = a.dcs[p];
-    il.dca = dsub(dmul(t.x, sc.cos_ad), dmul(t.y, sc.sin_ad));
-    il.dsa = dadd(dmul(t.y, sc.cos_ad), dmul(t.x, sc.sin_ad));
+    il.dca = __fma_rn(t.x, sc.cos_ad, -dmul(t.y, sc.sin_ad));
+    il.dsa = __fma_rn(t.y, sc.cos_ad, dmul(t.x, sc.sin_ad));
   }
   if constexpr (KIND == kKindCos2) {
-    il.card = (double)a.cnt_s[p];
+    il.cnt = a.cnt_s[p];
     il.dphi = a.dphi_s[p];
     if constexpr (PREC == kPrecFP32C) il.dphif = a.dphi_f[p];
   } else {
@@ -744,27 +753,27 @@ __device__ void epilogue_fp32x(const KArgs &a, int epi, const SysDesc &sd, const
   const int p = il.p;
   const longlong2 cq = a.ics[p];
   const double2 cs = make_double2(from_fixed(cq.x, kXQ), from_fixed(cq.y, kXQ));
-  const double ct = dsub(dmul(cs.x, sc.cos_ad), dmul(cs.y, sc.sin_ad));  // cos(phi_i + alpha)
-  const double st = dadd(dmul(cs.y, sc.cos_ad), dmul(cs.x, sc.sin_ad));  // sin(phi_i + alpha)
+  const double ct = __fma_rn(cs.x, sc.cos_ad, -dmul(cs.y, sc.sin_ad));  // cos(phi_i + alpha)
+  const double st = __fma_rn(cs.y, sc.cos_ad, dmul(cs.x, sc.sin_ad));   // sin(phi_i + alpha)
+  const Count cn = count_of(x.n);
   Acc<kPrecFP64> acc;
   acc.n = x.n;
   acc.s1 = 0.0;
   if constexpr (KIND == kKindSin) {
-    acc.s0 = x.n ? dsub(dmul(x.s, ct), dmul(x.c, st)) : 0.0;
+    acc.s0 = x.n ? __fma_rn(x.s, ct, -dmul(x.c, st)) : 0.0;
     if (epi == kEpiSrk1) {
       // what the second pass needs: this particle's sum of cosines and its
       // rate (the FP64 epilogue's value) times cos phi_i, sin phi_i
-      const double rate = x.n ? ddiv(dmul(sc.sigma, acc.s0), (double)x.n) : 0.0;
-      a.scos[p] = x.n ? dadd(dmul(x.c, ct), dmul(x.s, st)) : 0.0;
+      const double rate = x.n ? ddiv_by(dmul(sc.sigma, acc.s0), cn.n, cn.r) : 0.0;
+      a.scos[p] = x.n ? __fma_rn(x.c, ct, dmul(x.s, st)) : 0.0;
       a.iws[p] = make_longlong2(to_fixed(dmul(rate, cs.x), sc.xq2), to_fixed(dmul(rate, cs.y), sc.xq2));
     }
   } else {
     const double scs = a.scos[p];
     if (x.n) {
-      const double n = (double)x.n;
-      acc.s0 = ddiv(scs, n);
+      acc.s0 = ddiv_by(scs, cn.n, cn.r);
       // sum_j (d_j - d_i) cos(phi_j - theta_i) / n_i
-      acc.s1 = ddiv(dsub(dadd(dmul(x.c, ct), dmul(x.s, st)), dmul(il.dphi, scs)), n);
+      acc.s1 = ddiv_by(dsub(__fma_rn(x.c, ct, dmul(x.s, st)), dmul(il.dphi, scs)), cn.n, cn.r);
     } else {
       acc.s0 = 0.0;
     }

@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(256) k_vgather(KArgs a, int rk_form, int kq, d
     }
     if constexpr (PREC == kPrecFP64) {
       double s, c;
-      sincos(ph, &s, &c);
+      sincos_phase(ph, s, c);
       a.dcs[v] = make_double2(c, s);
     }
     double ex = x - a.vxb[v], ey = y - a.vyb[v];
