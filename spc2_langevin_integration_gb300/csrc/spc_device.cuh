@@ -118,6 +118,16 @@ __device__ __forceinline__ bool in_box(double x, double L) {
   return b < (unsigned long long)__double_as_longlong(L) || b == 0x8000000000000000ull;
 }
 
+// Both components' sum in one packed instruction (each rounded to nearest).
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 r;
+  asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tadd.rn.f32x2 x, x, y;\n\t"
+      "mov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+
 // Per-system constants, the reference's ChimeraSystem / PeriodicBoundaryConditions
 // members (ChimeraSystem.cpp:19-33, PeriodicBoundaryConditions.cpp:13-14).
 struct SysConst {

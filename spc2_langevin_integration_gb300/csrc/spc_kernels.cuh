@@ -422,6 +422,48 @@ __device__ __forceinline__ void add_pair(Acc<kPrecFP64> &acc, const SysConst &sc
     acc.s1 = __fma_rn(dsub(dj, il.dphi), t, acc.s1);
   }
 }
+// A particle's neighbours as words of bits (bit 31 of a word is its entry
+// `base`): next(bits, base) gives the next word that is not zero, cs(k), rate(k)
+// and phase(k) what entry k's pair needs.  U neighbours of a word are taken at
+// a time: their terms are independent, so only the additions wait for one
+// another (a dependent FP64 operation takes over 100 cycles, and the small
+// systems have one warp per SM).
+template <int KIND, int U, class Next, class Cs, class Rate, class Phase>
+__device__ __forceinline__ void walk_pairs(Acc<kPrecFP64> &acc, const SysConst &sc, const ILane &il, Next next,
+                                           Cs cs, Rate rate, Phase phase) {
+  uint32_t bits = 0u;
+  int base = 0;
+  while (bits != 0u || next(bits, base)) {
+    int k[U];
+    bool has[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      has[u] = bits != 0u;
+      const int t = __clz(bits);
+      k[u] = has[u] ? base + t : k[0];
+      bits &= ~(0x80000000u >> (t & 31));
+    }
+    double t[U], d[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const double2 cj = cs(k[u]);
+      t[u] = KIND == kKindSin ? __fma_rn(cj.y, il.dca, -dmul(cj.x, il.dsa))
+                              : __fma_rn(cj.x, il.dca, dmul(cj.y, il.dsa));
+      d[u] = KIND == kKindCos2 ? dsub(rate(k[u]), il.dphi) : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (small_term(t[u]))
+        t[u] = KIND == kKindSin ? sin_of_difference(phase(k[u]), il.phi, sc.alpha)
+                                : cos_of_difference(phase(k[u]), il.phi, sc.alpha);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (!has[u]) continue;
+      acc.s0 = dadd(acc.s0, t[u]);
+      if constexpr (KIND == kKindCos2) acc.s1 = __fma_rn(d[u], t[u], acc.s1);
+    }
+  }
+}
 template <int KIND>
 __device__ __forceinline__ void finish_pairs(Acc<kPrecFP64> &acc, const ILane &il) {
   if constexpr (KIND == kKindCos2) {
@@ -898,6 +940,7 @@ template <int PREC, int KIND, int T = kAllPairsThreads>
 __global__ void __launch_bounds__(T) k_allpairs_pass(KArgs a, int epi) {
   constexpr bool kPair64 = PREC == kPrecFP64 && KIND != kKindNb;
   constexpr int kWords = kAllPairsCap / kWarp;
+  constexpr int kAP64 = T == kAllPairsThreads ? 2 : 4;  // neighbours at a time: more where warps are few
   __shared__ __align__(16) float2 t_xy[kAllPairsCap];
   __shared__ double2 t_cs[kPair64 ? kAllPairsCap : 1];
   __shared__ double t_d[kPair64 && KIND == kKindCos2 ? kAllPairsCap : 1];
@@ -997,16 +1040,23 @@ __global__ void __launch_bounds__(T) k_allpairs_pass(KArgs a, int epi) {
         }
         t_w[wd][threadIdx.x] = bits & known;
       }
-      uint32_t bits = 0u;
-      for (int wd = -1;;) {
+      int wd = -1;
+      auto next = [&](uint32_t &bits, int &base) {
         while (bits == 0u && ++wd < nw) bits = t_w[wd][threadIdx.x];
-        if (bits == 0u) break;
-        const int t = __clz(bits), k = wd * kWarp + t;
-        bits ^= 0x80000000u >> t;
-        if constexpr (kPair64) {
-          add_pair<KIND>(acc, sc, il, t_cs[k], KIND == kKindCos2 ? t_d[k] : 0.0, [&]() { return a.sphi[jt + k]; });
-          acc.n++;
-        } else {
+        base = wd * kWarp;
+        if constexpr (kPair64) acc.n += __popc(bits);
+        return bits != 0u;
+      };
+      if constexpr (kPair64) {
+        walk_pairs<KIND, kAP64>(
+            acc, sc, il, next, [&](int k) { return t_cs[k]; }, [&](int k) { return t_d[KIND == kKindCos2 ? k : 0]; },
+            [&](int k) { return a.sphi[jt + k]; });
+      } else {
+        uint32_t bits = 0u;
+        int base = 0;
+        while (bits != 0u || next(bits, base)) {
+          const int t = __clz(bits), k = base + t;
+          bits ^= 0x80000000u >> t;
           float cc = 0.0f, ss = 0.0f, dj = 0.0f;
           if constexpr (PREC == kPrecFP32C) {
             cc = t_csf[k].x;

@@ -8,13 +8,12 @@
 // no barrier and no work per cell; every lane of a warp has a particle, and the
 // fused epilogue runs on full warps.
 //
-// A lane first tests a row's candidates, four at a time, which gives one bit
-// per candidate (d^2 < lo2: inside for certain; the reference's FP64 test
-// decides in the band, as everywhere).  Words with neighbours go to the lane's
-// list in shared memory with the slot of their first bit; then the lane walks
-// its list in order (rows top to bottom, ascending slots: the reference's
-// visiting order, ChimeraSystem.cpp:39-44) and adds its terms.  The SRK first
-// pass keeps the list for the second.
+// A lane tests a row's candidates, four at a time, which gives one bit per
+// candidate (d^2 < lo2: inside for certain; the reference's FP64 test decides
+// in the band, as everywhere), and walks the bits of each word of 32 (rows top
+// to bottom, ascending slots: the reference's visiting order,
+// ChimeraSystem.cpp:39-44).  The SRK first pass keeps the words with neighbours
+// for the second.
 //
 // The prefilter's x is relative to the first column of a block of 16 to 31
 // columns and its y to the cell row's edge, so a run of three cells needs no
@@ -23,10 +22,16 @@
 // d^2 is below 1e-5 rho^2 (31 columns of at most 1.25 rho, 2^-24 relative),
 // inside the band of 3e-5 rho^2.
 //
-// Bound by issue.  96-system Euler ensemble (681,278 particles, ~6 per cell),
-// FP32X: the pass and its epilogue take 216 us where one warp per cell took
-// 230 and a separate epilogue 170 (168 instructions per 32 tests, most of them
-// per cell); N = 1,024 in 100 cells, FP64: 29 us against 64.
+// Bound by the latency of the loads from L1 (its hit rate is 79%) and by issue
+// (43%).  96-system Euler ensemble (681,278 particles, ~6 per cell), FP32X: the
+// pass with its update takes 162 us, where one warp per cell took 230 and a
+// separate epilogue 170 (168 instructions per 32 tests, most of them per
+// cell).  Taking two neighbours of a word at a time gave 176 -> 171, ten CTAs
+// per SM (48 registers) 171 -> 162; FP32C (24 systems, 1.0 M particles) 168 ->
+// 160 and no gain from fewer registers.  CTAs of 256 and 512 threads and
+// prefetching the next row gave nothing.  FP64, N = 1,024 in 100 cells: 29 us
+// against 64; there the words are listed first (39 us when each word is walked
+// on its own).
 #pragma once
 
 #include "spc_tile.cuh"
@@ -34,7 +39,8 @@
 namespace spc {
 
 constexpr int kLaneThreads = 128;
-constexpr int kLaneWords = 16;  // words a lane collects before it walks them
+constexpr int kLaneWords = 16;  // words a lane collects (FP64) before it walks them
+constexpr int kLanePairs = 2;   // FP64: neighbours taken at a time
 // Saved lists: (bits, slot) pair w of particle p, in the particle's 16-byte
 // groups of nbmask (as mask_at, so that the passes of one batch share the
 // buffer).  A list of up to kLaneWords - 1 words ends with (0, 0); (0, 1) in
@@ -67,19 +73,17 @@ __device__ __forceinline__ LaneRuns lane_runs(int cx, int nc) {
   return r;
 }
 
-// One lane's sums.
+// One lane's sums (float forms): value() loads what a neighbour adds, add()
+// adds it if p.
 template <int PREC, int KIND>
 struct LaneSums;
 
+// FP64: the words are listed first and walked together, the lanes of a warp
+// running out of neighbours at about the same time.
 template <int KIND>
 struct LaneSums<kPrecFP64, KIND> {
   Acc<kPrecFP64> acc;
   __device__ void init() { acc.init(); }
-  __device__ void term(const KArgs &a, const SysConst &sc, const ILane &il, int j) {
-    add_pair<KIND>(acc, sc, il, a.dcs[j], KIND == kKindCos2 ? a.dphi_s[j] : 0.0, [&]() { return a.sphi[j]; });
-  }
-  __device__ void word_end(const ILane &) {}
-  __device__ void list_end() {}
   __device__ void finish(const KArgs &a, int epi, const SysDesc &sd, const ILane &il, int n, int q) {
     acc.n = n;
     finish_pairs<KIND>(acc, il);
@@ -87,30 +91,30 @@ struct LaneSums<kPrecFP64, KIND> {
   }
 };
 
-// FP32X: exact fixed-point sums, 64 bits over a list (at most 16 x 32
-// candidates) and 128 over the lists, so the result is bitwise that of the
-// cell-tile kernel.
+// FP32X: exact fixed-point sums, so the result is bitwise that of the
+// cell-tile kernel.  A word's neighbours add less than 2^57; after each word the
+// multiples of 2^57 move to a 32-bit count (2^57 each).
 template <int KIND>
 struct LaneSums<kPrecFP32X, KIND> {
   long long c, s;
-  __int128 tc, ts;
+  int ch, sh;
   __device__ void init() {
     c = s = 0;
-    tc = ts = 0;
+    ch = sh = 0;
   }
-  __device__ void term(const KArgs &a, const SysConst &, const ILane &, int j) {
-    const longlong2 v = KIND == kKindSin ? a.ics[j] : a.iws[j];
-    c += v.x;
-    s += v.y;
-  }
-  __device__ void word_end(const ILane &) {}
-  __device__ void list_end() {
-    tc += c;
-    ts += s;
-    c = s = 0;
+  typedef longlong2 Value;
+  __device__ static Value value(const KArgs &a, int j) { return KIND == kKindSin ? a.ics[j] : a.iws[j]; }
+  __device__ void add(const Value &v, bool p) { add2_if(c, s, v, p); }
+  __device__ void word_end(const ILane &) {
+    constexpr long long low = (1ll << 57) - 1;
+    ch += (int)(c >> 57);
+    sh += (int)(s >> 57);
+    c &= low;
+    s &= low;
   }
   __device__ void finish(const KArgs &a, int epi, const SysDesc &sd, const ILane &il, int n, int q) {
     const int qv = KIND == kKindSin ? kXQ : sd.sc.xq2;
+    const __int128 tc = ((__int128)ch << 57) + c, ts = ((__int128)sh << 57) + s;
     epilogue_fp32x<KIND>(a, epi, sd, il, XSums{from_fixed128(tc, qv), from_fixed128(ts, qv), n}, q);
   }
 };
@@ -125,15 +129,14 @@ struct LaneSums<kPrecFP32C, KIND> {
     bc = bs = bdc = bds = 0.0f;
     acc.init();
   }
-  __device__ void term(const KArgs &a, const SysConst &, const ILane &, int j) {
-    const float2 t = a.cs[j];
-    bc += t.x;
-    bs += t.y;
-    if constexpr (KIND == kKindCos2) {
-      const float d = a.dphi_f[j];
-      bdc = fmaf(d, t.x, bdc);
-      bds = fmaf(d, t.y, bds);
-    }
+  struct Value {
+    float2 cs;
+    float d;
+  };
+  __device__ static Value value(const KArgs &a, int j) { return {a.cs[j], KIND == kKindCos2 ? a.dphi_f[j] : 0.0f}; }
+  __device__ void add(const Value &v, bool p) {
+    addf2_if(bc, bs, v.cs.x, v.cs.y, p);
+    if constexpr (KIND == kKindCos2) fmaf2_if(bdc, bds, v.d, v.cs.x, v.cs.y, p);
   }
   __device__ void word_end(const ILane &il) {
     if constexpr (KIND == kKindSin) {
@@ -145,7 +148,6 @@ struct LaneSums<kPrecFP32C, KIND> {
     }
     bc = bs = bdc = bds = 0.0f;
   }
-  __device__ void list_end() {}
   __device__ void finish(const KArgs &a, int epi, const SysDesc &sd, const ILane &il, int n, int q) {
     acc.n = n;
     acc.s0 -= acc.c0;
@@ -155,9 +157,10 @@ struct LaneSums<kPrecFP32C, KIND> {
 };
 
 template <int PREC, int KIND>
-__global__ void __launch_bounds__(kLaneThreads) k_lane(KArgs a, int epi) {
-  __shared__ uint32_t s_bits[kLaneWords][kLaneThreads];
-  __shared__ int s_slot[kLaneWords][kLaneThreads];
+__global__ void __launch_bounds__(kLaneThreads, PREC == kPrecFP32X ? 10 : 1) k_lane(KArgs a, int epi) {
+  constexpr bool kList = PREC == kPrecFP64;
+  __shared__ uint32_t s_bits[kList ? kLaneWords : 1][kLaneThreads];
+  __shared__ int s_slot[kList ? kLaneWords : 1][kLaneThreads];
   const int tid = threadIdx.x;
   const int p = a.lane_p0 + blockIdx.x * blockDim.x + tid;
   if (p >= a.lane_p1) return;  // no barrier below
@@ -169,26 +172,45 @@ __global__ void __launch_bounds__(kLaneThreads) k_lane(KArgs a, int epi) {
   load_i<PREC, KIND>(a, sc, il, p, true);
   LaneSums<PREC, KIND> sums;
   sums.init();
-  int n = 0, nw = 0;
+  int n = 0;
   uint2 *saved = reinterpret_cast<uint2 *>(a.nbmask);
 
-  auto walk = [&]() {  // the listed words (none of them zero), in order
-    uint32_t bits = 0u;
-    int slot = 0;
-    for (int w = 0;;) {
-      if (bits == 0u) {
-        if (w > 0) sums.word_end(il);
-        if (w == nw) break;
-        bits = s_bits[w][tid];
-        slot = s_slot[w][tid];
-        ++w;
-      }
-      const int t = __clz(bits);
-      bits ^= 0x80000000u >> t;
-      sums.term(a, sc, il, slot + t);
+  int nw = 0;  // FP64: words listed
+  auto walk_list = [&]() {
+    if constexpr (kList) {
+      int w = -1;
+      walk_pairs<KIND, kLanePairs>(
+          sums.acc, sc, il,
+          [&](uint32_t &bits, int &base) {
+            if (++w >= nw) return false;
+            bits = s_bits[w][tid];
+            base = s_slot[w][tid];
+            return true;
+          },
+          [&](int j) { return a.dcs[j]; }, [&](int j) { return a.dphi_s[j]; }, [&](int j) { return a.sphi[j]; });
+      nw = 0;
     }
-    sums.list_end();
-    nw = 0;
+  };
+  // a word with neighbours; bit 31 is slot `slot`
+  auto take = [&](uint32_t bits, int slot) {
+    n += __popc(bits);
+    if constexpr (kList) {
+      s_bits[nw][tid] = bits;
+      s_slot[nw][tid] = slot;
+      ++nw;
+    } else {
+      while (bits != 0u) {  // two at a time: both loads are on their way together
+        const int t0 = __clz(bits);
+        bits ^= 0x80000000u >> t0;
+        const bool two = bits != 0u;
+        const int t1 = two ? __clz(bits) : t0;
+        bits &= ~(0x80000000u >> t1);
+        const auto v0 = sums.value(a, slot + t0), v1 = sums.value(a, slot + t1);
+        sums.add(v0, true);
+        sums.add(v1, two);
+      }
+      sums.word_end(il);
+    }
   };
 
   bool listed = false;  // pass 2: the first pass left its list
@@ -197,25 +219,22 @@ __global__ void __launch_bounds__(kLaneThreads) k_lane(KArgs a, int epi) {
       uint2 e = saved[saved_at(0, p, n_all)];
       listed = e.x != 0u || e.y == 0u;  // (0, 1): the list was too long
       if (listed)
-        while (e.x != 0u) {
-          s_bits[nw][tid] = e.x;
-          s_slot[nw][tid] = (int)e.y;
-          n += __popc(e.x);
-          ++nw;
-          e = saved[saved_at(nw, p, n_all)];
+        for (int w = 1; e.x != 0u; ++w) {
+          const uint2 next = saved[saved_at(w, p, n_all)];
+          take(e.x, (int)e.y);
+          e = next;
         }
     }
   }
   if (!listed) {
     int nsaved = 0;
-    auto put = [&](uint32_t bits, int slot) {
+    auto found = [&](uint32_t bits, int slot) {
       if (bits == 0u) return;
-      s_bits[nw][tid] = bits;
-      s_slot[nw][tid] = slot;
-      if (KIND == kKindSin && saved && nsaved < kLaneWords - 1)
-        saved[saved_at(nsaved, p, n_all)] = make_uint2(bits, (uint32_t)slot);
-      ++nsaved;
-      ++nw;
+      if (KIND == kKindSin && saved) {
+        if (nsaved < kLaneWords - 1) saved[saved_at(nsaved, p, n_all)] = make_uint2(bits, (uint32_t)slot);
+        ++nsaved;
+      }
+      take(bits, slot);
     };
     const float nlo = -sc.lo2, wid = undecided_width(sc.lo2, sc.hi2);
     const bool exact_all = sc.exact_all != 0;
@@ -241,13 +260,15 @@ __global__ void __launch_bounds__(kLaneThreads) k_lane(KArgs a, int epi) {
           const float x = in_a ? xa : xb;
           // up to three slots past the run's end are read (the array is padded) and masked
           const float2 *f = a.fxy + ((in_a ? a0 : b0 - la4) + base + done);
+          uint32_t o[4];
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
-            const float2 fj = f[u];
-            const uint32_t o = __float_as_uint(cutoff_offset(fj.x - x, fj.y - y, nlo));
-            bits = __funnelshift_l(o, bits, 1);
-            um = min(um, o);
+            const float2 d = add2(f[u], make_float2(-x, -y));
+            o[u] = __float_as_uint(cutoff_offset(d.x, d.y, nlo));
+            bits = __funnelshift_l(o[u], bits, 1);
           }
+          um = __vimin3_u32(um, o[0], o[1]);
+          um = __vimin3_u32(um, o[2], o[3]);
         }
         bits <<= kWarp - done;
         const uint32_t part_a = first_bits(min(max(la4 - base, 0), kWarp));
@@ -271,10 +292,9 @@ __global__ void __launch_bounds__(kLaneThreads) k_lane(KArgs a, int epi) {
           }
         }
         bits &= known;
-        n += __popc(bits);
-        put(bits & part_a, a0 + base);
-        put(bits & ~part_a, b0 - la4 + base);
-        if (nw > kLaneWords - 2) walk();
+        found(bits & part_a, a0 + base);
+        if (base + cnt > la4) found(bits & ~part_a, b0 - la4 + base);
+        if (kList && nw > kLaneWords - 2) walk_list();
       }
       a0 = na0, a1 = na1, b0 = nb0, b1 = nb1;
     }
@@ -285,7 +305,7 @@ __global__ void __launch_bounds__(kLaneThreads) k_lane(KArgs a, int epi) {
         saved[saved_at(0, p, n_all)] = make_uint2(0u, 1u);
     }
   }
-  walk();
+  walk_list();
   sums.finish(a, epi, sd, il, n, a.pidx[p]);
 }
 

@@ -1202,17 +1202,19 @@ __global__ void __launch_bounds__(kTileThreads64) k_tile_fp64(KArgs a, int epi) 
               m4[(size_t)g * n_all + p] =
                   make_uint4(s_w[4 * g][tid], s_w[4 * g + 1][tid], s_w[4 * g + 2][tid], s_w[4 * g + 3][tid]);
         }
-        uint32_t bits = 0u;
-        for (int w = -1;;) {
-          while (bits == 0u && ++w < nw) bits = s_w[w][tid];
-          if (bits == 0u) break;
-          const int t = __clz(bits), j = w * kWarp + t;
-          bits ^= 0x80000000u >> t;
-          add_pair<KIND>(acc, sc, il, s_cs[j], KIND == kKindCos2 ? s_d[j] : 0.0, [&]() {
-            int q;
-            return a.sphi[slot_of(st, rlo + j, q)];
-          });
-        }
+        int w = -1;
+        walk_pairs<KIND, 2>(
+            acc, sc, il,
+            [&](uint32_t &bits, int &base) {
+              while (bits == 0u && ++w < nw) bits = s_w[w][tid];
+              base = w * kWarp;
+              return bits != 0u;
+            },
+            [&](int j) { return s_cs[j]; }, [&](int j) { return s_d[KIND == kKindCos2 ? j : 0]; },
+            [&](int j) {
+              int q;
+              return a.sphi[slot_of(st, rlo + j, q)];
+            });
       }
       if (valid) {
         finish_pairs<KIND>(acc, il);
