@@ -973,10 +973,14 @@ int launch_pass_t(Engine *e, const KArgs &a, int epi) {
           if (a.units) SPC_CUDA(e, cudaStreamWaitEvent(st, e->join_ev, 0));
       }
       if (e->ncell_warp > 0) {
-        // one warp per CTA when that spreads the particles over more SMs
         const int np = a.lane_p1 - a.lane_p0;
-        const int threads = np >= 152 * 4 * kLaneThreads ? kLaneThreads : kWarp;
-        k_lane<PREC, KIND><<<blocks_for(np, threads), threads, 0, st>>>(a, epi);
+        if (np <= kLaneGroupMax<PREC>) {
+          k_lane<PREC, KIND, kLaneGroup><<<blocks_for((long long)np * kLaneGroup, kWarp), kWarp, 0, st>>>(a, epi);
+        } else {
+          // one warp per CTA when that spreads the particles over more SMs
+          const int threads = np >= 152 * 4 * kLaneThreads ? kLaneThreads : kWarp;
+          k_lane<PREC, KIND, 1><<<blocks_for(np, threads), threads, 0, st>>>(a, epi);
+        }
         SPC_LAUNCHED(e);
       }
       if constexpr (PREC == kPrecFP32X) {

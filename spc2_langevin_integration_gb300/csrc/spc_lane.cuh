@@ -24,14 +24,13 @@
 //
 // Bound by the latency of the loads from L1 (its hit rate is 79%) and by issue
 // (43%).  96-system Euler ensemble (681,278 particles, ~6 per cell), FP32X: the
-// pass with its update takes 162 us, where one warp per cell took 230 and a
+// pass with its update takes 165 us, where one warp per cell took 230 and a
 // separate epilogue 170 (168 instructions per 32 tests, most of them per
-// cell).  Taking two neighbours of a word at a time gave 176 -> 171, ten CTAs
-// per SM (48 registers) 171 -> 162; FP32C (24 systems, 1.0 M particles) 168 ->
-// 160 and no gain from fewer registers.  CTAs of 256 and 512 threads and
-// prefetching the next row gave nothing.  FP64, N = 1,024 in 100 cells: 29 us
-// against 64; there the words are listed first (39 us when each word is walked
-// on its own).
+// cell); FP32C (24 systems, 1.0 M particles): 166 us against 290.  Ten CTAs per
+// SM (48 registers), rows unrolled and two neighbours of a word at a time each
+// gave 3 to 15%; CTAs of 256 and 512 threads and prefetching the next row
+// nothing.  FP64, N = 1,024 in 100 cells: 20 us against 64; there the words are
+// listed first (10 us more when each word is walked on its own).
 #pragma once
 
 #include "spc_tile.cuh"
@@ -41,11 +40,24 @@ namespace spc {
 constexpr int kLaneThreads = 128;
 constexpr int kLaneWords = 16;  // words a lane collects (FP64) before it walks them
 constexpr int kLanePairs = 2;   // FP64: neighbours taken at a time
-// Saved lists: (bits, slot) pair w of particle p, in the particle's 16-byte
-// groups of nbmask (as mask_at, so that the passes of one batch share the
-// buffer).  A list of up to kLaneWords - 1 words ends with (0, 0); (0, 1) in
-// front says that it was longer.
-static_assert(kLaneWords * 2 == kMaskWords, "the saved lists fill the particles' mask words");
+// Few particles: a group of four lanes takes one.  Three of them test a row
+// each, and the FP64 terms of four neighbours are formed side by side (their
+// additions keep the order).  The sums are the same bit for bit: FP32X's are
+// exact, FP32C adds row by row either way.
+constexpr int kLaneGroup = 4;
+// Up to this many particles, where the GPU's schedulers would hold one or two
+// warps each (4 lanes and 1 lane per particle, Euler step in us at density
+// 1,000, rho = 0.1): FP64 1,024: 34.8 / 40.1, 12,288: 44.5 / 49.0, 16,384: 56.1
+// / 50.3; FP32C 1,024: 27.5 / 34.7, 32,768: 48.2 / 53.0, 49,152: 58.7 / 58.5;
+// FP32X 1,024: 29.7 / 39.3, 32,768: 55.6 / 58.7, 49,152: 69.2 / 64.5.
+template <int PREC>
+constexpr int kLaneGroupMax = PREC == kPrecFP64 ? 14336 : PREC == kPrecFP32C ? 45056 : 36864;
+// Saved words: row k of particle p has entries [5 k, 5 k + 5) of (bits, slot)
+// pairs, in the particle's 16-byte groups of nbmask (as mask_at, so that the
+// passes of one batch share the buffer).  (0, 0) ends a row; (0, 1) in front
+// says that it had more words, and the second pass tests it again.
+constexpr int kRowWords = 5;
+static_assert((3 * kRowWords + 1) * 2 <= kMaskWords, "three rows fit a particle's mask words");
 __device__ __forceinline__ size_t saved_at(int w, int p, int n) {
   return ((size_t)(w >> 1) * n + p) * 2 + (w & 1);
 }
@@ -112,6 +124,16 @@ struct LaneSums<kPrecFP32X, KIND> {
     c &= low;
     s &= low;
   }
+  __device__ void row_end() {}
+  __device__ void join_group(unsigned mask, int) {
+#pragma unroll
+    for (int o = 1; o < kLaneGroup; o <<= 1) {  // four times 2^57 at most
+      c += __shfl_xor_sync(mask, c, o);
+      s += __shfl_xor_sync(mask, s, o);
+      ch += __shfl_xor_sync(mask, ch, o);
+      sh += __shfl_xor_sync(mask, sh, o);
+    }
+  }
   __device__ void finish(const KArgs &a, int epi, const SysDesc &sd, const ILane &il, int n, int q) {
     const int qv = KIND == kKindSin ? kXQ : sd.sc.xq2;
     const __int128 tc = ((__int128)ch << 57) + c, ts = ((__int128)sh << 57) + s;
@@ -120,14 +142,17 @@ struct LaneSums<kPrecFP32X, KIND> {
 };
 
 // FP32C: a word's neighbours are summed in float, turned into the alignment
-// terms by angle addition and added with Kahan compensation.
+// terms by angle addition and added with Kahan compensation, and so are the
+// rows' sums.
 template <int KIND>
 struct LaneSums<kPrecFP32C, KIND> {
   float bc, bs, bdc, bds;
+  Acc<kPrecFP32C> tot;
   Acc<kPrecFP32C> acc;
   __device__ void init() {
     bc = bs = bdc = bds = 0.0f;
     acc.init();
+    tot.init();
   }
   struct Value {
     float2 cs;
@@ -148,21 +173,82 @@ struct LaneSums<kPrecFP32C, KIND> {
     }
     bc = bs = bdc = bds = 0.0f;
   }
+  // the row's compensated sums join the total
+  __device__ void row_end() {
+    join(acc);
+    acc.init();
+  }
+  __device__ void join(const Acc<kPrecFP32C> &row) {
+    kahan_add(tot.s0, tot.c0, row.s0);
+    kahan_add(tot.s0, tot.c0, -row.c0);
+    if constexpr (KIND == kKindCos2) {
+      kahan_add(tot.s1, tot.c1, row.s1);
+      kahan_add(tot.s1, tot.c1, -row.c1);
+    }
+  }
+  __device__ void join_group(unsigned mask, int lead) {
+    const Acc<kPrecFP32C> mine = acc;
+    for (int k = 0; k < 3; ++k) {
+      Acc<kPrecFP32C> row;
+      row.s0 = __shfl_sync(mask, mine.s0, lead + k);
+      row.c0 = __shfl_sync(mask, mine.c0, lead + k);
+      row.s1 = __shfl_sync(mask, mine.s1, lead + k);
+      row.c1 = __shfl_sync(mask, mine.c1, lead + k);
+      join(row);
+    }
+  }
   __device__ void finish(const KArgs &a, int epi, const SysDesc &sd, const ILane &il, int n, int q) {
     acc.n = n;
-    acc.s0 -= acc.c0;
-    acc.s1 -= acc.c1;
+    acc.s0 = tot.s0 - tot.c0;
+    acc.s1 = tot.s1 - tot.c1;
     epilogue<kPrecFP32C, KIND>(a, epi, sd, il, acc, q);
   }
 };
 
-template <int PREC, int KIND>
-__global__ void __launch_bounds__(kLaneThreads, PREC == kPrecFP32X ? 10 : 1) k_lane(KArgs a, int epi) {
+// Four lanes of a group walk one particle's words together (FP64): lane g
+// forms the term of the (g+1)-th remaining neighbour of the word, and all four
+// add the terms in order.  next(bits, base) as for walk_pairs.
+template <int KIND, class Next>
+__device__ __forceinline__ void walk_group(Acc<kPrecFP64> &acc, const KArgs &a, const SysConst &sc, const ILane &il,
+                                           int g, unsigned mask, int lead, Next next) {
+  uint32_t bits = 0u;
+  int base = 0;
+  while (bits != 0u || next(bits, base)) {
+    const int m = __popc(bits);
+    int j = il.p;
+#pragma unroll
+    for (int u = 0; u < kLaneGroup; ++u) {
+      const int t = __clz(bits);
+      if (u == g && u < m) j = base + t;
+      bits &= ~(0x80000000u >> (t & 31));
+    }
+    const double2 cj = a.dcs[j];
+    double t = KIND == kKindSin ? __fma_rn(cj.y, il.dca, -dmul(cj.x, il.dsa))
+                                : __fma_rn(cj.x, il.dca, dmul(cj.y, il.dsa));
+    const double d = KIND == kKindCos2 ? dsub(a.dphi_s[j], il.dphi) : 0.0;
+    if (g < m && small_term(t))
+      t = KIND == kKindSin ? sin_of_difference(a.sphi[j], il.phi, sc.alpha)
+                           : cos_of_difference(a.sphi[j], il.phi, sc.alpha);
+#pragma unroll
+    for (int u = 0; u < kLaneGroup; ++u) {
+      const double tu = __shfl_sync(mask, t, lead + u);
+      const double du = KIND == kKindCos2 ? __shfl_sync(mask, d, lead + u) : 0.0;
+      if (u >= m) continue;
+      acc.s0 = dadd(acc.s0, tu);
+      if constexpr (KIND == kKindCos2) acc.s1 = __fma_rn(du, tu, acc.s1);
+    }
+  }
+}
+
+// G lanes per particle: 1 or kLaneGroup.
+template <int PREC, int KIND, int G>
+__global__ void __launch_bounds__(kLaneThreads, PREC != kPrecFP64 && G == 1 ? 10 : 1) k_lane(KArgs a, int epi) {
   constexpr bool kList = PREC == kPrecFP64;
   __shared__ uint32_t s_bits[kList ? kLaneWords : 1][kLaneThreads];
   __shared__ int s_slot[kList ? kLaneWords : 1][kLaneThreads];
-  const int tid = threadIdx.x;
-  const int p = a.lane_p0 + blockIdx.x * blockDim.x + tid;
+  const int tid = threadIdx.x, g = tid % G, lead = tid % kWarp - g;
+  const unsigned group = ((1u << G) - 1u) << lead;  // the group's lanes (G > 1)
+  const int p = a.lane_p0 + (blockIdx.x * blockDim.x + tid) / G;
   if (p >= a.lane_p1) return;  // no barrier below
   const int n_all = a.n_active;
   const int c = cell_of_slot(a, p);
@@ -176,6 +262,7 @@ __global__ void __launch_bounds__(kLaneThreads, PREC == kPrecFP32X ? 10 : 1) k_l
   uint2 *saved = reinterpret_cast<uint2 *>(a.nbmask);
 
   int nw = 0;  // FP64: words listed
+  bool full = false;  // FP64, G > 1: the row has more words than the list
   auto walk_list = [&]() {
     if constexpr (kList) {
       int w = -1;
@@ -213,99 +300,148 @@ __global__ void __launch_bounds__(kLaneThreads, PREC == kPrecFP32X ? 10 : 1) k_l
     }
   };
 
-  bool listed = false;  // pass 2: the first pass left its list
-  if constexpr (KIND == kKindCos2) {
-    if (saved) {
-      uint2 e = saved[saved_at(0, p, n_all)];
-      listed = e.x != 0u || e.y == 0u;  // (0, 1): the list was too long
-      if (listed)
-        for (int w = 1; e.x != 0u; ++w) {
-          const uint2 next = saved[saved_at(w, p, n_all)];
-          take(e.x, (int)e.y);
-          e = next;
-        }
-    }
-  }
-  if (!listed) {
-    int nsaved = 0;
-    auto found = [&](uint32_t bits, int slot) {
-      if (bits == 0u) return;
-      if (KIND == kKindSin && saved) {
-        if (nsaved < kLaneWords - 1) saved[saved_at(nsaved, p, n_all)] = make_uint2(bits, (uint32_t)slot);
-        ++nsaved;
-      }
-      take(bits, slot);
-    };
-    const float nlo = -sc.lo2, wid = undecided_width(sc.lo2, sc.hi2);
-    const bool exact_all = sc.exact_all != 0;
-    const int nc = sc.nc, cl = c - sd.c0, cy = cl / nc, cx = cl - cy * nc;
-    const LaneRuns r = lane_runs(cx, nc);
-    const float xa = il.fx - (float)r.sa * sc.cell_f, xb = il.fx - (float)r.sb * sc.cell_f;
-    const int *row = a.cell_start + sd.c0 + adjust_cell(cy - 1, nc) * nc;
+  const float nlo = -sc.lo2, wid = undecided_width(sc.lo2, sc.hi2);
+  const bool exact_all = sc.exact_all != 0;
+  const int nc = sc.nc, cl = c - sd.c0, cy = cl / nc, cx = cl - cy * nc;
+  const LaneRuns r = lane_runs(cx, nc);
+  const float xa = il.fx - (float)r.sa * sc.cell_f, xb = il.fx - (float)r.sb * sc.cell_f;
+  // rows [k0, k1) of the stencil; flush: walk the FP64 list when it is full
+  auto rows = [&](int k0, int k1, bool flush) {
+    const int *row = a.cell_start + sd.c0 + adjust_cell(cy + k0 - 1, nc) * nc;
     int a0 = row[r.a0], a1 = row[r.a1], b0 = row[r.b0], b1 = row[r.b1];
-#pragma unroll 1
-    for (int k = 0; k < 3; ++k) {
+#pragma unroll(!kList && G == 1 ? 3 : 1)
+    for (int k = k0; k < k1; ++k) {
       // the next row's bounds, on their way while this row is tested
-      const int *next = a.cell_start + sd.c0 + adjust_cell(cy + k, nc) * nc;
+      const int *next = a.cell_start + sd.c0 + adjust_cell(cy + min(k, 1), nc) * nc;
       const int na0 = next[r.a0], na1 = next[r.a1], nb0 = next[r.b0], nb1 = next[r.b1];
-      const float y = il.fy - (float)(k - 1) * sc.cell_f;
-      // run a takes positions [0, la), run b [la4, la4 + lb)
-      const int la = a1 - a0, la4 = (la + 3) & ~3, total = la4 + (b1 - b0);
-      for (int base = 0; base < total; base += kWarp) {
-        const int cnt = min(kWarp, total - base);
-        uint32_t bits = 0u, um = 0xffffffffu;
-        int done = 0;
-        for (; done < cnt; done += 4) {
-          const bool in_a = base + done < la4;
-          const float x = in_a ? xa : xb;
-          // up to three slots past the run's end are read (the array is padded) and masked
-          const float2 *f = a.fxy + ((in_a ? a0 : b0 - la4) + base + done);
-          uint32_t o[4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const float2 d = add2(f[u], make_float2(-x, -y));
-            o[u] = __float_as_uint(cutoff_offset(d.x, d.y, nlo));
-            bits = __funnelshift_l(o[u], bits, 1);
-          }
-          um = __vimin3_u32(um, o[0], o[1]);
-          um = __vimin3_u32(um, o[2], o[3]);
+      // room for a row's saved words (with flush off the list starts empty)
+      if (kList && flush && nw > kLaneWords - kRowWords) walk_list();
+      bool listed = false;  // pass 2: the first pass left this row's words
+      if constexpr (KIND == kKindCos2) {
+        if (saved) {
+          uint2 e = saved[saved_at(k * kRowWords, p, n_all)];
+          listed = e.x != 0u || e.y == 0u;
+          if (listed)
+            for (int w = 1; e.x != 0u; ++w) {
+              const uint2 after = w < kRowWords ? saved[saved_at(k * kRowWords + w, p, n_all)] : make_uint2(0u, 0u);
+              take(e.x, (int)e.y);
+              e = after;
+            }
         }
-        bits <<= kWarp - done;
-        const uint32_t part_a = first_bits(min(max(la4 - base, 0), kWarp));
-        uint32_t known = first_bits(min(max(la - base, 0), kWarp)) | (first_bits(cnt) & ~part_a);
-        if (k == 1) {
-          const int self = (p < a1 && p >= a0 ? p - a0 : la4 + p - b0) - base;
-          if ((unsigned)self < (unsigned)kWarp) known &= ~(0x80000000u >> self);
-        }
-        // pairs the float test cannot decide: the reference's FP64 test
-        if (exact_all || um <= __float_as_uint(wid)) {
-          for (uint32_t ask = known; ask != 0u;) {
-            const int t = __clz(ask);
-            const uint32_t b = 0x80000000u >> t;
-            ask ^= b;
-            const bool in_a = base + t < la4;
-            const int j = (in_a ? a0 : b0 - la4) + base + t;
-            const float2 fj = a.fxy[j];
-            const float off = cutoff_offset(fj.x - (in_a ? xa : xb), fj.y - y, nlo);
-            if (exact_all || (off >= 0.0f && off <= wid))
-              bits = exact_within(sc, il.x, il.y, a.sx[j], a.sy[j]) ? bits | b : bits & ~b;
-          }
-        }
-        bits &= known;
-        found(bits & part_a, a0 + base);
-        if (base + cnt > la4) found(bits & ~part_a, b0 - la4 + base);
-        if (kList && nw > kLaneWords - 2) walk_list();
       }
+      if (!listed) {
+        int nsaved = 0;
+        auto found = [&](uint32_t bits, int slot) {
+          if (bits == 0u) return;
+          if (KIND == kKindSin && saved) {
+            if (nsaved < kRowWords) saved[saved_at(k * kRowWords + nsaved, p, n_all)] = make_uint2(bits, (uint32_t)slot);
+            ++nsaved;
+          }
+          take(bits, slot);
+        };
+        const float y = il.fy - (float)(k - 1) * sc.cell_f;
+        // run a takes positions [0, la), run b [la4, la4 + lb)
+        const int la = a1 - a0, la4 = (la + 3) & ~3, total = la4 + (b1 - b0);
+        for (int base = 0; base < total; base += kWarp) {
+          const int cnt = min(kWarp, total - base);
+          uint32_t bits = 0u, um = 0xffffffffu;
+          int done = 0;
+          for (; done < cnt; done += 4) {
+            const bool in_a = base + done < la4;
+            const float x = in_a ? xa : xb;
+            // up to three slots past the run's end are read (the array is padded) and masked
+            const float2 *f = a.fxy + ((in_a ? a0 : b0 - la4) + base + done);
+            uint32_t o[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const float2 d = add2(f[u], make_float2(-x, -y));
+              o[u] = __float_as_uint(cutoff_offset(d.x, d.y, nlo));
+              bits = __funnelshift_l(o[u], bits, 1);
+            }
+            um = __vimin3_u32(um, o[0], o[1]);
+            um = __vimin3_u32(um, o[2], o[3]);
+          }
+          bits <<= kWarp - done;
+          const uint32_t part_a = first_bits(min(max(la4 - base, 0), kWarp));
+          uint32_t known = first_bits(min(max(la - base, 0), kWarp)) | (first_bits(cnt) & ~part_a);
+          if (k == 1) {
+            const int self = (p < a1 && p >= a0 ? p - a0 : la4 + p - b0) - base;
+            if ((unsigned)self < (unsigned)kWarp) known &= ~(0x80000000u >> self);
+          }
+          // pairs the float test cannot decide: the reference's FP64 test
+          if (exact_all || um <= __float_as_uint(wid)) {
+            for (uint32_t ask = known; ask != 0u;) {
+              const int t = __clz(ask);
+              const uint32_t b = 0x80000000u >> t;
+              ask ^= b;
+              const bool in_a = base + t < la4;
+              const int j = (in_a ? a0 : b0 - la4) + base + t;
+              const float2 fj = a.fxy[j];
+              const float off = cutoff_offset(fj.x - (in_a ? xa : xb), fj.y - y, nlo);
+              if (exact_all || (off >= 0.0f && off <= wid))
+                bits = exact_within(sc, il.x, il.y, a.sx[j], a.sy[j]) ? bits | b : bits & ~b;
+            }
+          }
+          bits &= known;
+          found(bits & part_a, a0 + base);
+          if (base + cnt > la4) found(bits & ~part_a, b0 - la4 + base);
+          if (kList && nw > kLaneWords - 2) {
+            if (flush) {
+              walk_list();
+            } else {
+              full = true;
+              return;
+            }
+          }
+        }
+        if (KIND == kKindSin && saved) {
+          if (nsaved < kRowWords)
+            saved[saved_at(k * kRowWords + nsaved, p, n_all)] = make_uint2(0u, 0u);
+          else if (nsaved > kRowWords)
+            saved[saved_at(k * kRowWords, p, n_all)] = make_uint2(0u, 1u);
+        }
+      }
+      if constexpr (!kList && G == 1) sums.row_end();
       a0 = na0, a1 = na1, b0 = nb0, b1 = nb1;
     }
-    if (KIND == kKindSin && saved) {
-      if (nsaved < kLaneWords)
-        saved[saved_at(nsaved, p, n_all)] = make_uint2(0u, 0u);
-      else
-        saved[saved_at(0, p, n_all)] = make_uint2(0u, 1u);
+  };
+
+  if constexpr (G == 1) {
+    rows(0, 3, true);
+    walk_list();
+  } else {
+    bool alone = false;
+    if (g < 3) rows(g, g + 1, false);
+    if constexpr (kList) {
+      __syncwarp(group);
+      if (__any_sync(group, full)) {  // a very long row: the first lane walks as it tests
+        if (g != 0) return;
+        alone = true;
+        n = nw = 0;
+        rows(0, 3, true);
+        walk_list();
+      } else {
+        int row = 0, w = -1, words = __shfl_sync(group, nw, lead);
+        walk_group<KIND>(sums.acc, a, sc, il, g, group, lead, [&](uint32_t &bits, int &base) {
+          while (++w >= words) {
+            if (++row > 2) return false;
+            w = -1;
+            words = __shfl_sync(group, nw, lead + row);
+          }
+          bits = s_bits[w][tid - g + row];
+          base = s_slot[w][tid - g + row];
+          return true;
+        });
+      }
+    } else {
+      sums.join_group(group, lead);
     }
+    if (!alone) {
+#pragma unroll
+      for (int o = 1; o < G; o <<= 1) n += __shfl_xor_sync(group, n, o);
+    }
+    if (g != 0) return;
   }
-  walk_list();
   sums.finish(a, epi, sd, il, n, a.pidx[p]);
 }
 

@@ -71,3 +71,28 @@ def test_lane_lists_and_batches(n):
             b.admit(200, par(2, rho=1.2), init_state(200, L, 2))
             b.step(0.01, 3)
             assert np.array_equal(b.download(slot), alone[1])
+
+
+@pytest.mark.parametrize("precision", [abi.PRECISION_FP64, abi.PRECISION_FP32X, abi.PRECISION_FP32C])
+def test_four_lanes_and_one_lane_per_particle_agree_bitwise(precision):
+    """A system alone takes four lanes per particle; in a batch of 50,000
+    particles it takes one.  Rows of up to 90 neighbours (three words), and a
+    system whose rows have more words than the first pass keeps."""
+    L, n = 3.0, 3000
+    par = [abi.make_params(L=L, stepper=abi.STEPPER_SRK, precision=precision, seed=9, system_id=k, v0=0.02,
+                           sigma=1.3, rho=rho, alpha=1.1, D_phi=0.01) for k, rho in ((0, 0.2), (1, 0.3), (2, 0.6))]
+    states = [init_state(n, L, 700), init_state(n, L, 701), init_state(n, 1.5, 702)]
+    big = abi.make_params(L=8.0, stepper=abi.STEPPER_SRK, precision=precision, v0=0.02, sigma=1.0, rho=0.1,
+                          alpha=1.0, D_phi=0.01)
+    with abi.Batch(abi.STEPPER_SRK, precision, 4, 3 * n + 50000, 225 + 100 + 25 + 6400) as b:
+        b.set_tuning(abi.TUNE_SPARSE_BELOW, 1e9)
+        slots = [b.admit(n, p, st) for p, st in zip(par, states)]
+        b.admit(50000, big, init_state(50000, 8.0, 703))
+        b.step(0.01, 4)
+        got = [b.download(s) for s in slots]
+    for p, st, want in zip(par, states, got):
+        with abi.System(n, p) as s:
+            s.set_tuning(abi.TUNE_SPARSE_BELOW, 1e9)
+            s.upload_state(st)
+            s.step(0.01, 4)
+            assert np.array_equal(s.download_state(), want)
