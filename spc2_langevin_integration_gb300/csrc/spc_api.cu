@@ -1092,7 +1092,7 @@ int spc_batch_profile_steps(spc_batch *b, double dt, int32_t nsteps, double *out
 // cudaMalloc/cudaFree pair would synchronise the device, and hosts that must
 // not grow their device footprint after start-up.  spc_rhs_srk_noalloc serves
 // them: the caller passes device input and output buffers, and every
-// intermediate array (cell keys, the radix sort's buffers and histograms, the
+// intermediate array (cell keys, the sort's buffers and counts, the
 // cell table, the cell-order copies, the one-entry system table) lives in one
 // file-scope __device__ array of fixed size, resident on every GPU that loads
 // this library until the process exits.
@@ -1100,20 +1100,21 @@ namespace {
 
 constexpr int kNoAllocMaxN = 8192;       // particles per call
 constexpr int kNoAllocMaxCells = 16384;  // cells (nc * nc) per call
-constexpr int kNoAllocMaxTiles = (kNoAllocMaxN + kSortTile - 1) / kSortTile;
 
 constexpr size_t na_round(size_t b) { return (b + 255) / 256 * 256; }
 constexpr size_t kNaD = na_round(8ull * kNoAllocMaxN);   // one double per particle
 constexpr size_t kNaF = na_round(4ull * kNoAllocMaxN);   // one 32-bit value per particle
 constexpr size_t kNaF2 = na_round(8ull * kNoAllocMaxN);  // one float2 per particle
 constexpr size_t kNaCells = na_round(4ull * (kNoAllocMaxCells + 1));
-constexpr size_t kNaHist = na_round(4ull * (1u << 11) * kNoAllocMaxTiles);
+constexpr size_t kNaCount = 4ull * ((kNoAllocMaxCells + kScanChunk - 1) / kScanChunk * kScanChunk);
+constexpr size_t kNaStage = na_round(sizeof(StageRec) * kNoAllocMaxN);
 constexpr size_t kNaSys = na_round(sizeof(SysDesc));
-// x y phi omega | st_x st_y st_phi | sx sy sphi | dphi_s      (11 double arrays)
-// keys vals keys_alt vals_alt pidx cnt_s dphi_f sys_of_p      (8 32-bit arrays)
-// fxy cs (2 float2 arrays) | dcs (double2) | cell_start | sys_of_c | hist | system table | all-pairs cell | clamp counter
+// x y phi omega | sx sy sphi | dphi_s                         (8 double arrays)
+// keys arrival list skeys pidx cnt_s dphi_f sys_of_p          (8 32-bit arrays)
+// fxy cs (2 float2 arrays) | dcs (double2) | stage records | cell_start | sys_of_c | counts | chunk sums |
+// system table | all-pairs cell | clamp counter
 constexpr size_t kNoAllocBytes =
-    11 * kNaD + 8 * kNaF + 2 * kNaF2 + 2 * kNaD + 2 * kNaCells + kNaHist + kNaSys + 256 + 256;
+    8 * kNaD + 8 * kNaF + 2 * kNaF2 + 2 * kNaD + kNaStage + 2 * kNaCells + kNaCount + 256 + kNaSys + 256 + 256;
 
 constexpr int kNoAllocMaxDevices = 64;
 std::mutex g_noalloc_mu;
@@ -1234,17 +1235,14 @@ extern "C" int spc_rhs_srk_noalloc(const spc_params *p, int32_t n, const double 
   a.y = (double *)take(kNaD);
   a.phi = (double *)take(kNaD);
   a.omega = (double *)take(kNaD);
-  a.st_x = (double *)take(kNaD);
-  a.st_y = (double *)take(kNaD);
-  a.st_phi = (double *)take(kNaD);
   a.sx = (double *)take(kNaD);
   a.sy = (double *)take(kNaD);
   a.sphi = (double *)take(kNaD);
   a.dphi_s = (double *)take(kNaD);
   a.keys = (uint32_t *)take(kNaF);
-  a.vals = (uint32_t *)take(kNaF);
-  e.keys_alt = (uint32_t *)take(kNaF);
-  e.vals_alt = (uint32_t *)take(kNaF);
+  a.arrival = (int *)take(kNaF);
+  a.list = (int *)take(kNaF);
+  a.skeys = (uint32_t *)take(kNaF);
   a.pidx = (int *)take(kNaF);
   a.cnt_s = (int *)take(kNaF);
   a.dphi_f = (float *)take(kNaF);
@@ -1254,7 +1252,9 @@ extern "C" int spc_rhs_srk_noalloc(const spc_params *p, int32_t n, const double 
   a.dcs = (double2 *)take(2 * kNaD);
   a.cell_start = (int *)take(kNaCells);
   int *sys_of_c = (int *)take(kNaCells);
-  e.hist = (uint32_t *)take(kNaHist);
+  a.stg = (StageRec *)take(kNaStage);
+  a.cell_cnt = (int *)take(kNaCount);
+  e.part = (int *)take(256);
   SysDesc *sys = (SysDesc *)take(kNaSys);
   int *ap = (int *)take(256);
   unsigned long long *clamped = (unsigned long long *)take(256);
@@ -1263,7 +1263,6 @@ extern "C" int spc_rhs_srk_noalloc(const spc_params *p, int32_t n, const double 
   a.sys = sys;
   a.ap_cells = ap;
   a.clamped = clamped;
-  a.hist = e.hist;
   a.nbmask = nullptr;  // pass 2 re-tests candidates instead of reading masks
   a.out_d = d_derivative;
   a.out_a = d_additional;
@@ -1271,11 +1270,6 @@ extern "C" int spc_rhs_srk_noalloc(const spc_params *p, int32_t n, const double 
   e.nsys = 1;
   e.n_active = n;
   e.ncell_total = ncell;
-  e.ntiles = (n + kSortTile - 1) / kSortTile;
-  int bits = 1;
-  while (bits < 31 && (1u << bits) < (unsigned)std::max(ncell, 2)) ++bits;
-  e.sort_passes = (bits + 10) / 11;
-  e.radix_bits = (bits + e.sort_passes - 1) / e.sort_passes;
   e.has_cells = !sc.allpairs;
   a.nsys = 1;
   a.n_active = n;
@@ -1287,7 +1281,6 @@ extern "C" int spc_rhs_srk_noalloc(const spc_params *p, int32_t n, const double 
   a.n_ap = sc.allpairs ? 1 : 0;
   e.ap_items = sc.allpairs ? (n + kAllPairsThreads - 1) / kAllPairsThreads : 0;
   e.ap_items_small = sc.allpairs ? (n + kAllPairsThreadsSmall - 1) / kAllPairsThreadsSmall : 0;
-  a.hist_len = (1 << e.radix_bits) * e.ntiles;
   SysHost h;
   h.used = true;
   h.p = *p;
@@ -1300,10 +1293,10 @@ extern "C" int spc_rhs_srk_noalloc(const spc_params *p, int32_t n, const double 
   cudaError_t ce = set_kernel_attributes();
   if (ce != cudaSuccess) return fail(nullptr, SPC_ERR_CUDA, "kernel attributes: %s", cudaGetErrorString(ce));
   // the scratch keeps the previous call's contents: the clamp counter and the
-  // radix histogram table are accumulated into, and the system maps must read
+  // particles per cell are accumulated into, and the system maps must read
   // system 0, so they are cleared here
   ce = cudaMemsetAsync(clamped, 0, 8, e.stream);
-  if (ce == cudaSuccess) ce = cudaMemsetAsync(e.hist, 0, (size_t)a.hist_len * 4, e.stream);
+  if (ce == cudaSuccess) ce = cudaMemsetAsync(a.cell_cnt, 0, kNaCount, e.stream);
   if (ce == cudaSuccess) ce = cudaMemsetAsync(sys_of_p, 0, (size_t)n * 4, e.stream);
   if (ce == cudaSuccess) ce = cudaMemsetAsync(sys_of_c, 0, (size_t)ncell * 4, e.stream);
   if (ce != cudaSuccess) return fail(nullptr, SPC_ERR_CUDA, "clear scratch: %s", cudaGetErrorString(ce));

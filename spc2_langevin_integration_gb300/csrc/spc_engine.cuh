@@ -180,7 +180,7 @@ struct Engine {
   std::vector<void *> allocs;
   std::string err;
   // capacities
-  int pool_cap = 0, sys_cap = 0, cell_cap = 0, tile_cap = 0;
+  int pool_cap = 0, sys_cap = 0, cell_cap = 0;
   KArgs a{};
   SysDesc *d_sys = nullptr;
   int *d_ap = nullptr;      // cells of the all-pairs systems the all-pairs kernel integrates
@@ -191,7 +191,7 @@ struct Engine {
   int ap_items = 0, ap_items_all = 0;
   int ap_items_small = 0, ap_items_all_small = 0;
   unsigned long long *d_clamped = nullptr;
-  uint32_t *keys_alt = nullptr, *vals_alt = nullptr, *hist = nullptr, *part = nullptr;
+  int *part = nullptr;      // particles per chunk of keys (k_chunk_sums)
   double *aos = nullptr;  // AoS staging (12 x pool_cap doubles)
   double *order_part = nullptr;
   int order_blocks = 0;
@@ -202,7 +202,7 @@ struct Engine {
   int cells_used = 0;
   bool dirty = true;
   // current layout
-  int nsys = 0, n_active = 0, ncell_total = 0, ntiles = 0, radix_bits = 1, sort_passes = 1;
+  int nsys = 0, n_active = 0, ncell_total = 0;
   int ncell_tile = 0, ncell_warp = 0, ncell_va = 0;  // cells of the tile, warp and vortex-arrays systems
   bool has_cells = false;
   // tuning: cell-list systems with fewer than sparse_below particles per cell
@@ -304,20 +304,22 @@ cudaError_t vtile_attribute() {
                               (int)sizeof(VStage<PREC, KIND>));
 }
 
-// The 11-bit scatter and the Verlet passes need more than the default 48 KB of dynamic shared
+// The Verlet passes need more than the default 48 KB of dynamic shared
 // memory; the attribute is set with the device current (not a stream
 // operation, so never inside a capture).
 inline cudaError_t set_kernel_attributes() {
-  cudaError_t ce = cudaFuncSetAttribute(k_radix_scatter<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)scatter_smem_bytes(11));
-  if (ce == cudaSuccess)
-    ce = cudaFuncSetAttribute(k_radix_scatter<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)scatter_smem_bytes(11));
-  if (ce == cudaSuccess) ce = vtile_attribute<kPrecFP64, kKindSin>();
+  cudaError_t ce = vtile_attribute<kPrecFP64, kKindSin>();
   if (ce == cudaSuccess) ce = vtile_attribute<kPrecFP64, kKindCos2>();
   if (ce == cudaSuccess) ce = vtile_attribute<kPrecFP32C, kKindSin>();
   if (ce == cudaSuccess) ce = vtile_attribute<kPrecFP32C, kKindCos2>();
   return ce;
+}
+
+// Entries of the table of particles per key: whole chunks of the scan; the
+// float forms' sub-cells have two keys per cell.
+inline size_t count_entries(int precision, size_t cells) {
+  const size_t k = (precision != SPC_PRECISION_FP64 ? 2 : 1) * cells;
+  return (k + kScanChunk - 1) / kScanChunk * kScanChunk;
 }
 
 inline int engine_set_device(Engine *e) {
@@ -329,7 +331,7 @@ inline int engine_set_device(Engine *e) {
 inline void engine_footprint(int stepper, int precision, long long *per_particle, long long *per_cell) {
   long long b = 4 * 8;                       // x, y, phi, omega
   if (stepper == SPC_STEPPER_RK4) b += 12 * 8;  // k1..k4
-  b += 3 * 8 + 4 * 4 + 3 * 8 + 8 + 4 + 8 + 4 + 4 + 4;  // stage, sort, cell order, fxy, pidx, dphi, cnt, sys_of_p
+  b += 32 + 4 * 4 + 3 * 8 + 8 + 4 + 8 + 4 + 4;  // stage, sort, cell order, fxy, pidx, dphi, cnt, sys_of_p
   if (precision == SPC_PRECISION_FP32C) b += 8 + 4 + (long long)kMaskWords * 4;  // cs, dphi_f, masks
   if (precision == SPC_PRECISION_FP32X)
     b += 16 + 16 + 8 + 16 + 4 + (long long)kMaskWords * 4;  // ics, iws, scos, xsum, xcnt, masks
@@ -338,10 +340,10 @@ inline void engine_footprint(int stepper, int precision, long long *per_particle
   if (precision == SPC_PRECISION_FP64) b += 8 + 8 + 4;                          // vortex-arrays outputs
   if (precision != SPC_PRECISION_FP32C) b += 16;                                // dcs
   if (precision == SPC_PRECISION_FP64 && stepper == SPC_STEPPER_SRK) b += (long long)kMaskWords * 4;  // masks
-  b += 12 * 8 + 4 + 4;                       // AoS staging, histogram share
+  b += 12 * 8;                               // AoS staging
   *per_particle = b;
-  // cell_start, sys_of_c; float forms: unit list (two halves' worth), flag, sub-cell split and flag
-  *per_cell = 4 + 4 + (precision != SPC_PRECISION_FP64 ? 2 * kSplitRounds * 8 + 1 + 4 + 1 : 0);
+  // cell_start, sys_of_c, counts; float forms: unit list (two halves' worth), flag, sub-cell split and flag
+  *per_cell = 4 + 4 + 4 + (precision != SPC_PRECISION_FP64 ? 4 + 2 * kSplitRounds * 8 + 1 + 4 + 1 : 0);
 }
 
 inline int engine_init(Engine *e, int stepper, int precision, int pool_cap, int sys_cap, int cell_cap) {
@@ -355,7 +357,6 @@ inline int engine_init(Engine *e, int stepper, int precision, int pool_cap, int 
   SPC_CUDA(e, cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking));
   const size_t N = (size_t)pool_cap;
   KArgs &a = e->a;
-  e->tile_cap = (int)((N + kSortTile - 1) / kSortTile);
   SPC_TRY(dalloc(e, &a.x, N));
   SPC_TRY(dalloc(e, &a.y, N));
   SPC_TRY(dalloc(e, &a.phi, N));
@@ -368,13 +369,11 @@ inline int engine_init(Engine *e, int stepper, int precision, int pool_cap, int 
       SPC_TRY(dalloc(e, &a.ky[q], N));
       SPC_TRY(dalloc(e, &a.kphi[q], N));
     }
-  SPC_TRY(dalloc(e, &a.st_x, N));
-  SPC_TRY(dalloc(e, &a.st_y, N));
-  SPC_TRY(dalloc(e, &a.st_phi, N));
+  SPC_TRY(dalloc(e, &a.stg, N));
   SPC_TRY(dalloc(e, &a.keys, N));
-  SPC_TRY(dalloc(e, &a.vals, N));
-  SPC_TRY(dalloc(e, &e->keys_alt, N));
-  SPC_TRY(dalloc(e, &e->vals_alt, N));
+  SPC_TRY(dalloc(e, &a.arrival, N));
+  SPC_TRY(dalloc(e, &a.list, N));
+  SPC_TRY(dalloc(e, &a.skeys, N));
   SPC_TRY(dalloc(e, &a.sx, N));
   SPC_TRY(dalloc(e, &a.sy, N));
   SPC_TRY(dalloc(e, &a.sphi, N));
@@ -426,9 +425,9 @@ inline int engine_init(Engine *e, int stepper, int precision, int pool_cap, int 
   SPC_TRY(dalloc(e, &a.cell_start, (size_t)cell_cap + 1));
   SPC_TRY(dalloc(e, &sys_of_c, (size_t)cell_cap));
   a.sys_of_c = sys_of_c;
-  // radix histogram table: up to 2^11 digits per tile, plus group partials
-  SPC_TRY(dalloc(e, &e->hist, (size_t)(1 << 11) * e->tile_cap));
-  SPC_TRY(dalloc(e, &e->part, (size_t)(1 << 11) * ((e->tile_cap + kScanGroup - 1) / kScanGroup)));
+  const size_t nkeys = count_entries(precision, (size_t)cell_cap);
+  SPC_TRY(dalloc(e, &a.cell_cnt, nkeys));
+  SPC_TRY(dalloc(e, &e->part, nkeys / kScanChunk));
   SPC_TRY(dalloc(e, &e->d_sys, (size_t)sys_cap));
   SPC_TRY(dalloc(e, &e->d_ap, (size_t)sys_cap));
   SPC_TRY(dalloc(e, &e->d_ap_all, (size_t)sys_cap));
@@ -439,10 +438,9 @@ inline int engine_init(Engine *e, int stepper, int precision, int pool_cap, int 
   a.sys = e->d_sys;
   a.ap_cells = e->d_ap;
   a.clamped = e->d_clamped;
-  a.hist = e->hist;
   cudaStream_t st = e->stream;
   SPC_CUDA(e, cudaMemsetAsync(omega, 0, N * 8, st));
-  SPC_CUDA(e, cudaMemsetAsync(e->hist, 0, (size_t)(1 << 11) * e->tile_cap * 4, st));
+  SPC_CUDA(e, cudaMemsetAsync(a.cell_cnt, 0, nkeys * 4, st));
   SPC_CUDA(e, cudaMemsetAsync(e->d_clamped, 0, 8, st));
   if (a.unit_done) {
     SPC_CUDA(e, cudaMemsetAsync(a.unit_done, 0, N * 4, st));
@@ -678,8 +676,8 @@ inline bool subcells_on(const Engine *e) {
 // keeps the cached graphs, whose kernels read the rewritten tables.
 inline std::vector<long long> launch_shape(const Engine *e) {
   const KArgs &a = e->a;
-  return {e->nsys, e->n_active, e->ncell_total, e->ntiles, e->radix_bits, e->sort_passes, e->ncell_tile,
-          e->ncell_warp, e->ncell_va, e->n_ap_all, e->has_cells, a.n_ap, a.tile_split, a.hist_len,
+  return {e->nsys, e->n_active, e->ncell_total, e->ncell_tile,
+          e->ncell_warp, e->ncell_va, e->n_ap_all, e->has_cells, a.n_ap, a.tile_split,
           e->ap_items, e->ap_items_all, e->ap_items_small, e->ap_items_all_small, a.units != nullptr,
           a.cell_mid != nullptr, a.lane_p0, a.lane_p1};
 }
@@ -731,14 +729,7 @@ inline int engine_layout(Engine *e) {
   e->nsys = (int)table.size();
   e->n_active = dense;
   e->ncell_total = cells;
-  e->ntiles = std::max(1, (dense + kSortTile - 1) / kSortTile);
-  // sub-cells: two sort keys per cell
-  const bool sub = subcells_on(e);
-  const int nkeys = sub ? 2 * cells : cells;
-  int bits = 1;
-  while (bits < 31 && (1u << bits) < (unsigned)std::max(nkeys, 2)) ++bits;
-  e->sort_passes = (bits + 10) / 11;
-  e->radix_bits = (bits + e->sort_passes - 1) / e->sort_passes;
+  const bool sub = subcells_on(e);  // two sort keys per cell
   e->has_cells = ncell_tile + ncell_warp > 0;
   e->n_ap_all = (int)ap_all.size();
   KArgs &a = e->a;
@@ -755,7 +746,6 @@ inline int engine_layout(Engine *e) {
   a.va_c0 = e->ncell_tile + e->ncell_warp;
   a.va_c1 = a.va_c0 + e->ncell_va;
   a.n_ap = (int)ap.size();
-  a.hist_len = (1 << e->radix_bits) * e->ntiles;
   if (e->nsys > 0) {
     SPC_CUDA(e, cudaMemcpyAsync(e->d_sys, table.data(), table.size() * sizeof(SysDesc),
                                 cudaMemcpyHostToDevice, e->stream));
@@ -769,8 +759,6 @@ inline int engine_layout(Engine *e) {
     k_layout_maps<<<blocks_for(g, 256), 256, 0, e->stream>>>(e->d_sys, e->nsys, e->n_active, e->ncell_total,
                                                              (int *)a.sys_of_p, (int *)a.sys_of_c);
     SPC_LAUNCHED(e);
-    // the histogram table must be zero before the next stage kernel
-    SPC_CUDA(e, cudaMemsetAsync(e->hist, 0, (size_t)(1 << 11) * e->tile_cap * 4, e->stream));
     // host-side copies above read pageable memory: finish before `table` dies
     SPC_CUDA(e, cudaStreamSynchronize(e->stream));
   }
@@ -825,8 +813,6 @@ inline int eval_stage(Engine *e, KArgs &a, int rk_form, int kq, double kcdt, boo
   k_verlet_build<<<std::min(std::max(e->ncell_total, 1), 152 * 16), kVThreads, 0, st>>>(b);
   SPC_LAUNCHED(e);
   mark(e, 3);
-  a.skeys = b.skeys;
-  a.svals = b.svals;
   return SPC_OK;
 }
 
@@ -836,42 +822,27 @@ inline int eval_stage(Engine *e, KArgs &a, int rk_form, int kq, double kcdt, boo
 inline int eval_cells(Engine *e, KArgs &a, int prec, int rk_form, int kq, double kcdt, bool marks) {
   const int n = e->n_active;
   cudaStream_t st = e->stream;
-  const int bits = e->radix_bits;
-  k_stage<<<blocks_for(n, kStageThreads), kStageThreads, 0, st>>>(a, rk_form, kq, kcdt, bits, e->hist);
+  k_stage<<<blocks_for(n, kStageThreads), kStageThreads, 0, st>>>(a, rk_form, kq, kcdt);
   SPC_LAUNCHED(e);
   if (marks) mark(e, 1);
-  uint32_t *kin = a.keys, *vin = a.vals, *kout = e->keys_alt, *vout = e->vals_alt;
-  for (int pass = 0; pass < e->sort_passes; ++pass) {
-    const int shift = pass * bits;
-    if (pass > 0) k_radix_hist<<<e->ntiles, kSortThreads, 0, st>>>(kin, n, shift, bits, e->hist, a.gate);
-    if (e->ntiles <= kScanGroup) {
-      k_scan_digits<<<1, kScanThreads, 0, st>>>(e->hist, e->ntiles, bits, a.gate);
-    } else {
-      const int ng = (e->ntiles + kScanGroup - 1) / kScanGroup;
-      const dim3 grid(ng, blocks_for(1 << bits, 256));
-      k_scan_group_sums<<<grid, 256, 0, st>>>(e->hist, e->ntiles, bits, e->part, a.gate);
-      k_scan_digits<<<1, kScanThreads, 0, st>>>(e->part, ng, bits, a.gate);
-      k_scan_group_apply<<<grid, 256, 0, st>>>(e->hist, e->ntiles, bits, e->part, a.gate);
-    }
-    if (e->ntiles < kScatterSplitBelow)
-      k_radix_scatter<4><<<e->ntiles * 4, kSortThreads, scatter_smem_bytes(bits), st>>>(
-          kin, vin, kout, vout, n, shift, bits, e->hist, a.gate);
-    else
-      k_radix_scatter<1><<<e->ntiles, kSortThreads, scatter_smem_bytes(bits), st>>>(
-          kin, vin, kout, vout, n, shift, bits, e->hist, a.gate);
-    SPC_LAUNCHED(e);
-    std::swap(kin, kout);
-    std::swap(vin, vout);
+  const int nkeys = a.cell_mid ? 2 * e->ncell_total : e->ncell_total;
+  if (nkeys <= kScanOneCta) {
+    k_scan_cells<<<1, kScanThreads, 0, st>>>(a.cell_cnt, nkeys, e->ncell_total, n, a.cell_start, a.cell_mid, a.gate);
+  } else {
+    const int chunks = blocks_for(nkeys, kScanChunk);
+    k_chunk_sums<<<chunks, kScanThreads, 0, st>>>(a.cell_cnt, e->part, a.gate);
+    k_scan_chunks<<<chunks, kScanThreads, 0, st>>>(a.cell_cnt, e->part, nkeys, e->ncell_total, n, a.cell_start,
+                                                   a.cell_mid, a.gate);
   }
+  k_place<<<blocks_for(n, 256), 256, 0, st>>>(a.keys, a.arrival, n, a.cell_start, a.cell_mid, a.list, a.gate);
+  SPC_LAUNCHED(e);
   if (marks) mark(e, 2);
-  a.skeys = kin;
-  a.svals = vin;
   if (prec == kPrecFP32C)
-    k_gather<kPrecFP32C><<<blocks_for(n + 1, 256), 256, 0, st>>>(a);
+    k_gather<kPrecFP32C><<<blocks_for(n, 256), 256, 0, st>>>(a);
   else if (prec == kPrecFP32X)
-    k_gather<kPrecFP32X><<<blocks_for(n + 1, 256), 256, 0, st>>>(a);
+    k_gather<kPrecFP32X><<<blocks_for(n, 256), 256, 0, st>>>(a);
   else
-    k_gather<kPrecFP64><<<blocks_for(n + 1, 256), 256, 0, st>>>(a);
+    k_gather<kPrecFP64><<<blocks_for(n, 256), 256, 0, st>>>(a);
   SPC_LAUNCHED(e);
   if (a.units && e->ncell_tile > 0 && !e->verlet) {  // the cell units of this evaluation
     if (e->precision == SPC_PRECISION_FP32C)

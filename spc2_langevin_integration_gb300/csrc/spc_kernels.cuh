@@ -4,7 +4,7 @@
 // One evaluation (the reference's EvaluateInteractionsWithLinkedList,
 // ChimeraSystem.cpp:258-426 / :429-645) runs as:
 //   k_stage   stage state s + k_coef*dt*k_prev, copy-wrap, cell key  (ChimeraSystem.cpp:270-309)
-//   sort      stable radix sort of (global cell key, index)           (:335-338)
+//   sort      stable counting sort by global cell key (spc_sort.cuh)  (:335-338)
 //   k_gather  particles into cell order + float prefilter coordinates
 //   k_tile_*  (spc_tile.cuh) one CTA per cell: the 3x3 stencil in the
 //             reference's order, the exact FP64 cutoff, the alignment sums,
@@ -63,6 +63,14 @@ struct SysDesc {
   int budget;             // steps of the current call it takes; later steps leave it frozen
 };
 
+// A particle's stage state and cell key, one 32-byte sector: the gather reads
+// them in cell order.
+struct alignas(32) StageRec {
+  double x, y, phi;
+  uint32_t key;
+  int sys;
+};
+
 struct KArgs {
   const SysDesc *sys;
   int nsys;
@@ -79,9 +87,12 @@ struct KArgs {
   const double *omega;
   double *kx[kKSlots], *ky[kKSlots], *kphi[kKSlots];
   // stage (dense order)
-  double *st_x, *st_y, *st_phi;
-  uint32_t *keys, *vals;             // unsorted (global cell key, dense index)
-  const uint32_t *skeys, *svals;     // sorted
+  StageRec *stg;
+  uint32_t *keys;                    // global cell key (dense order)
+  int *arrival;                      // number of the particle among its cell's arrivals (dense order)
+  int *cell_cnt;                     // particles per key (zero between evaluations, padded to kScanChunk)
+  int *list;                         // dense indices by cell, in order of arrival
+  uint32_t *skeys;                   // key of each cell-order slot
   int *cell_start;
   // Sub-cells (SPC_TUNE_SUBCELLS; null when off): the sort key is 2c + h, h = 1
   // for the upper half of cell c (row_offset at least half a cell), and the
@@ -121,8 +132,6 @@ struct KArgs {
   longlong2 *part_x;
   int *part_n;
   int *unit_done;
-  uint32_t *hist;                    // radix histogram table (zeroed by k_gather)
-  int hist_len;
   const int *ap_cells;               // global cells of the all-pairs systems
   int n_ap;
   // parity / diagnostics outputs, indexed by pool slot
@@ -183,65 +192,54 @@ constexpr double kNearHalf = 0x1p-20;
 // the SRK form, whose stage state is the state itself (:456-458).  With
 // sub-cells the key also carries the half of the cell (the upper half when
 // the stage y is at least half a cell above the cell's lower edge).
-// With hist_bits > 0 the kernel also counts the first radix digit per sort
-// tile into hist (tile-major [tile][digit], zero on entry): a block-local
-// shared histogram, then one global atomic per non-empty bin.
+// It also counts the key's particles and numbers its arrivals (spc_sort.cuh).
 constexpr int kStageThreads = 256;
 
-constexpr int kMaxHistBits = 11;
-
-__global__ void __launch_bounds__(kStageThreads)
-    k_stage(KArgs a, int rk_form, int kq, double kcdt, int hist_bits, uint32_t *hist) {
+__global__ void __launch_bounds__(kStageThreads) k_stage(KArgs a, int rk_form, int kq, double kcdt) {
   if (a.gate && *a.gate == 0) return;
-  __shared__ uint32_t h[1 << kMaxHistBits];
-  const int R = 1 << hist_bits;
   const int d = blockIdx.x * blockDim.x + threadIdx.x;
-  if (hist_bits > 0) {
-    for (int k = threadIdx.x; k < R; k += blockDim.x) h[k] = 0;
-    __syncthreads();
-  }
   if (a.cell_mid)  // this evaluation's near flags (set by k_gather)
     for (int c = d; c < a.ncell_total; c += gridDim.x * blockDim.x) a.cell_near[c] = 0;
-  if (d < a.n_active) {
-    const SysDesc &sd = a.sys[a.sys_of_p[d]];
-    const SysConst &sc = sd.sc;
-    const int q = sd.pool_p0 + (d - sd.dense_p0);
-    double x = a.x[q], y = a.y[q], ph = a.phi[q];
-    if (rk_form) {
-      const double kx = kq >= 0 ? a.kx[kq][q] : 0.0;
-      const double ky = kq >= 0 ? a.ky[kq][q] : 0.0;
-      const double kp = kq >= 0 ? a.kphi[kq][q] : 0.0;
-      x = dadd(x, dmul(kcdt, kx));
-      y = dadd(y, dmul(kcdt, ky));
-      ph = dadd(ph, dmul(kcdt, kp));
-    }
-    uint32_t key;
-    if (sc.allpairs) {
-      // all pairs use the unwrapped stage positions (ChimeraSystem.cpp:135-153)
-      key = a.cell_mid ? 2u * (uint32_t)sd.c0 : (uint32_t)sd.c0;
-    } else {
-      wrap_if_outside(sc, x, y);
-      int clamped = 0;
-      const int cx = cell_coord(sc, x, clamped);
-      const int cy = cell_coord(sc, y, clamped);
-      if (clamped) atomicAdd(a.clamped, 1ull);
-      key = (uint32_t)(sd.c0 + cy * sc.nc + cx);
-      if (a.cell_mid) key = 2u * key + (row_offset(sc, y, cy) >= 0.5 * sc.cell ? 1u : 0u);
-    }
-    a.st_x[d] = x;
-    a.st_y[d] = y;
-    a.st_phi[d] = ph;
-    a.keys[d] = key;
-    a.vals[d] = (uint32_t)d;
-    if (hist_bits > 0) atomicAdd(&h[key & (R - 1)], 1u);
+  if (d >= a.n_active) return;
+  const int s = a.sys_of_p[d];
+  const SysDesc &sd = a.sys[s];
+  const SysConst &sc = sd.sc;
+  const int i = d - sd.dense_p0, q = sd.pool_p0 + i;
+  double x = a.x[q], y = a.y[q], ph = a.phi[q];
+  if (rk_form) {
+    const double kx = kq >= 0 ? a.kx[kq][q] : 0.0;
+    const double ky = kq >= 0 ? a.ky[kq][q] : 0.0;
+    const double kp = kq >= 0 ? a.kphi[kq][q] : 0.0;
+    x = dadd(x, dmul(kcdt, kx));
+    y = dadd(y, dmul(kcdt, ky));
+    ph = dadd(ph, dmul(kcdt, kp));
   }
-  if (hist_bits > 0) {
-    __syncthreads();
-    // a block of 256 lies inside one sort tile of 2048
-    uint32_t *row = hist + (size_t)(blockIdx.x * blockDim.x / kSortTile) * R;
-    for (int k = threadIdx.x; k < R; k += blockDim.x)
-      if (h[k]) atomicAdd(&row[k], h[k]);
+  uint32_t key;
+  int arrival = i;
+  if (sc.allpairs) {
+    // all pairs use the unwrapped stage positions (ChimeraSystem.cpp:135-153),
+    // in index order
+    key = a.cell_mid ? 2u * (uint32_t)sd.c0 : (uint32_t)sd.c0;
+    if (i == 0) a.cell_cnt[key] = sc.n;
+  } else {
+    wrap_if_outside(sc, x, y);
+    int clamped = 0;
+    const int cx = cell_coord(sc, x, clamped);
+    const int cy = cell_coord(sc, y, clamped);
+    if (clamped) atomicAdd(a.clamped, 1ull);
+    key = (uint32_t)(sd.c0 + cy * sc.nc + cx);
+    if (a.cell_mid) key = 2u * key + (row_offset(sc, y, cy) >= 0.5 * sc.cell ? 1u : 0u);
+    arrival = atomicAdd(&a.cell_cnt[key], 1);
   }
+  StageRec r;
+  r.x = x;
+  r.y = y;
+  r.phi = ph;
+  r.key = key;
+  r.sys = s;
+  a.stg[d] = r;
+  a.keys[d] = key;
+  a.arrival[d] = arrival;
 }
 
 // Phase reduced to about [-pi, pi] in double, then float (FP32C trig input).
@@ -260,34 +258,33 @@ __device__ __forceinline__ int block_first(int cx, int nc) {
 template <int PREC>
 __global__ void k_gather(KArgs a) {
   if (a.gate && *a.gate == 0) return;
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  const int n = a.n_active;
-  if (p > n) return;
-  // the cell start table of the sorted keys (one thread per slot and one past the end)
-  if (a.cell_mid)
-    half_bounds_at(a.skeys, n, a.ncell_total, a.cell_start, a.cell_mid, p);
-  else
-    cell_bounds_at(a.skeys, n, a.ncell_total, a.cell_start, p);
-  // leave the first-digit histogram table zero for the next stage kernel
-  for (int k = p; k < a.hist_len; k += n + 1) a.hist[k] = 0u;
-  if (p == n) {
-    if (a.unit_count) *a.unit_count = 0;  // this evaluation's cell units (k_list_units)
-    return;
-  }
-  const int d = (int)a.svals[p];
-  const SysDesc &sd = a.sys[a.sys_of_p[d]];
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= a.n_active) return;
+  if (t == 0 && a.unit_count) *a.unit_count = 0;  // this evaluation's cell units (k_list_units)
+  const int d = a.list[t];
+  const StageRec r = a.stg[d];
+  const SysDesc &sd = a.sys[r.sys];
   const SysConst &sc = sd.sc;
-  const double x = a.st_x[d], y = a.st_y[d], ph = a.st_phi[d];
+  const double x = r.x, y = r.y, ph = r.phi;
+  int p = t;  // cell-order slot: the cell's indices below d come before it
+  if (!sc.allpairs) {
+    const int c0 = key_start(r.key, a.cell_start, a.cell_mid), c1 = key_end(r.key, a.cell_start, a.cell_mid);
+    p = c0;
+#pragma unroll 4
+    for (int k = c0; k < c1; ++k) p += a.list[k] < d ? 1 : 0;
+  }
+  a.skeys[p] = r.key;
   a.sx[p] = x;
   a.sy[p] = y;
   a.sphi[p] = ph;
   a.pidx[p] = sd.pool_p0 + (d - sd.dense_p0);
+  const int cell = (int)(a.cell_mid ? r.key >> 1 : r.key);
   if (a.vsys) {  // Verlet build: remember each slot's system and cell until the next build
-    a.vsys[p] = a.sys_of_p[d];
-    a.vcell[p] = cell_of_slot(a, p);
+    a.vsys[p] = r.sys;
+    a.vcell[p] = cell;
   }
   if (!sc.allpairs) {
-    const int key = cell_of_slot(a, p) - sd.c0;
+    const int key = cell - sd.c0;
     const int cx = key % sc.nc, cy = key / sc.nc;
     const int ox = p >= a.lane_p0 && p < a.lane_p1 ? block_first(cx, sc.nc) : cx;
     a.fxy[p] = make_float2((float)__fma_rn(-(double)ox, sc.cell, x), (float)__fma_rn(-(double)cy, sc.cell, y));

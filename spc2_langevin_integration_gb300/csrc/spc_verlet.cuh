@@ -2,7 +2,7 @@
 // ChimeraSystem.cpp:648-903; rebuild rule ChimeraSystemPtr.cpp:902-927).
 //
 // A build bins the stage positions into the rho-cells exactly as the cell-list
-// path does (stage, radix sort, gather), which fixes a cell order, the
+// path does (stage, sort, gather), which fixes a cell order, the
 // "Verlet order" v, until the next build.  For every particle the build then
 // lists, in the order of a (2R+1) x (2R+1) cell stencil (R = ceil(r_max / cell
 // side), rows of cells top to bottom, ascending index inside a cell), every
