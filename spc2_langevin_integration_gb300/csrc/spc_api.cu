@@ -196,12 +196,6 @@ int spc_create(const spc_params *p, int32_t n, spc_handle **out) {
     const double want = std::max(2.0 * mean, mean + 8.0 * std::sqrt(mean)) + 64.0;
     rc = engine_init_verlet(&h->e, ((int)want + 31) / 32 * 32);
   }
-  if (rc == SPC_OK && p->model == SPC_MODEL_VORTEX_ARRAYS && p->stepper == SPC_STEPPER_SRK) {
-    // pairs within rho: about pi rho^2 n / L^2 per particle
-    const double mean = 3.141592653589793 * p->rho * p->rho * (double)n / (p->L * p->L);
-    const double want = std::max(2.0 * mean, mean + 8.0 * std::sqrt(mean)) + 64.0;
-    rc = engine_init_va_cache(&h->e, ((int)std::min(want, (double)n) + 31) / 32 * 32);
-  }
   if (rc == SPC_OK) rc = engine_admit(&h->e, *p, n, -1, &h->slot);
   if (rc == SPC_OK) {
     Engine &e = h->e;
@@ -1106,7 +1100,7 @@ constexpr size_t kNaD = na_round(8ull * kNoAllocMaxN);   // one double per parti
 constexpr size_t kNaF = na_round(4ull * kNoAllocMaxN);   // one 32-bit value per particle
 constexpr size_t kNaF2 = na_round(8ull * kNoAllocMaxN);  // one float2 per particle
 constexpr size_t kNaCells = na_round(4ull * (kNoAllocMaxCells + 1));
-constexpr size_t kNaCount = 4ull * ((kNoAllocMaxCells + kScanChunk - 1) / kScanChunk * kScanChunk);
+constexpr size_t kNaCount = 4ull * (kNoAllocMaxCells + kScanChunk + (kSpreadKeys << kSpreadShift));
 constexpr size_t kNaStage = na_round(sizeof(StageRec) * kNoAllocMaxN);
 constexpr size_t kNaSys = na_round(sizeof(SysDesc));
 // x y phi omega | sx sy sphi | dphi_s                         (8 double arrays)
@@ -1275,7 +1269,6 @@ extern "C" int spc_rhs_srk_noalloc(const spc_params *p, int32_t n, const double 
   a.n_active = n;
   a.ncell_total = ncell;
   a.ncell_tile = sc.allpairs ? 0 : ncell;  // cell-tile kernels only
-  a.va_c0 = a.va_c1 = ncell;
   e.ncell_tile = a.ncell_tile;
   e.ncell_warp = 0;
   a.n_ap = sc.allpairs ? 1 : 0;

@@ -159,9 +159,13 @@ struct SysConst {
   int va;
   double mu_plus, mu_minus, xi_a, xi_r, kappa;
   float va_r2;    // float dr^2 above this: beyond rho and xi_r for certain
-  // vortex arrays: w = rho - xi_a and xi_a^2 as the model computes them, and
-  // the reciprocals of w, xi_a and xi_a^2 rounded to nearest (ddiv_by)
-  double va_w, va_xa2, va_rw, va_rxa, va_rxa2;
+  int va_near;    // rho and xi_r are at most L / 4
+  // vortex arrays: the largest squares whose rounded roots are within xi_a, rho
+  // and xi_r, the smallest whose roots reach xi_a and rho, L / 2, and the
+  // strengths' coefficients: mu_+ / xi_a^2, -4 mu_- / w^2 (w = rho - xi_a), the
+  // derivatives' 2 mu_+ / xi_a^2 and -4 mu_- / w^2 times v0, rho + xi_a, 2 D
+  double va_t_xia, va_t_rho, va_t_xir, va_s_xia, va_s_rho, va_hL;
+  double va_c1, va_c2, va_g1, va_g2, va_xr, va_2D;
 };
 
 // PeriodicBoundaryConditions::ClassAEffectiveParticleDistance (PeriodicBoundaryConditions.cpp:22-35):

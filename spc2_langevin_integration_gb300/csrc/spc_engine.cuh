@@ -53,6 +53,22 @@ inline int noise_per_particle(int stepper) {
   }
 }
 
+// The largest double whose correctly rounded root is at most r, and the
+// smallest whose root is at least r (r >= 0 and finite): the root is monotonic,
+// so comparing squares with them is comparing roots with r.
+inline double largest_square(double r) {
+  double t = r * r;
+  while (std::sqrt(t) > r) t = std::nextafter(t, 0.0);
+  while (std::sqrt(std::nextafter(t, HUGE_VAL)) <= r) t = std::nextafter(t, HUGE_VAL);
+  return t;
+}
+inline double smallest_square(double r) {
+  double t = r * r;
+  while (std::sqrt(t) < r) t = std::nextafter(t, HUGE_VAL);
+  while (t > 0.0 && std::sqrt(std::nextafter(t, 0.0)) >= r) t = std::nextafter(t, 0.0);
+  return t;
+}
+
 // Per-system constants from the public parameters (ChimeraSystem.cpp:19-33).
 inline SysConst make_sysconst(const spc_params &p, int n) {
   SysConst sc{};
@@ -96,12 +112,20 @@ inline SysConst make_sysconst(const spc_params &p, int n) {
     sc.kappa = p.kappa;
     const double rm = std::max(p.rho, p.xi_r);
     sc.va_r2 = (float)(rm * rm * (1.0 + 3e-5));
-    // IEEE double arithmetic on the host: the same roundings as the device's
-    sc.va_w = p.rho - p.xi_a;
-    sc.va_xa2 = p.xi_a * p.xi_a;
-    sc.va_rw = 1.0 / sc.va_w;
-    sc.va_rxa = 1.0 / p.xi_a;
-    sc.va_rxa2 = 1.0 / sc.va_xa2;
+    sc.va_near = rm <= 0.25 * p.L;
+    sc.va_t_xia = largest_square(p.xi_a);
+    sc.va_t_rho = largest_square(p.rho);
+    sc.va_t_xir = largest_square(p.xi_r);
+    sc.va_s_xia = smallest_square(p.xi_a);
+    sc.va_s_rho = smallest_square(p.rho);
+    sc.va_hL = 0.5 * p.L;
+    const double w = p.rho - p.xi_a;
+    sc.va_c1 = p.mu_plus / (p.xi_a * p.xi_a);
+    sc.va_c2 = -4.0 * p.mu_minus / (w * w);
+    sc.va_g1 = p.v0 * (2.0 * sc.va_c1);
+    sc.va_g2 = p.v0 * sc.va_c2;
+    sc.va_xr = p.rho + p.xi_a;
+    sc.va_2D = 2.0 * p.D_phi;
   }
   // Verlet rows over a (2R+1)^2 stencil of rho-cells; needs 2R+1 distinct cells
   if (p.neighbour == SPC_NEIGHBOUR_VERLET && !sc.allpairs && !sc.va) {
@@ -319,7 +343,7 @@ inline cudaError_t set_kernel_attributes() {
 // float forms' sub-cells have two keys per cell.
 inline size_t count_entries(int precision, size_t cells) {
   const size_t k = (precision != SPC_PRECISION_FP64 ? 2 : 1) * cells;
-  return (k + kScanChunk - 1) / kScanChunk * kScanChunk;
+  return std::max((k + kScanChunk - 1) / kScanChunk * kScanChunk, (size_t)kSpreadKeys << kSpreadShift);
 }
 
 inline int engine_set_device(Engine *e) {
@@ -337,7 +361,7 @@ inline void engine_footprint(int stepper, int precision, long long *per_particle
     b += 16 + 16 + 8 + 16 + 4 + (long long)kMaskWords * 4;  // ics, iws, scos, xsum, xcnt, masks
   if (precision != SPC_PRECISION_FP64)  // cell units: round sums, counts, chunk counters, list
     b += kSplitRounds * ((precision == SPC_PRECISION_FP32X ? 16 : 8) + 4) + 4 + kSplitRounds * 8 / 32;
-  if (precision == SPC_PRECISION_FP64) b += 8 + 8 + 4;                          // vortex-arrays outputs
+  if (precision == SPC_PRECISION_FP64) b += 4;                                  // vortex-arrays partner counts
   if (precision != SPC_PRECISION_FP32C) b += 16;                                // dcs
   if (precision == SPC_PRECISION_FP64 && stepper == SPC_STEPPER_SRK) b += (long long)kMaskWords * 4;  // masks
   b += 12 * 8;                               // AoS staging
@@ -382,8 +406,6 @@ inline int engine_init(Engine *e, int stepper, int precision, int pool_cap, int 
   SPC_TRY(dalloc(e, &a.dphi_s, N));
   SPC_TRY(dalloc(e, &a.cnt_s, N));
   if (precision == SPC_PRECISION_FP64) {  // vortex-arrays pass-1 outputs
-    SPC_TRY(dalloc(e, &a.va_vx, N));
-    SPC_TRY(dalloc(e, &a.va_vy, N));
     SPC_TRY(dalloc(e, &a.va_cnt2, N));
     if (stepper == SPC_STEPPER_SRK) SPC_TRY(dalloc(e, &a.nbmask, (size_t)kMaskWords * N));
   }
@@ -457,18 +479,6 @@ inline int engine_init(Engine *e, int stepper, int precision, int pool_cap, int 
   e->slot_layout.assign(sys_cap, -1);
   e->free_ranges.clear();
   e->free_ranges.push_back({0, pool_cap});
-  return SPC_OK;
-}
-
-// Vortex-arrays SRK single systems: room for the first pass's records of
-// `cap` pairs within rho per particle (32 B each), within a budget of 4 GB;
-// beyond it (or beyond cap pairs) the second pass recomputes them.
-inline int engine_init_va_cache(Engine *e, int cap) {
-  const size_t N = (size_t)e->pool_cap;
-  cap = std::max(32, cap);
-  if ((size_t)cap * N * 4 * sizeof(double) > ((size_t)4 << 30)) return SPC_OK;
-  SPC_TRY(dalloc(e, &e->a.vacache, (size_t)cap * N * 4));
-  e->a.vacap = cap;
   return SPC_OK;
 }
 
@@ -679,7 +689,7 @@ inline std::vector<long long> launch_shape(const Engine *e) {
   return {e->nsys, e->n_active, e->ncell_total, e->ncell_tile,
           e->ncell_warp, e->ncell_va, e->n_ap_all, e->has_cells, a.n_ap, a.tile_split,
           e->ap_items, e->ap_items_all, e->ap_items_small, e->ap_items_all_small, a.units != nullptr,
-          a.cell_mid != nullptr, a.lane_p0, a.lane_p1};
+          a.cell_mid != nullptr, a.lane_p0, a.lane_p1, a.va_p1};
 }
 
 inline int engine_layout(Engine *e) {
@@ -693,7 +703,7 @@ inline int engine_layout(Engine *e) {
   // cell-tile systems first, then particle-per-lane, vortex-arrays and all-pairs
   // systems, so that each neighbour kernel covers one contiguous range of cells
   // and, for the lane kernel, of cell-order slots
-  int ncell_tile = 0, ncell_warp = 0, ncell_va = 0, lane_p0 = 0, lane_p1 = 0;
+  int ncell_tile = 0, ncell_warp = 0, ncell_va = 0, lane_p0 = 0, lane_p1 = 0, va_p1 = 0;
   e->ap_items = e->ap_items_all = 0;
   e->ap_items_small = e->ap_items_all_small = 0;
   for (int cls = 0; cls < 4; ++cls) {
@@ -722,6 +732,7 @@ inline int engine_layout(Engine *e) {
     }
     if (cls == 0) lane_p0 = dense;
     if (cls == 1) lane_p1 = dense;
+    if (cls == 2) va_p1 = dense;
   }
   e->ncell_tile = ncell_tile;
   e->ncell_warp = ncell_warp;
@@ -743,8 +754,7 @@ inline int engine_layout(Engine *e) {
   a.cell_near = sub ? e->cell_near_buf : nullptr;
   a.lane_p0 = lane_p0;
   a.lane_p1 = e->verlet ? lane_p0 : lane_p1;  // Verlet passes serve every cell-list system
-  a.va_c0 = e->ncell_tile + e->ncell_warp;
-  a.va_c1 = a.va_c0 + e->ncell_va;
+  a.va_p1 = e->verlet ? lane_p0 : va_p1;
   a.n_ap = (int)ap.size();
   if (e->nsys > 0) {
     SPC_CUDA(e, cudaMemcpyAsync(e->d_sys, table.data(), table.size() * sizeof(SysDesc),
@@ -784,7 +794,7 @@ inline int eval_stage(Engine *e, KArgs &a, int rk_form, int kq, double kcdt, boo
   if (!verlet_ok) {
     a.cell_mid = nullptr;
     a.cell_near = nullptr;
-    a.lane_p0 = a.lane_p1 = 0;  // every prefilter coordinate relative to its own cell
+    a.lane_p0 = a.lane_p1 = a.va_p1 = 0;  // every prefilter coordinate relative to its own cell
     // they run the FP64 gather and pass: cos / sin of the phases go behind
     // the results in the AoS staging area (12 doubles per pool particle)
     a.dcs = reinterpret_cast<double2 *>(e->aos + (((size_t)e->pool_cap + 1) & ~(size_t)1));
@@ -822,19 +832,23 @@ inline int eval_stage(Engine *e, KArgs &a, int rk_form, int kq, double kcdt, boo
 inline int eval_cells(Engine *e, KArgs &a, int prec, int rk_form, int kq, double kcdt, bool marks) {
   const int n = e->n_active;
   cudaStream_t st = e->stream;
+  const int nkeys = a.cell_mid ? 2 * e->ncell_total : e->ncell_total;
+  a.cnt_shift = count_shift(nkeys);
   k_stage<<<blocks_for(n, kStageThreads), kStageThreads, 0, st>>>(a, rk_form, kq, kcdt);
   SPC_LAUNCHED(e);
   if (marks) mark(e, 1);
-  const int nkeys = a.cell_mid ? 2 * e->ncell_total : e->ncell_total;
+  const bool placed = nkeys <= kScanOneCta && n <= kPlaceInScan;
   if (nkeys <= kScanOneCta) {
-    k_scan_cells<<<1, kScanThreads, 0, st>>>(a.cell_cnt, nkeys, e->ncell_total, n, a.cell_start, a.cell_mid, a.gate);
+    k_scan_cells<<<1, kScanThreads, 0, st>>>(a.cell_cnt, a.cnt_shift, nkeys, e->ncell_total, n, a.cell_start,
+                                             a.cell_mid, a.gate, a.keys, a.arrival, a.list, placed ? n : 0);
   } else {
     const int chunks = blocks_for(nkeys, kScanChunk);
     k_chunk_sums<<<chunks, kScanThreads, 0, st>>>(a.cell_cnt, e->part, a.gate);
     k_scan_chunks<<<chunks, kScanThreads, 0, st>>>(a.cell_cnt, e->part, nkeys, e->ncell_total, n, a.cell_start,
                                                    a.cell_mid, a.gate);
   }
-  k_place<<<blocks_for(n, 256), 256, 0, st>>>(a.keys, a.arrival, n, a.cell_start, a.cell_mid, a.list, a.gate);
+  if (!placed)
+    k_place<<<blocks_for(n, 256), 256, 0, st>>>(a.keys, a.arrival, n, a.cell_start, a.cell_mid, a.list, a.gate);
   SPC_LAUNCHED(e);
   if (marks) mark(e, 2);
   if (prec == kPrecFP32C)
@@ -902,7 +916,9 @@ int launch_pass_t(Engine *e, const KArgs &a, int epi) {
   }
   if constexpr (PREC == kPrecFP64 && KIND != kKindNb) {
     if (e->ncell_va > 0) {
-      k_va_pass<KIND><<<std::min(e->ncell_va, 152 * 64), kVAThreads, 0, st>>>(a, epi);
+      const int np = a.va_p1 - a.lane_p1;
+      const int threads = np >= 152 * 4 * kLaneThreads ? kLaneThreads : kWarp;
+      k_va_pass<KIND><<<blocks_for(np, threads), threads, 0, st>>>(a, epi);
       SPC_LAUNCHED(e);
     }
   }

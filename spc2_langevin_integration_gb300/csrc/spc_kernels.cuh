@@ -78,8 +78,7 @@ struct KArgs {
   int ncell_total;
   int ncell_tile;                    // cells [0, ncell_tile): cell-tile kernels
   int tile_split;                    // cell-tile kernels: CTAs per cell (0 or 1: one)
-  int va_c0, va_c1;                  // [ncell_tile, va_c0): lane kernel; [va_c0, va_c1): vortex arrays
-  int lane_p0, lane_p1;              // cell-order slots of the lane kernel's systems
+  int lane_p0, lane_p1, va_p1;       // cell-order slots [lane_p0, lane_p1): lane kernel; [lane_p1, va_p1): vortex arrays
   const int *sys_of_p;               // dense index -> system
   const int *sys_of_c;               // global cell -> system
   // state pool (structure of arrays)
@@ -90,7 +89,8 @@ struct KArgs {
   StageRec *stg;
   uint32_t *keys;                    // global cell key (dense order)
   int *arrival;                      // number of the particle among its cell's arrivals (dense order)
-  int *cell_cnt;                     // particles per key (zero between evaluations, padded to kScanChunk)
+  int *cell_cnt;                     // key k's particles at [k << cnt_shift] (zero between evaluations)
+  int cnt_shift;
   int *list;                         // dense indices by cell, in order of arrival
   uint32_t *skeys;                   // key of each cell-order slot
   int *cell_start;
@@ -103,8 +103,8 @@ struct KArgs {
   uint8_t *cell_near;
   // cell order
   double *sx, *sy, *sphi;
-  float2 *fxy;                       // prefilter coordinates relative to the cell origin (lane kernel's
-                                     // systems: x relative to the column block's), kFxyPad entries more
+  float2 *fxy;                       // prefilter coordinates relative to the cell origin (slots [lane_p0,
+                                     // va_p1): x relative to the column block's), kFxyPad entries more
   float2 *cs;                        // FP32C: (cos phi, sin phi)
   double2 *dcs;                      // FP64 passes: (cos phi, sin phi) of the stage phase
   longlong2 *ics;                    // FP32X: (cos phi, sin phi) in fixed point (2^kXQ)
@@ -116,7 +116,6 @@ struct KArgs {
   double *dphi_s;                    // SRK pass 1 phase rate, cell order
   float *dphi_f;                     // same, float (FP32C)
   int *cnt_s;                        // n_i, cell order
-  double *va_vx, *va_vy;             // vortex arrays: pass-1 velocity components, cell order
   int *va_cnt2;                      // vortex arrays: cohesion partners, cell order
   uint32_t *nbmask;                  // pass-1 neighbour bitmasks for the SRK second pass (mask_at), or null
   // Cell units of the float cell-tile passes (SPC_TUNE_CELL_UNITS; units
@@ -151,11 +150,6 @@ struct KArgs {
   const int *gate;                   // binning kernels return at once when *gate == 0
   int *vsys, *vcell;                 // build: system and cell of each cell-order slot
   uint16_t *vrows;                   // row entry k of slot v at vrows[((k / 8) * n_active + v) * 8 + k % 8]
-  // vortex-arrays SRK (single systems): the first pass's record of slot p's
-  // k-th pair within rho (k < vacap): strength, its derivative, sin and cos of
-  // the phase difference at vacache[(k * n_active + p) * 4 + 0..3], or null
-  double *vacache;
-  int vacap;
   int *vrowlen;                      // entries of each row, -1: overflow (scan the stencil)
   int vcap;                          // row limit of the current build
   double *vxb, *vyb;                 // stage positions at the build
@@ -220,7 +214,7 @@ __global__ void __launch_bounds__(kStageThreads) k_stage(KArgs a, int rk_form, i
     // all pairs use the unwrapped stage positions (ChimeraSystem.cpp:135-153),
     // in index order
     key = a.cell_mid ? 2u * (uint32_t)sd.c0 : (uint32_t)sd.c0;
-    if (i == 0) a.cell_cnt[key] = sc.n;
+    if (i == 0) a.cell_cnt[(size_t)key << a.cnt_shift] = sc.n;
   } else {
     wrap_if_outside(sc, x, y);
     int clamped = 0;
@@ -229,7 +223,7 @@ __global__ void __launch_bounds__(kStageThreads) k_stage(KArgs a, int rk_form, i
     if (clamped) atomicAdd(a.clamped, 1ull);
     key = (uint32_t)(sd.c0 + cy * sc.nc + cx);
     if (a.cell_mid) key = 2u * key + (row_offset(sc, y, cy) >= 0.5 * sc.cell ? 1u : 0u);
-    arrival = atomicAdd(&a.cell_cnt[key], 1);
+    arrival = atomicAdd(&a.cell_cnt[(size_t)key << a.cnt_shift], 1);
   }
   StageRec r;
   r.x = x;
@@ -286,7 +280,7 @@ __global__ void k_gather(KArgs a) {
   if (!sc.allpairs) {
     const int key = cell - sd.c0;
     const int cx = key % sc.nc, cy = key / sc.nc;
-    const int ox = p >= a.lane_p0 && p < a.lane_p1 ? block_first(cx, sc.nc) : cx;
+    const int ox = p >= a.lane_p0 && p < a.va_p1 ? block_first(cx, sc.nc) : cx;
     a.fxy[p] = make_float2((float)__fma_rn(-(double)ox, sc.cell, x), (float)__fma_rn(-(double)cy, sc.cell, y));
     if (a.cell_mid && fabs(row_offset(sc, y, cy) - 0.5 * sc.cell) < kNearHalf * sc.cell)
       a.cell_near[sd.c0 + key] = 1;

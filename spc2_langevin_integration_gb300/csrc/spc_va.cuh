@@ -2,62 +2,46 @@
 // model (DynamicalSystems/VortexArraysSystemPtr.cpp).
 //
 // Per candidate pair the model needs the exact distance dr = sqrt(dx^2 + dy^2)
-// and, for cohesion, the bearing atan2(dy, dx): pass 1 sums the alignment
-// (dr <= xi_a), anti-alignment (xi_a < dr <= rho) and cohesion (dr <= xi_r)
-// terms with their three counts (:472-488); pass 2 (the stochastic
-// Runge-Kutta form) sums the additional derivative (:695-728) from the pass-1
-// derivatives of both particles.  One CTA takes one cell: the candidates of
-// its 3x3 stencil (the reference's visiting order, ChimeraSystem-style
-// linked list :446-473; all of the system's particles in index order when
-// rho > L/4, :164-183) are staged in shared memory, and each thread walks
-// them for one particle in order, so every sum keeps the reference's order.
-// A float test on cell-relative coordinates drops candidates beyond
-// max(rho, xi_r) for certain; every other candidate is decided and evaluated
-// in FP64 exactly as the reference writes it.
+// and, for cohesion, the bearing of j from i: pass 1 sums the alignment (dr <=
+// xi_a), anti-alignment (xi_a < dr <= rho) and cohesion (dr <= xi_r) terms with
+// their counts (:472-488); pass 2 (the stochastic Runge-Kutta form) sums the
+// additional derivative (:695-728) from the pass-1 rates of both particles.
+//
+// One lane takes one particle, as in the particle-per-lane passes (spc_lane.cuh):
+// a float test drops candidates beyond max(rho, xi_r) for certain, the rest
+// become bits, and the lanes walk their bits together (the reference's visiting
+// order; all of the system's particles in index order when rho > L/4,
+// :164-183).  The pair terms are FP64 with few operations of that pipe, which
+// bounds these passes:
+//  * the cutoffs compare dr^2 with the largest square whose root is within the
+//    cutoff (the rounded root is monotonic, so the sets are those of dr);
+//  * the minimum image of two positions of neighbouring cells is dx or dx -+ L;
+//  * sin and cos of phi_j - phi_i and of the bearing minus phi_i come from the
+//    particles' cos and sin, (dx, dy) / dr and the angle-difference identities
+//    (a small sine or cosine is evaluated as the reference writes it, as in
+//    add_pair), and the strengths from their polynomials' coefficients;
+//  * the quotients by the counts are taken once of each sum.
+// 19 operations a pair in pass 1 and 36 in pass 2, where sincos, atan2, quotients
+// and minimum images took about 100 and 60 with 32 bytes a pair kept between the
+// passes.  N = 12,800, L = 4, rho = 0.2: {VA1} and {VA2} us, before 1,338 and
+// 1,143.
 #pragma once
 
-#include "spc_tile.cuh"
+#include "spc_lane.cuh"
 
 namespace spc {
 
-constexpr int kVAThreads = 64;
-constexpr int kVACap = 512;  // candidates staged per round
-
-// AlignmentStrength (VortexArraysSystemPtr.cpp:737-749); the divisions by
-// the constants xi_a^2 and w = rho - xi_a use their precomputed reciprocals
-// (ddiv_by: the same correctly rounded quotients)
-__device__ __forceinline__ double va_strength(const SysConst &sc, double r) {
-  if (r < sc.xi_a) return dmul(sc.mu_plus, dsub(1.0, ddiv_by(dmul(r, r), sc.va_xa2, sc.va_rxa2)));
-  if (r < sc.rho) {
-    const double w = sc.va_w, rw = sc.va_rw;
-    return ddiv_by(ddiv_by(dmul(dmul(dmul(-sc.mu_minus, 4.0), dsub(r, sc.xi_a)), dsub(sc.rho, r)), w, rw), w, rw);
-  }
-  return 0.0;
-}
-
-// AlignmentStrengthDerivative (VortexArraysSystemPtr.cpp:751-763)
-__device__ __forceinline__ double va_strength_derivative(const SysConst &sc, double r) {
-  if (r < sc.xi_a)
-    return dmul(sc.mu_plus, ddiv_by(ddiv_by(dmul(-2.0, r), sc.xi_a, sc.va_rxa), sc.xi_a, sc.va_rxa));
-  if (r < sc.rho) {
-    const double w = sc.va_w, rw = sc.va_rw;
-    return ddiv_by(ddiv_by(dmul(dmul(-sc.mu_minus, 4.0), dadd(dadd(dmul(-2.0, r), sc.rho), sc.xi_a)), w, rw),
-                   w, rw);
-  }
-  return 0.0;
-}
-
 // Per-particle results of a pass.
 struct VAAcc {
-  double align, anti, coh;  // pass 1
-  int c0, c1, c2;
-  double a0, a1;            // pass 2
+  double align, coh;      // pass 1: (anti-)alignment, cohesion
+  int c01, c2;            // their partners
+  double a0, a1, b0, b1;  // pass 2: the additional terms, (anti-)alignment and cohesion
 };
 
 // Fused epilogue of the vortex-arrays passes for the particle at cell-order
 // slot p, pool slot q.
 template <int KIND>
-__device__ void va_epilogue(const KArgs &a, int epi, const SysDesc &sd, int p, int q, double phi,
+__device__ void va_epilogue(const KArgs &a, int epi, const SysDesc &sd, int p, int q, double2 cs,
                             const VAAcc &r) {
   const SysConst &sc = sd.sc;
   const bool live = a.step_off < sd.budget;
@@ -66,25 +50,24 @@ __device__ void va_epilogue(const KArgs &a, int epi, const SysDesc &sd, int p, i
   const double dt = a.dt;
   double z0 = 0.0, z1 = 0.0;
   const bool draws = (epi == kEpiEulerPtr || epi == kEpiSrk2) && !a.noise && live;
+  // velocity components (VortexArraysSystemPtr.cpp:491-504)
+  const double d0 = dmul(sc.v0, cs.x), d1 = dmul(sc.v0, cs.y);
   if (draws) philox_normal2(sd.seed, sd.system_id, step, (uint32_t)i, z0, z1);
   if constexpr (KIND == kKindSin) {
-    // k_next / derivative (VortexArraysSystemPtr.cpp:491-504): velocity
-    // components always; the phase rate only when there are (anti-)alignment
-    // partners, then the cohesion mean added on top
-    const double d0 = dmul(sc.v0, cos(phi)), d1 = dmul(sc.v0, sin(phi));
-    const int c01 = r.c0 + r.c1;
+    // k_next / derivative: velocity components always; the phase rate only
+    // when there are (anti-)alignment partners, then the cohesion mean added
+    // on top
     auto rate_from = [&](double prev) {
       double v = prev;
-      if (c01 > 0) v = ddiv(dadd(r.align, r.anti), (double)c01);
-      if (r.c2 > 0) v = dadd(v, ddiv(r.coh, (double)r.c2));
+      const Count n1 = count_of(r.c01), n2 = count_of(r.c2);
+      if (r.c01 > 0) v = ddiv_by(r.align, n1.n, n1.r);
+      if (r.c2 > 0) v = dadd(v, ddiv_by(r.coh, n2.n, n2.r));
       return v;
     };
     if (epi == kEpiSrk1) {
       a.dphi_s[p] = rate_from(0.0);  // the stepper zero-fills derivative
-      a.cnt_s[p] = c01;
+      a.cnt_s[p] = r.c01;
       a.va_cnt2[p] = r.c2;
-      a.va_vx[p] = d0;
-      a.va_vy[p] = d1;
     } else if (epi == kEpiEulerPtr) {
       if (!live) return;
       // StochasticEulerStepperPtr.hpp:56-76
@@ -116,9 +99,20 @@ __device__ void va_epilogue(const KArgs &a, int epi, const SysDesc &sd, int p, i
     }
   } else {
     // additional_derivative[i][0] *= sqrt(2 D) (VortexArraysSystemPtr.cpp:732)
-    const double A0 = dmul(r.a0, sc.s2D);
-    const double A1 = r.a1;
-    const double d0 = a.va_vx[p], d1 = a.va_vy[p], d2 = a.dphi_s[p];
+    // the neighbours within a cutoff are those the first pass counted
+    const int c01 = a.cnt_s[p], c2 = a.va_cnt2[p];
+    const Count n1 = count_of(c01), n2 = count_of(c2);
+    double s0 = 0.0, A1 = 0.0;
+    if (c01 > 0) {
+      s0 = ddiv_by(r.a0, n1.n, n1.r);
+      A1 = ddiv_by(r.a1, n1.n, n1.r);
+    }
+    if (c2 > 0) {
+      s0 = dadd(s0, ddiv_by(r.b0, n2.n, n2.r));
+      A1 = dadd(A1, ddiv_by(r.b1, n2.n, n2.r));
+    }
+    const double A0 = dmul(s0, sc.s2D);
+    const double d2 = a.dphi_s[p];
     if (epi == kEpiSrk2Out) {
       a.out_d[3 * (size_t)q] = d0;
       a.out_d[3 * (size_t)q + 1] = d1;
@@ -147,179 +141,172 @@ __device__ void va_epilogue(const KArgs &a, int epi, const SysDesc &sd, int p, i
   }
 }
 
-template <int KIND>
-struct VAStage {
-  float2 xy[kVACap];  // x+shift, y+shift (prefilter; cell-list systems)
-  double phi[kVACap];
-  int slot[kVACap];
-  // pass 2: the candidates' pass-1 derivatives
-  double vx[KIND == kKindCos2 ? kVACap : 1], vy[KIND == kKindCos2 ? kVACap : 1];
-  double dd[KIND == kKindCos2 ? kVACap : 1];
-};
+
+// a <= b for doubles that are not negative (b not NaN), by their bit patterns
+__device__ __forceinline__ bool le_bits(double a, double b) {
+  return (unsigned long long)__double_as_longlong(a) <= (unsigned long long)__double_as_longlong(b);
+}
+
+// xj - xi by minimum image (PeriodicBoundaryConditions.cpp:22-35).  `near`: the
+// pair passed the float test of a cell list with both cutoffs up to L/4, so the
+// difference is within L/4 of 0 or of -+L, and the reference's truncated
+// quotient is 0 or +-1.
+__device__ __forceinline__ double va_image(const SysConst &sc, double xj, double xi, bool near) {
+  const double d = dsub(xj, xi);
+  if (!near) return min_image_1d(d, sc.rL, sc.L);
+  const int hi = __double2hiint(d) & 0x7fffffff;
+  return hi > __double2hiint(sc.va_hL) ? dsub(d, copysign(sc.L, d)) : d;
+}
+
+__device__ __noinline__ double va_bearing(double dx, double dy, double phi) { return dsub(atan2(dy, dx), phi); }
+__device__ __noinline__ double sin_library(double v) { return sin(v); }
+__device__ __noinline__ double cos_library(double v) { return cos(v); }
+
+// sin and cos of (bearing - phi_i)
+__device__ __forceinline__ void va_bearing_sincos(double dx, double dy, double dr, double2 ci, double phii, double &s,
+                                                  double &c) {
+  if (dr == 0.0) {
+    const double t = va_bearing(dx, dy, phii);
+    s = sin_library(t);
+    c = cos_library(t);
+    return;
+  }
+  s = ddiv(__fma_rn(dy, ci.x, -dmul(dx, ci.y)), dr);
+  c = ddiv(__fma_rn(dx, ci.x, dmul(dy, ci.y)), dr);
+  if (small_term(s)) s = sin_library(va_bearing(dx, dy, phii));
+  if (small_term(c)) c = cos_library(va_bearing(dx, dy, phii));
+}
 
 template <int KIND>
-__global__ void __launch_bounds__(kVAThreads) k_va_pass(KArgs a, int epi) {
-  __shared__ VAStage<KIND> sm;
+__global__ void __launch_bounds__(kLaneThreads) k_va_pass(KArgs a, int epi) {
+  __shared__ uint32_t s_bits[kLaneWords][kLaneThreads];
+  __shared__ int s_slot[kLaneWords][kLaneThreads];
   const int tid = threadIdx.x;
-  const int n_all = a.n_active;
-  for (int c = a.va_c0 + blockIdx.x; c < a.va_c1; c += gridDim.x) {
-    const int cb = a.cell_start[c], ce = a.cell_start[c + 1];
-    if (cb == ce) continue;
-    const SysDesc &sd = a.sys[a.sys_of_c[c]];
-    const SysConst &sc = sd.sc;
-    const bool ap = sc.allpairs != 0;
-    Stencil st;
-    if (ap) {  // one cell holding the whole system, in index order
-#pragma unroll
-      for (int k = 0; k < 9; ++k) st.start[k] = cb;
-      st.prefix[0] = 0;
-#pragma unroll
-      for (int k = 1; k < 10; ++k) st.prefix[k] = ce - cb;
+  const int p = a.lane_p1 + blockIdx.x * blockDim.x + tid;
+  if (p >= a.va_p1) return;  // no barrier below
+  const int cell = cell_of_slot(a, p);
+  const SysDesc &sd = a.sys[a.sys_of_c[cell]];
+  const SysConst &sc = sd.sc;
+  const bool ap = sc.allpairs != 0, near = !ap && sc.va_near;
+  const double xi = a.sx[p], yi = a.sy[p], phii = a.sphi[p];
+  const double2 ci = a.dcs[p];
+  const double ddi = KIND == kKindCos2 ? a.dphi_s[p] : 0.0;
+  VAAcc r{0.0, 0.0, 0, 0, 0.0, 0.0, 0.0, 0.0};
+
+  auto pair = [&](int j) {
+    const double dx = va_image(sc, a.sx[j], xi, near), dy = va_image(sc, a.sy[j], yi, near);
+    const double dr2 = dadd(dmul(dx, dx), dmul(dy, dy));
+    const bool align = le_bits(dr2, sc.va_t_xia), rho_pair = le_bits(dr2, sc.va_t_rho);
+    const bool coh = le_bits(dr2, sc.va_t_xir);
+    const bool term = KIND == kKindSin ? align || rho_pair : rho_pair;
+    if (!(term || coh)) return;
+    const double dr = sqrt_pos(dr2);
+    const double2 cj = a.dcs[j];
+    // AlignmentStrength (:737-749) and, over dr, AlignmentStrengthDerivative (:751-763)
+    const bool in1 = !le_bits(sc.va_s_xia, dr2), in2 = !in1 && !le_bits(sc.va_s_rho, dr2);
+    const double f = in1 ? __fma_rn(dr2, -sc.va_c1, sc.mu_plus)
+                         : (in2 ? dmul(dmul(sc.va_c2, dsub(dr, sc.xi_a)), dsub(sc.rho, dr)) : 0.0);
+    if constexpr (KIND == kKindSin) {
+      // VortexArraysSystemPtr.cpp:475-488
+      if (term) {
+        double sn = __fma_rn(cj.y, ci.x, -dmul(cj.x, ci.y));
+        if (small_term(sn)) sn = sin_of_difference(a.sphi[j], phii, 0.0);
+        r.align = __fma_rn(f, sn, r.align);
+        ++r.c01;
+      }
+      if (coh) {
+        double s, c;
+        va_bearing_sincos(dx, dy, dr, ci, phii, s, c);
+        r.coh = dadd(r.coh, dmul(-sc.kappa, s));
+        ++r.c2;
+      }
     } else {
-      stencil_of(a, sd, c, st);
+      // VortexArraysSystemPtr.cpp:706-728
+      const double ex = dsub(cj.x, ci.x), ey = dsub(cj.y, ci.y);  // times v0: the velocity difference
+      if (rho_pair) {
+        double sp = __fma_rn(cj.y, ci.x, -dmul(cj.x, ci.y)), cp = __fma_rn(cj.x, ci.x, dmul(cj.y, ci.y));
+        if (small_term(sp)) sp = sin_of_difference(a.sphi[j], phii, 0.0);
+        if (small_term(cp)) cp = cos_of_difference(a.sphi[j], phii, 0.0);
+        // the strength's derivative over dr, times v0; at dr = 0 the reference divides 0 by 0
+        double g = in1 ? -sc.va_g1 : 0.0;
+        if (in2) g = ddiv(dmul(sc.va_g2, __fma_rn(-2.0, dr, sc.va_xr)), dr);
+        if (dr == 0.0) g = __longlong_as_double(0x7ff8000000000000ll);
+        const double fc = dmul(f, cp);
+        r.a0 = dsub(r.a0, fc);
+        const double q = __fma_rn(__fma_rn(ex, dx, dmul(ey, dy)), g, dmul(-sc.va_2D, f));
+        r.a1 = __fma_rn(q, sp, r.a1);
+        r.a1 = __fma_rn(dsub(a.dphi_s[j], ddi), fc, r.a1);
+      }
+      if (coh) {
+        double s, c;
+        va_bearing_sincos(dx, dy, dr, ci, phii, s, c);
+        r.b0 = __fma_rn(sc.kappa, c, r.b0);
+        const double turn = ddiv(dmul(sc.v0, __fma_rn(ey, dx, -dmul(ex, dy))), dr2);
+        r.b1 = __fma_rn(dmul(-sc.kappa, dsub(turn, ddi)), c, r.b1);
+        r.b1 = __fma_rn(dmul(sc.kappa, sc.D), s, r.b1);
+      }
     }
-    const int total = st.prefix[9];
-    const int rounds = (total + kVACap - 1) / kVACap;
-    for (int ig = cb; ig < ce; ig += kVAThreads) {
-      const int p = ig + tid;
-      const bool valid = p < ce;
-      double xi = 0.0, yi = 0.0, phii = 0.0;
-      float fx = 0.0f, fy = 0.0f;
-      double vxi = 0.0, vyi = 0.0, ddi = 0.0, norm1 = 0.0, norm2 = 0.0, rn1 = 1.0, rn2 = 1.0;
-      if (valid) {
-        xi = a.sx[p];
-        yi = a.sy[p];
-        phii = a.sphi[p];
+  };
+
+  int nw = 0;
+  auto walk = [&]() {
+    uint32_t bits = 0u;
+    int slot = 0;
+    for (int w = 0;;) {
+      if (bits == 0u) {
+        if (w == nw) break;
+        bits = s_bits[w][tid];
+        slot = s_slot[w][tid];
+        ++w;
+      }
+      const int t = __clz(bits);
+      bits ^= 0x80000000u >> t;
+      pair(slot + t);
+    }
+    nw = 0;
+  };
+  auto put = [&](uint32_t bits, int slot) {
+    if ((unsigned)(p - slot) < (unsigned)kWarp) bits &= ~(0x80000000u >> (p - slot));  // not itself
+    if (bits == 0u) return;
+    s_bits[nw][tid] = bits;
+    s_slot[nw][tid] = slot;
+    ++nw;
+  };
+
+  const int nc = sc.nc, cl = cell - sd.c0, cy = cl / nc, cx = cl - cy * nc;
+  const LaneRuns rn = lane_runs(cx, nc);
+  const float2 fi = ap ? make_float2(0.0f, 0.0f) : a.fxy[p];
+  const float xa = fi.x - (float)rn.sa * sc.cell_f, xb = fi.x - (float)rn.sb * sc.cell_f;
+  for (int k = ap ? 2 : 0; k < 3; ++k) {
+    const float y = fi.y - (float)(k - 1) * sc.cell_f;
+    const int *row = a.cell_start + sd.c0 + (ap ? 0 : adjust_cell(cy + k - 1, nc) * nc);
+#pragma unroll 1
+    for (int run = 0; run < (ap ? 1 : 2); ++run) {
+      const int j0 = ap ? row[0] : row[run ? rn.b0 : rn.a0], j1 = ap ? row[1] : row[run ? rn.b1 : rn.a1];
+      const float x = run ? xb : xa;
+      for (int base = j0; base < j1; base += kWarp) {
+        const int cnt = min(kWarp, j1 - base);
+        uint32_t bits = 0xffffffffu;
         if (!ap) {
-          const float2 f = a.fxy[p];
-          fx = f.x;
-          fy = f.y;
+          // sign of d^2 - va_r2 (rounded outwards): beyond rho and xi_r for certain when clear
+          int done = 0;
+          for (; done < cnt; done += 4) {
+            const float2 *f = a.fxy + base + done;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const float2 d = add2(f[u], make_float2(-x, -y));
+              bits = __funnelshift_l(__float_as_uint(cutoff_offset(d.x, d.y, -sc.va_r2)), bits, 1);
+            }
+          }
+          bits <<= kWarp - done;
         }
-        if constexpr (KIND == kKindCos2) {
-          vxi = a.va_vx[p];
-          vyi = a.va_vy[p];
-          ddi = a.dphi_s[p];
-          norm1 = (double)a.cnt_s[p];   // neighborhood_cardinality_[i][0] + [i][1]
-          norm2 = (double)a.va_cnt2[p]; // neighborhood_cardinality_[i][2]
-          rn1 = drcp(norm1);            // used only when norm1 > 0 (ddiv_by)
-          rn2 = drcp(norm2);
-        }
+        put(bits & first_bits(cnt), base);
+        if (nw == kLaneWords) walk();
       }
-      const int self = (ap ? 0 : st.prefix[4]) + (p - cb);
-      VAAcc r{0.0, 0.0, 0.0, 0, 0, 0, 0.0, 0.0};
-      int kr = 0;  // pairs within rho so far: the index of this particle's pair records
-      for (int rr = 0; rr < rounds; ++rr) {
-        const int rlo = rr * kVACap, rcnt = min(kVACap, total - rlo);
-        if (rounds > 1 || ig == cb) {
-          __syncthreads();
-          for (int k = tid; k < rcnt; k += blockDim.x) {
-            int q;
-            const int pj = slot_of(st, rlo + k, q);
-            if (!ap) {
-              const float2 f = a.fxy[pj];
-              sm.xy[k] = make_float2(f.x + shift_x(q, sc.cell_f), f.y + shift_y(q, sc.cell_f));
-            }
-            sm.phi[k] = a.sphi[pj];
-            sm.slot[k] = pj;
-            if constexpr (KIND == kKindCos2) {
-              sm.vx[k] = a.va_vx[pj];
-              sm.vy[k] = a.va_vy[pj];
-              sm.dd[k] = a.dphi_s[pj];
-            }
-          }
-          __syncthreads();
-        }
-        if (!valid) continue;
-        for (int j = 0; j < rcnt; ++j) {
-          if (rlo + j == self) continue;
-          if (!ap) {
-            const float2 cj = sm.xy[j];
-            const float ex = cj.x - fx, ey = cj.y - fy;
-            if (fmaf(ex, ex, ey * ey) > sc.va_r2) continue;  // beyond rho and xi_r for certain
-          }
-          // ClassAEffectiveParticleDistance on the (copy-wrapped) stage positions
-          const int pj = sm.slot[j];
-          const double dx = min_image_1d(dsub(a.sx[pj], xi), sc.rL, sc.L);
-          const double dy = min_image_1d(dsub(a.sy[pj], yi), sc.rL, sc.L);
-          const double dr = dsqrt(dadd(dmul(dx, dx), dmul(dy, dy)));
-          const double phij = sm.phi[j];
-          // a pair within rho has a record for the second SRK pass (single
-          // systems): the same strength, derivative, sin and cos bit for bit
-          const bool rho_pair = dr <= sc.rho;
-          double *rec = (rho_pair && a.vacache && kr < a.vacap) ? a.vacache + ((size_t)kr * n_all + p) * 4 : nullptr;
-          kr += rho_pair ? 1 : 0;
-          if constexpr (KIND == kKindSin) {
-            // VortexArraysSystemPtr.cpp:475-488
-            if (dr <= sc.xi_a || rho_pair) {
-              double as, sn;
-              if (rec) {
-                double cn;
-                sincos(dsub(phij, phii), &sn, &cn);  // the bits of sin and cos
-                as = va_strength(sc, dr);
-                rec[0] = as;
-                rec[1] = va_strength_derivative(sc, dr);
-                rec[2] = sn;
-                rec[3] = cn;
-              } else {
-                as = va_strength(sc, dr);
-                sn = sin(dsub(phij, phii));
-              }
-              if (dr <= sc.xi_a) {
-                r.align = dadd(r.align, dmul(as, sn));
-                ++r.c0;
-              } else {
-                r.anti = dadd(r.anti, dmul(as, sn));
-                ++r.c1;
-              }
-            }
-            if (dr <= sc.xi_r) {
-              r.coh = dadd(r.coh, dmul(-sc.kappa, sin(dsub(atan2(dy, dx), phii))));
-              ++r.c2;
-            }
-          } else {
-            // VortexArraysSystemPtr.cpp:706-728
-            if (rho_pair && (norm1 > 0.0)) {
-              double cp, sp, as, asd;
-              if (rec) {  // the first pass's values
-                as = rec[0];
-                asd = rec[1];
-                sp = rec[2];
-                cp = rec[3];
-              } else {
-                cp = cos(dsub(phij, phii));
-                sp = sin(dsub(phij, phii));
-                as = va_strength(sc, dr);
-                asd = va_strength_derivative(sc, dr);
-              }
-              // every quotient by norm1 or dr as ddiv would give it (ddiv_by)
-              const double rdr = drcp(dr);
-              r.a0 = dadd(r.a0, ddiv_by(dmul(-as, cp), norm1, rn1));
-              const double gx = ddiv_by(dmul(dmul(dsub(sm.vx[j], vxi), asd), dx), dr, rdr);
-              const double gy = ddiv_by(dmul(dmul(dsub(sm.vy[j], vyi), asd), dy), dr, rdr);
-              const double t1 = ddiv_by(dmul(dadd(gx, gy), sp), norm1, rn1);
-              const double t2 = ddiv_by(dmul(dmul(dsub(sm.dd[j], ddi), as), cp), norm1, rn1);
-              const double t3 = ddiv_by(dmul(dmul(dmul(2.0, sc.D), sp), as), norm1, rn1);
-              r.a1 = dadd(r.a1, dsub(dadd(t1, t2), t3));
-            }
-            if ((dr <= sc.xi_r) && (norm2 > 0.0)) {
-              const double th = atan2(dy, dx);
-              const double cq = cos(dsub(th, phii)), sq = sin(dsub(th, phii));
-              const double rdr = drcp(dr);
-              r.a0 = dadd(r.a0, ddiv_by(dmul(sc.kappa, cq), norm2, rn2));
-              const double inner =
-                  dsub(dadd(ddiv_by(ddiv_by(dmul(dsub(sm.vx[j], vxi), -dy), dr, rdr), dr, rdr),
-                            ddiv_by(ddiv_by(dmul(dsub(sm.vy[j], vyi), dx), dr, rdr), dr, rdr)),
-                       ddi);
-              const double u1 = ddiv_by(dmul(dmul(-sc.kappa, inner), cq), norm2, rn2);
-              const double u2 = ddiv_by(dmul(dmul(sc.kappa, sc.D), sq), norm2, rn2);
-              r.a1 = dadd(r.a1, dadd(u1, u2));
-            }
-          }
-        }
-      }
-      if (valid) va_epilogue<KIND>(a, epi, sd, p, a.pidx[p], phii, r);
     }
   }
+  walk();
+  va_epilogue<KIND>(a, epi, sd, p, a.pidx[p], ci, r);
 }
 
 }  // namespace spc
