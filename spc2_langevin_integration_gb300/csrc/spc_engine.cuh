@@ -880,6 +880,12 @@ void launch_allpairs(const KArgs &a, int epi, int items, int items_small, cudaSt
         <<<std::min(items_small, 152 * 32), kAllPairsThreadsSmall, 0, st>>>(a, epi);
 }
 
+// CTA width of the lane kernels at one lane per particle: one warp while that
+// spreads the particles over more SMs (up to 8 warps an SM; past it the lists of
+// one-warp CTAs take the SM's shared memory: FP64 N = 65,536 74 us a step
+// with them, 58 with four warps).
+inline int lane_threads(int np) { return np > 152 * 8 * kWarp ? kLaneThreads : kWarp; }
+
 template <int PREC, int KIND>
 int launch_pass_t(Engine *e, const KArgs &a, int epi) {
   cudaStream_t st = e->stream;
@@ -917,8 +923,14 @@ int launch_pass_t(Engine *e, const KArgs &a, int epi) {
   if constexpr (PREC == kPrecFP64 && KIND != kKindNb) {
     if (e->ncell_va > 0) {
       const int np = a.va_p1 - a.lane_p1;
-      const int threads = np >= 152 * 4 * kLaneThreads ? kLaneThreads : kWarp;
-      k_va_pass<KIND><<<blocks_for(np, threads), threads, 0, st>>>(a, epi);
+      if (np <= kVAGroupMax) {
+        k_va_pass<KIND, kLaneGroup><<<blocks_for((long long)np * kLaneGroup, kWarp), kWarp, 0, st>>>(a, epi);
+      } else {
+        // one warp per CTA while an SM's shared memory holds all of its warps
+        // (N = 51,200: 1,348 us a step, with four warps 1,536)
+        const int threads = np > 152 * 13 * kWarp ? kLaneThreads : kWarp;
+        k_va_pass<KIND, 1><<<blocks_for(np, threads), threads, 0, st>>>(a, epi);
+      }
       SPC_LAUNCHED(e);
     }
   }
@@ -964,8 +976,7 @@ int launch_pass_t(Engine *e, const KArgs &a, int epi) {
         if (np <= kLaneGroupMax<PREC>) {
           k_lane<PREC, KIND, kLaneGroup><<<blocks_for((long long)np * kLaneGroup, kWarp), kWarp, 0, st>>>(a, epi);
         } else {
-          // one warp per CTA when that spreads the particles over more SMs
-          const int threads = np >= 152 * 4 * kLaneThreads ? kLaneThreads : kWarp;
+          const int threads = lane_threads(np);
           k_lane<PREC, KIND, 1><<<blocks_for(np, threads), threads, 0, st>>>(a, epi);
         }
         SPC_LAUNCHED(e);

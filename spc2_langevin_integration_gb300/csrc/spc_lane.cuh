@@ -45,13 +45,14 @@ constexpr int kLanePairs = 2;   // FP64: neighbours taken at a time
 // additions keep the order).  The sums are the same bit for bit: FP32X's are
 // exact, FP32C adds row by row either way.
 constexpr int kLaneGroup = 4;
-// Up to this many particles, where the GPU's schedulers would hold one or two
-// warps each (4 lanes and 1 lane per particle, Euler step in us at density
-// 1,000, rho = 0.1): FP64 1,024: 34.8 / 40.1, 12,288: 44.5 / 49.0, 16,384: 56.1
-// / 50.3; FP32C 1,024: 27.5 / 34.7, 32,768: 48.2 / 53.0, 49,152: 58.7 / 58.5;
-// FP32X 1,024: 29.7 / 39.3, 32,768: 55.6 / 58.7, 49,152: 69.2 / 64.5.
+// Up to this many particles, where the GPU's schedulers would hold a few warps
+// each (4 lanes and 1 lane per particle, Euler step in us at density 1,000, rho
+// = 0.1): FP64 1,024: 27.1 / 34.2, 12,288: 34.3 / 40.0, 16,384: 46.0 / 42.3;
+// FP32C 1,024: 20.8 / 29.8, 65,536: 45.3 / 47.1, 81,920: 53.1 / 49.7; FP32X
+// 1,024: 24.1 / 33.8, 32,768: 41.8 / 44.3, 49,152: 53.5 / 49.0.
 template <int PREC>
-constexpr int kLaneGroupMax = PREC == kPrecFP64 ? 14336 : PREC == kPrecFP32C ? 45056 : 36864;
+constexpr int kLaneGroupMax = PREC == kPrecFP64 ? 14336 : PREC == kPrecFP32C ? 73728 : 38912;
+
 // Saved words: row k of particle p has entries [5 k, 5 k + 5) of (bits, slot)
 // pairs, in the particle's 16-byte groups of nbmask (as mask_at, so that the
 // passes of one batch share the buffer).  (0, 0) ends a row; (0, 1) in front
@@ -205,39 +206,41 @@ struct LaneSums<kPrecFP32C, KIND> {
   }
 };
 
-// Four lanes of a group walk one particle's words together (FP64): lane g
-// forms the term of the (g+1)-th remaining neighbour of the word, and all four
-// add the terms in order.  next(bits, base) as for walk_pairs.
-template <int KIND, class Next>
-__device__ __forceinline__ void walk_group(Acc<kPrecFP64> &acc, const KArgs &a, const SysConst &sc, const ILane &il,
-                                           int g, unsigned mask, int lead, Next next) {
-  uint32_t bits = 0u;
-  int base = 0;
-  while (bits != 0u || next(bits, base)) {
-    const int m = __popc(bits);
-    int j = il.p;
-#pragma unroll
-    for (int u = 0; u < kLaneGroup; ++u) {
-      const int t = __clz(bits);
-      if (u == g && u < m) j = base + t;
-      bits &= ~(0x80000000u >> (t & 31));
-    }
-    const double2 cj = a.dcs[j];
-    double t = KIND == kKindSin ? __fma_rn(cj.y, il.dca, -dmul(cj.x, il.dsa))
-                                : __fma_rn(cj.x, il.dca, dmul(cj.y, il.dsa));
-    const double d = KIND == kKindCos2 ? dsub(a.dphi_s[j], il.dphi) : 0.0;
-    if (g < m && small_term(t))
-      t = KIND == kKindSin ? sin_of_difference(a.sphi[j], il.phi, sc.alpha)
-                           : cos_of_difference(a.sphi[j], il.phi, sc.alpha);
-#pragma unroll
-    for (int u = 0; u < kLaneGroup; ++u) {
-      const double tu = __shfl_sync(mask, t, lead + u);
-      const double du = KIND == kKindCos2 ? __shfl_sync(mask, d, lead + u) : 0.0;
-      if (u >= m) continue;
-      acc.s0 = dadd(acc.s0, tu);
-      if constexpr (KIND == kKindCos2) acc.s1 = __fma_rn(du, tu, acc.s1);
-    }
+// The words that a group's first three lanes listed (lane k: row k), one after
+// the other, for walks in which the whole warp stays together: a group whose
+// words are used up idles until the last one's are.  skip: an empty list.
+struct GroupWords {
+  int w0, w1, w2, i;
+  __device__ GroupWords(int nw, int lead, bool skip) {
+    w0 = __shfl_sync(0xffffffffu, nw, lead);
+    w1 = w0 + __shfl_sync(0xffffffffu, nw, lead + 1);
+    w2 = w1 + __shfl_sync(0xffffffffu, nw, lead + 2);
+    if (skip) w0 = w1 = w2 = 0;
+    i = 0;
   }
+  // the next word when `bits` is used up; col: the first lane's column
+  __device__ void next(const uint32_t (*s_bits)[kLaneThreads], const int (*s_slot)[kLaneThreads], int col,
+                       uint32_t &bits, int &slot) {
+    if (bits != 0u || i >= w2) return;
+    const int row = i < w0 ? 0 : (i < w1 ? 1 : 2);
+    const int w = i - (row == 0 ? 0 : (row == 1 ? w0 : w1));
+    bits = s_bits[w][col + row];
+    slot = s_slot[w][col + row];
+    ++i;
+  }
+};
+
+// Lane g's neighbour of the word's next four (slot of bit 31: `slot`; `none`
+// when there are fewer); they leave the word.
+__device__ __forceinline__ int group_pick(uint32_t &bits, int slot, int g, int m, int none) {
+  int j = none;
+#pragma unroll
+  for (int u = 0; u < kLaneGroup; ++u) {
+    const int t = __clz(bits);
+    if (u == g && u < m) j = slot + t;
+    bits &= ~(0x80000000u >> (t & 31));
+  }
+  return j;
 }
 
 // G lanes per particle: 1 or kLaneGroup.
@@ -247,9 +250,10 @@ __global__ void __launch_bounds__(kLaneThreads, PREC != kPrecFP64 && G == 1 ? 10
   __shared__ uint32_t s_bits[kList ? kLaneWords : 1][kLaneThreads];
   __shared__ int s_slot[kList ? kLaneWords : 1][kLaneThreads];
   const int tid = threadIdx.x, g = tid % G, lead = tid % kWarp - g;
-  const unsigned group = ((1u << G) - 1u) << lead;  // the group's lanes (G > 1)
-  const int p = a.lane_p0 + (blockIdx.x * blockDim.x + tid) / G;
-  if (p >= a.lane_p1) return;  // no barrier below
+  const int p_own = a.lane_p0 + (blockIdx.x * blockDim.x + tid) / G;
+  if (G == 1 && p_own >= a.lane_p1) return;  // no barrier below
+  // groups: the warps stay whole, lanes past the end repeat the last particle
+  const int p = min(p_own, a.lane_p1 - 1);
   const int n_all = a.n_active;
   const int c = cell_of_slot(a, p);
   const SysDesc &sd = a.sys[a.sys_of_c[c]];
@@ -410,37 +414,50 @@ __global__ void __launch_bounds__(kLaneThreads, PREC != kPrecFP64 && G == 1 ? 10
     rows(0, 3, true);
     walk_list();
   } else {
-    bool alone = false;
+    constexpr unsigned kAll = 0xffffffffu;
     if (g < 3) rows(g, g + 1, false);
+    bool alone = false;
     if constexpr (kList) {
-      __syncwarp(group);
-      if (__any_sync(group, full)) {  // a very long row: the first lane walks as it tests
-        if (g != 0) return;
-        alone = true;
-        n = nw = 0;
-        rows(0, 3, true);
-        walk_list();
-      } else {
-        int row = 0, w = -1, words = __shfl_sync(group, nw, lead);
-        walk_group<KIND>(sums.acc, a, sc, il, g, group, lead, [&](uint32_t &bits, int &base) {
-          while (++w >= words) {
-            if (++row > 2) return false;
-            w = -1;
-            words = __shfl_sync(group, nw, lead + row);
+      __syncwarp();
+      alone = ((__ballot_sync(kAll, full) >> lead) & ((1u << G) - 1u)) != 0u;  // a very long row
+      GroupWords words(nw, lead, alone);
+      uint32_t bits = 0u;
+      int slot = 0;
+      while (true) {
+        words.next(s_bits, s_slot, tid - g, bits, slot);
+        const int m = __popc(bits);
+        if (!__any_sync(kAll, m > 0)) break;
+        const int j = group_pick(bits, slot, g, m, p);
+        const double2 cj = a.dcs[j];
+        double t = KIND == kKindSin ? __fma_rn(cj.y, il.dca, -dmul(cj.x, il.dsa))
+                                    : __fma_rn(cj.x, il.dca, dmul(cj.y, il.dsa));
+        const double d = KIND == kKindCos2 ? dsub(a.dphi_s[j], il.dphi) : 0.0;
+        if (g < m && small_term(t))
+          t = KIND == kKindSin ? sin_of_difference(a.sphi[j], il.phi, sc.alpha)
+                               : cos_of_difference(a.sphi[j], il.phi, sc.alpha);
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < G; ++u) {
+          const double tu = __shfl_sync(kAll, t, lead + u);
+          const double du = KIND == kKindCos2 ? __shfl_sync(kAll, d, lead + u) : 0.0;
+          if (u < m) {
+            sums.acc.s0 = dadd(sums.acc.s0, tu);
+            if constexpr (KIND == kKindCos2) sums.acc.s1 = __fma_rn(du, tu, sums.acc.s1);
           }
-          bits = s_bits[w][tid - g + row];
-          base = s_slot[w][tid - g + row];
-          return true;
-        });
+        }
       }
     } else {
-      sums.join_group(group, lead);
+      __syncwarp();
+      sums.join_group(kAll, lead);
     }
-    if (!alone) {
 #pragma unroll
-      for (int o = 1; o < G; o <<= 1) n += __shfl_xor_sync(group, n, o);
+    for (int o = 1; o < G; o <<= 1) n += __shfl_xor_sync(kAll, n, o);
+    if (g != 0 || p_own >= a.lane_p1) return;
+    if (alone) {  // the first lane walks as it tests
+      n = nw = 0;
+      rows(0, 3, true);
+      walk_list();
     }
-    if (g != 0) return;
   }
   sums.finish(a, epi, sd, il, n, a.pidx[p]);
 }

@@ -23,8 +23,7 @@
 //  * the quotients by the counts are taken once of each sum.
 // 19 operations a pair in pass 1 and 36 in pass 2, where sincos, atan2, quotients
 // and minimum images took about 100 and 60 with 32 bytes a pair kept between the
-// passes.  N = 12,800, L = 4, rho = 0.2: {VA1} and {VA2} us, before 1,338 and
-// 1,143.
+// passes.  N = 12,800, L = 4, rho = 0.2: 149 and 288 us, before 1,338 and 1,143.
 #pragma once
 
 #include "spc_lane.cuh"
@@ -177,13 +176,30 @@ __device__ __forceinline__ void va_bearing_sincos(double dx, double dy, double d
   if (small_term(c)) c = cos_library(va_bearing(dx, dy, phii));
 }
 
-template <int KIND>
+// What one pair adds: pass 1 (anti-)alignment x and cohesion u, pass 2 x and y
+// to the additional terms, u and v of cohesion.
+struct VATerm {
+  bool term, coh;
+  double x, y, u, v;
+};
+
+// G lanes per particle: one, or a group of four, three of which test a row of
+// the stencil each (or a third of an all-pairs system) and all of which form
+// pair terms side by side.  The terms are added in the reference's order either
+// way, so both give the same bits.  Few particles take groups: SRK step of N =
+// 12,800, L = 4 652 us with one lane, 456 with four; N = 25,600 820
+// and 943; N = 51,200 1,348 and 1,656.
+constexpr int kVAGroupMax = 19200;
+
+template <int KIND, int G>
 __global__ void __launch_bounds__(kLaneThreads) k_va_pass(KArgs a, int epi) {
   __shared__ uint32_t s_bits[kLaneWords][kLaneThreads];
   __shared__ int s_slot[kLaneWords][kLaneThreads];
-  const int tid = threadIdx.x;
-  const int p = a.lane_p1 + blockIdx.x * blockDim.x + tid;
-  if (p >= a.va_p1) return;  // no barrier below
+  const int tid = threadIdx.x, g = tid % G, lead = tid % kWarp - g;
+  const int p_own = a.lane_p1 + (blockIdx.x * blockDim.x + tid) / G;
+  if (G == 1 && p_own >= a.va_p1) return;  // no barrier below
+  // groups: the warps stay whole, lanes past the end repeat the last particle
+  const int p = min(p_own, a.va_p1 - 1);
   const int cell = cell_of_slot(a, p);
   const SysDesc &sd = a.sys[a.sys_of_c[cell]];
   const SysConst &sc = sd.sc;
@@ -193,63 +209,75 @@ __global__ void __launch_bounds__(kLaneThreads) k_va_pass(KArgs a, int epi) {
   const double ddi = KIND == kKindCos2 ? a.dphi_s[p] : 0.0;
   VAAcc r{0.0, 0.0, 0, 0, 0.0, 0.0, 0.0, 0.0};
 
-  auto pair = [&](int j) {
+  auto term_of = [&](int j, bool wanted) {
+    VATerm t{false, false, 0.0, 0.0, 0.0, 0.0};
     const double dx = va_image(sc, a.sx[j], xi, near), dy = va_image(sc, a.sy[j], yi, near);
     const double dr2 = dadd(dmul(dx, dx), dmul(dy, dy));
     const bool align = le_bits(dr2, sc.va_t_xia), rho_pair = le_bits(dr2, sc.va_t_rho);
-    const bool coh = le_bits(dr2, sc.va_t_xir);
-    const bool term = KIND == kKindSin ? align || rho_pair : rho_pair;
-    if (!(term || coh)) return;
+    t.term = wanted && (KIND == kKindSin ? align || rho_pair : rho_pair);
+    t.coh = wanted && le_bits(dr2, sc.va_t_xir);
     const double dr = sqrt_pos(dr2);
     const double2 cj = a.dcs[j];
     // AlignmentStrength (:737-749) and, over dr, AlignmentStrengthDerivative (:751-763)
     const bool in1 = !le_bits(sc.va_s_xia, dr2), in2 = !in1 && !le_bits(sc.va_s_rho, dr2);
     const double f = in1 ? __fma_rn(dr2, -sc.va_c1, sc.mu_plus)
                          : (in2 ? dmul(dmul(sc.va_c2, dsub(dr, sc.xi_a)), dsub(sc.rho, dr)) : 0.0);
+    double sp = __fma_rn(cj.y, ci.x, -dmul(cj.x, ci.y));
+    if (wanted && small_term(sp)) sp = sin_of_difference(a.sphi[j], phii, 0.0);
     if constexpr (KIND == kKindSin) {
-      // VortexArraysSystemPtr.cpp:475-488
-      if (term) {
-        double sn = __fma_rn(cj.y, ci.x, -dmul(cj.x, ci.y));
-        if (small_term(sn)) sn = sin_of_difference(a.sphi[j], phii, 0.0);
-        r.align = __fma_rn(f, sn, r.align);
-        ++r.c01;
-      }
-      if (coh) {
+      t.x = dmul(f, sp);  // VortexArraysSystemPtr.cpp:475-485
+      if (t.coh) {        // :486-488
         double s, c;
         va_bearing_sincos(dx, dy, dr, ci, phii, s, c);
-        r.coh = dadd(r.coh, dmul(-sc.kappa, s));
-        ++r.c2;
+        t.u = dmul(-sc.kappa, s);
       }
     } else {
       // VortexArraysSystemPtr.cpp:706-728
+      double cp = __fma_rn(cj.x, ci.x, dmul(cj.y, ci.y));
+      if (wanted && small_term(cp)) cp = cos_of_difference(a.sphi[j], phii, 0.0);
       const double ex = dsub(cj.x, ci.x), ey = dsub(cj.y, ci.y);  // times v0: the velocity difference
-      if (rho_pair) {
-        double sp = __fma_rn(cj.y, ci.x, -dmul(cj.x, ci.y)), cp = __fma_rn(cj.x, ci.x, dmul(cj.y, ci.y));
-        if (small_term(sp)) sp = sin_of_difference(a.sphi[j], phii, 0.0);
-        if (small_term(cp)) cp = cos_of_difference(a.sphi[j], phii, 0.0);
-        // the strength's derivative over dr, times v0; at dr = 0 the reference divides 0 by 0
-        double g = in1 ? -sc.va_g1 : 0.0;
-        if (in2) g = ddiv(dmul(sc.va_g2, __fma_rn(-2.0, dr, sc.va_xr)), dr);
-        if (dr == 0.0) g = __longlong_as_double(0x7ff8000000000000ll);
-        const double fc = dmul(f, cp);
-        r.a0 = dsub(r.a0, fc);
-        const double q = __fma_rn(__fma_rn(ex, dx, dmul(ey, dy)), g, dmul(-sc.va_2D, f));
-        r.a1 = __fma_rn(q, sp, r.a1);
-        r.a1 = __fma_rn(dsub(a.dphi_s[j], ddi), fc, r.a1);
-      }
-      if (coh) {
+      // the strength's derivative over dr, times v0; at dr = 0 the reference divides 0 by 0
+      double gr = in1 ? -sc.va_g1 : 0.0;
+      if (in2) gr = ddiv(dmul(sc.va_g2, __fma_rn(-2.0, dr, sc.va_xr)), dr);
+      if (dr == 0.0) gr = __longlong_as_double(0x7ff8000000000000ll);
+      const double q = __fma_rn(__fma_rn(ex, dx, dmul(ey, dy)), gr, dmul(-sc.va_2D, f));
+      t.x = dmul(f, cp);
+      t.y = __fma_rn(dsub(a.dphi_s[j], ddi), t.x, dmul(q, sp));
+      if (t.coh) {
         double s, c;
         va_bearing_sincos(dx, dy, dr, ci, phii, s, c);
-        r.b0 = __fma_rn(sc.kappa, c, r.b0);
         const double turn = ddiv(dmul(sc.v0, __fma_rn(ey, dx, -dmul(ex, dy))), dr2);
-        r.b1 = __fma_rn(dmul(-sc.kappa, dsub(turn, ddi)), c, r.b1);
-        r.b1 = __fma_rn(dmul(sc.kappa, sc.D), s, r.b1);
+        t.u = dmul(sc.kappa, c);
+        t.v = __fma_rn(dmul(-sc.kappa, dsub(turn, ddi)), c, dmul(dmul(sc.kappa, sc.D), s));
+      }
+    }
+    return t;
+  };
+  auto add = [&](bool term, bool coh, double x, double y, double u, double v) {
+    if constexpr (KIND == kKindSin) {
+      if (term) {
+        r.align = dadd(r.align, x);
+        ++r.c01;
+      }
+      if (coh) {
+        r.coh = dadd(r.coh, u);
+        ++r.c2;
+      }
+    } else {
+      if (term) {
+        r.a0 = dsub(r.a0, x);
+        r.a1 = dadd(r.a1, y);
+      }
+      if (coh) {
+        r.b0 = dadd(r.b0, u);
+        r.b1 = dadd(r.b1, v);
       }
     }
   };
 
-  int nw = 0;
-  auto walk = [&]() {
+  int nw = 0;         // words listed
+  bool full = false;  // G > 1: the row has more words than the list
+  auto walk = [&]() {  // this lane's words, in order
     uint32_t bits = 0u;
     int slot = 0;
     for (int w = 0;;) {
@@ -261,7 +289,8 @@ __global__ void __launch_bounds__(kLaneThreads) k_va_pass(KArgs a, int epi) {
       }
       const int t = __clz(bits);
       bits ^= 0x80000000u >> t;
-      pair(slot + t);
+      const VATerm v = term_of(slot + t, true);
+      add(v.term, v.coh, v.x, v.y, v.u, v.v);
     }
     nw = 0;
   };
@@ -277,35 +306,94 @@ __global__ void __launch_bounds__(kLaneThreads) k_va_pass(KArgs a, int epi) {
   const LaneRuns rn = lane_runs(cx, nc);
   const float2 fi = ap ? make_float2(0.0f, 0.0f) : a.fxy[p];
   const float xa = fi.x - (float)rn.sa * sc.cell_f, xb = fi.x - (float)rn.sb * sc.cell_f;
-  for (int k = ap ? 2 : 0; k < 3; ++k) {
-    const float y = fi.y - (float)(k - 1) * sc.cell_f;
-    const int *row = a.cell_start + sd.c0 + (ap ? 0 : adjust_cell(cy + k - 1, nc) * nc);
+  // rows [k0, k1) of the stencil, or thirds of an all-pairs system; flush: walk
+  // the list when it is full
+  auto rows = [&](int k0, int k1, bool flush) {
 #pragma unroll 1
-    for (int run = 0; run < (ap ? 1 : 2); ++run) {
-      const int j0 = ap ? row[0] : row[run ? rn.b0 : rn.a0], j1 = ap ? row[1] : row[run ? rn.b1 : rn.a1];
-      const float x = run ? xb : xa;
-      for (int base = j0; base < j1; base += kWarp) {
-        const int cnt = min(kWarp, j1 - base);
-        uint32_t bits = 0xffffffffu;
-        if (!ap) {
-          // sign of d^2 - va_r2 (rounded outwards): beyond rho and xi_r for certain when clear
-          int done = 0;
-          for (; done < cnt; done += 4) {
-            const float2 *f = a.fxy + base + done;
+    for (int k = k0; k < k1; ++k) {
+      const float y = fi.y - (float)(k - 1) * sc.cell_f;
+      const int *row = a.cell_start + sd.c0 + (ap ? 0 : adjust_cell(cy + k - 1, nc) * nc);
+#pragma unroll 1
+      for (int run = 0; run < (ap ? 1 : 2); ++run) {
+        int j0, j1;
+        if (ap) {
+          const long long m = row[1] - row[0];
+          j0 = row[0] + (int)(m * k / 3);
+          j1 = row[0] + (int)(m * (k + 1) / 3);
+        } else {
+          j0 = row[run ? rn.b0 : rn.a0];
+          j1 = row[run ? rn.b1 : rn.a1];
+        }
+        const float x = run ? xb : xa;
+        for (int base = j0; base < j1; base += kWarp) {
+          const int cnt = min(kWarp, j1 - base);
+          uint32_t bits = 0xffffffffu;
+          if (!ap) {
+            // sign of d^2 - va_r2 (rounded outwards): beyond rho and xi_r for certain when clear
+            int done = 0;
+            for (; done < cnt; done += 4) {
+              const float2 *f = a.fxy + base + done;
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              const float2 d = add2(f[u], make_float2(-x, -y));
-              bits = __funnelshift_l(__float_as_uint(cutoff_offset(d.x, d.y, -sc.va_r2)), bits, 1);
+              for (int u = 0; u < 4; ++u) {
+                const float2 d = add2(f[u], make_float2(-x, -y));
+                bits = __funnelshift_l(__float_as_uint(cutoff_offset(d.x, d.y, -sc.va_r2)), bits, 1);
+              }
+            }
+            bits <<= kWarp - done;
+          }
+          put(bits & first_bits(cnt), base);
+          if (nw == kLaneWords) {
+            if (flush) {
+              walk();
+            } else {
+              full = true;
+              return;
             }
           }
-          bits <<= kWarp - done;
         }
-        put(bits & first_bits(cnt), base);
-        if (nw == kLaneWords) walk();
       }
     }
+  };
+
+  if constexpr (G == 1) {
+    rows(0, 3, true);
+    walk();
+  } else {
+    constexpr unsigned kAll = 0xffffffffu;
+    if (g < 3) rows(g, g + 1, false);
+    __syncwarp();
+    const bool alone = ((__ballot_sync(kAll, full) >> lead) & ((1u << G) - 1u)) != 0u;  // a very long row
+    GroupWords words(nw, lead, alone);
+    uint32_t bits = 0u;
+    int slot = 0;
+    while (true) {
+      words.next(s_bits, s_slot, tid - g, bits, slot);
+      const int m = __popc(bits);
+      if (!__any_sync(kAll, m > 0)) break;
+      const int j = group_pick(bits, slot, g, m, p);
+      const VATerm t = term_of(j, g < m);
+      __syncwarp();
+      const unsigned terms = __ballot_sync(kAll, t.term) >> lead, all_cohs = __ballot_sync(kAll, t.coh);
+      const unsigned cohs = all_cohs >> lead;
+#pragma unroll
+      for (int u = 0; u < G; ++u) {
+        const double x = __shfl_sync(kAll, t.x, lead + u);
+        const double y = KIND == kKindCos2 ? __shfl_sync(kAll, t.y, lead + u) : 0.0;
+        double cu = 0.0, cv = 0.0;
+        if (all_cohs != 0u) {  // the same for the whole warp
+          cu = __shfl_sync(kAll, t.u, lead + u);
+          if constexpr (KIND == kKindCos2) cv = __shfl_sync(kAll, t.v, lead + u);
+        }
+        add((terms >> u) & 1u, (cohs >> u) & 1u, x, y, cu, cv);
+      }
+    }
+    if (g != 0 || p_own >= a.va_p1) return;
+    if (alone) {  // the first lane walks as it tests
+      nw = 0;
+      rows(0, 3, true);
+      walk();
+    }
   }
-  walk();
   va_epilogue<KIND>(a, epi, sd, p, a.pidx[p], ci, r);
 }
 
