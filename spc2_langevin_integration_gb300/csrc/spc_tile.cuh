@@ -714,30 +714,29 @@ struct TileRedX {
 
 // One block of 32 staged candidates against one particle (FP32X): the float
 // test, the fixed-point sums of the inside candidates, their bits, and the
-// smallest |d^2 - mid| for the undecided check (as block32).
+// smallest offset pattern for the undecided check (as test32).  Packed
+// subtraction and predicates taken from the offset's sign: vortex N = 65,536
+// clustered, cell units, pass 1 with its epilogue 79 -> 72 us.  (The FP32C block
+// gains nothing from them: 41 against 43 us.)
 template <bool SELF>
-__device__ __forceinline__ void block32x(const float2 *__restrict__ s_xy, const longlong2 *__restrict__ s_v,
-                                         int j0, int self, float fxi, float fyi, float nmid, float nband,
-                                         long long &C, long long &S, uint32_t &bits, float &mn) {
+__device__ __forceinline__ void block32x(const float2 *__restrict__ s_xy, const longlong2 *__restrict__ s_v, int j0,
+                                         int self, float2 nxy, float nlo, long long &C, long long &S, uint32_t &bits,
+                                         uint32_t &um) {
+  uint32_t b = 0u;
 #pragma unroll
   for (int t = 0; t < kWarp; ++t) {
-    const float2 cj = s_xy[j0 + t];
-    const float dx = cj.x - fxi, dy = cj.y - fyi;
-    float off = cutoff_offset(dx, dy, nmid);
-    bool in = off < nband;
-    if (SELF) {
-      in = in && (j0 + t != self);
-      off = (j0 + t != self) ? off : 3.0e38f;
-    }
-    mn = fminf(mn, fabsf(off));
-    add2_if(C, S, s_v[j0 + t], in);
-    bits |= (uint32_t)in << t;
+    const float2 d = add2(s_xy[j0 + t], nxy);
+    uint32_t o = __float_as_uint(cutoff_offset(d.x, d.y, nlo));
+    if (SELF) o = (j0 + t != self) ? o : 0x7f000000u;
+    um = min(um, o);
+    add2_if_neg(C, S, s_v[j0 + t], o);
+    b = __funnelshift_l(o, b, 1);
   }
+  bits = __brev(b);
 }
 
 // Stage candidates [rlo, rlo + rcnt) of the stencil list (padded to rpad) for
-// the FP32X passes (with part_fp32x, for the units kernel; the cell-tile
-// kernel keeps the same code inline, as stage_fp32c says).
+// the FP32X passes.
 template <int KIND>
 __device__ __forceinline__ void stage_fp32x(const KArgs &a, const SysConst &sc, const Stencil &st, int rlo,
                                             int rcnt, int rpad, float2 *s_xy, longlong2 *s_v) {
@@ -762,7 +761,7 @@ template <int KIND>
 __device__ __forceinline__ void part_fp32x(const KArgs &a, const SysConst &sc, const Stencil &st,
                                            const float2 *s_xy, const longlong2 *s_v, TileRedX &red, int c0,
                                            int ig, int li, int gi, int rlo, int rcnt, int jlo, int jhi,
-                                           int part, bool masked, bool exact_all, float band, float nmid) {
+                                           int part, bool masked, bool exact_all, float nlo, float wid) {
   const int n_all = a.n_active;
   const bool valid = li < gi;
   const int p = ig + li;
@@ -775,6 +774,7 @@ __device__ __forceinline__ void part_fp32x(const KArgs &a, const SysConst &sc, c
     xi = a.sx[p];
     yi = a.sy[p];
   }
+  const float2 nxy = make_float2(-fxi, -fyi);
   const int self = st.prefix[4] + (p - c0) - rlo;
   long long C = 0, Sn = 0;
   int n = 0;
@@ -807,25 +807,24 @@ __device__ __forceinline__ void part_fp32x(const KArgs &a, const SysConst &sc, c
     }
   } else {
     for (int j0 = jlo; j0 < jhi; j0 += kWarp) {
-      float mn = 3.0e38f;
-      uint32_t bits = 0u;
+      uint32_t bits = 0u, um = 0xffffffffu;
       const bool self_block = (unsigned)(self - j0) < (unsigned)kWarp;
       if (!exact_all) {
         if (__any_sync(0xffffffffu, self_block))
-          block32x<true>(s_xy, s_v, j0, self, fxi, fyi, nmid, -band, C, Sn, bits, mn);
+          block32x<true>(s_xy, s_v, j0, self, nxy, nlo, C, Sn, bits, um);
         else
-          block32x<false>(s_xy, s_v, j0, self, fxi, fyi, nmid, -band, C, Sn, bits, mn);
+          block32x<false>(s_xy, s_v, j0, self, nxy, nlo, C, Sn, bits, um);
       }
       // pairs the float test cannot decide: the reference's FP64 test
-      const bool amb = valid && (exact_all || mn <= band);
+      const bool amb = valid && (exact_all || um <= __float_as_uint(wid));
       if (__any_sync(0xffffffffu, amb)) {
         if (amb) {
           for (int t = 0; t < kWarp; ++t) {
             const int j = j0 + t;
             if (j == self || j >= rcnt) continue;
-            const float2 cj = s_xy[j];
-            const float dx = cj.x - fxi, dy = cj.y - fyi;
-            if (!(exact_all || fabsf(cutoff_offset(dx, dy, nmid)) <= band)) continue;
+            const float2 d = add2(s_xy[j], nxy);
+            const float off = cutoff_offset(d.x, d.y, nlo);
+            if (!(exact_all || (off >= 0.0f && off <= wid))) continue;
             int q;
             const int pj = slot_of(st, rlo + j, q);
             if (!exact_within(sc, xi, yi, a.sx[pj], a.sy[pj])) continue;
@@ -847,14 +846,12 @@ __device__ __forceinline__ void part_fp32x(const KArgs &a, const SysConst &sc, c
   }
 }
 
-// UNITS: unit cells are left to the units kernel (a separate instantiation, so
-// that the kernel without cell units compiles exactly as before).
+// UNITS: unit cells are left to the units kernel.
 template <int KIND, bool UNITS>
 __global__ void __launch_bounds__(kTileThreads32, kTileMinBlocks32) k_tile_fp32x(KArgs a, int epi) {
-  __shared__ float2 s_xy[kTileCapX];     // x+shift, y+shift (padded to 32)
-  __shared__ longlong2 s_v[kTileCapX];   // pass 1: ics, pass 2: iws of the candidate
+  __shared__ float2 s_xy[kTileCapX];  // x+shift, y+shift (padded to 32)
+  __shared__ longlong2 s_v[kTileCapX];          // pass 1: ics, pass 2: iws of the candidate
   __shared__ TileRedX red;
-  const int n_all = a.n_active;
   const int tid = threadIdx.x, w = tid / kWarp, lane = tid % kWarp;
   const int nitems = tile_items(a);
   for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
@@ -867,8 +864,7 @@ __global__ void __launch_bounds__(kTileThreads32, kTileMinBlocks32) k_tile_fp32x
     const SysDesc &sd = a.sys[a.sys_of_c[c]];
     const SysConst &sc = sd.sc;
     if (sc.allpairs) continue;
-    const float lo2 = sc.lo2, hi2 = sc.hi2;
-    const float band = 0.5f * (hi2 - lo2), nmid = -0.5f * (hi2 + lo2);
+    const float nlo = -sc.lo2, wid = undecided_width(sc.lo2, sc.hi2);
     const bool exact_all = sc.exact_all != 0;
     Stencil st;
     stencil_of(a, sd, c, st);
@@ -885,108 +881,16 @@ __global__ void __launch_bounds__(kTileThreads32, kTileMinBlocks32) k_tile_fp32x
         const int rpad = (rcnt + kWarp - 1) & ~(kWarp - 1);
         if (rounds > 1 || ig == cb) {
           __syncthreads();
-          for (int k = tid; k < rpad; k += blockDim.x) {
-            if (k < rcnt) {
-              int q;
-              const int pj = slot_of(st, rlo + k, q);
-              const float2 f = a.fxy[pj];
-              s_xy[k] = make_float2(f.x + shift_x(q, sc.cell_f), f.y + shift_y(q, sc.cell_f));
-              s_v[k] = KIND == kKindSin ? a.ics[pj] : a.iws[pj];
-            } else {  // padding: far away, never a neighbour, never near the cutoff
-              s_xy[k] = make_float2(3.0e18f, 3.0e18f);
-              s_v[k] = make_longlong2(0, 0);
-            }
-          }
+          stage_fp32x<KIND>(a, sc, st, rlo, rcnt, rpad, s_xy, s_v);
           __syncthreads();
         }
         const int chunks = (gi + kWarp - 1) / kWarp;
         const int S = chunks >= 4 ? 1 : (chunks == 1 ? 4 : 2);
-        const int items = chunks * S;
-        for (int item = w; item < items; item += kTileThreads32 / kWarp) {
+        for (int item = w; item < chunks * S; item += kTileThreads32 / kWarp) {
           const int chunk = item / S, part = item % S;
-          const int li = chunk * kWarp + lane;
-          const bool valid = li < gi;
-          const int p = ig + li;
-          float fxi = 3.0e30f, fyi = 3.0e30f;
-          double xi = 0.0, yi = 0.0;
-          if (valid) {
-            const float2 f = a.fxy[p];
-            fxi = f.x;
-            fyi = f.y;
-            xi = a.sx[p];
-            yi = a.sy[p];
-          }
-          const int self = st.prefix[4] + (p - c0) - rlo;
-          const int jlo = split_point(rpad, part, S), jhi = split_point(rpad, part + 1, S);
-          long long C = 0, Sn = 0;
-          int n = 0;
-          if (KIND == kKindCos2 && masked) {
-            // pass 2 over the neighbour bitmask of pass 1 (same staged list)
-            const uint4 *m4 = reinterpret_cast<const uint4 *>(a.nbmask);
-            const uint4 none = make_uint4(0u, 0u, 0u, 0u);
-            const int w0 = jlo / kWarp, w1 = jhi / kWarp;
-            int g = w0 >> 2;
-            uint4 cur = (valid && w0 < w1) ? m4[(size_t)g * n_all + p] : none;
-            uint4 nxt = (valid && ((g + 1) << 2) < w1) ? m4[(size_t)(g + 1) * n_all + p] : none;
-            for (int j0 = jlo; j0 < jhi; j0 += kWarp) {
-              const int wd = j0 / kWarp;
-              if ((wd >> 2) != g) {
-                ++g;
-                cur = nxt;
-                nxt = (valid && ((g + 1) << 2) < w1) ? m4[(size_t)(g + 1) * n_all + p] : none;
-              }
-              const int sub = wd & 3;
-              const uint32_t bits = sub == 0 ? cur.x : sub == 1 ? cur.y : sub == 2 ? cur.z : cur.w;
-#pragma unroll
-              for (int t = 0; t < kWarp; ++t) {
-                if ((bits >> t) & 1u) {
-                  const longlong2 v = s_v[j0 + t];
-                  C += v.x;
-                  Sn += v.y;
-                }
-              }
-              n += __popc(bits);
-            }
-          } else {
-            for (int j0 = jlo; j0 < jhi; j0 += kWarp) {
-              float mn = 3.0e38f;
-              uint32_t bits = 0u;
-              const bool self_block = (unsigned)(self - j0) < (unsigned)kWarp;
-              if (!exact_all) {
-                if (__any_sync(0xffffffffu, self_block))
-                  block32x<true>(s_xy, s_v, j0, self, fxi, fyi, nmid, -band, C, Sn, bits, mn);
-                else
-                  block32x<false>(s_xy, s_v, j0, self, fxi, fyi, nmid, -band, C, Sn, bits, mn);
-              }
-              // pairs the float test cannot decide: the reference's FP64 test
-              const bool amb = valid && (exact_all || mn <= band);
-              if (__any_sync(0xffffffffu, amb)) {
-                if (amb) {
-                  for (int t = 0; t < kWarp; ++t) {
-                    const int j = j0 + t;
-                    if (j == self || j >= rcnt) continue;
-                    const float2 cj = s_xy[j];
-                    const float dx = cj.x - fxi, dy = cj.y - fyi;
-                    if (!(exact_all || fabsf(cutoff_offset(dx, dy, nmid)) <= band)) continue;
-                    int q;
-                    const int pj = slot_of(st, rlo + j, q);
-                    if (!exact_within(sc, xi, yi, a.sx[pj], a.sy[pj])) continue;
-                    const longlong2 v = s_v[j];
-                    C += v.x;
-                    Sn += v.y;
-                    bits |= 1u << t;
-                  }
-                }
-              }
-              n += __popc(bits);
-              if (KIND == kKindSin && masked && valid) a.nbmask[mask_at(j0 / kWarp, p, n_all)] = bits;
-            }
-          }
-          if (valid) {
-            red.c[part][li] = C;
-            red.s[part][li] = Sn;
-            red.n[part][li] = n;
-          }
+          part_fp32x<KIND>(a, sc, st, s_xy, s_v, red, c0, ig, chunk * kWarp + lane, gi, rlo, rcnt,
+                           split_point(rpad, part, S), split_point(rpad, part + 1, S), part, masked, exact_all, nlo,
+                           wid);
         }
         __syncthreads();
         if (tid < gi) {
@@ -1029,8 +933,7 @@ __global__ void __launch_bounds__(kTileThreads32, kTileMinBlocks32) k_units_fp32
     const int g1 = half == 0 ? a.cell_mid[c] : a.cell_start[c + 1];
     const SysDesc &sd = a.sys[a.sys_of_c[c]];
     const SysConst &sc = sd.sc;
-    const float lo2 = sc.lo2, hi2 = sc.hi2;
-    const float band = 0.5f * (hi2 - lo2), nmid = -0.5f * (hi2 + lo2);
+    const float nlo = -sc.lo2, wid = undecided_width(sc.lo2, sc.hi2);
     const bool exact_all = sc.exact_all != 0;
     const int qv = KIND == kKindSin ? kXQ : sc.xq2;
     Stencil st;
@@ -1046,7 +949,7 @@ __global__ void __launch_bounds__(kTileThreads32, kTileMinBlocks32) k_units_fp32
     stage_fp32x<KIND>(a, sc, st, rlo, rcnt, rpad, s_xy, s_v);
     __syncthreads();
     part_fp32x<KIND>(a, sc, st, s_xy, s_v, red, c0, ig, lane, gi, rlo, rcnt, split_point(rpad, w, 4),
-                     split_point(rpad, w + 1, 4), w, masked, exact_all, band, nmid);
+                     split_point(rpad, w + 1, 4), w, masked, exact_all, nlo, wid);
     __syncthreads();
     long long uc = 0, us = 0;
     int un = 0;
