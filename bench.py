@@ -55,13 +55,13 @@ ALG_BYTES_STEP = 168 + 8      # survey accounting for the whole SRK step (+ omeg
 PHASE_KERNELS = {
     "fp32c": {"stage": ["k_stage"], "sort": ["k_scan_digits", "k_radix_scatter"],
               "gather": ["k_gather<1>", "k_list_units (cell units on)"],
-              "pass1": ["k_tile_fp32c<0>", "k_units_fp32c<0> (cell units on)", "k_lane<1, 0>"],
-              "pass2": ["k_tile_fp32c<1>", "k_units_fp32c<1> (cell units on)", "k_lane<1, 1>"]},
+              "pass1": ["k_tile_float<1, 0>", "k_units_float<1, 0> (cell units on)", "k_lane<1, 0>"],
+              "pass2": ["k_tile_float<1, 1>", "k_units_float<1, 1> (cell units on)", "k_lane<1, 1>"]},
     "fp32x": {"stage": ["k_stage"], "sort": ["k_scan_digits", "k_radix_scatter"],
               "gather": ["k_gather<2>", "k_list_units (cell units on)"],
-              "pass1": ["k_tile_fp32x<0>", "k_units_fp32x<0> (cell units on)", "k_lane<2, 0>",
+              "pass1": ["k_tile_float<2, 0>", "k_units_float<2, 0> (cell units on)", "k_lane<2, 0>",
                         "k_epilogue_fp32x<0>"],
-              "pass2": ["k_tile_fp32x<1>", "k_units_fp32x<1> (cell units on)", "k_lane<2, 1>",
+              "pass2": ["k_tile_float<2, 1>", "k_units_float<2, 1> (cell units on)", "k_lane<2, 1>",
                         "k_epilogue_fp32x<1>"]},
     "fp64": {"stage": ["k_stage"], "sort": ["k_scan_digits", "k_radix_scatter"],
              "gather": ["k_gather<0>", "k_vgather<0>"], "pass1": ["k_vtile<0,0>", "k_tile_fp64<0>"],

@@ -1104,11 +1104,11 @@ constexpr size_t kNaCount = 4ull * (kNoAllocMaxCells + kScanChunk + (kSpreadKeys
 constexpr size_t kNaStage = na_round(sizeof(StageRec) * kNoAllocMaxN);
 constexpr size_t kNaSys = na_round(sizeof(SysDesc));
 // x y phi omega | sx sy sphi | dphi_s                         (8 double arrays)
-// keys arrival list skeys pidx cnt_s dphi_f sys_of_p          (8 32-bit arrays)
-// fxy cs (2 float2 arrays) | dcs (double2) | stage records | cell_start | sys_of_c | counts | chunk sums |
+// keys arrival list skeys pidx cnt_s dphi_f scos_f sys_of_p   (9 32-bit arrays)
+// fxy cs (2 float2 arrays) | dcs (double2), dig, wdig (16 bytes each) | stage records | cell_start | sys_of_c | counts | chunk sums |
 // system table | all-pairs cell | clamp counter
 constexpr size_t kNoAllocBytes =
-    8 * kNaD + 8 * kNaF + 2 * kNaF2 + 2 * kNaD + kNaStage + 2 * kNaCells + kNaCount + 256 + kNaSys + 256 + 256;
+    8 * kNaD + 9 * kNaF + 2 * kNaF2 + 6 * kNaD + kNaStage + 2 * kNaCells + kNaCount + 256 + kNaSys + 256 + 256;
 
 constexpr int kNoAllocMaxDevices = 64;
 std::mutex g_noalloc_mu;
@@ -1240,10 +1240,13 @@ extern "C" int spc_rhs_srk_noalloc(const spc_params *p, int32_t n, const double 
   a.pidx = (int *)take(kNaF);
   a.cnt_s = (int *)take(kNaF);
   a.dphi_f = (float *)take(kNaF);
+  a.scos_f = (float *)take(kNaF);
   int *sys_of_p = (int *)take(kNaF);
   a.fxy = (float2 *)take(kNaF2);
   a.cs = (float2 *)take(kNaF2);
   a.dcs = (double2 *)take(2 * kNaD);
+  a.dig = (uint4 *)take(2 * kNaD);
+  a.wdig = (uint4 *)take(2 * kNaD);
   a.cell_start = (int *)take(kNaCells);
   int *sys_of_c = (int *)take(kNaCells);
   a.stg = (StageRec *)take(kNaStage);
@@ -1269,6 +1272,7 @@ extern "C" int spc_rhs_srk_noalloc(const spc_params *p, int32_t n, const double 
   a.n_active = n;
   a.ncell_total = ncell;
   a.ncell_tile = sc.allpairs ? 0 : ncell;  // cell-tile kernels only
+  a.lane_p0 = a.lane_p1 = a.va_p1 = sc.allpairs ? 0 : n;
   e.ncell_tile = a.ncell_tile;
   e.ncell_warp = 0;
   a.n_ap = sc.allpairs ? 1 : 0;

@@ -69,13 +69,6 @@ __device__ __forceinline__ void add2_if(long long &c, long long &s, longlong2 v,
       : "+l"(c), "+l"(s)
       : "l"(v.x), "l"(v.y), "r"((int)p));
 }
-// the same when the sign bit of a float offset's pattern is set: the predicate
-// is formed in one instruction
-__device__ __forceinline__ void add2_if_neg(long long &c, long long &s, longlong2 v, uint32_t o) {
-  asm("{\n\t.reg .pred q;\n\tsetp.lt.s32 q, %4, 0;\n\t@q add.s64 %0, %0, %2;\n\t@q add.s64 %1, %1, %3;\n\t}"
-      : "+l"(c), "+l"(s)
-      : "l"(v.x), "l"(v.y), "r"(o));
-}
 // the same for float sums: c += x, s += y when p (each rounded to nearest,
 // as the plain adds)
 __device__ __forceinline__ void addf2_if(float &c, float &s, float x, float y, bool p) {

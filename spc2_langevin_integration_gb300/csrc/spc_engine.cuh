@@ -28,6 +28,7 @@
 #include "spc_kernels.cuh"
 #include "spc_sort.cuh"
 #include "spc_tile.cuh"
+#include "spc_ftile.cuh"
 #include "spc_lane.cuh"
 #include "spc_verlet.cuh"
 #include "spc_va.cuh"
@@ -356,11 +357,11 @@ inline void engine_footprint(int stepper, int precision, long long *per_particle
   long long b = 4 * 8;                       // x, y, phi, omega
   if (stepper == SPC_STEPPER_RK4) b += 12 * 8;  // k1..k4
   b += 32 + 4 * 4 + 3 * 8 + 8 + 4 + 8 + 4 + 4;  // stage, sort, cell order, fxy, pidx, dphi, cnt, sys_of_p
-  if (precision == SPC_PRECISION_FP32C) b += 8 + 4 + (long long)kMaskWords * 4;  // cs, dphi_f, masks
+  if (precision == SPC_PRECISION_FP32C) b += 8 + 4 + 16 + 16 + 4 + (long long)kMaskWords * 4;  // cs, dphi_f, digits, scos_f, masks
   if (precision == SPC_PRECISION_FP32X)
-    b += 16 + 16 + 8 + 16 + 4 + (long long)kMaskWords * 4;  // ics, iws, scos, xsum, xcnt, masks
+    b += 16 + 16 + 32 + 32 + 8 + 16 + 4 + (long long)kMaskWords * 4;  // ics, iws, digits, scos, xsum, xcnt, masks
   if (precision != SPC_PRECISION_FP64)  // cell units: round sums, counts, chunk counters, list
-    b += kSplitRounds * ((precision == SPC_PRECISION_FP32X ? 16 : 8) + 4) + 4 + kSplitRounds * 8 / 32;
+    b += kSplitRounds * (16 + 4) + 4 + kSplitRounds * 8 / 32;
   if (precision == SPC_PRECISION_FP64) b += 4;                                  // vortex-arrays partner counts
   if (precision != SPC_PRECISION_FP32C) b += 16;                                // dcs
   if (precision == SPC_PRECISION_FP64 && stepper == SPC_STEPPER_SRK) b += (long long)kMaskWords * 4;  // masks
@@ -417,7 +418,9 @@ inline int engine_init(Engine *e, int stepper, int precision, int pool_cap, int 
     SPC_TRY(dalloc(e, &a.cs, N));
     SPC_TRY(dalloc(e, &a.dphi_f, N));
     SPC_TRY(dalloc(e, &a.nbmask, (size_t)kMaskWords * N));
-    SPC_TRY(dalloc(e, &a.part_f, (size_t)kSplitRounds * N));
+    SPC_TRY(dalloc(e, &a.dig, N));
+    SPC_TRY(dalloc(e, &a.wdig, N));
+    SPC_TRY(dalloc(e, &a.scos_f, N));
   }
   if (precision == SPC_PRECISION_FP32X) {
     SPC_TRY(dalloc(e, &a.ics, N));
@@ -426,7 +429,8 @@ inline int engine_init(Engine *e, int stepper, int precision, int pool_cap, int 
     SPC_TRY(dalloc(e, &a.xsum, N));
     SPC_TRY(dalloc(e, &a.xcnt, N));
     SPC_TRY(dalloc(e, &a.nbmask, (size_t)kMaskWords * N));
-    SPC_TRY(dalloc(e, &a.part_x, (size_t)kSplitRounds * N));
+    SPC_TRY(dalloc(e, &a.dig, 2 * N));
+    SPC_TRY(dalloc(e, &a.wdig, 2 * N));
   }
   if (precision != SPC_PRECISION_FP64) {
     // a unit cell of n_c particles lists ceil(n_c / 32) x (at most
@@ -438,6 +442,7 @@ inline int engine_init(Engine *e, int stepper, int precision, int pool_cap, int 
     SPC_TRY(dalloc(e, &e->cell_near_buf, (size_t)cell_cap));
     SPC_TRY(dalloc(e, &a.unit_count, 1));
     SPC_TRY(dalloc(e, &a.cell_unit, (size_t)cell_cap));
+    SPC_TRY(dalloc(e, &a.part_x, (size_t)kSplitRounds * N));
     SPC_TRY(dalloc(e, &a.part_n, (size_t)kSplitRounds * N));
     SPC_TRY(dalloc(e, &a.unit_done, N));
     SPC_CUDA(e, cudaStreamCreateWithFlags(&e->side, cudaStreamNonBlocking));
@@ -947,24 +952,16 @@ int launch_pass_t(Engine *e, const KArgs &a, int epi) {
             // against 3, 4, 6, 7 and 10 per SM, the most units in flight won.
             SPC_CUDA(e, cudaEventRecord(e->fork_ev, st));
             SPC_CUDA(e, cudaStreamWaitEvent(e->side, e->fork_ev, 0));
-            if constexpr (PREC == kPrecFP32C)
-              k_units_fp32c<KIND><<<152 * 16, kTileThreads32, 0, e->side>>>(a, epi);
-            else
-              k_units_fp32x<KIND><<<152 * 16, kTileThreads32, 0, e->side>>>(a, epi);
+            k_units_float<PREC, KIND><<<152 * 16, kTileThreads32, 0, e->side>>>(a, epi);
             SPC_LAUNCHED(e);
             SPC_CUDA(e, cudaEventRecord(e->join_ev, e->side));
           }
         }
-        if constexpr (PREC == kPrecFP32C) {
+        if constexpr ((PREC == kPrecFP32C || PREC == kPrecFP32X) && KIND != kKindNb) {
           if (a.units)
-            k_tile_fp32c<KIND, true><<<grid, kTileThreads32, 0, st>>>(a, epi);
+            k_tile_float<PREC, KIND, true><<<grid, kTileThreads32, 0, st>>>(a, epi);
           else
-            k_tile_fp32c<KIND, false><<<grid, kTileThreads32, 0, st>>>(a, epi);
-        } else if constexpr (PREC == kPrecFP32X) {
-          if (a.units)
-            k_tile_fp32x<KIND, true><<<grid, kTileThreads32, 0, st>>>(a, epi);
-          else
-            k_tile_fp32x<KIND, false><<<grid, kTileThreads32, 0, st>>>(a, epi);
+            k_tile_float<PREC, KIND, false><<<grid, kTileThreads32, 0, st>>>(a, epi);
         } else
           k_tile_fp64<KIND><<<grid, kTileThreads64, 0, st>>>(a, epi);
         SPC_LAUNCHED(e);

@@ -24,6 +24,8 @@
 // the same kernels.
 #pragma once
 
+#include <cuda_fp16.h>
+
 #include "spc_device.cuh"
 #include "spc_sort.cuh"
 
@@ -108,6 +110,11 @@ struct KArgs {
   float2 *cs;                        // FP32C: (cos phi, sin phi)
   double2 *dcs;                      // FP64 passes: (cos phi, sin phi) of the stage phase
   longlong2 *ics;                    // FP32X: (cos phi, sin phi) in fixed point (2^kXQ)
+  // float forms, cell-tile slots: the values of the two passes as digits in
+  // halves, 16 bytes (FP32X: 32) a slot (float_digits, fixed_digits); FP32C SRK:
+  // pass-1 sum_j cos(phi_j - phi_i - alpha)
+  uint4 *dig, *wdig;
+  float *scos_f;
   longlong2 *iws;                    // FP32X SRK: phase rate times (cos phi, sin phi), fixed point (2^xq2)
   double *scos;                      // FP32X SRK: pass-1 sum_j cos(phi_j - phi_i - alpha), cell order
   double2 *xsum;                     // FP32X: a pass's exact neighbour sums (c, s), cell order
@@ -121,13 +128,12 @@ struct KArgs {
   // Cell units of the float cell-tile passes (SPC_TUNE_CELL_UNITS; units
   // null when off): the units k_list_units lists for the units kernel
   // (cell, unit), their count (zeroed by k_gather), per staging
-  // round r and cell-order slot p at [r * n_active + p] a unit's sums (FP32C:
-  // float pair, FP32X: fixed-point pair) and counts, and a completion counter
+  // round r and cell-order slot p at [r * n_active + p] a unit's sums (fixed-point
+  // pair) and counts, and a completion counter
   // per 32-particle chunk, indexed by its first slot (zero between launches).
   int2 *units;
   int *unit_count;
   uint8_t *cell_unit;  // per cell-tile cell: 1 if it runs as units (written with the list)
-  float2 *part_f;
   longlong2 *part_x;
   int *part_n;
   int *unit_done;
@@ -249,6 +255,41 @@ __device__ __forceinline__ int block_first(int cx, int nc) {
   return min(cx >> 4, max((nc >> 4) - 1, 0)) << 4;
 }
 
+// A candidate's record for the float cell-tile passes (spc_ftile.cuh): signed
+// digits, each exact in a half, whose sums the tensor cores keep exact.
+// FP32C: three digits in base 4096 each of x and y (|x|, |y| <= 1 up to float
+// rounding; units of 2^-35), 1, and 1 if either is not finite.
+__device__ __forceinline__ uint32_t halves(float lo, float hi) {
+  const __half2 h = __floats2half2_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t *>(&h);
+}
+__device__ __forceinline__ uint4 float_digits(float x, float y) {
+  const bool bad = !(fabsf(x) < 1.5f && fabsf(y) < 1.5f);
+  if (bad) x = y = 0.0f;
+  const float x2 = rintf(x * 2048.0f), rx = fmaf(x, 2048.0f, -x2) * 4096.0f, x1 = rintf(rx);
+  const float y2 = rintf(y * 2048.0f), ry = fmaf(y, 2048.0f, -y2) * 4096.0f, y1 = rintf(ry);
+  return make_uint4(halves(x2, x1), halves(rintf((rx - x1) * 4096.0f), y2),
+                    halves(y1, rintf((ry - y1) * 4096.0f)), halves(1.0f, bad ? 1.0f : 0.0f));
+}
+// FP32X: five digits in base 2048 each of x and y (|x|, |y| < 2^54), lowest
+// first, 1, zeros.
+__device__ __forceinline__ void fixed_digits(longlong2 v, uint4 *to) {
+  float d[10];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    long long r = h ? v.y : v.x;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int low = (int)((uint32_t)r << 21) >> 21;
+      d[5 * h + k] = (float)low;
+      r = (r - low) >> 11;
+    }
+    d[5 * h + 4] = (float)(int)r;
+  }
+  to[0] = make_uint4(halves(d[0], d[1]), halves(d[2], d[3]), halves(d[4], d[5]), halves(d[6], d[7]));
+  to[1] = make_uint4(halves(d[8], d[9]), halves(1.0f, 0.0f), 0u, 0u);
+}
+
 template <int PREC>
 __global__ void k_gather(KArgs a) {
   if (a.gate && *a.gate == 0) return;
@@ -264,8 +305,14 @@ __global__ void k_gather(KArgs a) {
   if (!sc.allpairs) {
     const int c0 = key_start(r.key, a.cell_start, a.cell_mid), c1 = key_end(r.key, a.cell_start, a.cell_mid);
     p = c0;
+    int k = c0;
+    for (; k < c1 && (k & 3); ++k) p += a.list[k] < d ? 1 : 0;
 #pragma unroll 4
-    for (int k = c0; k < c1; ++k) p += a.list[k] < d ? 1 : 0;
+    for (; k + 3 < c1; k += 4) {
+      const int4 v = *reinterpret_cast<const int4 *>(a.list + k);
+      p += (v.x < d ? 1 : 0) + (v.y < d ? 1 : 0) + (v.z < d ? 1 : 0) + (v.w < d ? 1 : 0);
+    }
+    for (; k < c1; ++k) p += a.list[k] < d ? 1 : 0;
   }
   a.skeys[p] = r.key;
   a.sx[p] = x;
@@ -289,11 +336,14 @@ __global__ void k_gather(KArgs a) {
     float s, c;
     sincosf(reduced_phase_f(ph), &s, &c);
     a.cs[p] = make_float2(c, s);
+    if (p < a.lane_p0) a.dig[p] = float_digits(c, s);
   }
   if constexpr (PREC == kPrecFP32X) {
     double s, c;
     sincos_phase(ph, s, c);
-    a.ics[p] = make_longlong2(to_fixed(c, kXQ), to_fixed(s, kXQ));
+    const longlong2 v = make_longlong2(to_fixed(c, kXQ), to_fixed(s, kXQ));
+    a.ics[p] = v;
+    if (p < a.lane_p0) fixed_digits(v, a.dig + 2 * (size_t)p);
     if (sc.allpairs) a.dcs[p] = make_double2(c, s);  // its passes are the FP64 ones
   }
   if constexpr (PREC == kPrecFP64) {
@@ -779,7 +829,9 @@ struct XSums {
 // and the FP64 epilogue finishes the step with the plain form's formulas and
 // normals.  The SRK second pass's per-term divisions by n_i
 // (ChimeraSystem.cpp:634-637) become one division of each sum.
-template <int KIND>
+// TILE: a slot of the cell-tile passes, which take the second pass's values as
+// digits.
+template <int KIND, bool TILE = false>
 __device__ void epilogue_fp32x(const KArgs &a, int epi, const SysDesc &sd, const ILane &il, const XSums &x,
                                int q) {
   const SysConst &sc = sd.sc;
@@ -799,7 +851,11 @@ __device__ void epilogue_fp32x(const KArgs &a, int epi, const SysDesc &sd, const
       // rate (the FP64 epilogue's value) times cos phi_i, sin phi_i
       const double rate = x.n ? ddiv_by(dmul(sc.sigma, acc.s0), cn.n, cn.r) : 0.0;
       a.scos[p] = x.n ? __fma_rn(x.c, ct, dmul(x.s, st)) : 0.0;
-      a.iws[p] = make_longlong2(to_fixed(dmul(rate, cs.x), sc.xq2), to_fixed(dmul(rate, cs.y), sc.xq2));
+      const longlong2 w = make_longlong2(to_fixed(dmul(rate, cs.x), sc.xq2), to_fixed(dmul(rate, cs.y), sc.xq2));
+      if constexpr (TILE)
+        fixed_digits(w, a.wdig + 2 * (size_t)p);
+      else
+        a.iws[p] = w;
     }
   } else {
     const double scs = a.scos[p];
@@ -829,7 +885,7 @@ __global__ void __launch_bounds__(256) k_epilogue_fp32x(KArgs a, int epi, int n)
   load_i<kPrecFP32X, KIND>(a, sc, il, p, true);
   const double2 v = a.xsum[p];
   const XSums x{v.x, v.y, a.xcnt[p]};
-  epilogue_fp32x<KIND>(a, epi, sd, il, x, a.pidx[p]);
+  epilogue_fp32x<KIND, true>(a, epi, sd, il, x, a.pidx[p]);
 }
 
 constexpr int kPassWarps = 4;

@@ -75,7 +75,7 @@ def test_lane_lists_and_batches(n):
 
 @pytest.mark.parametrize("precision", [abi.PRECISION_FP64, abi.PRECISION_FP32X, abi.PRECISION_FP32C])
 def test_four_lanes_and_one_lane_per_particle_agree_bitwise(precision):
-    """A system alone takes four lanes per particle; in a batch of 50,000
+    """A system alone takes four lanes per particle; in a batch of 89,000
     particles it takes one.  Rows of up to 90 neighbours (three words), and a
     system whose rows have more words than the first pass keeps."""
     L, n = 3.0, 3000
@@ -84,10 +84,10 @@ def test_four_lanes_and_one_lane_per_particle_agree_bitwise(precision):
     states = [init_state(n, L, 700), init_state(n, L, 701), init_state(n, 1.5, 702)]
     big = abi.make_params(L=8.0, stepper=abi.STEPPER_SRK, precision=precision, v0=0.02, sigma=1.0, rho=0.1,
                           alpha=1.0, D_phi=0.01)
-    with abi.Batch(abi.STEPPER_SRK, precision, 4, 3 * n + 50000, 225 + 100 + 25 + 6400) as b:
+    with abi.Batch(abi.STEPPER_SRK, precision, 4, 3 * n + 80000, 225 + 100 + 25 + 6400) as b:
         b.set_tuning(abi.TUNE_SPARSE_BELOW, 1e9)
         slots = [b.admit(n, p, st) for p, st in zip(par, states)]
-        b.admit(50000, big, init_state(50000, 8.0, 703))
+        b.admit(80000, big, init_state(80000, 8.0, 703))
         b.step(0.01, 4)
         got = [b.download(s) for s in slots]
     for p, st, want in zip(par, states, got):
