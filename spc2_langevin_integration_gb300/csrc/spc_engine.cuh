@@ -395,7 +395,7 @@ inline int engine_init(Engine *e, int stepper, int precision, int pool_cap, int 
       SPC_TRY(dalloc(e, &a.kphi[q], N));
     }
   SPC_TRY(dalloc(e, &a.stg, N));
-  SPC_TRY(dalloc(e, &a.keys, N));
+  SPC_TRY(dalloc(e, &a.keys, N + 4));  // read four at a time
   SPC_TRY(dalloc(e, &a.arrival, N));
   SPC_TRY(dalloc(e, &a.list, N));
   SPC_TRY(dalloc(e, &a.skeys, N));
@@ -839,30 +839,42 @@ inline int eval_cells(Engine *e, KArgs &a, int prec, int rk_form, int kq, double
   cudaStream_t st = e->stream;
   const int nkeys = a.cell_mid ? 2 * e->ncell_total : e->ncell_total;
   a.cnt_shift = count_shift(nkeys);
+  const bool ranked = n <= kRankMax && nkeys <= kScanOneCta;
+  if (ranked) a.cell_cnt = nullptr;  // nothing is counted
   k_stage<<<blocks_for(n, kStageThreads), kStageThreads, 0, st>>>(a, rk_form, kq, kcdt);
   SPC_LAUNCHED(e);
   if (marks) mark(e, 1);
-  const bool placed = nkeys <= kScanOneCta && n <= kPlaceInScan;
-  if (nkeys <= kScanOneCta) {
-    k_scan_cells<<<1, kScanThreads, 0, st>>>(a.cell_cnt, a.cnt_shift, nkeys, e->ncell_total, n, a.cell_start,
-                                             a.cell_mid, a.gate, a.keys, a.arrival, a.list, placed ? n : 0);
+  if (ranked) {
+    if (marks) mark(e, 2);
+    const int blocks = blocks_for((long long)(n + nkeys) * kRankLanes, kRankThreads);
+    if (prec == kPrecFP32C)
+      k_rank_gather<kPrecFP32C><<<blocks, kRankThreads, 0, st>>>(a, nkeys);
+    else if (prec == kPrecFP32X)
+      k_rank_gather<kPrecFP32X><<<blocks, kRankThreads, 0, st>>>(a, nkeys);
+    else
+      k_rank_gather<kPrecFP64><<<blocks, kRankThreads, 0, st>>>(a, nkeys);
+    SPC_LAUNCHED(e);
   } else {
-    const int chunks = blocks_for(nkeys, kScanChunk);
-    k_chunk_sums<<<chunks, kScanThreads, 0, st>>>(a.cell_cnt, e->part, a.gate);
-    k_scan_chunks<<<chunks, kScanThreads, 0, st>>>(a.cell_cnt, e->part, nkeys, e->ncell_total, n, a.cell_start,
-                                                   a.cell_mid, a.gate);
-  }
-  if (!placed)
+    if (nkeys <= kScanOneCta) {
+      k_scan_cells<<<1, kScanThreads, 0, st>>>(a.cell_cnt, a.cnt_shift, nkeys, e->ncell_total, n, a.cell_start,
+                                               a.cell_mid, a.gate);
+    } else {
+      const int chunks = blocks_for(nkeys, kScanChunk);
+      k_chunk_sums<<<chunks, kScanThreads, 0, st>>>(a.cell_cnt, e->part, a.gate);
+      k_scan_chunks<<<chunks, kScanThreads, 0, st>>>(a.cell_cnt, e->part, nkeys, e->ncell_total, n, a.cell_start,
+                                                     a.cell_mid, a.gate);
+    }
     k_place<<<blocks_for(n, 256), 256, 0, st>>>(a.keys, a.arrival, n, a.cell_start, a.cell_mid, a.list, a.gate);
-  SPC_LAUNCHED(e);
-  if (marks) mark(e, 2);
-  if (prec == kPrecFP32C)
-    k_gather<kPrecFP32C><<<blocks_for(n, 256), 256, 0, st>>>(a);
-  else if (prec == kPrecFP32X)
-    k_gather<kPrecFP32X><<<blocks_for(n, 256), 256, 0, st>>>(a);
-  else
-    k_gather<kPrecFP64><<<blocks_for(n, 256), 256, 0, st>>>(a);
-  SPC_LAUNCHED(e);
+    SPC_LAUNCHED(e);
+    if (marks) mark(e, 2);
+    if (prec == kPrecFP32C)
+      k_gather<kPrecFP32C><<<blocks_for(n, 256), 256, 0, st>>>(a);
+    else if (prec == kPrecFP32X)
+      k_gather<kPrecFP32X><<<blocks_for(n, 256), 256, 0, st>>>(a);
+    else
+      k_gather<kPrecFP64><<<blocks_for(n, 256), 256, 0, st>>>(a);
+    SPC_LAUNCHED(e);
+  }
   if (a.units && e->ncell_tile > 0 && !e->verlet) {  // the cell units of this evaluation
     if (e->precision == SPC_PRECISION_FP32C)
       k_list_units<kTileCap><<<blocks_for(e->ncell_tile, 128), 128, 0, st>>>(a);

@@ -22,8 +22,8 @@
 // Bound by latency (few keys) or by scattered 32-byte sectors.  Against a radix
 // sort of (key, index) pairs by 8- to 11-bit digits, in us for stage + sort +
 // gather: 96-system ensemble (681,278 particles, 110,312 cells) 145 -> 94, N =
-// 2^22 in 65,536 cells 541 -> 335, N = 65,536 in 1,024 cells 37 -> 31, N = 1,024
-// in 100 cells 30 -> 25.
+// 2^22 in 65,536 cells 541 -> 335, N = 65,536 in 1,024 cells 37 -> 31.
+// Up to kRankMax particles k_rank_gather takes the place of 2 to 4.
 #pragma once
 
 #include "spc_device.cuh"
@@ -135,35 +135,22 @@ __device__ __forceinline__ int key_end(uint32_t k, const int *__restrict__ start
   return mid && !(k & 1u) ? mid[k >> 1] : start[(mid ? k >> 1 : k) + 1];
 }
 
-__device__ __forceinline__ void place(int d, const uint32_t *__restrict__ keys, const int *__restrict__ arrival,
-                                      const int *start, const int *mid, int *__restrict__ list) {
-  list[key_start(keys[d], start, mid) + arrival[d]] = d;
-}
-
 __global__ void k_place(const uint32_t *__restrict__ keys, const int *__restrict__ arrival, int n, const int *start,
                         const int *mid, int *__restrict__ list, const int *gate) {
   if (gate && *gate == 0) return;
   const int d = blockIdx.x * blockDim.x + threadIdx.x;
-  if (d < n) place(d, keys, arrival, start, mid, list);
+  if (d < n) list[key_start(keys[d], start, mid) + arrival[d]] = d;
 }
 
-// One CTA scans all keys and, with place_n > 0, places that many particles
-// itself: one launch less, 1 us of a step of up to 1,024 particles; even at
-// 2,048, and 1 us more at 4,096.
-constexpr int kPlaceInScan = kScanThreads;
-
+// One CTA scans all keys.
 __global__ void __launch_bounds__(kScanThreads)
-    k_scan_cells(int *cnt, int shift, int nkeys, int ncell, int n, int *start, int *mid, const int *gate,
-                 const uint32_t *__restrict__ keys, const int *__restrict__ arrival, int *__restrict__ list,
-                 int place_n) {
+    k_scan_cells(int *cnt, int shift, int nkeys, int ncell, int n, int *start, int *mid, const int *gate) {
   if (gate && *gate == 0) return;
   __shared__ int wsum[kWarp + 1];
   int before = 0;
   for (int k0 = 0; k0 < nkeys; k0 += kScanChunk)
     before += scan_chunk(cnt, shift, nkeys, k0, before, start, mid, wsum);
   if (threadIdx.x == 0) start[ncell] = n;
-  __syncthreads();
-  for (int d = threadIdx.x; d < place_n; d += kScanThreads) place(d, keys, arrival, start, mid, list);
 }
 
 }  // namespace spc

@@ -16,7 +16,7 @@ pytestmark = pytest.mark.gpu
 PRM = dict(v0=0.01, sigma=1.1, alpha=0.8, D_phi=0.01)
 
 
-@pytest.mark.parametrize("n,nc", [(1023, 10), (1024, 10), (1025, 10), (3000, 64), (3000, 65), (3000, 110), (3000, 111)])
+@pytest.mark.parametrize("n,nc", [(1023, 10), (1024, 10), (1025, 10), (2047, 10), (2048, 44), (2049, 10), (2000, 110), (2000, 111), (3000, 64), (3000, 65), (3000, 110), (3000, 111)])
 def test_neighbour_sets_across_the_sorts_branches(n, nc):
     L, rho = 1.0, 1.0 / (nc + 0.25)
     st = init_state(n, L, 40 + nc)
