@@ -908,7 +908,7 @@ int launch_pass_t(Engine *e, const KArgs &a, int epi) {
   cudaStream_t st = e->stream;
   if constexpr (KIND == kKindNb) {
     // diagnostics count neighbours within rho for every model: the all-pairs
-    // kernel takes every all-pairs system, the cell kernel every cell list
+    // kernel takes every all-pairs system, the cell-tile kernel every cell list
     KArgs b = a;
     b.ap_cells = e->d_ap_all;
     b.n_ap = e->n_ap_all;
@@ -917,8 +917,9 @@ int launch_pass_t(Engine *e, const KArgs &a, int epi) {
       SPC_LAUNCHED(e);
     }
     if (e->ncell_total > e->n_ap_all) {
-      k_cell_pass<PREC, KIND><<<std::min(blocks_for(e->ncell_total, kPassWarps), 152 * 64), kPassThreads, 0,
-                                st>>>(b, epi);
+      b.ncell_tile = e->ncell_total;
+      b.tile_split = 1;
+      k_tile_fp64<KIND><<<std::min(e->ncell_total, 152 * 256), kTileThreads64, 0, st>>>(b, epi);
       SPC_LAUNCHED(e);
     }
     return SPC_OK;

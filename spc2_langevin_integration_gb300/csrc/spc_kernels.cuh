@@ -939,79 +939,6 @@ __global__ void __launch_bounds__(256) k_epilogue_fp32x(KArgs a, int epi, int n)
   epilogue_fp32x<KIND, true>(a, epi, sd, il, x, a.pidx[p]);
 }
 
-constexpr int kPassWarps = 4;
-constexpr int kPassThreads = kPassWarps * kWarp;
-constexpr int kIPL = 2;  // i particles per lane: a warp covers a 64-particle cell tile
-
-// Neighbour diagnostics (counts, lists in visiting order, local order
-// parameter): one warp per cell tile, two particles per lane, the 9 stencil
-// cells in the reference's order (ChimeraSystem.cpp:39-44) and within each the
-// members in ascending index, 32 candidates at a time through shared memory.
-// Decisions as everywhere: float prefilter, the reference's FP64 test near the
-// cutoff.
-template <int PREC, int KIND>
-__global__ void __launch_bounds__(kPassThreads) k_cell_pass(KArgs a, int epi) {
-  __shared__ float4 stage[kPassWarps][kWarp];
-  const int w = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
-  const int gwarp = blockIdx.x * kPassWarps + w;
-  const int nwarps = gridDim.x * kPassWarps;
-  for (int c = gwarp; c < a.ncell_total; c += nwarps) {
-    const SysDesc &sd = a.sys[a.sys_of_c[c]];
-    const SysConst &sc = sd.sc;
-    if (sc.allpairs) continue;
-    const int nc = sc.nc;
-    const bool exact_all = sc.exact_all != 0;
-    const int cb = a.cell_start[c], ce = a.cell_start[c + 1];
-    const int cl = c - sd.c0, cx = cl % nc, cy = cl / nc;
-    for (int base = cb; base < ce; base += kIPL * kWarp) {
-      ILane il[kIPL];
-      Acc<PREC> acc[kIPL];
-      long long wpos[kIPL];
-#pragma unroll
-      for (int k = 0; k < kIPL; ++k) {
-        const int p = base + k * kWarp + lane;
-        load_i<PREC, KIND>(a, sc, il[k], p, p < ce);
-        acc[k].init();
-        wpos[k] = (a.list_idx && il[k].valid) ? a.list_off[a.pidx[p]] : 0;
-      }
-      for (int q = 0; q < 9; ++q) {
-        const int ox = (q % 3) - 1, oy = (q / 3) - 1;  // {-1,-1},{0,-1},{1,-1},{-1,0},...
-        const int cj = sd.c0 + adjust_cell(cy + oy, nc) * nc + adjust_cell(cx + ox, nc);
-        const int ja = a.cell_start[cj], jb = a.cell_start[cj + 1];
-        const float shx = (float)ox * sc.cell_f, shy = (float)oy * sc.cell_f;
-        for (int jbase = ja; jbase < jb; jbase += kWarp) {
-          const int pl = jbase + lane;
-          __syncwarp();
-          if (pl < jb) {
-            const float2 f = a.fxy[pl];
-            stage[w][lane] = make_float4(f.x + shx, f.y + shy, 0.0f, 0.0f);
-          }
-          __syncwarp();
-          const int cnt = min(kWarp, jb - jbase);
-          for (int t = 0; t < cnt; ++t) {
-            const float4 cj4 = stage[w][t];
-            const int pj = jbase + t;
-#pragma unroll
-            for (int k = 0; k < kIPL; ++k) {
-              if (!il[k].valid || pj == il[k].p) continue;
-              const float dx = cj4.x - il[k].fx, dy = cj4.y - il[k].fy;
-              const float d2 = dx * dx + dy * dy;
-              if (exact_all || d2 <= sc.hi2) {
-                const bool in = (!exact_all && d2 < sc.lo2) ||
-                                exact_within(sc, il[k].x, il[k].y, a.sx[pj], a.sy[pj]);
-                if (in) accept_pair<PREC, KIND>(a, sd, il[k], acc[k], pj, 0.0f, 0.0f, 0.0f, wpos[k]);
-              }
-            }
-          }
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < kIPL; ++k)
-        if (il[k].valid) epilogue<PREC, KIND>(a, epi, sd, il[k], acc[k], a.pidx[il[k].p]);
-    }
-  }
-}
-
 // All pairs (rho > L/4): ChimeraSystem.cpp:117-255.  An all-pairs system's
 // particles form one cell, in index order.  A work item is one block of T
 // particles of one such system, so a large system spreads over many CTAs;

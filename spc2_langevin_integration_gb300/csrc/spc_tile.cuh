@@ -203,6 +203,10 @@ __global__ void k_list_units(KArgs a) {
 // 250 us (sines per pair and a queue of accepted candidates before; 137 MB
 // of kept cosines are gone).  704 candidates per round leave room for 7 CTAs
 // per SM in pass 2.
+// The neighbour diagnostics (kKindNb: counts, lists in visiting order, local
+// order parameters) are the same walk.  Order parameters of N = 65,536 at 64 a
+// cell, with upload and readback: 550 -> 278 us against a warp per cell that
+// added on the lanes that accept a candidate (even, 2% slower, at 3 a cell).
 constexpr int kTileWords64 = kTileCap64 / kWarp;
 static_assert(kTileCap64 % kWarp == 0 && (kTileWords64 + 3) / 4 * 4 <= kMaskWords, "FP64 staging round");
 
@@ -241,6 +245,7 @@ __global__ void __launch_bounds__(kTileThreads64) k_tile_fp64(KArgs a, int epi) 
       }
       Acc<kPrecFP64> acc;
       acc.init();
+      long long wpos = KIND == kKindNb && a.list_idx && valid ? a.list_off[a.pidx[p]] : 0;
       for (int r = 0; r < rounds; ++r) {
         const int rlo = r * kTileCap64, rcnt = min(kTileCap64, total - rlo);
         const int nw = (rcnt + kWarp - 1) / kWarp;
@@ -302,18 +307,39 @@ __global__ void __launch_bounds__(kTileThreads64) k_tile_fp64(KArgs a, int epi) 
                   make_uint4(s_w[4 * g][tid], s_w[4 * g + 1][tid], s_w[4 * g + 2][tid], s_w[4 * g + 3][tid]);
         }
         int w = -1;
-        walk_pairs<KIND, 2>(
-            acc, sc, il,
-            [&](uint32_t &bits, int &base) {
-              while (bits == 0u && ++w < nw) bits = s_w[w][tid];
-              base = w * kWarp;
-              return bits != 0u;
-            },
-            [&](int j) { return s_cs[j]; }, [&](int j) { return s_d[KIND == kKindCos2 ? j : 0]; },
-            [&](int j) {
+        auto next = [&](uint32_t &bits, int &base) {
+          while (bits == 0u && ++w < nw) bits = s_w[w][tid];
+          base = w * kWarp;
+          return bits != 0u;
+        };
+        if constexpr (KIND == kKindNb) {  // diagnostics
+          uint32_t bits = 0u;
+          int base = 0;
+          if (a.list_idx) {
+            while (bits != 0u || next(bits, base)) {
+              const int t = __clz(bits);
+              bits &= ~(0x80000000u >> t);
               int q;
-              return a.sphi[slot_of(st, rlo + j, q)];
-            });
+              a.list_idx[wpos++] = a.pidx[slot_of(st, rlo + base + t, q)] - sd.pool_p0;
+            }
+          } else if (a.out_r) {
+            while (bits != 0u || next(bits, base)) {
+              const int t = __clz(bits);
+              bits &= ~(0x80000000u >> t);
+              const double2 cj = s_cs[base + t];
+              acc.s0 = dadd(acc.s0, cj.x);
+              acc.s1 = dadd(acc.s1, cj.y);
+            }
+          }
+        } else {
+          walk_pairs<KIND, 2>(
+              acc, sc, il, next, [&](int j) { return s_cs[j]; },
+              [&](int j) { return s_d[KIND == kKindCos2 ? j : 0]; },
+              [&](int j) {
+                int q;
+                return a.sphi[slot_of(st, rlo + j, q)];
+              });
+        }
       }
       if (valid) {
         finish_pairs<KIND>(acc, il);
