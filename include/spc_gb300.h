@@ -72,9 +72,11 @@ enum { SPC_NEIGHBOUR_CELL = 0, SPC_NEIGHBOUR_VERLET = 1 };
 /* Precision.  FP64: every value and operation in double, the neighbour terms
  * added in the reference's order; a term's sine or cosine of the phase
  * difference comes from each particle's sine and cosine by the
- * angle-difference identity, within ~4e-16 of the exact value.  FP32C: neighbour sums, sin/cos and stage updates in float with
- * compensated (Kahan) accumulation; the cutoff / minimum-image decision, the
- * wrapped positions and the accumulated phase stay double.
+ * angle-difference identity, within ~4e-16 of the exact value.
+ * FP32C: sin/cos and stage updates in float; neighbour sums exact in units of
+ * 2^-35 (cell-tile passes) or float with compensated (Kahan) accumulation (the
+ * others); the cutoff / minimum-image decision, the wrapped positions and the
+ * accumulated phase stay double.
  * FP32X: the per-pair work stays off the FP64 pipe (float prefilter, the
  * exact FP64 test only near the cutoff), and the neighbour sums are exact:
  * each particle's cos phi and sin phi (and, for the SRK second pass, the
@@ -214,8 +216,8 @@ int spc_diagnostics(spc_handle *h, int64_t *clamped_cells, int64_t *verlet_rebui
 
 /* Per-phase device time of nsteps steps (no graph), measured with CUDA
  * events on the handle's stream between kernel groups.  out_ms receives
- * the average milliseconds per step of: [0] stage + cell keys, [1] radix
- * sort, [2] cell bounds + cell-order gather, [3] first neighbour pass
+ * the average milliseconds per step of: [0] stage + cell keys, [1] sort
+ * by cell (0 up to 2,048 particles), [2] cell-order gather, [3] first neighbour pass
  * (with its fused epilogue), [4] second neighbour pass (SRK) or the other
  * RK4 passes, [5] the whole step.  On a Verlet handle [0] is the refresh of
  * the Verlet-order state (with the displacement test), [1] the cell binning
@@ -245,9 +247,8 @@ int spc_profile_steps(spc_handle *h, double dt, int32_t nsteps, double *out_ms, 
  * groups), each unit on its own CTA in a second launch of each pass, beside
  * the cell-tile kernel; 0 (the default) runs every cell as whole particle
  * groups.  It pays on clustered states, where whole groups leave most SMs
- * idle at the end of a pass.  With 1, FP32X results are unchanged (exact
- * sums) and FP32C sums are added in another fixed order; either way they do
- * not depend on SPC_TUNE_TILE_SPLIT.  Refused for FP64 handles.
+ * idle at the end of a pass.  Results are unchanged (the sums of the float
+ * cell-tile passes are exact).  Refused for FP64 handles.
  * SPC_TUNE_SUBCELLS (FP32C and FP32X cell-list handles; the cell-size
  * dimension): 1 bins each cell of side L/int(L/rho) into a lower and an
  * upper half and runs the cells of at most 8 staging rounds as cell units of
@@ -255,8 +256,7 @@ int spc_profile_steps(spc_handle *h, double dt, int32_t nsteps, double *out_ms, 
  * near half of the row beyond it: the far half is more than a cell side
  * (>= rho) away, so about 7.5 of the 9 stencil cells are tested.  0 (the
  * default) keeps whole cells.  The neighbour sets are those of whole cells:
- * FP32X results are unchanged, FP32C sums are added in another fixed
- * order.  (An excluded pair could only count as a neighbour if the cell side
+ * results are unchanged.  (An excluded pair could only count as a neighbour if the cell side
  * equalled rho to within rounding and the pair lay within rounding of the
  * cutoff, across the half boundary, with |dx| below ~1e-8 rho.)  Neighbour
  * diagnostics keep whole cells.  Refused for FP64 and Verlet handles.

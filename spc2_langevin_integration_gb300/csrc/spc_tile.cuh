@@ -200,9 +200,8 @@ __global__ void k_list_units(KArgs a) {
 // one-round cells in nbmask and the second pass tests nothing again.
 // Bound by the FP64 pipe (3 operations per pair in pass 1, 5 in pass 2).
 // Vortex SRK, N = 65,536: pass 1 2.04 ms -> 171 us, pass 2 0.92 ms ->
-// 250 us (sines per pair and a queue of accepted candidates before; 137 MB
-// of kept cosines are gone).  704 candidates per round leave room for 7 CTAs
-// per SM in pass 2.
+// 250 us (against sines per pair and a queue of accepted candidates).  704
+// candidates per round leave room for 7 CTAs per SM in pass 2.
 // The neighbour diagnostics (kKindNb: counts, lists in visiting order, local
 // order parameters) are the same walk.  Order parameters of N = 65,536 at 64 a
 // cell, with upload and readback: 550 -> 278 us against a warp per cell that
