@@ -375,14 +375,16 @@ struct RowSums<kPrecFP32C> {
     bad += v[7];
   }
   __device__ longlong2 pair() const { return make_longlong2(c, s); }
-  __device__ int count() const { return bad ? -1 : n; }
+  // a round's count, complemented when a neighbour's value was not finite
+  __device__ int count() const { return bad ? ~n : n; }
   __device__ void add(longlong2 v, int m) {
     c += v.x;
     s += v.y;
-    if (m < 0)
+    if (m < 0) {
       bad = 1;
-    else
-      n += m;
+      m = ~m;
+    }
+    n += m;
   }
 };
 template <>
