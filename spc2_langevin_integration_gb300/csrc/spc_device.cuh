@@ -49,6 +49,16 @@ __device__ __forceinline__ double dsqrt(double a) { return __dsqrt_rn(a); }
 constexpr int kXQ = 52;
 __device__ __forceinline__ long long to_fixed(double v, int q) { return double_to_fixed(v, q); }
 __device__ __forceinline__ double from_fixed(long long v, int q) { return fixed_to_double(v, q); }
+// A pair of values: both kNotFixed when either has no fixed-point form (its
+// phase is not finite), which the neighbour passes turn into sums of NaN.
+__device__ __forceinline__ longlong2 to_fixed2(double x, double y, int q) {
+  const longlong2 v = make_longlong2(to_fixed(x, q), to_fixed(y, q));
+  return v.x == kNotFixed || v.y == kNotFixed ? make_longlong2(kNotFixed, kNotFixed) : v;
+}
+__device__ __forceinline__ double2 from_fixed2(longlong2 v, int q) {
+  const double nan = __longlong_as_double(0x7ff8000000000000ll);
+  return v.x == kNotFixed ? make_double2(nan, nan) : make_double2(from_fixed(v.x, q), from_fixed(v.y, q));
+}
 // A particle's whole sum over several staging rounds is kept in 128 bits, so
 // it is one exact integer whatever the kernel's round size, and converted to
 // double once: one rounding when it fits 64 bits (always below 2^11

@@ -12,7 +12,7 @@
 //               a float's own rounding is 2^-25), 1 (the count), and 1 for a
 //               value that is not finite, whose digits are 0
 //   FP32X (16): five digits each, base 2048, of the 64-bit fixed-point values,
-//               1 (the count), zeros
+//               1 (the count), 1 for a value that is not finite, zeros
 // A warp takes 32 particles (rows) and 32 candidates at a time; its
 // lanes hold the tests in the layout of mma.sync's A operand (lane 4 g + t:
 // rows g + 8 k, candidates 8 m + 2 t and the next), so a test becomes an A
@@ -390,7 +390,7 @@ struct RowSums<kPrecFP32C> {
 template <>
 struct RowSums<kPrecFP32X> {
   __int128 c = 0, s = 0;
-  int n = 0;
+  int n = 0, bad = 0;
   __device__ void add(const int (&v)[12]) {
     long long p = v[4], q = v[9];
 #pragma unroll
@@ -401,12 +401,17 @@ struct RowSums<kPrecFP32X> {
     c += p;
     s += q;
     n += v[10];
+    bad += v[11];
   }
   __device__ longlong2 pair() const { return make_longlong2((long long)c, (long long)s); }  // one round
-  __device__ int count() const { return n; }
+  __device__ int count() const { return bad ? ~n : n; }
   __device__ void add(longlong2 v, int m) {
     c += v.x;
     s += v.y;
+    if (m < 0) {
+      bad = 1;
+      m = ~m;
+    }
     n += m;
   }
 };
@@ -470,7 +475,8 @@ template <int KIND>
 __device__ __forceinline__ void finish_row(const KArgs &a, int epi, const SysDesc &sd, int p,
                                            const RowSums<kPrecFP32X> &sum) {
   const int qv = KIND == kKindSin ? kXQ : sd.sc.xq2;
-  a.xsum[p] = make_double2(from_fixed128(sum.c, qv), from_fixed128(sum.s, qv));
+  const double nan = __longlong_as_double(0x7ff8000000000000ll);
+  a.xsum[p] = sum.bad ? make_double2(nan, nan) : make_double2(from_fixed128(sum.c, qv), from_fixed128(sum.s, qv));
   a.xcnt[p] = sum.n;
 }
 

@@ -279,9 +279,11 @@ __device__ __forceinline__ uint4 float_digits(float x, float y) {
                     halves(y1, rintf((ry - y1) * 4096.0f)), halves(1.0f, bad ? 1.0f : 0.0f));
 }
 // FP32X: five digits in base 2048 each of x and y (|x|, |y| < 2^54), lowest
-// first, 1, zeros.
+// first, 1, and 1 if they are kNotFixed, zeros.
 __device__ __forceinline__ void fixed_digits(longlong2 v, uint4 *to) {
   float d[10];
+  const bool bad = v.x == kNotFixed;
+  if (bad) v = make_longlong2(0, 0);
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     long long r = h ? v.y : v.x;
@@ -294,7 +296,7 @@ __device__ __forceinline__ void fixed_digits(longlong2 v, uint4 *to) {
     d[5 * h + 4] = (float)(int)r;
   }
   to[0] = make_uint4(halves(d[0], d[1]), halves(d[2], d[3]), halves(d[4], d[5]), halves(d[6], d[7]));
-  to[1] = make_uint4(halves(d[8], d[9]), halves(1.0f, 0.0f), 0u, 0u);
+  to[1] = make_uint4(halves(d[8], d[9]), halves(1.0f, bad ? 1.0f : 0.0f), 0u, 0u);
 }
 
 // Dense particle d into cell-order slot p.
@@ -330,7 +332,7 @@ __device__ __forceinline__ void gather_to(const KArgs &a, int d, const StageRec 
   if constexpr (PREC == kPrecFP32X) {
     double s, c;
     sincos_phase(ph, s, c);
-    const longlong2 v = make_longlong2(to_fixed(c, kXQ), to_fixed(s, kXQ));
+    const longlong2 v = to_fixed2(c, s, kXQ);
     a.ics[p] = v;
     if (p < a.lane_p0) fixed_digits(v, a.dig + 2 * (size_t)p);
     if (sc.allpairs) a.dcs[p] = make_double2(c, s);  // its passes are the FP64 ones
@@ -887,8 +889,7 @@ __device__ void epilogue_fp32x(const KArgs &a, int epi, const SysDesc &sd, const
                                int q) {
   const SysConst &sc = sd.sc;
   const int p = il.p;
-  const longlong2 cq = a.ics[p];
-  const double2 cs = make_double2(from_fixed(cq.x, kXQ), from_fixed(cq.y, kXQ));
+  const double2 cs = from_fixed2(a.ics[p], kXQ);
   const double ct = __fma_rn(cs.x, sc.cos_ad, -dmul(cs.y, sc.sin_ad));  // cos(phi_i + alpha)
   const double st = __fma_rn(cs.y, sc.cos_ad, dmul(cs.x, sc.sin_ad));   // sin(phi_i + alpha)
   const Count cn = count_of(x.n);
@@ -902,7 +903,7 @@ __device__ void epilogue_fp32x(const KArgs &a, int epi, const SysDesc &sd, const
       // rate (the FP64 epilogue's value) times cos phi_i, sin phi_i
       const double rate = x.n ? ddiv_by(dmul(sc.sigma, acc.s0), cn.n, cn.r) : 0.0;
       a.scos[p] = x.n ? __fma_rn(x.c, ct, dmul(x.s, st)) : 0.0;
-      const longlong2 w = make_longlong2(to_fixed(dmul(rate, cs.x), sc.xq2), to_fixed(dmul(rate, cs.y), sc.xq2));
+      const longlong2 w = to_fixed2(dmul(rate, cs.x), dmul(rate, cs.y), sc.xq2);
       if constexpr (TILE)
         fixed_digits(w, a.wdig + 2 * (size_t)p);
       else

@@ -106,24 +106,28 @@ struct LaneSums<kPrecFP64, KIND> {
 
 // FP32X: exact fixed-point sums, so the result is bitwise that of the
 // cell-tile kernel.  A word's neighbours add less than 2^57; after each word the
-// multiples of 2^57 move to a 32-bit count (2^57 each).
+// multiples of 2^57 move to a 32-bit count (2^57 each).  A value that is not
+// finite (kNotFixed) is found by the smallest high word of the neighbours'.
 template <int KIND>
 struct LaneSums<kPrecFP32X, KIND> {
   long long c, s;
-  int ch, sh;
+  int ch, sh, low;
   __device__ void init() {
     c = s = 0;
-    ch = sh = 0;
+    ch = sh = low = 0;
   }
   typedef longlong2 Value;
   __device__ static Value value(const KArgs &a, int j) { return KIND == kKindSin ? a.ics[j] : a.iws[j]; }
-  __device__ void add(const Value &v, bool p) { add2_if(c, s, v, p); }
+  __device__ void add(const Value &v, bool p) {
+    add2_if(c, s, v, p);
+    low = min(low, (int)(v.x >> 32));  // a v that is not added has been
+  }
   __device__ void word_end(const ILane &) {
-    constexpr long long low = (1ll << 57) - 1;
+    constexpr long long rest = (1ll << 57) - 1;
     ch += (int)(c >> 57);
     sh += (int)(s >> 57);
-    c &= low;
-    s &= low;
+    c &= rest;
+    s &= rest;
   }
   __device__ void row_end() {}
   __device__ void join_group(unsigned mask, int) {
@@ -133,12 +137,16 @@ struct LaneSums<kPrecFP32X, KIND> {
       s += __shfl_xor_sync(mask, s, o);
       ch += __shfl_xor_sync(mask, ch, o);
       sh += __shfl_xor_sync(mask, sh, o);
+      low = min(low, __shfl_xor_sync(mask, low, o));
     }
   }
   __device__ void finish(const KArgs &a, int epi, const SysDesc &sd, const ILane &il, int n, int q) {
     const int qv = KIND == kKindSin ? kXQ : sd.sc.xq2;
     const __int128 tc = ((__int128)ch << 57) + c, ts = ((__int128)sh << 57) + s;
-    epilogue_fp32x<KIND>(a, epi, sd, il, XSums{from_fixed128(tc, qv), from_fixed128(ts, qv), n}, q);
+    const double nan = __longlong_as_double(0x7ff8000000000000ll);
+    const bool bad = low == (int)(kNotFixed >> 32);
+    epilogue_fp32x<KIND>(a, epi, sd, il,
+                         XSums{bad ? nan : from_fixed128(tc, qv), bad ? nan : from_fixed128(ts, qv), n}, q);
   }
 };
 

@@ -155,16 +155,18 @@ SPC_MATH_FN double sqrt_pos(double x) {
   return x == 0.0 ? 0.0 : g;
 }
 
-// RN(v 2^q) as an integer, |v 2^q| < 2^52: to nearest, ties to even, by
-// integer instructions (the scaling is exact, so this is the rounding of the
-// scaled value).
+// RN(v 2^q) as an integer: to nearest, ties to even, by integer instructions
+// (the scaling is exact, so this is the rounding of the scaled value).
+// kNotFixed when v is not finite or |v 2^q| is 2^62 or more.
+constexpr long long kNotFixed = -0x7fffffffffffffffll - 1;
 SPC_MATH_FN long long double_to_fixed(double v, int q) {
   const std::uint64_t b = double_to_bits(v);
   const int e = static_cast<int>((b >> 52) & 0x7ff);
   const int drop = 1075 - e - q;  // bits below the unit
+  if (e == 0x7ff || drop < -9) return kNotFixed;
   if (drop > 54 || e == 0) return 0;
   const std::uint64_t m = (b & 0xfffffffffffffull) | (1ull << 52);
-  std::uint64_t r = m;
+  std::uint64_t r = drop < 0 ? m << -drop : m;
   if (drop > 0) {
     r = m >> drop;
     const std::uint64_t rest = m << (64 - drop), half = 1ull << 63;
