@@ -47,6 +47,9 @@ __device__ __forceinline__ double dsqrt(double a) { return __dsqrt_rn(a); }
 // 2^62 in magnitude, so the integer sums are exact, and the conversion back
 // (one rounding to double) is the only error of a round's sum.
 constexpr int kXQ = 52;
+// Phase rates take units of 2^-xq2, xq2 = 51 - e for |sigma| <= 2^e, e up to
+// kSigmaBits: the conversions' powers of two and a sum's value stay normal.
+constexpr int kSigmaBits = 900;
 __device__ __forceinline__ long long to_fixed(double v, int q) { return double_to_fixed(v, q); }
 __device__ __forceinline__ double from_fixed(long long v, int q) { return fixed_to_double(v, q); }
 // A pair of values: both kNotFixed when either has no fixed-point form (its

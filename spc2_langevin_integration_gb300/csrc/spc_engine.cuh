@@ -101,7 +101,7 @@ inline SysConst make_sysconst(const spc_params &p, int n) {
   {
     // |phase rate| <= |sigma| (sigma times a mean of sines): 2^e >= |sigma|
     int e = 0;
-    while (e < 40 && std::ldexp(1.0, e) < std::fabs(p.sigma)) ++e;
+    while (e < kSigmaBits && std::ldexp(1.0, e) < std::fabs(p.sigma)) ++e;
     sc.xq2 = kXQ - e - 1;  // one more bit of headroom for the rate's rounding
   }
   if (p.model == SPC_MODEL_VORTEX_ARRAYS) {

@@ -13,7 +13,7 @@
 // FP32X neighbour kernels otherwise hardly use.
 //
 // Valid for results in the normal range, 2^-1022 <= |v 2^-q| < 2^1024, which
-// holds for every q the FP32X form uses (11 <= q <= 52) and any nonzero v.
+// holds for every q the FP32X form uses (-849 <= q <= 52) and any nonzero v.
 // Plain C++ as well, so the host test compares it with the C conversion.
 #pragma once
 

@@ -1,5 +1,6 @@
 // double_to_fixed (csrc/spc_math.h) outside the range of its usual values:
-// not finite, and up to and beyond 2^62 units.
+// not finite, and up to and beyond 2^62 units; and fixed_to_double
+// (csrc/spc_fixed.h) with units far above one.
 #include <cmath>
 #include <cstdio>
 #include <initializer_list>
@@ -26,6 +27,9 @@ int main() {
     for (int e : {62, 63, 64, 200})
       for (double m : {1.0, -1.0}) expect(std::ldexp(m, e - q), q, spc::kNotFixed);
   }
+  for (int q : {52, 0, -1, -300, -849})
+    for (long long v : {1ll, -1ll, 3ll, (1ll << 52) + 1, (1ll << 62) + 129, -(1ll << 62) - 257})
+      if (spc::fixed_to_double(v, q) != std::ldexp((double)v, -q)) ++bad;
   std::printf(bad ? "FAILED\n" : "ok\n");
   return bad ? 1 : 0;
 }
