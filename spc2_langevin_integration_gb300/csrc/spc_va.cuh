@@ -149,11 +149,12 @@ __device__ __forceinline__ bool le_bits(double a, double b) {
 // xj - xi by minimum image (PeriodicBoundaryConditions.cpp:22-35).  `near`: the
 // pair passed the float test of a cell list with both cutoffs up to L/4, so the
 // difference is within L/4 of 0 or of -+L, and the reference's truncated
-// quotient is 0 or +-1.
+// quotient is 0 or +-1, but +-2 at a difference of L itself (a copy that wraps
+// to exactly L, against x = 0), which the general form takes.
 __device__ __forceinline__ double va_image(const SysConst &sc, double xj, double xi, bool near) {
   const double d = dsub(xj, xi);
-  if (!near) return min_image_1d(d, sc.rL, sc.L);
   const int hi = __double2hiint(d) & 0x7fffffff;
+  if (!near || hi >= __double2hiint(sc.L)) return min_image_1d(d, sc.rL, sc.L);
   return hi > __double2hiint(sc.va_hL) ? dsub(d, copysign(sc.L, d)) : d;
 }
 
