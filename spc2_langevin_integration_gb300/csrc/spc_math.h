@@ -138,7 +138,8 @@ SPC_MATH_FN double neg2_log53(std::uint64_t A) {
   return add_rn(T, add_rn(R, low));
 }
 
-// sqrt(x), x = 0 or 2^-60 < x < 2^60.
+// sqrt(x), x = 0 or 2^-900 < x < 2^1000 (the remainder of the last step is then
+// normal).
 SPC_MATH_FN double sqrt_pos(double x) {
 #if defined(__CUDA_ARCH__)
   double y;

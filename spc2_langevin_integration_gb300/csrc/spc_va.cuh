@@ -162,10 +162,14 @@ __device__ __noinline__ double va_bearing(double dx, double dy, double phi) { re
 __device__ __noinline__ double sin_library(double v) { return sin(v); }
 __device__ __noinline__ double cos_library(double v) { return cos(v); }
 
+// dr2 < 2^-900 (0 among them): its root, and (dx, dy) over it, would not have a
+// double's precision by the short forms.
+__device__ __forceinline__ bool va_tiny(double dr2) { return __double2hiint(dr2) < 0x07b00000; }
+
 // sin and cos of (bearing - phi_i)
-__device__ __forceinline__ void va_bearing_sincos(double dx, double dy, double dr, double2 ci, double phii, double &s,
-                                                  double &c) {
-  if (dr == 0.0) {
+__device__ __forceinline__ void va_bearing_sincos(double dx, double dy, double dr, bool tiny, double2 ci, double phii,
+                                                  double &s, double &c) {
+  if (tiny) {
     const double t = va_bearing(dx, dy, phii);
     s = sin_library(t);
     c = cos_library(t);
@@ -217,7 +221,8 @@ __global__ void __launch_bounds__(kLaneThreads) k_va_pass(KArgs a, int epi) {
     const bool align = le_bits(dr2, sc.va_t_xia), rho_pair = le_bits(dr2, sc.va_t_rho);
     t.term = wanted && (KIND == kKindSin ? align || rho_pair : rho_pair);
     t.coh = wanted && le_bits(dr2, sc.va_t_xir);
-    const double dr = sqrt_pos(dr2);
+    const bool tiny = va_tiny(dr2);
+    const double dr = tiny ? dsqrt(dr2) : sqrt_pos(dr2);
     const double2 cj = a.dcs[j];
     // AlignmentStrength (:737-749) and, over dr, AlignmentStrengthDerivative (:751-763)
     const bool in1 = !le_bits(sc.va_s_xia, dr2), in2 = !in1 && !le_bits(sc.va_s_rho, dr2);
@@ -229,7 +234,7 @@ __global__ void __launch_bounds__(kLaneThreads) k_va_pass(KArgs a, int epi) {
       t.x = dmul(f, sp);  // VortexArraysSystemPtr.cpp:475-485
       if (t.coh) {        // :486-488
         double s, c;
-        va_bearing_sincos(dx, dy, dr, ci, phii, s, c);
+        va_bearing_sincos(dx, dy, dr, tiny, ci, phii, s, c);
         t.u = dmul(-sc.kappa, s);
       }
     } else {
@@ -246,7 +251,7 @@ __global__ void __launch_bounds__(kLaneThreads) k_va_pass(KArgs a, int epi) {
       t.y = __fma_rn(dsub(a.dphi_s[j], ddi), t.x, dmul(q, sp));
       if (t.coh) {
         double s, c;
-        va_bearing_sincos(dx, dy, dr, ci, phii, s, c);
+        va_bearing_sincos(dx, dy, dr, tiny, ci, phii, s, c);
         const double turn = ddiv(dmul(sc.v0, __fma_rn(ey, dx, -dmul(ex, dy))), dr2);
         t.u = dmul(sc.kappa, c);
         t.v = __fma_rn(dmul(-sc.kappa, dsub(turn, ddi)), c, dmul(dmul(sc.kappa, sc.D), s));
