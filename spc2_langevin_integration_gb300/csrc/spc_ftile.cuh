@@ -425,11 +425,11 @@ __device__ __forceinline__ void take_row(const TileMem<PREC> &s, RowSums<PREC> &
   sum.add(v);
 }
 
-// v 2^-35 as an unevaluated sum of two floats
+// v 2^-35 as an unevaluated sum of two floats: v rounded to float, and the rest
+// rounded to float (the whole within 2^-48 of v).
 __device__ __forceinline__ float2 two_floats(long long v) {
-  const float a = (float)(v >> 22) * 0x1p-13f, b = (float)(int)(v & 0x3fffff) * 0x1p-35f;
-  const float h = a + b, bb = h - a;
-  return make_float2(h, (a - (h - bb)) + (b - bb));
+  const float h = __ll2float_rn(v);
+  return make_float2(h * 0x1p-35f, __ll2float_rn(v - __float2ll_rn(h)) * 0x1p-35f);
 }
 // x u + y v for such sums x and y
 __device__ __forceinline__ float dot2(float2 x, float u, float2 y, float v) {
