@@ -72,7 +72,9 @@ enum { SPC_NEIGHBOUR_CELL = 0, SPC_NEIGHBOUR_VERLET = 1 };
 /* Precision.  FP64: every value and operation in double, the neighbour terms
  * added in the reference's order; a term's sine or cosine of the phase
  * difference comes from each particle's sine and cosine by the
- * angle-difference identity, within ~4e-16 of the exact value.
+ * angle-difference identity, within ~4e-16 of the exact value; for |alpha| <
+ * 0.5 (and in VORTEX_ARRAYS) the rates between aligned phases, whose sines are
+ * small, are as close as the sines of the differences would give them.
  * FP32C: sin/cos and stage updates in float; neighbour sums exact in units of
  * 2^-35 (cell-tile passes) or float with compensated (Kahan) accumulation (the
  * others); the cutoff / minimum-image decision, the wrapped positions and the

@@ -1098,6 +1098,7 @@ constexpr int kNoAllocMaxCells = 16384;  // cells (nc * nc) per call
 constexpr size_t na_round(size_t b) { return (b + 255) / 256 * 256; }
 constexpr size_t kNaD = na_round(8ull * kNoAllocMaxN);   // one double per particle
 constexpr size_t kNaF = na_round(4ull * kNoAllocMaxN);   // one 32-bit value per particle
+constexpr size_t kNaH = na_round(2ull * kNoAllocMaxN);   // one 16-bit value per particle
 constexpr size_t kNaF2 = na_round(8ull * kNoAllocMaxN);  // one float2 per particle
 constexpr size_t kNaCells = na_round(4ull * (kNoAllocMaxCells + 1));
 constexpr size_t kNaCount = 4ull * (kNoAllocMaxCells + kScanChunk + (kSpreadKeys << kSpreadShift));
@@ -1105,10 +1106,10 @@ constexpr size_t kNaStage = na_round(sizeof(StageRec) * kNoAllocMaxN);
 constexpr size_t kNaSys = na_round(sizeof(SysDesc));
 // x y phi omega | sx sy sphi | dphi_s                         (8 double arrays)
 // keys arrival list skeys pidx cnt_s dphi_f scos_f sys_of_p   (9 32-bit arrays)
-// fxy cs (2 float2 arrays) | dcs (double2), dig, wdig (16 bytes each) | stage records | cell_start | sys_of_c | counts | chunk sums |
-// system table | all-pairs cell | clamp counter
+// fxy cs (2 float2 arrays) | dcs (double2), dig, wdig (16 bytes each) | rests (16-bit) | stage records | cell_start |
+// sys_of_c | counts | chunk sums | system table | all-pairs cell | clamp counter
 constexpr size_t kNoAllocBytes =
-    8 * kNaD + 9 * kNaF + 2 * kNaF2 + 6 * kNaD + kNaStage + 2 * kNaCells + kNaCount + 256 + kNaSys + 256 + 256;
+    8 * kNaD + 9 * kNaF + 2 * kNaF2 + 6 * kNaD + kNaH + kNaStage + 2 * kNaCells + kNaCount + 256 + kNaSys + 256 + 256;
 
 constexpr int kNoAllocMaxDevices = 64;
 std::mutex g_noalloc_mu;
@@ -1247,6 +1248,7 @@ extern "C" int spc_rhs_srk_noalloc(const spc_params *p, int32_t n, const double 
   a.dcs = (double2 *)take(2 * kNaD);
   a.dig = (uint4 *)take(2 * kNaD);
   a.wdig = (uint4 *)take(2 * kNaD);
+  a.rest = (uint16_t *)take(kNaH);
   a.cell_start = (int *)take(kNaCells);
   int *sys_of_c = (int *)take(kNaCells);
   a.stg = (StageRec *)take(kNaStage);
@@ -1268,6 +1270,7 @@ extern "C" int spc_rhs_srk_noalloc(const spc_params *p, int32_t n, const double 
   e.n_active = n;
   e.ncell_total = ncell;
   e.has_cells = !sc.allpairs;
+  e.any_rest = sc.rest_on != 0;
   a.nsys = 1;
   a.n_active = n;
   a.ncell_total = ncell;

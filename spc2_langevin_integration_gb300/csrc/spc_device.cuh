@@ -105,6 +105,22 @@ __device__ __forceinline__ void sincos_phase(double ph, double &s, double &c) {
     sincos_library(ph, &s, &c);
 }
 
+// A phase's sector (of 16) and rest (sincos_with_rest; units of 2^-64, offset
+// 2,048) in 16 bits, for pair terms that keep their relative accuracy between
+// aligned phases (sine_rest).  Phases beyond the table's range have no rest:
+// their own last place is above 2^-33.
+constexpr uint32_t kNoRest = 2048u;
+__device__ __forceinline__ uint16_t sincos_phase_rest(double ph, double &s, double &c) {
+  if (!phase_in_range(ph)) {
+    sincos_library(ph, &s, &c);
+    return kNoRest;
+  }
+  int k;
+  double rest;
+  sincos_with_rest(ph, s, c, k, rest);
+  return (uint16_t)((((k + 4) >> 3) & 15) << 12 | (small_to_int(rest, 64) + (int)kNoRest));
+}
+
 // A neighbour count as a double with its reciprocal rounded to nearest, for
 // ddiv_by: a table of the usual counts in place of a conversion and a division
 // (about ten operations of the FP64 pipe).
@@ -179,6 +195,10 @@ struct SysConst {
   // derivatives' 2 mu_+ / xi_a^2 and -4 mu_- / w^2 times v0, rho + xi_a, 2 D
   double va_t_xia, va_t_rho, va_t_xir, va_s_xia, va_s_rho, va_hL;
   double va_c1, va_c2, va_g1, va_g2, va_xr, va_2D;
+  // FP64 pair sums: |alpha| < kRestAlpha, so that aligned phases have small
+  // sines; alpha in sectors; the angle by which alpha exceeds that of (cos_ad, sin_ad)
+  int rest_on, rest_sector;
+  double rest_alpha;
 };
 
 // PeriodicBoundaryConditions::ClassAEffectiveParticleDistance (PeriodicBoundaryConditions.cpp:22-35):

@@ -98,6 +98,10 @@ inline SysConst make_sysconst(const spc_params &p, int n) {
   sc.s2D = std::sqrt(2.0 * p.D_phi);  // correctly rounded, as the device's sqrt
   sc.cos_ad = std::cos(p.alpha);
   sc.sin_ad = std::sin(p.alpha);
+  sc.rest_on = std::fabs(p.alpha) < kRestAlpha || p.model == SPC_MODEL_VORTEX_ARRAYS;
+  sc.rest_sector = sc.rest_on ? (int)std::lrint(p.alpha * (8.0 / 3.141592653589793)) : 0;
+  sc.rest_alpha = (double)(sc.cos_ad * (sinl((long double)p.alpha) - sc.sin_ad) -
+                           sc.sin_ad * (cosl((long double)p.alpha) - sc.cos_ad));
   {
     // |phase rate| <= |sigma| (sigma times a mean of sines): 2^e >= |sigma|
     int e = 0;
@@ -230,6 +234,7 @@ struct Engine {
   int nsys = 0, n_active = 0, ncell_total = 0;
   int ncell_tile = 0, ncell_warp = 0, ncell_va = 0;  // cells of the tile, warp and vortex-arrays systems
   bool has_cells = false;
+  bool any_rest = false, lane_rest = false;  // a system (of the lane passes) has rests (SysConst::rest_on)
   // tuning: cell-list systems with fewer than sparse_below particles per cell
   // (on average) run the particle-per-lane passes
   double sparse_below = kSparseBelowDefault;
@@ -363,7 +368,7 @@ inline void engine_footprint(int stepper, int precision, long long *per_particle
   if (precision != SPC_PRECISION_FP64)  // cell units: round sums, counts, chunk counters, list
     b += kSplitRounds * (16 + 4) + 4 + kSplitRounds * 8 / 32;
   if (precision == SPC_PRECISION_FP64) b += 4;                                  // vortex-arrays partner counts
-  if (precision != SPC_PRECISION_FP32C) b += 16;                                // dcs
+  if (precision != SPC_PRECISION_FP32C) b += 16 + 2;                            // dcs, rests
   if (precision == SPC_PRECISION_FP64 && stepper == SPC_STEPPER_SRK) b += (long long)kMaskWords * 4;  // masks
   b += 12 * 8;                               // AoS staging
   *per_particle = b;
@@ -410,7 +415,10 @@ inline int engine_init(Engine *e, int stepper, int precision, int pool_cap, int 
     SPC_TRY(dalloc(e, &a.va_cnt2, N));
     if (stepper == SPC_STEPPER_SRK) SPC_TRY(dalloc(e, &a.nbmask, (size_t)kMaskWords * N));
   }
-  if (precision != SPC_PRECISION_FP32C) SPC_TRY(dalloc(e, &a.dcs, N));
+  if (precision != SPC_PRECISION_FP32C) {
+    SPC_TRY(dalloc(e, &a.dcs, N));
+    SPC_TRY(dalloc(e, &a.rest, N));
+  }
   int *sys_of_p = nullptr, *sys_of_c = nullptr;
   SPC_TRY(dalloc(e, &sys_of_p, N));
   a.sys_of_p = sys_of_p;
@@ -694,7 +702,7 @@ inline std::vector<long long> launch_shape(const Engine *e) {
   return {e->nsys, e->n_active, e->ncell_total, e->ncell_tile,
           e->ncell_warp, e->ncell_va, e->n_ap_all, e->has_cells, a.n_ap, a.tile_split,
           e->ap_items, e->ap_items_all, e->ap_items_small, e->ap_items_all_small, a.units != nullptr,
-          a.cell_mid != nullptr, a.lane_p0, a.lane_p1, a.va_p1};
+          a.cell_mid != nullptr, a.lane_p0, a.lane_p1, a.va_p1, e->any_rest, e->lane_rest};
 }
 
 inline int engine_layout(Engine *e) {
@@ -711,6 +719,7 @@ inline int engine_layout(Engine *e) {
   int ncell_tile = 0, ncell_warp = 0, ncell_va = 0, lane_p0 = 0, lane_p1 = 0, va_p1 = 0;
   e->ap_items = e->ap_items_all = 0;
   e->ap_items_small = e->ap_items_all_small = 0;
+  e->any_rest = e->lane_rest = false;
   for (int cls = 0; cls < 4; ++cls) {
     for (int slot : e->order) {
       const SysHost &h = e->slots[slot];
@@ -731,8 +740,12 @@ inline int engine_layout(Engine *e) {
       }
       dense += h.n;
       cells += h.ncell;
+      e->any_rest |= h.sc.rest_on != 0;
       if (cls == 0) ncell_tile += h.ncell;
-      if (cls == 1) ncell_warp += h.ncell;
+      if (cls == 1) {
+        ncell_warp += h.ncell;
+        e->lane_rest |= h.sc.rest_on != 0;
+      }
       if (cls == 2) ncell_va += h.ncell;
     }
     if (cls == 0) lane_p0 = dense;
@@ -786,7 +799,7 @@ inline void mark(Engine *e, int slot) {
   if (e->profiling) cudaEventRecord(e->prof_ev[slot], e->stream);
 }
 
-inline int eval_cells(Engine *e, KArgs &a, int prec, int rk_form, int kq, double kcdt, bool marks = true);
+inline int eval_cells(Engine *e, KArgs &a, int prec, bool rests, int rk_form, int kq, double kcdt, bool marks = true);
 
 // One evaluation's binning.  Verlet engines: refresh the Verlet-order copies
 // of the stage state and rebuild the rows when the displacement test (or a
@@ -806,9 +819,9 @@ inline int eval_stage(Engine *e, KArgs &a, int rk_form, int kq, double kcdt, boo
   }
   if (!verlet_ok) {
     if (e->verlet) e->verlet_stale = true;
-    return eval_cells(e, a, kPrecFP64, rk_form, kq, kcdt);
+    return eval_cells(e, a, kPrecFP64, false, rk_form, kq, kcdt);
   }
-  if (!e->verlet) return eval_cells(e, a, e->precision, rk_form, kq, kcdt);
+  if (!e->verlet) return eval_cells(e, a, e->precision, e->any_rest, rk_form, kq, kcdt);
   const int n = e->n_active;
   cudaStream_t st = e->stream;
   // the gather and the rebuild see the build tables; the caller's arguments
@@ -823,7 +836,7 @@ inline int eval_stage(Engine *e, KArgs &a, int rk_form, int kq, double kcdt, boo
     k_vgather<kPrecFP64><<<blocks_for(n, 256), 256, 0, st>>>(b, rk_form, kq, kcdt);
   SPC_LAUNCHED(e);
   mark(e, 1);
-  SPC_TRY(eval_cells(e, b, e->precision, rk_form, kq, kcdt, false));
+  SPC_TRY(eval_cells(e, b, e->precision, e->any_rest, rk_form, kq, kcdt, false));
   mark(e, 2);
   k_verlet_build<<<std::min(std::max(e->ncell_total, 1), 152 * 16), kVThreads, 0, st>>>(b);
   SPC_LAUNCHED(e);
@@ -832,9 +845,9 @@ inline int eval_stage(Engine *e, KArgs &a, int rk_form, int kq, double kcdt, boo
 }
 
 // Cell-list binning: stage, sort, cell bounds, cell-order gather (for the
-// passes of precision prec).  marks: record the profiling events after each
-// part.
-inline int eval_cells(Engine *e, KArgs &a, int prec, int rk_form, int kq, double kcdt, bool marks) {
+// passes of precision prec; rests: with the rests of the systems that have
+// them).  marks: record the profiling events after each part.
+inline int eval_cells(Engine *e, KArgs &a, int prec, bool rests, int rk_form, int kq, double kcdt, bool marks) {
   const int n = e->n_active;
   cudaStream_t st = e->stream;
   const int nkeys = a.cell_mid ? 2 * e->ncell_total : e->ncell_total;
@@ -848,11 +861,13 @@ inline int eval_cells(Engine *e, KArgs &a, int prec, int rk_form, int kq, double
     if (marks) mark(e, 2);
     const int blocks = blocks_for((long long)(n + nkeys) * kRankLanes, kRankThreads);
     if (prec == kPrecFP32C)
-      k_rank_gather<kPrecFP32C><<<blocks, kRankThreads, 0, st>>>(a, nkeys);
+      k_rank_gather<kPrecFP32C, false><<<blocks, kRankThreads, 0, st>>>(a, nkeys);
     else if (prec == kPrecFP32X)
-      k_rank_gather<kPrecFP32X><<<blocks, kRankThreads, 0, st>>>(a, nkeys);
+      k_rank_gather<kPrecFP32X, true><<<blocks, kRankThreads, 0, st>>>(a, nkeys);
+    else if (rests)
+      k_rank_gather<kPrecFP64, true><<<blocks, kRankThreads, 0, st>>>(a, nkeys);
     else
-      k_rank_gather<kPrecFP64><<<blocks, kRankThreads, 0, st>>>(a, nkeys);
+      k_rank_gather<kPrecFP64, false><<<blocks, kRankThreads, 0, st>>>(a, nkeys);
     SPC_LAUNCHED(e);
   } else {
     if (nkeys <= kScanOneCta) {
@@ -868,11 +883,13 @@ inline int eval_cells(Engine *e, KArgs &a, int prec, int rk_form, int kq, double
     SPC_LAUNCHED(e);
     if (marks) mark(e, 2);
     if (prec == kPrecFP32C)
-      k_gather<kPrecFP32C><<<blocks_for(n, 256), 256, 0, st>>>(a);
+      k_gather<kPrecFP32C, false><<<blocks_for(n, 256), 256, 0, st>>>(a);
     else if (prec == kPrecFP32X)
-      k_gather<kPrecFP32X><<<blocks_for(n, 256), 256, 0, st>>>(a);
+      k_gather<kPrecFP32X, true><<<blocks_for(n, 256), 256, 0, st>>>(a);
+    else if (rests)
+      k_gather<kPrecFP64, true><<<blocks_for(n, 256), 256, 0, st>>>(a);
     else
-      k_gather<kPrecFP64><<<blocks_for(n, 256), 256, 0, st>>>(a);
+      k_gather<kPrecFP64, false><<<blocks_for(n, 256), 256, 0, st>>>(a);
     SPC_LAUNCHED(e);
   }
   if (a.units && e->ncell_tile > 0 && !e->verlet) {  // the cell units of this evaluation
@@ -902,6 +919,17 @@ void launch_allpairs(const KArgs &a, int epi, int items, int items_small, cudaSt
 // one-warp CTAs take the SM's shared memory: FP64 N = 65,536 74 us a step
 // with them, 58 with four warps).
 inline int lane_threads(int np) { return np > 152 * 8 * kWarp ? kLaneThreads : kWarp; }
+
+template <int PREC, int KIND, bool REST>
+void launch_lane(const KArgs &a, int epi, cudaStream_t st) {
+  const int np = a.lane_p1 - a.lane_p0;
+  if (np <= kLaneGroupMax<PREC>) {
+    k_lane<PREC, KIND, kLaneGroup, REST><<<blocks_for((long long)np * kLaneGroup, kWarp), kWarp, 0, st>>>(a, epi);
+  } else {
+    const int threads = lane_threads(np);
+    k_lane<PREC, KIND, 1, REST><<<blocks_for(np, threads), threads, 0, st>>>(a, epi);
+  }
+}
 
 template <int PREC, int KIND>
 int launch_pass_t(Engine *e, const KArgs &a, int epi) {
@@ -982,12 +1010,13 @@ int launch_pass_t(Engine *e, const KArgs &a, int epi) {
           if (a.units) SPC_CUDA(e, cudaStreamWaitEvent(st, e->join_ev, 0));
       }
       if (e->ncell_warp > 0) {
-        const int np = a.lane_p1 - a.lane_p0;
-        if (np <= kLaneGroupMax<PREC>) {
-          k_lane<PREC, KIND, kLaneGroup><<<blocks_for((long long)np * kLaneGroup, kWarp), kWarp, 0, st>>>(a, epi);
+        if constexpr (PREC == kPrecFP64 && KIND == kKindSin) {
+          if (e->lane_rest)
+            launch_lane<PREC, KIND, true>(a, epi, st);
+          else
+            launch_lane<PREC, KIND, false>(a, epi, st);
         } else {
-          const int threads = lane_threads(np);
-          k_lane<PREC, KIND, 1><<<blocks_for(np, threads), threads, 0, st>>>(a, epi);
+          launch_lane<PREC, KIND, false>(a, epi, st);
         }
         SPC_LAUNCHED(e);
       }

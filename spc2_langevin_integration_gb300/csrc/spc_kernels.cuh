@@ -109,6 +109,7 @@ struct KArgs {
                                      // va_p1): x relative to the column block's), kFxyPad entries more
   float2 *cs;                        // FP32C: (cos phi, sin phi)
   double2 *dcs;                      // FP64 passes: (cos phi, sin phi) of the stage phase
+  uint16_t *rest;                    // and their rests (sincos_phase_rest)
   longlong2 *ics;                    // FP32X: (cos phi, sin phi) in fixed point (2^kXQ)
   // float forms, cell-tile slots: the values of the two passes as digits in
   // halves, 16 bytes (FP32X: 32) a slot (float_digits, fixed_digits); FP32C SRK:
@@ -299,8 +300,20 @@ __device__ __forceinline__ void fixed_digits(longlong2 v, uint4 *to) {
   to[1] = make_uint4(halves(d[8], d[9]), halves(1.0f, bad ? 1.0f : 0.0f), 0u, 0u);
 }
 
+// What the FP64 passes need of a phase, for slot p.
+// REST: false when no system has rests (rest_on).
+template <bool REST>
+__device__ __forceinline__ void gather_cs64(const KArgs &a, const SysConst &sc, double ph, int p) {
+  double s, c;
+  if (REST && sc.rest_on)
+    a.rest[p] = sincos_phase_rest(ph, s, c);
+  else
+    sincos_phase(ph, s, c);
+  a.dcs[p] = make_double2(c, s);
+}
+
 // Dense particle d into cell-order slot p.
-template <int PREC>
+template <int PREC, bool REST>
 __device__ __forceinline__ void gather_to(const KArgs &a, int d, const StageRec &r, int p) {
   const SysDesc &sd = a.sys[r.sys];
   const SysConst &sc = sd.sc;
@@ -335,16 +348,12 @@ __device__ __forceinline__ void gather_to(const KArgs &a, int d, const StageRec 
     const longlong2 v = to_fixed2(c, s, kXQ);
     a.ics[p] = v;
     if (p < a.lane_p0) fixed_digits(v, a.dig + 2 * (size_t)p);
-    if (sc.allpairs) a.dcs[p] = make_double2(c, s);  // its passes are the FP64 ones
+    if (sc.allpairs) gather_cs64<REST>(a, sc, ph, p);  // its passes are the FP64 ones
   }
-  if constexpr (PREC == kPrecFP64) {
-    double s, c;
-    sincos_phase(ph, s, c);
-    a.dcs[p] = make_double2(c, s);
-  }
+  if constexpr (PREC == kPrecFP64) gather_cs64<REST>(a, sc, ph, p);
 }
 
-template <int PREC>
+template <int PREC, bool REST>
 __global__ void k_gather(KArgs a) {
   if (a.gate && *a.gate == 0) return;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -365,7 +374,7 @@ __global__ void k_gather(KArgs a) {
     }
     for (; k < c1; ++k) p += a.list[k] < d ? 1 : 0;
   }
-  gather_to<PREC>(a, d, r, p);
+  gather_to<PREC, REST>(a, d, r, p);
 }
 
 // Few particles: no counting and no list.  Sixteen lanes count the particles
@@ -380,7 +389,7 @@ constexpr int kRankMax = 2048;
 constexpr int kRankLanes = 16, kRankThreads = 32;
 static_assert(kRankMax <= 1 << kRankBits && (uint64_t)kScanOneCta << kRankBits < 0xffffffffu, "ranks fit 32 bits");
 
-template <int PREC>
+template <int PREC, bool REST>
 __global__ void __launch_bounds__(kRankThreads) k_rank_gather(KArgs a, int nkeys) {
   if (a.gate && *a.gate == 0) return;
   const int n = a.n_active;
@@ -401,7 +410,7 @@ __global__ void __launch_bounds__(kRankThreads) k_rank_gather(KArgs a, int nkeys
   for (int off = 1; off < kRankLanes; off <<= 1) p += __shfl_xor_sync(0xffffffffu, p, off);
   if (sub != 0) return;
   if (q < n)
-    gather_to<PREC>(a, q, a.stg[q], p);
+    gather_to<PREC, REST>(a, q, a.stg[q], p);
   else if (q < n + nkeys)
     (a.cell_mid && (key & 1u) ? a.cell_mid : a.cell_start)[a.cell_mid ? key >> 1 : key] = p;
 }
@@ -415,7 +424,8 @@ template <>
 struct Acc<kPrecFP64> {
   double s0, s1;  // sin sum | cos/n sum, (dphi) cos/n sum | cos, sin sums
   int n;
-  __device__ void init() { s0 = 0.0; s1 = 0.0; n = 0; }
+  long long rest; // sin sum: the terms' rests, in units of 2^-68 (sine_rest; up to 2^17 each)
+  __device__ void init() { s0 = 0.0; s1 = 0.0; n = 0; rest = 0; }
 };
 
 template <>
@@ -472,6 +482,10 @@ struct ILane {
   double dphi;  // pass 2: own phase rate
   float ca, sa; // FP32C: cos(phi + alpha), sin(phi + alpha)
   double dca, dsa;  // FP64: the same in double
+  bool rest;        // FP64 pass 1: sine_rest, with the sectors that are near and
+  int rest_from, rest_own;  // the own rest (units of 2^-68, with the offset)
+  uint32_t dsa_lo, dsa_hi;  // dsa's significand and exponent, for rest_of_product
+  int dsa_e;
   float dphif;
 };
 
@@ -488,7 +502,44 @@ struct ILane {
 // phases.  The terms are added in the reference's order as before; the mean of
 // 200 terms is 2.4e-17 (uniform phases, before 2.9e-17) to 3.5e-16 (aligned,
 // alpha = 1.45: the same as before) from the exact one.  Vortex SRK step,
-// N = 65,536: 2.96 -> 0.45 ms on the cell list.
+// N = 65,536: 2.96 -> 0.45 ms on the cell list (0.47 with the rests below).
+//
+// Between aligned phases (alpha small) 3.5e-16 is far more than the rounding of
+// the small sine that the reference gets.  Three things make up that error: the
+// rounding of the particles' cosines and sines, which turns either by up to
+// 2^-53.4; that of (dca, dsa); and that of one product.  The first two are kept
+// as an angle per particle (rest), the third is found by an integer product, and
+// where the phases are within two sectors of 22.5 degrees (the cosine of the
+// difference is near 1) their sum goes to an integer, so that it depends on no
+// order.  Mean of 200 terms, error against 64 bits over that of the sines of the
+// differences, phases spread by sd about one phase, alpha = 0: sd 3e-4 54 -> 1.1,
+// 1e-3 47 -> 1.0, 1e-2 6.7 -> 1.1, 0.1 1.2 -> 1.0 (20 terms: 170, 139, 18, 2.2 ->
+// at most 1.3); alpha = 0.1, sd 1e-2: 1.3 -> 1.0.  From |alpha| = 0.5 on the
+// reference's own rounding of the difference is as large, and nothing is kept.
+// Some 25 integer instructions a pair, beside the 48 cycles that the FP64 pipe
+// takes for a warp's pair, and 26 FP64 operations a particle in the gather: vortex
+// SRK, N = 65,536, pass 1 171 -> 189 us and gather 6 -> 9 (with the product's rest
+// by a fused multiply-add, pass 1 was 220).
+constexpr double kRestAlpha = 0.5;
+constexpr uint32_t kRestNear = 5u << 12;
+// (c dsa - p) 2^68, p = RN(c dsa), |p| <= 1, by integers: the product of the
+// significands from its last place of p on, modulo 2^64, is what rounding left of
+// it, a signed number of 52 or 53 bits.
+__device__ __forceinline__ int rest_of_product(const ILane &il, double c, double p) {
+  const int hi = __double2hiint(c), ep = (__double2hiint(p) >> 20) & 0x7ff;
+  const uint32_t lo = (uint32_t)__double2loint(c), mh = ((uint32_t)hi & 0xfffffu) | 0x100000u;
+  const uint64_t low = (uint64_t)lo * il.dsa_lo;
+  const uint32_t up = (uint32_t)(low >> 32) + lo * il.dsa_hi + mh * il.dsa_lo;
+  const int carry = ep - ((hi >> 20) & 0x7ff) - il.dsa_e;  // 1: 53 bits
+  const int x = (int)__funnelshift_l((uint32_t)low, up, 12 - carry);
+  const int v = x >> min((unsigned)(1039 - ep), 31u);
+  return __double2hiint(p) < 0 ? -v : v;
+}
+// What the term fma(cj.y, dca, -p), p = RN(cj.x dsa), lacks; w: j's rest.
+__device__ __forceinline__ int sine_rest(const ILane &il, uint32_t w, double cjx, double p) {
+  const int v = (int)((w & 0xfffu) << 4) - il.rest_own - rest_of_product(il, cjx, p);
+  return ((w - (uint32_t)il.rest_from) & 0xffffu) < kRestNear ? v : 0;
+}
 __device__ __noinline__ double sin_of_difference(double pj, double pi, double alpha) {
   return sin(dsub(dsub(pj, pi), alpha));
 }
@@ -500,14 +551,19 @@ __device__ __forceinline__ bool small_term(double t) {
   return (unsigned)(__double2hiint(t) & 0x7fffffff) < 0x3f400000u;
 }
 // One accepted pair: pass 1 adds the sine, pass 2 the cosine and the cosine
-// weighted by the difference of the phase rates.  phase() gives phi_j.  The
-// second pass's quotients by n_i are taken once of each sum (finish_pairs).
-template <int KIND, class Phase>
+// weighted by the difference of the phase rates.  phase() gives phi_j, rest() its
+// rest.  The second pass's quotients by n_i are taken once of each sum
+// (finish_pairs).
+template <int KIND, class Phase, class Rest>
 __device__ __forceinline__ void add_pair(Acc<kPrecFP64> &acc, const SysConst &sc, const ILane &il, double2 cj,
-                                         double dj, Phase phase) {
+                                         double dj, Phase phase, Rest rest) {
   if constexpr (KIND == kKindSin) {
-    double t = __fma_rn(cj.y, il.dca, -dmul(cj.x, il.dsa));
-    if (small_term(t)) t = sin_of_difference(phase(), il.phi, sc.alpha);
+    const double p = dmul(cj.x, il.dsa);
+    double t = __fma_rn(cj.y, il.dca, -p);
+    if (small_term(t))
+      t = sin_of_difference(phase(), il.phi, sc.alpha);
+    else if (il.rest)
+      acc.rest += sine_rest(il, rest(), cj.x, p);
     acc.s0 = dadd(acc.s0, t);
   } else {
     double t = __fma_rn(cj.x, il.dca, dmul(cj.y, il.dsa));
@@ -517,14 +573,14 @@ __device__ __forceinline__ void add_pair(Acc<kPrecFP64> &acc, const SysConst &sc
   }
 }
 // A particle's neighbours as words of bits (bit 31 of a word is its entry
-// `base`): next(bits, base) gives the next word that is not zero, cs(k), rate(k)
-// and phase(k) what entry k's pair needs.  U neighbours of a word are taken at
+// `base`): next(bits, base) gives the next word that is not zero, cs(k), rate(k),
+// phase(k) and rest(k) what entry k's pair needs.  U neighbours of a word are taken at
 // a time: their terms are independent, so only the additions wait for one
 // another (a dependent FP64 operation takes over 100 cycles, and the small
 // systems have one warp per SM).
-template <int KIND, int U, class Next, class Cs, class Rate, class Phase>
+template <int KIND, int U, bool REST, class Next, class Cs, class Rate, class Phase, class Rest>
 __device__ __forceinline__ void walk_pairs(Acc<kPrecFP64> &acc, const SysConst &sc, const ILane &il, Next next,
-                                           Cs cs, Rate rate, Phase phase) {
+                                           Cs cs, Rate rate, Phase phase, Rest rest) {
   uint32_t bits = 0u;
   int base = 0;
   while (bits != 0u || next(bits, base)) {
@@ -538,21 +594,31 @@ __device__ __forceinline__ void walk_pairs(Acc<kPrecFP64> &acc, const SysConst &
       bits &= ~(0x80000000u >> (t & 31));
     }
     double t[U], d[U];
+    int r[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const double2 cj = cs(k[u]);
-      t[u] = KIND == kKindSin ? __fma_rn(cj.y, il.dca, -dmul(cj.x, il.dsa))
-                              : __fma_rn(cj.x, il.dca, dmul(cj.y, il.dsa));
+      r[u] = 0;
+      if constexpr (KIND == kKindSin) {
+        const double p = dmul(cj.x, il.dsa);
+        t[u] = __fma_rn(cj.y, il.dca, -p);
+        if (REST && il.rest) r[u] = sine_rest(il, rest(k[u]), cj.x, p);
+      } else {
+        t[u] = __fma_rn(cj.x, il.dca, dmul(cj.y, il.dsa));
+      }
       d[u] = KIND == kKindCos2 ? dsub(rate(k[u]), il.dphi) : 0.0;
     }
 #pragma unroll
     for (int u = 0; u < U; ++u)
-      if (small_term(t[u]))
+      if (small_term(t[u])) {
         t[u] = KIND == kKindSin ? sin_of_difference(phase(k[u]), il.phi, sc.alpha)
                                 : cos_of_difference(phase(k[u]), il.phi, sc.alpha);
+        r[u] = 0;
+      }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       if (!has[u]) continue;
+      if constexpr (KIND == kKindSin) acc.rest += r[u];
       acc.s0 = dadd(acc.s0, t[u]);
       if constexpr (KIND == kKindCos2) acc.s1 = __fma_rn(d[u], t[u], acc.s1);
     }
@@ -560,7 +626,9 @@ __device__ __forceinline__ void walk_pairs(Acc<kPrecFP64> &acc, const SysConst &
 }
 template <int KIND>
 __device__ __forceinline__ void finish_pairs(Acc<kPrecFP64> &acc, const ILane &il) {
-  if constexpr (KIND == kKindCos2) {
+  if constexpr (KIND == kKindSin) {
+    if (acc.rest != 0) acc.s0 = __fma_rn((double)acc.rest, 0x1p-68, acc.s0);
+  } else if constexpr (KIND == kKindCos2) {
     if (il.cnt > 0) {
       const Count n = count_of(il.cnt);
       acc.s0 = ddiv_by(acc.s0, n.n, n.r);
@@ -603,7 +671,8 @@ __device__ __forceinline__ void accept_pair(const KArgs &a, const SysDesc &sd, c
                                             float dphij_f, long long &wpos) {
   if constexpr (KIND == kKindSin) {
     if constexpr (PREC == kPrecFP64) {
-      add_pair<KIND>(acc, sd.sc, il, a.dcs[pj], 0.0, [&]() { return a.sphi[pj]; });  // ChimeraSystem.cpp:412
+      add_pair<KIND>(acc, sd.sc, il, a.dcs[pj], 0.0, [&]() { return a.sphi[pj]; },
+                     [&]() { return (uint32_t)a.rest[pj]; });  // ChimeraSystem.cpp:412
     } else {
       // sin(phi_j - (phi_i + alpha)) by the angle-difference identity
       kahan_add(acc.s0, acc.c0, cjs * il.ca - cjc * il.sa);
@@ -611,7 +680,8 @@ __device__ __forceinline__ void accept_pair(const KArgs &a, const SysDesc &sd, c
     acc.n++;
   } else if constexpr (KIND == kKindCos2) {
     if constexpr (PREC == kPrecFP64) {
-      add_pair<KIND>(acc, sd.sc, il, a.dcs[pj], a.dphi_s[pj], [&]() { return a.sphi[pj]; });  // :634-637
+      add_pair<KIND>(acc, sd.sc, il, a.dcs[pj], a.dphi_s[pj], [&]() { return a.sphi[pj]; },
+                     []() { return 0u; });  // :634-637
     } else {
       const float c = cjc * il.ca + cjs * il.sa;
       kahan_add(acc.s0, acc.c0, c);
@@ -831,10 +901,12 @@ __device__ void epilogue(const KArgs &a, int epi, const SysDesc &sd, const ILane
   }
 }
 
-template <int PREC, int KIND>
+// REST: false when no system of the launch has rests (rest_on).
+template <int PREC, int KIND, bool REST = true>
 __device__ __forceinline__ void load_i(const KArgs &a, const SysConst &sc, ILane &il, int p, bool valid) {
   il.p = p;
   il.valid = valid;
+  il.rest = REST && PREC == kPrecFP64 && KIND == kKindSin && valid && sc.rest_on;
   if (!valid) return;
   il.x = a.sx[p];
   il.y = a.sy[p];
@@ -853,8 +925,23 @@ __device__ __forceinline__ void load_i(const KArgs &a, const SysConst &sc, ILane
   }
   if constexpr (PREC == kPrecFP64 && KIND != kKindNb) {
     const double2 t = a.dcs[p];
-    il.dca = __fma_rn(t.x, sc.cos_ad, -dmul(t.y, sc.sin_ad));
-    il.dsa = __fma_rn(t.y, sc.cos_ad, dmul(t.x, sc.sin_ad));
+    const double u = dmul(t.y, sc.sin_ad), v = dmul(t.x, sc.sin_ad);
+    il.dca = __fma_rn(t.x, sc.cos_ad, -u);
+    il.dsa = __fma_rn(t.y, sc.cos_ad, v);
+    if (REST && KIND == kKindSin && il.rest) {
+      const uint32_t w = a.rest[p];
+      il.rest_from = (int)(w & 0xf000u) + ((sc.rest_sector - 2) << 12);
+      il.rest_own = (int)((w & 0xfffu) << 4);
+      const int hi = __double2hiint(il.dsa), e = (hi >> 20) & 0x7ff;
+      il.dsa_lo = (uint32_t)__double2loint(il.dsa);
+      il.dsa_hi = e ? ((uint32_t)hi & 0xfffffu) | 0x100000u : 0u;
+      il.dsa_e = e - 1023;
+      if (sc.alpha != 0.0) {  // and that of (dca, dsa), from what its roundings left
+        const double cl = dsub(dsub(__fma_rn(t.x, sc.cos_ad, -il.dca), u), __fma_rn(t.y, sc.sin_ad, -u));
+        const double sl = dadd(dadd(__fma_rn(t.y, sc.cos_ad, -il.dsa), v), __fma_rn(t.x, sc.sin_ad, -v));
+        il.rest_own += small_to_int(dadd(__fma_rn(il.dca, sl, -dmul(il.dsa, cl)), sc.rest_alpha), 68);
+      }
+    }
   }
   if constexpr (KIND == kKindCos2) {
     il.cnt = a.cnt_s[p];
@@ -970,6 +1057,7 @@ __global__ void __launch_bounds__(T) k_allpairs_pass(KArgs a, int epi) {
   __shared__ __align__(16) float2 t_xy[kAllPairsCap];
   __shared__ double2 t_cs[kPair64 ? kAllPairsCap : 1];
   __shared__ double t_d[kPair64 && KIND == kKindCos2 ? kAllPairsCap : 1];
+  __shared__ uint16_t t_r[kPair64 && KIND == kKindSin ? kAllPairsCap : 1];
   __shared__ float2 t_csf[PREC == kPrecFP32C ? kAllPairsCap : 1];
   __shared__ float t_df[PREC == kPrecFP32C && KIND == kKindCos2 ? kAllPairsCap : 1];
   __shared__ uint32_t t_out[kWords];   // candidates outside the box (first_bits order)
@@ -1017,6 +1105,8 @@ __global__ void __launch_bounds__(T) k_allpairs_pass(KArgs a, int epi) {
           if constexpr (kPair64) {
             t_cs[k] = a.dcs[j];
             if constexpr (KIND == kKindCos2) t_d[k] = a.dphi_s[j];
+            if constexpr (KIND == kKindSin)
+              if (sc.rest_on) t_r[k] = a.rest[j];
           }
           if constexpr (PREC == kPrecFP32C) {
             t_csf[k] = a.cs[j];
@@ -1074,9 +1164,10 @@ __global__ void __launch_bounds__(T) k_allpairs_pass(KArgs a, int epi) {
         return bits != 0u;
       };
       if constexpr (kPair64) {
-        walk_pairs<KIND, kAP64>(
+        walk_pairs<KIND, kAP64, true>(
             acc, sc, il, next, [&](int k) { return t_cs[k]; }, [&](int k) { return t_d[KIND == kKindCos2 ? k : 0]; },
-            [&](int k) { return a.sphi[jt + k]; });
+            [&](int k) { return a.sphi[jt + k]; },
+            [&](int k) { return (uint32_t)t_r[KIND == kKindSin ? k : 0]; });
       } else {
         uint32_t bits = 0u;
         int base = 0;

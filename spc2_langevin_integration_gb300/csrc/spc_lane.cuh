@@ -251,8 +251,10 @@ __device__ __forceinline__ int group_pick(uint32_t &bits, int slot, int g, int m
   return j;
 }
 
-// G lanes per particle: 1 or kLaneGroup.
-template <int PREC, int KIND, int G>
+// G lanes per particle: 1 or kLaneGroup.  REST (FP64 pass 1): some system has
+// rests.  (The gather and this kernel compiled without them: an Euler step of N =
+// 1,024 at alpha = 1.45 takes 25.2 us, 26.7 with a test at run time.)
+template <int PREC, int KIND, int G, bool REST = false>
 __global__ void __launch_bounds__(kLaneThreads, PREC != kPrecFP64 && G == 1 ? 10 : 1) k_lane(KArgs a, int epi) {
   constexpr bool kList = PREC == kPrecFP64;
   __shared__ uint32_t s_bits[kList ? kLaneWords : 1][kLaneThreads];
@@ -267,7 +269,7 @@ __global__ void __launch_bounds__(kLaneThreads, PREC != kPrecFP64 && G == 1 ? 10
   const SysDesc &sd = a.sys[a.sys_of_c[c]];
   const SysConst &sc = sd.sc;
   ILane il;
-  load_i<PREC, KIND>(a, sc, il, p, true);
+  load_i<PREC, KIND, REST>(a, sc, il, p, true);
   LaneSums<PREC, KIND> sums;
   sums.init();
   int n = 0;
@@ -278,7 +280,7 @@ __global__ void __launch_bounds__(kLaneThreads, PREC != kPrecFP64 && G == 1 ? 10
   auto walk_list = [&]() {
     if constexpr (kList) {
       int w = -1;
-      walk_pairs<KIND, kLanePairs>(
+      walk_pairs<KIND, kLanePairs, REST>(
           sums.acc, sc, il,
           [&](uint32_t &bits, int &base) {
             if (++w >= nw) return false;
@@ -286,7 +288,8 @@ __global__ void __launch_bounds__(kLaneThreads, PREC != kPrecFP64 && G == 1 ? 10
             base = s_slot[w][tid];
             return true;
           },
-          [&](int j) { return a.dcs[j]; }, [&](int j) { return a.dphi_s[j]; }, [&](int j) { return a.sphi[j]; });
+          [&](int j) { return a.dcs[j]; }, [&](int j) { return a.dphi_s[j]; }, [&](int j) { return a.sphi[j]; },
+          [&](int j) { return (uint32_t)a.rest[j]; });
       nw = 0;
     }
   };
@@ -437,12 +440,16 @@ __global__ void __launch_bounds__(kLaneThreads, PREC != kPrecFP64 && G == 1 ? 10
         if (!__any_sync(kAll, m > 0)) break;
         const int j = group_pick(bits, slot, g, m, p);
         const double2 cj = a.dcs[j];
-        double t = KIND == kKindSin ? __fma_rn(cj.y, il.dca, -dmul(cj.x, il.dsa))
-                                    : __fma_rn(cj.x, il.dca, dmul(cj.y, il.dsa));
+        const double pr = KIND == kKindSin ? -dmul(cj.x, il.dsa) : dmul(cj.y, il.dsa);
+        double t = __fma_rn(KIND == kKindSin ? cj.y : cj.x, il.dca, pr);
         const double d = KIND == kKindCos2 ? dsub(a.dphi_s[j], il.dphi) : 0.0;
-        if (g < m && small_term(t))
-          t = KIND == kKindSin ? sin_of_difference(a.sphi[j], il.phi, sc.alpha)
-                               : cos_of_difference(a.sphi[j], il.phi, sc.alpha);
+        if (g < m) {
+          if (small_term(t))
+            t = KIND == kKindSin ? sin_of_difference(a.sphi[j], il.phi, sc.alpha)
+                                 : cos_of_difference(a.sphi[j], il.phi, sc.alpha);
+          else if (REST && il.rest)
+            sums.acc.rest += sine_rest(il, a.rest[j], cj.x, -pr);
+        }
         __syncwarp();
 #pragma unroll
         for (int u = 0; u < G; ++u) {
@@ -459,7 +466,10 @@ __global__ void __launch_bounds__(kLaneThreads, PREC != kPrecFP64 && G == 1 ? 10
       sums.join_group(kAll, lead);
     }
 #pragma unroll
-    for (int o = 1; o < G; o <<= 1) n += __shfl_xor_sync(kAll, n, o);
+    for (int o = 1; o < G; o <<= 1) {
+      n += __shfl_xor_sync(kAll, n, o);
+      if constexpr (REST) sums.acc.rest += __shfl_xor_sync(kAll, sums.acc.rest, o);
+    }
     if (g != 0 || p_own >= a.lane_p1) return;
     if (alone) {  // the first lane walks as it tests
       n = nw = 0;

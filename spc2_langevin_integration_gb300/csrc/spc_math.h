@@ -109,6 +109,39 @@ SPC_MATH_FN void sincos_in_range(double ph, double &s, double &c) {
   circle_point(static_cast<int>(double_to_bits(t)), d, s, c);
 }
 
+// The same sine and cosine, bit for bit, with the point's number k and the angle
+// `rest` by which the phase exceeds that of the rounded pair (|rest| < 2^-53.4,
+// within 2^-59): every rounding on the way kept as a second double.  26 more
+// operations.
+SPC_MATH_FN void sincos_with_rest(double ph, double &s, double &c, int &k, double &rest) {
+  const double t = fma_rn(ph, 0x1.45f306dc9c883p+4, kRoundMagic);  // 64 / pi
+  const double n = add_rn(t, -kRoundMagic);
+  const double d1 = fma_rn(-n, 0x1.921fb54442d18p-5, ph);  // exact
+  const double d = fma_rn(-n, 0x1.1a62633145c07p-59, d1);
+  const double dl = fma_rn(-n, 0x1.1a62633145c07p-59, add_rn(d1, -d));
+  k = static_cast<int>(double_to_bits(t)) & 127;
+  const double4_t p = kCircle[k];
+  const double d2 = mul_rn(d, d), d3 = mul_rn(d, d2);
+  const double cm1 = mul_rn(d2, fma_rn(d2, fma_rn(d2, -1.0 / 720.0, 1.0 / 24.0), -0.5));
+  const double q = fma_rn(d2, fma_rn(d2, -1.0 / 5040.0, 1.0 / 120.0), -1.0 / 6.0);
+  const double sn = fma_rn(d3, q, d);
+  const double snl = add_rn(fma_rn(d3, q, add_rn(d, -sn)), dl);
+  const double ic = fma_rn(-p.y, sn, p.z), is = fma_rn(p.x, sn, p.w);
+  const double wc = fma_rn(p.x, cm1, ic), ws = fma_rn(p.y, cm1, is);
+  c = add_rn(p.x, wc);
+  s = add_rn(p.y, ws);
+  const double icl = add_rn(fma_rn(-p.y, sn, -ic), p.z), isl = add_rn(fma_rn(p.x, sn, -is), p.w);
+  const double wcl = add_rn(fma_rn(p.x, cm1, add_rn(ic, -wc)), fma_rn(-p.y, snl, icl));
+  const double wsl = add_rn(fma_rn(p.y, cm1, add_rn(is, -ws)), fma_rn(p.x, snl, isl));
+  const double cl = add_rn(add_rn(add_rn(p.x, -c), wc), wcl), sl = add_rn(add_rn(add_rn(p.y, -s), ws), wsl);
+  rest = fma_rn(c, sl, -mul_rn(s, cl));
+}
+
+// RN(v 2^q) for |v 2^q| < 2^31, by one addition.
+SPC_MATH_FN int small_to_int(double v, int q) {
+  return static_cast<int>(double_to_bits(add_rn(v, kRoundMagic * pow2i(-q))));
+}
+
 // cos and sin of 2 pi b 2^-53, b < 2^53.
 SPC_MATH_FN void sincos_turn53(std::uint64_t b, double &s, double &c) {
   const std::uint64_t k = (b + (1ull << 45)) >> 46;

@@ -199,8 +199,8 @@ __global__ void k_list_units(KArgs a) {
 // FP64 terms run on ~90% full warps.  The SRK first pass keeps the words of
 // one-round cells in nbmask and the second pass tests nothing again.
 // Bound by the FP64 pipe (3 operations per pair in pass 1, 5 in pass 2).
-// Vortex SRK, N = 65,536: pass 1 2.04 ms -> 171 us, pass 2 0.92 ms ->
-// 250 us (against sines per pair and a queue of accepted candidates).  704
+// Vortex SRK, N = 65,536: pass 1 2.04 ms -> 171 us (189 with the terms' rests,
+// for alpha below 0.5), pass 2 0.92 ms -> 250 us (against sines per pair and a queue of accepted candidates).  704
 // candidates per round leave room for 7 CTAs per SM in pass 2.
 // The neighbour diagnostics (kKindNb: counts, lists in visiting order, local
 // order parameters) are the same walk.  Order parameters of N = 65,536 at 64 a
@@ -214,6 +214,7 @@ __global__ void __launch_bounds__(kTileThreads64) k_tile_fp64(KArgs a, int epi) 
   __shared__ __align__(16) float2 s_xy[kTileCap64];  // x+shift, y+shift (prefilter; padded to 32)
   __shared__ double2 s_cs[kTileCap64];               // cos, sin of the stage phase
   __shared__ double s_d[KIND == kKindCos2 ? kTileCap64 : 1];  // pass 2: phase rate
+  __shared__ uint16_t s_r[KIND == kKindSin ? kTileCap64 : 1];  // pass 1: rest of the phase
   __shared__ uint32_t s_w[(kTileWords64 + 3) / 4 * 4][kTileThreads64];
   const int tid = threadIdx.x;
   const int n_all = a.n_active;
@@ -256,6 +257,8 @@ __global__ void __launch_bounds__(kTileThreads64) k_tile_fp64(KArgs a, int epi) 
               const int pj = slot_of(st, rlo + k, q);
               s_cs[k] = a.dcs[pj];
               if constexpr (KIND == kKindCos2) s_d[k] = a.dphi_s[pj];
+              if constexpr (KIND == kKindSin)
+                if (sc.rest_on) s_r[k] = a.rest[pj];
               if (KIND == kKindCos2 && masked) continue;
               const float2 f = a.fxy[pj];
               s_xy[k] = make_float2(f.x + shift_x(q, sc.cell_f), f.y + shift_y(q, sc.cell_f));
@@ -331,13 +334,14 @@ __global__ void __launch_bounds__(kTileThreads64) k_tile_fp64(KArgs a, int epi) 
             }
           }
         } else {
-          walk_pairs<KIND, 2>(
+          walk_pairs<KIND, 2, true>(
               acc, sc, il, next, [&](int j) { return s_cs[j]; },
               [&](int j) { return s_d[KIND == kKindCos2 ? j : 0]; },
               [&](int j) {
                 int q;
                 return a.sphi[slot_of(st, rlo + j, q)];
-              });
+              },
+              [&](int j) { return (uint32_t)s_r[KIND == kKindSin ? j : 0]; });
         }
       }
       if (valid) {

@@ -19,7 +19,9 @@
 //  * sin and cos of phi_j - phi_i and of the bearing minus phi_i come from the
 //    particles' cos and sin, (dx, dy) / dr and the angle-difference identities
 //    (a small sine or cosine is evaluated as the reference writes it, as in
-//    add_pair), and the strengths from their polynomials' coefficients;
+//    add_pair; phi_j - phi_i by the differences of cos and sin and with what
+//    their roundings left), and the strengths from their polynomials'
+//    coefficients;
 //  * the quotients by the counts are taken once of each sum.
 // 19 operations a pair in pass 1 and 36 in pass 2, where sincos, atan2, quotients
 // and minimum images took about 100 and 60 with 32 bytes a pair kept between the
@@ -212,6 +214,8 @@ __global__ void __launch_bounds__(kLaneThreads) k_va_pass(KArgs a, int epi) {
   const double xi = a.sx[p], yi = a.sy[p], phii = a.sphi[p];
   const double2 ci = a.dcs[p];
   const double ddi = KIND == kKindCos2 ? a.dphi_s[p] : 0.0;
+  const uint32_t ri = a.rest[p], rest_from = (ri & 0xf000u) - (2u << 12);
+  const int rest_own = (int)(ri & 0xfffu);
   VAAcc r{0.0, 0.0, 0, 0, 0.0, 0.0, 0.0, 0.0};
 
   auto term_of = [&](int j, bool wanted) {
@@ -228,7 +232,13 @@ __global__ void __launch_bounds__(kLaneThreads) k_va_pass(KArgs a, int epi) {
     const bool in1 = !le_bits(sc.va_s_xia, dr2), in2 = !in1 && !le_bits(sc.va_s_rho, dr2);
     const double f = in1 ? __fma_rn(dr2, -sc.va_c1, sc.mu_plus)
                          : (in2 ? dmul(dmul(sc.va_c2, dsub(dr, sc.xi_a)), dsub(sc.rho, dr)) : 0.0);
-    double sp = __fma_rn(cj.y, ci.x, -dmul(cj.x, ci.y));
+    // the products of the differences round like the small sine of aligned phases
+    // does; what the rounded cosines and sines lack is added (see sine_rest)
+    const double ex = dsub(cj.x, ci.x), ey = dsub(cj.y, ci.y);
+    double sp = __fma_rn(ey, ci.x, -dmul(ex, ci.y));
+    const uint32_t rj = a.rest[j];
+    if (((rj - rest_from) & 0xffffu) < kRestNear)
+      sp = __fma_rn((double)((int)(rj & 0xfffu) - rest_own), 0x1p-64, sp);
     if (wanted && small_term(sp)) sp = sin_of_difference(a.sphi[j], phii, 0.0);
     if constexpr (KIND == kKindSin) {
       t.x = dmul(f, sp);  // VortexArraysSystemPtr.cpp:475-485
@@ -241,7 +251,7 @@ __global__ void __launch_bounds__(kLaneThreads) k_va_pass(KArgs a, int epi) {
       // VortexArraysSystemPtr.cpp:706-728
       double cp = __fma_rn(cj.x, ci.x, dmul(cj.y, ci.y));
       if (wanted && small_term(cp)) cp = cos_of_difference(a.sphi[j], phii, 0.0);
-      const double ex = dsub(cj.x, ci.x), ey = dsub(cj.y, ci.y);  // times v0: the velocity difference
+      // ex, ey times v0: the velocity difference
       // the strength's derivative over dr, times v0; at dr = 0 the reference divides 0 by 0
       double gr = in1 ? -sc.va_g1 : 0.0;
       if (in2) gr = ddiv(dmul(sc.va_g2, __fma_rn(-2.0, dr, sc.va_xr)), dr);

@@ -77,7 +77,7 @@ __device__ __forceinline__ int vstencil_entry(const int *s_prefix, int ncells, i
 template <int PREC, int KIND, bool BUILD>
 __device__ __forceinline__ void vstage_round(const KArgs &a, const SysConst &sc, const int *s_start,
                                              const int *s_prefix, int rlo, int rcnt, float4 *c4,
-                                             float2 *xy, float *df, double2 *dcs, double *dd) {
+                                             float2 *xy, float *df, double2 *dcs, double *dd, uint16_t *rest) {
   const int R = sc.vR, D = 2 * R + 1;
   for (int k = threadIdx.x; k < rcnt; k += blockDim.x) {
     const int g = rlo + k;
@@ -95,6 +95,8 @@ __device__ __forceinline__ void vstage_round(const KArgs &a, const SysConst &sc,
     if constexpr (!BUILD && PREC == kPrecFP64) {
       dcs[k] = a.dcs[pj];
       if constexpr (KIND == kKindCos2) dd[k] = a.dphi_s[pj];
+      if constexpr (KIND == kKindSin)
+        if (sc.rest_on) rest[k] = a.rest[pj];
     }
   }
 }
@@ -151,7 +153,7 @@ __global__ void __launch_bounds__(kVThreads) k_verlet_build(KArgs a) {
         const int rlo = r * kVStage32, rcnt = min(kVStage32, total - rlo);
         __syncthreads();
         vstage_round<kPrecFP64, kKindSin, true>(a, sc, s_start, s_prefix, rlo, rcnt, nullptr, s_xy,
-                                                nullptr, nullptr, nullptr);
+                                                nullptr, nullptr, nullptr, nullptr);
         __syncthreads();
         if (valid && !over) {
           for (int j = 0; j < rcnt; ++j) {
@@ -214,11 +216,7 @@ __global__ void __launch_bounds__(256) k_vgather(KArgs a, int rk_form, int kq, d
       sincosf(reduced_phase_f(ph), &s, &c);
       a.cs[v] = make_float2(c, s);
     }
-    if constexpr (PREC == kPrecFP64) {
-      double s, c;
-      sincos_phase(ph, s, c);
-      a.dcs[v] = make_double2(c, s);
-    }
+    if constexpr (PREC == kPrecFP64) gather_cs64<true>(a, sc, ph, v);
     double ex = x - a.vxb[v], ey = y - a.vyb[v];
     ex = ex > hL ? ex - sc.L : (ex < -hL ? ex + sc.L : ex);
     ey = ey > hL ? ey - sc.L : (ey < -hL ? ey + sc.L : ey);
@@ -248,6 +246,7 @@ struct VStage<kPrecFP64, KIND> {
   float2 xy[kCap];
   double2 dcs[kCap];  // cos, sin of the stage phase
   double dd[KIND == kKindCos2 ? kCap : 1];
+  uint16_t rest[KIND == kKindSin ? kCap : 1];  // pass 1 (16 bits: five CTAs' worth fit an SM, at 32 four would)
 };
 
 template <int PREC, int KIND>
@@ -337,7 +336,8 @@ __global__ void __launch_bounds__(kVThreads) k_vtile(KArgs a, int epi) {
             }
           } else {
             add_pair<KIND>(acc, sc, il, sm.dcs[j], KIND == kKindCos2 ? sm.dd[j] : 0.0,
-                           [&]() { return a.sphi[vslot_of(sc, s_start, s_prefix, g)]; });
+                           [&]() { return a.sphi[vslot_of(sc, s_start, s_prefix, g)]; },
+                           [&]() { return (uint32_t)sm.rest[KIND == kKindSin ? j : 0]; });
           }
           bits |= 1u << (k & (kWarp - 1));
         }
@@ -358,10 +358,10 @@ __global__ void __launch_bounds__(kVThreads) k_vtile(KArgs a, int epi) {
         __syncthreads();
         if constexpr (PREC == kPrecFP32C)
           vstage_round<PREC, KIND, false>(a, sc, s_start, s_prefix, rlo, rcnt, sm.c4, nullptr, sm.df,
-                                          nullptr, nullptr);
+                                          nullptr, nullptr, nullptr);
         else
           vstage_round<PREC, KIND, false>(a, sc, s_start, s_prefix, rlo, rcnt, nullptr, sm.xy, nullptr,
-                                          sm.dcs, sm.dd);
+                                          sm.dcs, sm.dd, sm.rest);
         __syncthreads();
         if (!valid) continue;
         if constexpr (kWalk) {
@@ -398,7 +398,7 @@ __global__ void __launch_bounds__(kVThreads) k_vtile(KArgs a, int epi) {
             int w = -1;
             uint32_t ahead = nw > 0 ? a.nbmask[v] : 0u;  // word w + 1
             auto staged = [&](int e) { return (int)a.vrows[((size_t)(e >> 3) * n_all + v) * 8 + (e & 7)]; };
-            walk_pairs<KIND, 2>(
+            walk_pairs<KIND, 2, true>(
                 acc, sc, il,
                 [&](uint32_t &b, int &base) {
                   while (b == 0u && ++w < nw) {
@@ -410,7 +410,8 @@ __global__ void __launch_bounds__(kVThreads) k_vtile(KArgs a, int epi) {
                 },
                 [&](int e) { return sm.dcs[staged(e)]; },
                 [&](int e) { return KIND == kKindCos2 ? sm.dd[staged(e)] : 0.0; },
-                [&](int e) { return a.sphi[vslot_of(sc, s_start, s_prefix, staged(e))]; });
+                [&](int e) { return a.sphi[vslot_of(sc, s_start, s_prefix, staged(e))]; },
+                [&](int e) { return (uint32_t)sm.rest[KIND == kKindSin ? staged(e) : 0]; });
             continue;
           }
         }
@@ -460,7 +461,8 @@ __global__ void __launch_bounds__(kVThreads) k_vtile(KArgs a, int epi) {
                     }
                   } else {
                     add_pair<KIND>(acc, sc, il, sm.dcs[j], KIND == kKindCos2 ? sm.dd[j] : 0.0,
-                           [&]() { return a.sphi[vslot_of(sc, s_start, s_prefix, j)]; });
+                                   [&]() { return a.sphi[vslot_of(sc, s_start, s_prefix, j)]; },
+                                   [&]() { return (uint32_t)sm.rest[KIND == kKindSin ? j : 0]; });
                   }
                   bits |= 1u << (kk & (kWarp - 1));
                 }
