@@ -517,7 +517,7 @@ struct ILane {
 // at most 1.3); alpha = 0.1, sd 1e-2: 1.3 -> 1.0.  From |alpha| = 0.5 on the
 // reference's own rounding of the difference is as large, and nothing is kept.
 // Some 25 integer instructions a pair, beside the 48 cycles that the FP64 pipe
-// takes for a warp's pair, and 26 FP64 operations a particle in the gather: vortex
+// takes for a warp's pair, and 28 FP64 operations a particle in the gather: vortex
 // SRK, N = 65,536, pass 1 171 -> 189 us and gather 6 -> 9 (with the product's rest
 // by a fused multiply-add, pass 1 was 220).
 constexpr double kRestAlpha = 0.5;

@@ -111,7 +111,7 @@ SPC_MATH_FN void sincos_in_range(double ph, double &s, double &c) {
 
 // The same sine and cosine, bit for bit, with the point's number k and the angle
 // `rest` by which the phase exceeds that of the rounded pair (|rest| < 2^-53.4,
-// within 2^-59): every rounding on the way kept as a second double.  26 more
+// within 2^-62): every rounding on the way kept as a second double.  28 more
 // operations.
 SPC_MATH_FN void sincos_with_rest(double ph, double &s, double &c, int &k, double &rest) {
   const double t = fma_rn(ph, 0x1.45f306dc9c883p+4, kRoundMagic);  // 64 / pi
@@ -130,7 +130,8 @@ SPC_MATH_FN void sincos_with_rest(double ph, double &s, double &c, int &k, doubl
   const double wc = fma_rn(p.x, cm1, ic), ws = fma_rn(p.y, cm1, is);
   c = add_rn(p.x, wc);
   s = add_rn(p.y, ws);
-  const double icl = add_rn(fma_rn(-p.y, sn, -ic), p.z), isl = add_rn(fma_rn(p.x, sn, -is), p.w);
+  const double icl = fma_rn(-p.w, sn, add_rn(fma_rn(-p.y, sn, -ic), p.z));
+  const double isl = fma_rn(p.z, sn, add_rn(fma_rn(p.x, sn, -is), p.w));
   const double wcl = add_rn(fma_rn(p.x, cm1, add_rn(ic, -wc)), fma_rn(-p.y, snl, icl));
   const double wsl = add_rn(fma_rn(p.y, cm1, add_rn(is, -ws)), fma_rn(p.x, snl, isl));
   const double cl = add_rn(add_rn(add_rn(p.x, -c), wc), wcl), sl = add_rn(add_rn(add_rn(p.y, -s), ws), wsl);
