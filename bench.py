@@ -15,9 +15,11 @@ time, `value`) and wall clock around the C-ABI call cycle with pinned host
 buffers (upload, replays, download: `e2e`); between bench steps the global
 and local order parameters (the drift series against FP64).  `value` is the
 fastest form whose drift from FP64 in this run stays within 1e-4 (`form`
-names it); every form's figures are under `forms`.
+names it); every form's figures are under `forms`.  The line stays below
+LINE_BYTES; the tuner's choices, the per-step times and the order-parameter
+series of every form go to the file that --details names.
 
-  python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
+  python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference] [--details FILE]
 """
 from __future__ import annotations
 
@@ -1109,8 +1111,40 @@ def drift_of(ref_series, series):
             "points": len(a), "every_steps": int(a[0, 0])}
 
 
+# Readers of the line keep the last 3,000 characters of the output.
+LINE_BYTES = 2600
+
+
+def rounded(v, digits=7):
+    """v with its floats rounded to so many significant digits."""
+    if isinstance(v, dict):
+        return {k: rounded(x, digits) for k, x in v.items()}
+    if isinstance(v, (list, tuple)):
+        return [rounded(x, digits) for x in v]
+    return float(f"{v:.{digits}g}") if isinstance(v, float) else v
+
+
+def line_of(out):
+    """The JSON line of a whole run: `out` without the long parts, which are
+    per-form details, the kernels' and the timing's descriptions."""
+    line = dict(out)
+    line["forms"] = {name: {k: f[k] for k in ("value", "e2e", "ms_per_step")}
+                     for name, f in out["forms"].items()}
+    for name, f in out["forms"].items():
+        if "drift_vs_fp64" in f:
+            line["forms"][name]["max_dR"] = f["drift_vs_fp64"]["max_dR"]
+    roof = out["roofline"]
+    line["roofline"] = {k: roof[k] for k in ("bound", "kernel", "achieved", "peak", "peak_kind", "unit", "frac",
+                                             "traffic", "alg_bytes_per_launch")}
+    line["roofline"]["phase_us"] = {k: v * 1e3 for k, v in roof["phase_ms_run_mean"].items()}
+    line["roofline"].update({k: roof["compute"][k] for k in ("candidate_tests_per_s", "pair_terms_per_s")})
+    return json.dumps(rounded(line))
+
+
 def main():
     ap = argparse.ArgumentParser()
+    ap.add_argument("--details", default=None, metavar="FILE",
+                    help="also write everything the whole-run bench recorded to this JSON file")
     ap.add_argument("--gpus", type=int, default=1)
     ap.add_argument("--steps", type=int, default=10)
     ap.add_argument("--warmup", type=int, default=3)
@@ -1368,7 +1402,7 @@ def main():
     n_total = w["n"] * world
     config = {"workload": w["name"], "N": w["n"], "L": w["L"], "stepper": "srk",
               "model": "vortex (alignment + natural frequencies)",
-              "neighbour": "autotuned per precision (cell list or Verlet rows; see autotune)",
+              "neighbour": "autotuned per precision (cell list or Verlet rows)",
               "dt": w["dt"], "sim_steps_per_bench_step": SIM_STEPS_PER_BENCH_STEP,
               "l2": "flushed between bench steps (512 MB write, outside the timed events)",
               "parallelism": f"replicas{world}"}
@@ -1389,7 +1423,8 @@ def main():
         print(json.dumps({
             "impl": "reference", "metric": "particle-steps/s", "value": v,
             "unit": "particle-steps/s", "n_gpus": args.gpus, "steps": args.steps,
-            "warmup": args.warmup, "higher_is_better": True, "scaling": "weak",
+            "warmup": args.warmup, "ms_per_step": w["n"] / v * 1e3,  # one simulation step
+            "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None, "dtype": "f64", "data": "synthetic", "config": config,
             "cpu_baseline": {"kind": cb["kind"], "cores": 1, "sample": cb["sample"], "value": v},
             # one system uses one core; every core, one replica each:
@@ -1525,7 +1560,10 @@ def main():
     if rank == 0 and not args.no_cpu_baseline:
         out["cpu_baseline"] = cpu_baseline(w)
     if rank == 0:
-        print(json.dumps(out))
+        if args.details:
+            with open(args.details, "w") as f:
+                json.dump(out, f)
+        print(line_of(out))
     if dist is not None:
         dist.destroy_process_group()
 
