@@ -669,24 +669,15 @@ template <int PREC, int KIND>
 __device__ __forceinline__ void accept_pair(const KArgs &a, const SysDesc &sd, const ILane &il,
                                             Acc<PREC> &acc, int pj, float cjc, float cjs,
                                             float dphij_f, long long &wpos) {
+  static_assert(PREC == kPrecFP32C || KIND == kKindNb, "FP64 sums: walk_pairs");
   if constexpr (KIND == kKindSin) {
-    if constexpr (PREC == kPrecFP64) {
-      add_pair<KIND>(acc, sd.sc, il, a.dcs[pj], 0.0, [&]() { return a.sphi[pj]; },
-                     [&]() { return (uint32_t)a.rest[pj]; });  // ChimeraSystem.cpp:412
-    } else {
-      // sin(phi_j - (phi_i + alpha)) by the angle-difference identity
-      kahan_add(acc.s0, acc.c0, cjs * il.ca - cjc * il.sa);
-    }
+    // sin(phi_j - (phi_i + alpha)) by the angle-difference identity
+    kahan_add(acc.s0, acc.c0, cjs * il.ca - cjc * il.sa);
     acc.n++;
   } else if constexpr (KIND == kKindCos2) {
-    if constexpr (PREC == kPrecFP64) {
-      add_pair<KIND>(acc, sd.sc, il, a.dcs[pj], a.dphi_s[pj], [&]() { return a.sphi[pj]; },
-                     []() { return 0u; });  // :634-637
-    } else {
-      const float c = cjc * il.ca + cjs * il.sa;
-      kahan_add(acc.s0, acc.c0, c);
-      kahan_add(acc.s1, acc.c1, (dphij_f - il.dphif) * c);
-    }
+    const float c = cjc * il.ca + cjs * il.sa;
+    kahan_add(acc.s0, acc.c0, c);
+    kahan_add(acc.s1, acc.c1, (dphij_f - il.dphif) * c);
     acc.n++;
   } else {
     if (a.list_idx) a.list_idx[wpos++] = a.pidx[pj] - sd.pool_p0;

@@ -417,11 +417,13 @@ __global__ void __launch_bounds__(kVThreads) k_vtile(KArgs a, int epi) {
         }
         if (rows && rounds == 1 && !exact_all) {
           // the common case: every row entry is in the one staged round.
-          // Chunks of 8 entries, unrolled, the next chunk loaded ahead.
+          // Chunks of 8 entries, unrolled, the next chunk loaded ahead.  (FP64 with
+          // pass-1 bits takes the walk above.)
+          const bool saved = PREC == kPrecFP32C && masked;
           for (int c8 = 0; c8 * 8 < len; ++c8) {
             const uint4 ch = cur;
             if ((c8 + 1) * 8 < len) cur = chunks[(size_t)(c8 + 1) * n_all + v];
-            if (KIND == kKindCos2 && masked && (c8 & 3) == 0)
+            if (KIND == kKindCos2 && saved && (c8 & 3) == 0)
               word = a.nbmask[(size_t)(c8 >> 2) * n_all + v];
 #pragma unroll
             for (int t = 0; t < 8; ++t) {
@@ -429,7 +431,7 @@ __global__ void __launch_bounds__(kVThreads) k_vtile(KArgs a, int epi) {
               if (kk < len) {
                 const int j = chunk_entry(ch, t);
                 bool in;
-                if (KIND == kKindCos2 && masked) {
+                if (KIND == kKindCos2 && saved) {
                   in = (word >> (kk & (kWarp - 1))) & 1u;
                 } else {
                   float cx, cy;
@@ -475,7 +477,7 @@ __global__ void __launch_bounds__(kVThreads) k_vtile(KArgs a, int epi) {
                 if constexpr (KIND == kKindCos2) kahan_add(acc.s1, acc.c1, b1);
                 b0 = b1 = 0.0f;
               }
-              if (KIND == kKindSin && masked) a.nbmask[(size_t)(c8 >> 2) * n_all + v] = bits;
+              if (KIND == kKindSin && saved) a.nbmask[(size_t)(c8 >> 2) * n_all + v] = bits;
               bits = 0u;
             }
           }
