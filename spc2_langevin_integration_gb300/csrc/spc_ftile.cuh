@@ -425,9 +425,15 @@ __device__ __forceinline__ void take_row(const TileMem<PREC> &s, RowSums<PREC> &
   sum.add(v);
 }
 
-// v 2^-35 as an unevaluated sum of two floats: v rounded to float, and the rest
-// rounded to float (the whole within 2^-48 of v).
+// v 2^-35 as an unevaluated sum of two floats (the whole within 2^-48 of v): below
+// 2,048 from two parts that are exact, else v rounded to float and the rest.
 __device__ __forceinline__ float2 two_floats(long long v) {
+  const long long up = v >> 22;
+  if ((unsigned long long)(up + (1ll << 24)) < 1ull << 25) {
+    const float a = (float)(int)up * 0x1p-13f, b = (float)(int)(v & 0x3fffff) * 0x1p-35f;
+    const float h = a + b, bb = h - a;
+    return make_float2(h, (a - (h - bb)) + (b - bb));
+  }
   const float h = __ll2float_rn(v);
   return make_float2(h * 0x1p-35f, __ll2float_rn(v - __float2ll_rn(h)) * 0x1p-35f);
 }
