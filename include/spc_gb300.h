@@ -351,8 +351,8 @@ int spc_philox4x32_10(const uint32_t ctr[4], const uint32_t key[2], uint32_t out
  * the reference writes it). */
 int spc_check_division(int64_t n, const double *a, const double *b, int64_t *mismatches);
 
-/* Self-check of the library's sine and cosine (no reference counterpart): for
- * i < n, sin(x[i]) and cos(x[i]) from separate launches against one
+/* Self-check of CUDA's sine and cosine, which phases of 2^20 and more take (no
+ * reference counterpart): for i < n, sin(x[i]) and cos(x[i]) from separate launches against one
  * sincos(x[i]); *mismatches counts the values whose results differ in any
  * bit. */
 int spc_check_sincos(int64_t n, const double *x, int64_t *mismatches);
@@ -429,7 +429,7 @@ int spc_batch_retune(spc_batch *b, double dt, int32_t trial_steps, spc_tuning *c
  * start-up.  The caller passes device buffers: d_state (3N doubles, AoS),
  * d_derivative (3N) and d_additional (2N); the work is enqueued on `stream`
  * (a cudaStream_t, NULL for the default stream) and the call returns without
- * waiting.  Intermediates live in one static device array of about 1.2 MB
+ * waiting.  Intermediates live in one static device array of about 1.9 MB
  * that every GPU loading the library keeps until the process exits; limits:
  * n <= 8192 particles and int(L/rho)^2 <= 16384 cells, larger sizes return
  * SPC_ERR_CAPACITY.  The Chimera and vortex models are supported; the

